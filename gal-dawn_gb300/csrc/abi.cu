@@ -140,7 +140,7 @@ void destroy(dawn_graph* g) {
   DevBuf* bufs[] = {&g->ss_queues, &g->ss_segs, &g->bs_segs, &g->ss_bitmaps, &g->ss_ctl, &g->ss_sources, &g->ss_scratch,
                     &g->bs_words, &g->bs_queues, &g->bs_ctl, &g->bs_sources, &g->ul_static, &g->hv_static, &g->hv_segoff, &g->hv_acc, &g->hv_tasks, &g->cc_out,
                     &g->dist_stage, &g->pt_voff, &g->pt_tasks, &g->pt_sources, &g->pt_ctl, &g->pt_scratch, &g->pt_rows,
-                    &g->sel_slot, &g->wt_col, &g->wt_val, &g->mw_block, &g->mw_masks,
+                    &g->sel_slot, &g->nf_ctl, &g->nf_queue, &g->nf_segbuf, &g->nf_masks, &g->wt_col, &g->wt_val, &g->mw_block, &g->mw_masks,
                     &g->mw_ctl, &g->mw_sources, &g->bc_levels, &g->bc_terms, &g->bc_range, &g->bc_out,
                     &g->bc_heavy, &g->bc_part};
   for (DevBuf* b : bufs) dawn::release(*b);
@@ -230,6 +230,10 @@ dawn_status sssp_device_impl(dawn_graph* g, const int32_t* sources, int32_t nsrc
     DAWN_CUDA(cudaEventRecord(g->ev1, g->stream));
     dawn::SsCtl c;
     DAWN_CHECK(dawn::download_ctl(g, &c));
+    if (c.err) {
+      dawn::set_error("weighted traversal: a device wait ran out");
+      return c.err;
+    }
     st->levels = c.total_levels;
     st->push_levels = c.total_push;
     st->pull_levels = c.total_pull;

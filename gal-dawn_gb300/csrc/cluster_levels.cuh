@@ -1,8 +1,8 @@
-// Shared pieces of the small-frontier cluster kernels (bfs_small,
-// sssp_small): one cluster of kSmallCtas CTAs runs level after level of a
-// single-source traversal inside one launch, each CTA keeping the vertices
-// its warps add to the next frontier in a shared-memory slice that the
-// whole cluster reads at the next level through distributed shared memory.
+// Pieces of the small-frontier cluster kernel (bfs_small): one cluster of
+// kSmallCtas CTAs runs level after level of a single-source traversal inside
+// one launch, each CTA keeping the vertices its warps add to the next
+// frontier in a shared-memory slice that the whole cluster reads at the next
+// level through distributed shared memory.
 #pragma once
 
 #include "dawn_device.cuh"

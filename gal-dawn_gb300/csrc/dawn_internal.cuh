@@ -210,6 +210,10 @@ struct dawn_graph {
   dawn::DevBuf mw_masks;    // 3 x n uint64 improved-source masks
   dawn::DevBuf mw_ctl;
   dawn::DevBuf mw_sources;
+  dawn::DevBuf nf_ctl, nf_queue, nf_segbuf, nf_masks;  // ordered weighted traversal (nearfar.cu)
+  int32_t nf_max_deg = -1;  // longest out-row (-1: shape not read yet)
+  int64_t nf_segs = 0;      // segments of the long out-rows
+  double nf_mean_weight = 0.0;
   dawn::DevBuf wt_col;      // weighted in-edge CSR (rows of t_row_ptr): tail vertex
   dawn::DevBuf wt_val;      // and weight of each in-edge, built on the first weighted pull
   dawn::SsCtl* h_ctl = nullptr;  // pinned: [0] upload staging, [1] download
@@ -236,7 +240,7 @@ struct dawn_graph {
   int32_t static_seg = 0;       // pull_seg the static pull lists were built with
   bool auto_learned = false;    // DAWN_VARIANT_AUTO batched calls use the learned selector
   bool l2_persist = false;      // DAWN_OPT_L2_PERSIST: persisting L2 window on the frontier words
-  bool small_levels = true;     // DAWN_OPT_SMALL_LEVELS: small frontiers as cluster levels
+  bool small_levels = true;     // DAWN_OPT_SMALL_LEVELS: small BFS frontiers as cluster levels
   // Learned selector.  The decide kernels take the slot's address as a
   // launch argument (fixed for the handle's life, so captured graphs stay
   // valid) and prefetch it while they read the control block.
@@ -298,6 +302,17 @@ dawn_status tune_cache_load(const char* path);
 // (d_dist nsrc x n, the single-source encoding)
 dawn_status sssp_batched(dawn_graph* g, const int32_t* sources, int32_t nsrc, void* d_dist);
 dawn_status sssp_batched_stats(dawn_graph* g, dawn_stats* st, int32_t nsrc);
+
+// nearfar.cu: weighted distances from nb sources (device list) by ordered
+// relaxation in one persistent launch.  D[(v << shift) + s] receives the
+// distance of vertex v from source s (shift 0 for one source, else
+// nearfar_shift(nb)).  The steps taken are added to *levels_out and *push_out
+// (device); *err_out (device) receives DAWN_ERR_TIMEOUT when a wait ran out.
+dawn_status nearfar_run(dawn_graph* g, const int32_t* d_sources, int32_t nb, int shift, int32_t* D,
+                        int32_t* levels_out, int32_t* push_out, int32_t* err_out);
+int nearfar_shift(int32_t nb);
+// Whether batches of up to 64 of nsrc sources run through nearfar_run.
+dawn_status nearfar_batch_fits(dawn_graph* g, int32_t nsrc, bool* fits);
 
 // bc.cu: BCDAWN betweenness summed over the sources into d_bc (n doubles).
 dawn_status betweenness(dawn_graph* g, const int32_t* sources, int32_t nsrc, double* d_bc, dawn_stats* st);

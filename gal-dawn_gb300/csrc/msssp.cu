@@ -31,6 +31,8 @@
 // and is relaxed again only through a self loop.  Any relaxation order
 // reaches the same fixed point, so the distances equal the single-source
 // traversal's.
+#include <algorithm>
+
 #include "dawn_device.cuh"
 
 namespace dawn {
@@ -54,6 +56,7 @@ struct MwCtl {
   int32_t* dist_base;           // nsrc x n output (source-major)
   const int32_t* sources;
   int32_t total_levels, total_push, total_pull;
+  int32_t err;                  // status of an ordered batch (0 = none)
 };
 
 __device__ __forceinline__ int32_t relax(int32_t d, int32_t w, bool is_float) {
@@ -663,34 +666,36 @@ __global__ void mw_decide(MwCtl* __restrict__ ctl, int32_t n, long long m, int c
 // read with coalesced 16-byte loads (512 bytes per warp load, all sixteen
 // issued before the first is waited on), transposed through a padded
 // shared-memory tile and written as one 128-byte run per source row.
+// K words per vertex: kBatch, or the power of two that an ordered batch uses.
 constexpr int kEmitBlock = 128;
-constexpr int kEmitPitch = kBatch + 1;  // words per tile row: column reads hit 32 banks
 
+template <int K>
 __global__ void __launch_bounds__(kEmitBlock) mw_emit(MwCtl* __restrict__ ctl, const int32_t* __restrict__ D,
                                                       const int32_t* __restrict__ row_ptr, int32_t inf, int32_t n) {
+  constexpr int kEmitPitch = K + 1;  // words per tile row: column reads hit 32 banks
   __shared__ int32_t s_tile[kEmitBlock / 32][32 * kEmitPitch];
   const int batch = ctl->batch;
   const int nb = min(kBatch, ctl->nsrc - batch * kBatch);
   int32_t* dist = ctl->dist_base + (size_t)batch * kBatch * n;
   int32_t* tile = s_tile[threadIdx.x >> 5];
   const int lane = lane_id();
-  constexpr int kVecs = 32 * kBatch / 4;  // 16-byte pieces of 32 rows
+  constexpr int kVecs = 32 * K / 4;  // 16-byte pieces of 32 rows
   unsigned long long reached = 0;
   const size_t nwarps = (size_t)gridDim.x * (kEmitBlock / 32);
   for (size_t v0 = ((size_t)blockIdx.x * (kEmitBlock / 32) + (threadIdx.x >> 5)) * 32; v0 < (size_t)n;
        v0 += nwarps * 32) {
     const int rows = (int)min((size_t)32, (size_t)n - v0);
-    const int4* src = reinterpret_cast<const int4*>(D + v0 * kBatch);
+    const int4* src = reinterpret_cast<const int4*>(D + v0 * K);
     int4 x[kVecs / 32];
 #pragma unroll
     for (int i = 0; i < kVecs / 32; i++) {
-      const int j = i * 32 + lane;  // piece j: row j / 16, words 4 (j % 16) ..
-      x[i] = j / (kBatch / 4) < rows ? __ldcs(src + j) : make_int4(inf, inf, inf, inf);
+      const int j = i * 32 + lane;  // piece j: row j / (K / 4), words 4 (j % (K / 4)) ..
+      x[i] = j / (K / 4) < rows ? __ldcs(src + j) : make_int4(inf, inf, inf, inf);
     }
 #pragma unroll
     for (int i = 0; i < kVecs / 32; i++) {
       const int j = i * 32 + lane;
-      int32_t* t = tile + (j / (kBatch / 4)) * kEmitPitch + (j % (kBatch / 4)) * 4;
+      int32_t* t = tile + (j / (K / 4)) * kEmitPitch + (j % (K / 4)) * 4;
       t[0] = x[i].x;
       t[1] = x[i].y;
       t[2] = x[i].z;
@@ -732,12 +737,42 @@ void probe_mw(const void* p, LevelProbe* out) {
   out->unvisited_edges = 0;
 }
 
+// Batches through the ordered traversal (nearfar.cu), which leaves the
+// distances in the vertex-major block that mw_emit writes out.
+dawn_status run_ordered(dawn_graph* g, const int32_t* sources, int32_t nsrc, void* d_dist) {
+  const int shift = nearfar_shift(std::min(kBatch, nsrc));
+  DAWN_CHECK(ensure(g->mw_block, sizeof(int32_t) * ((size_t)g->n << shift), g->stream));
+  DAWN_CHECK(ensure(g->mw_ctl, sizeof(MwCtl), g->stream));
+  DAWN_CHECK(ensure(g->mw_sources, sizeof(int32_t) * (size_t)nsrc, g->stream));
+  DAWN_CUDA(cudaMemcpyAsync(g->mw_sources.p, sources, sizeof(int32_t) * nsrc, cudaMemcpyHostToDevice, g->stream));
+  MwCtl c = {};
+  c.nsrc = nsrc;
+  c.dist_base = static_cast<int32_t*>(d_dist);
+  DAWN_CUDA(cudaMemcpyAsync(g->mw_ctl.p, &c, sizeof(MwCtl), cudaMemcpyHostToDevice, g->stream));
+  MwCtl* ctl = g->mw_ctl.as<MwCtl>();
+  int32_t* D = g->mw_block.as<int32_t>();
+  const int32_t inf = g->wtype == DAWN_W_F32 ? 0x7f7fffff : 0x7fffffff;
+  auto* const emit = shift == 6 ? mw_emit<64> : shift == 5 ? mw_emit<32> : shift == 4 ? mw_emit<16>
+                     : shift == 3 ? mw_emit<8> : mw_emit<4>;
+  for (int32_t b0 = 0; b0 < nsrc; b0 += kBatch) {
+    DAWN_CHECK(nearfar_run(g, g->mw_sources.as<int32_t>() + b0, std::min(kBatch, nsrc - b0), shift, D,
+                           &ctl->total_levels, &ctl->total_push, &ctl->err));
+    emit<<<g->geo.sms * 8, kEmitBlock, 0, g->stream>>>(ctl, D, g->row_ptr, inf, g->n);
+    mw_next<<<1, 32, 0, g->stream>>>(ctl);
+    DAWN_CUDA(cudaGetLastError());
+  }
+  return DAWN_OK;
+}
+
 }  // namespace
 
 dawn_status sssp_batched(dawn_graph* g, const int32_t* sources, int32_t nsrc, void* d_dist) {
   const int32_t n = g->n;
   const size_t nn = (size_t)n;
   const int is_float = g->wtype == DAWN_W_F32;
+  bool ordered = false;
+  if (!g->force_variant && !g->trace) DAWN_CHECK(nearfar_batch_fits(g, nsrc, &ordered));
+  if (ordered) return run_ordered(g, sources, nsrc, d_dist);
   const size_t segcap = seg_capacity(n, g->m);
   DAWN_CHECK(ensure(g->mw_block, sizeof(int32_t) * kBatch * nn, g->stream));
   DAWN_CHECK(ensure(g->mw_masks, sizeof(unsigned long long) * 3 * nn, g->stream));
@@ -825,7 +860,7 @@ dawn_status sssp_batched(dawn_graph* g, const int32_t* sources, int32_t nsrc, vo
                  "mw_pull", kModePull};
   fam.body[2] = {(const void*)mw_decide, decide_args, dim3(1), dim3(32), "mw_decide"};
   fam.npost = 2;
-  fam.post[0] = {(const void*)mw_emit, emit_args, dim3(sms * 8), dim3(kEmitBlock), "mw_emit"};
+  fam.post[0] = {(const void*)mw_emit<kBatch>, emit_args, dim3(sms * 8), dim3(kEmitBlock), "mw_emit"};
   fam.post[1] = {(const void*)mw_next, next_args, dim3(1), dim3(32), "mw_next"};
   fam.ctl = a.ctl;
   fam.ctl_bytes = sizeof(MwCtl);
@@ -845,6 +880,10 @@ dawn_status sssp_batched_stats(dawn_graph* g, dawn_stats* st, int32_t nsrc) {
   MwCtl h;
   DAWN_CUDA(cudaMemcpyAsync(&h, g->mw_ctl.p, sizeof(MwCtl), cudaMemcpyDeviceToHost, g->stream));
   DAWN_CUDA(cudaStreamSynchronize(g->stream));
+  if (h.err) {
+    set_error("weighted traversal: a device wait ran out");
+    return h.err;
+  }
   st->edges_traversed = (int64_t)h.reached;
   st->levels = h.total_levels;
   st->push_levels = h.total_push;

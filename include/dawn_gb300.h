@@ -197,9 +197,9 @@ dawn_status dawn_multi_closeness(dawn_graph* g, const int32_t* source_offset,
  * neighbour, as the reference CPU path does (src/algorithm/cpu/sssp.cpp:41-45).
  * As with dawn_bfs, a NULL dist returns only the statistics.
  * variant: DAWN_VARIANT_PUSH or DAWN_VARIANT_DO run one traversal per
- * source; any other value (AUTO) runs two or more sources 64 per batched
- * traversal (a vertex-major 64-distance block, one relaxation pass per
- * edge for all sources of the batch).  The distances are the same. */
+ * source; any other value (AUTO) runs two or more sources up to 64 per
+ * batched traversal.  The distances are the same.  stats->levels counts the
+ * relaxation steps, however the library orders them. */
 dawn_status dawn_sssp(dawn_graph* g, const int32_t* sources, int32_t nsrc,
                       void* dist, int32_t variant, dawn_stats* stats);
 dawn_status dawn_sssp_device(dawn_graph* g, const int32_t* sources,
@@ -267,14 +267,13 @@ dawn_status dawn_closeness(dawn_graph* g, const int32_t* sources,
  *                          carve-out shrinks the L2 the gathers also use), even
  *                          at scales 21 and 24. */
 #define DAWN_OPT_L2_PERSIST 8
-/*   DAWN_OPT_SMALL_LEVELS  1 (default): single-source traversals (BFS with
- *                          DAWN_VARIANT_DO, weighted distances with
- *                          DAWN_VARIANT_DO / PUSH) run stretches of levels
- *                          whose frontier holds at most 8192 vertices and
- *                          32768 out-edges, and no row of 128 entries or
- *                          more, inside one launch of a thread-block cluster
+/*   DAWN_OPT_SMALL_LEVELS  1 (default): single-source hop traversals
+ *                          (DAWN_VARIANT_DO) run stretches of levels whose
+ *                          frontier holds at most 8192 vertices and 32768
+ *                          out-edges, and no row of 128 entries or more,
+ *                          inside one launch of a thread-block cluster
  *                          (8 CTAs, one cluster barrier per level), instead
- *                          of two launches per level.  0: every level is its
+ *                          of a launch per level.  0: every level is its
  *                          own launch.  Distances are the same. */
 #define DAWN_OPT_SMALL_LEVELS 9
 
