@@ -154,7 +154,7 @@ struct PartTask {
   int32_t part;    // part index
   int32_t src0;    // first source, an index into the call's source list
   int32_t nsrc;    // sources in the task (1..64)
-  int32_t pad;
+  int32_t bits;    // word width of a single-CTA task (16 or 32), else 0
   long long out0;  // output offset of the task's first distance row
 };
 // One distance row of the multi-graph output (closeness reduction).
@@ -254,9 +254,12 @@ struct dawn_graph {
   // disjoint-union parts (dawn_graph_set_parts)
   std::vector<int32_t> pt_off;   // nparts + 1 vertex offsets (empty: no parts)
   std::vector<long long> pt_pos; // row_ptr at those offsets (edge positions)
-  dawn::DevBuf pt_voff, pt_tasks, pt_sources, pt_ctl, pt_scratch, pt_rows;
+  dawn::DevBuf pt_voff, pt_ctl, pt_scratch, pt_small, pt_tcol, pt_toff, pt_rows;  // pt_ctl: control blocks, tasks, sources
+  size_t pt_small_smem = 0, pt_small_words = 0, pt_small_slot = 0;  // single-CTA tasks (bytes)
+  int32_t pt_small_threads = 0, pt_small_ctas = 0;
   size_t pt_slot_words = 0;
-  int32_t pt_slots = 0, pt_maxn = 0;
+  int32_t pt_slots = 0, pt_maxn = 0, pt_exec_maxn = 0;
+  bool pt_cluster_ready = false;  // cluster scratch made for the current parts
   int32_t pt_cluster = 1;  // CTAs per task of the multi-graph launch
   cudaGraphExec_t pt_exec = nullptr;
 
