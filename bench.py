@@ -64,10 +64,10 @@ L2_BYTES = 129 * 2 ** 20
 _CAPTURE = ("ncu launch list of one RMAT-22 x 64 step, bitset variant, traced form: "
             "dram__bytes_read.sum + dram__bytes_write.sum per launch")
 NCU_TRAFFIC = {
-    "bs_pull": {"bytes": 337.8e6, "launches": 5, "file": "gal-dawn_gb300/csrc/msbfs.cu", "sha": "8765e77b47788482",
+    "bs_pull": {"bytes": 333.3e6, "launches": 5, "file": "gal-dawn_gb300/csrc/msbfs.cu", "sha": "50899047f5781c4a",
                 "source": _CAPTURE},
-    "bs_emit_dist": {"bytes": 1178.3e6, "launches": 1, "file": "gal-dawn_gb300/csrc/msbfs.cu",
-                     "sha": "8765e77b47788482", "source": _CAPTURE},
+    "bs_emit_dist": {"bytes": 1177.8e6, "launches": 1, "file": "gal-dawn_gb300/csrc/msbfs.cu",
+                     "sha": "50899047f5781c4a", "source": _CAPTURE},
 }
 # L1/TEX global-load sectors of the level-3 pull (every in-edge unfinished)
 # from `ncu --set full` of the 64-source pull (143,753,817 sectors,
@@ -1038,11 +1038,9 @@ def main():
     if checks:
         parity = {"config": f"rmat{args.scale} x {NSRC} sources", "equal": all(checks.values()),
                   "sources": NSRC, "against": cpu["kind"] + " MSSP_CPU::run", "checked": checks}
-    # Kernels one graph-mode step launches: clear and init, the four body
-    # kernels (pull, push scatter, push update, decide) at every level (those
-    # of the other direction return at once), emit and next.
-    levels = len({(r["run"], r["level"]) for r in recs if r["level"] >= 1})
-    launches = 2 + 4 * levels + 2
+    # Kernels one step launches: the persistent traversal and the distance
+    # emission, once per source batch.
+    launches = 2 * len({r["run"] for r in recs})
     line = {"metric": METRIC, "value": round(value, 3), "unit": "GTEPS", "n_gpus": ws, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": round(ms_step, 4), "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "int32", "data": "synthetic (seeded RMAT)",

@@ -51,10 +51,6 @@ void drop_graphs(dawn_graph* g) {
   if (g->sssp_exec) cudaGraphExecDestroy(g->sssp_exec);
   if (g->mw_exec) cudaGraphExecDestroy(g->mw_exec);
   g->bfs_exec = g->sssp_exec = g->mw_exec = nullptr;
-  for (cudaGraphExec_t& e : g->bs_exec) {
-    if (e) cudaGraphExecDestroy(e);
-    e = nullptr;
-  }
 }
 
 }  // namespace dawn
@@ -138,7 +134,7 @@ void destroy(dawn_graph* g) {
   dawn::pool_free(g->col, g->stream);
   if (g->val) dawn::pool_free(g->val, g->stream);
   DevBuf* bufs[] = {&g->ss_queues, &g->ss_segs, &g->bs_segs, &g->ss_bitmaps, &g->ss_ctl, &g->ss_sources, &g->ss_scratch,
-                    &g->bs_words, &g->bs_queues, &g->bs_ctl, &g->bs_sources, &g->ul_static, &g->hv_static, &g->hv_segoff, &g->hv_acc, &g->hv_tasks, &g->cc_out,
+                    &g->bs_words, &g->bs_queues, &g->bs_ctl, &g->ul_static, &g->hv_static, &g->hv_segoff, &g->hv_acc, &g->hv_tasks, &g->cc_out,
                     &g->dist_stage, &g->pt_voff, &g->pt_ctl, &g->pt_scratch, &g->pt_small, &g->pt_tcol, &g->pt_toff, &g->pt_rows,
                     &g->sel_slot, &g->nf_ctl, &g->nf_queue, &g->nf_segbuf, &g->nf_masks, &g->wt_col, &g->wt_val, &g->mw_block, &g->mw_masks,
                     &g->mw_ctl, &g->mw_sources, &g->bc_levels, &g->bc_terms, &g->bc_range, &g->bc_out,
@@ -147,8 +143,6 @@ void destroy(dawn_graph* g) {
   if (g->stream) cudaStreamSynchronize(g->stream);
   if (g->bfs_exec) cudaGraphExecDestroy(g->bfs_exec);
   if (g->sssp_exec) cudaGraphExecDestroy(g->sssp_exec);
-  for (cudaGraphExec_t e : g->bs_exec)
-    if (e) cudaGraphExecDestroy(e);
   if (g->pt_exec) cudaGraphExecDestroy(g->pt_exec);
   if (g->mw_exec) cudaGraphExecDestroy(g->mw_exec);
   dawn::pinned_slot_release(g->h_ctl);

@@ -68,6 +68,17 @@ __device__ __forceinline__ int num_warps() {
   return (int)((gridDim.x * blockDim.x) >> 5);
 }
 
+// The CTAs that work on a phase together: all of a launch, or as many as a
+// phase of a persistent launch takes.  Consecutive warp indices lie in
+// different CTAs, so that short lists spread over the SMs.
+struct Team {
+  int cta, ctas;
+  __device__ __forceinline__ int warp() const { return (int)(threadIdx.x >> 5) * ctas + cta; }
+  __device__ __forceinline__ int warps() const { return ctas * (int)(blockDim.x >> 5); }
+  __device__ __forceinline__ size_t thread() const { return cta * (size_t)blockDim.x + threadIdx.x; }
+  __device__ __forceinline__ size_t threads() const { return ctas * (size_t)blockDim.x; }
+};
+
 }  // namespace dawn
 
 namespace dawn {
@@ -87,13 +98,12 @@ constexpr int kWarpRow = 32;  // rows with at least this many entries use the wh
 // round of the grid, so a short queue is spread over all warps instead of
 // being walked by a few (64 rows of 16 edges: 64 warps, not two).
 template <bool kCoherent = false, class Op>
-__device__ __forceinline__ void warp_expand(const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ qin,
+__device__ __forceinline__ void warp_expand(int gw, int nw, const int32_t* __restrict__ row_ptr, const int32_t* qin,
                                             int qn, int* s_excl, int* s_rs, int* s_v, Op&& op) {
   const int lane = lane_id();
-  const int nw = num_warps();
   int per = 32;
   while (per > 1 && (long long)(per >> 1) * nw >= qn) per >>= 1;
-  for (int base = global_warp() * per; base < qn; base += nw * per) {
+  for (int base = gw * per; base < qn; base += nw * per) {
     const int idx = base + lane;
     int32_t v = -1;
     int rs = 0, re = 0;
@@ -135,6 +145,11 @@ __device__ __forceinline__ void warp_expand(const int32_t* __restrict__ row_ptr,
     }
     __syncwarp();
   }
+}
+template <bool kCoherent = false, class Op>
+__device__ __forceinline__ void warp_expand(const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ qin,
+                                            int qn, int* s_excl, int* s_rs, int* s_v, Op&& op) {
+  warp_expand<kCoherent>(global_warp(), num_warps(), row_ptr, qin, qn, s_excl, s_rs, s_v, op);
 }
 
 }  // namespace dawn
@@ -210,10 +225,10 @@ __device__ __forceinline__ int long_vertices(unsigned long long lpack) { return 
 // Deals segments to warps (one segment per warp at a time, one lane per
 // edge).  op(v, k, valid) as in warp_expand; kCoherent as there.
 template <bool kCoherent = false, class Op>
-__device__ __forceinline__ void seg_expand(const int32_t* __restrict__ row_ptr, const Seg* __restrict__ segs,
+__device__ __forceinline__ void seg_expand(int gw, int nw, const int32_t* __restrict__ row_ptr, const Seg* segs,
                                            int nsegs, Op&& op) {
   const int lane = lane_id();
-  for (int i = global_warp(); i < nsegs; i += num_warps()) {
+  for (int i = gw; i < nsegs; i += nw) {
     Seg sg;
     if (kCoherent) {
       sg.v = __ldcg(&segs[i].v);
@@ -224,6 +239,11 @@ __device__ __forceinline__ void seg_expand(const int32_t* __restrict__ row_ptr, 
     const int e = min(sg.k0 + kSeg, row_ptr[sg.v + 1]);
     for (int k0 = sg.k0; k0 < e; k0 += 32) op(sg.v, k0 + lane, k0 + lane < e);
   }
+}
+template <bool kCoherent = false, class Op>
+__device__ __forceinline__ void seg_expand(const int32_t* __restrict__ row_ptr, const Seg* __restrict__ segs,
+                                           int nsegs, Op&& op) {
+  seg_expand<kCoherent>(global_warp(), num_warps(), row_ptr, segs, nsegs, op);
 }
 
 }  // namespace dawn

@@ -222,8 +222,7 @@ struct dawn_graph {
   // batched bitset workspace
   dawn::DevBuf bs_words;    // visit / frontier / next words
   dawn::DevBuf bs_queues;   // active + touched queues
-  dawn::DevBuf bs_ctl;
-  dawn::DevBuf bs_sources;
+  dawn::DevBuf bs_ctl;          // control block, then the call's sources
   dawn::DevBuf bs_segs;         // 3 x seg_capacity long-row segments
   dawn::DevBuf ul_static;       // light pull rows: 0 < in-degree < kPullHeavy, id order
   int32_t ul_static_size = 0;
@@ -275,7 +274,6 @@ struct dawn_graph {
   int32_t sssp_exec_weighted = -1;
   cudaGraphExec_t mw_exec = nullptr;  // batched weighted traversal
   int32_t mw_exec_float = -1;
-  cudaGraphExec_t bs_exec[3] = {nullptr, nullptr, nullptr};  // bitset width 1, 2, 4
 
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 
@@ -353,6 +351,12 @@ dawn_status sssp_single(dawn_graph* g, const int32_t* sources, int32_t nsrc,
 // runtime.cu
 dawn_status ss_run(dawn_graph* g, SsFamily& fam, int32_t nsrc,
                    cudaGraphExec_t* exec_cache);
+// Traced form of a family's runs: its kernels one by one, timed.
+dawn_status ss_run_traced(dawn_graph* g, SsFamily& fam, int32_t nruns);
+// A kernel whose CTAs wait for each other, with the family's L2 window if it
+// has one.
+dawn_status launch_cooperative(const SsFamily& fam, const void* fn, int ctas, int threads, void** args,
+                               cudaStream_t s);
 dawn_status upload_ctl(dawn_graph* g, const SsCtl& c);
 dawn_status download_ctl(dawn_graph* g, SsCtl* out);
 // CTAs of a persistent grid: the SM count times the resident CTAs per SM,

@@ -31,6 +31,8 @@
 // pair rather than a read-modify-write of every set bit's slice, and the
 // final pass leaves those entries alone.
 #include <algorithm>
+#include <cstring>
+#include <vector>
 
 #include "dawn_device.cuh"
 #include "selector.cuh"
@@ -75,12 +77,57 @@ struct BsCtl {
   int32_t pad3;
   long long m;                  // CSR entries (selector input)
   unsigned long long total_reached;
-  int32_t total_levels, total_push, total_pull, pad2;
+  int32_t total_levels, total_push, total_pull;
+  int32_t err;                  // persistent launch: a wait ran out
   // 1 = the level that wrote this slot's frontier words kept no active list
   // (a dense push update: the next level is then a pull, which needs none,
   // and the slot is cleared densely when it goes stale); aq_size holds the
   // count only
-  int32_t unlisted[3], pad5;
+  int32_t unlisted[3];
+  // persistent launch: the words that all CTAs poll (BsStep), and the
+  // arrivals of all phases so far
+  struct __align__(128) {
+    unsigned long long word[16];
+  } sync;
+  struct __align__(128) {
+    uint32_t n;
+  } arrive;
+};
+
+// What a CTA has to know to work on a level, from the control block (one
+// launch per step) or from the words of the persistent launch: nine of 48
+// bits, each tagged with the phase's generation in its top 16, so that one
+// load per lane brings them all and a torn read shows in the tags.
+struct BsStep {
+  int32_t ctas, phase;
+  uint32_t arrived;                           // arrivals before the phase
+  int32_t L, dense;
+  int32_t qn, ln;                             // frontier: listed vertices, long-row segments
+  int32_t stale, stale_segs, stale_unlisted;  // the slot to clear
+  int32_t tn;                                 // update: vertices touched
+  int32_t ul_cur, un, hs_cur, hn;             // pull: the lists and their sizes
+  int32_t nf;                                 // frontier vertices
+};
+
+struct BsArgs {
+  BsCtl* ctl;
+  const int32_t *row_ptr, *col, *t_row_ptr, *t_col;
+  const int32_t *ul_static, *hv_static, *hv_segoff;  // pull lists of the graph
+  u64 *words, *visit, *fr, *nxt, *slices;
+  u64* hv_acc;
+  int2* hv_tasks;
+  int32_t *aq, *tq, *ul;
+  uint32_t* tbm;
+  Seg* segs;
+  size_t segcap, nwords;
+  long long m;
+  int32_t n, ul_static_size, hv_count, hv_segs, pull_seg;
+  int32_t nbits, force;
+  int32_t batch;                // -1: the control block's (one launch per step)
+  // where levels from kDeepLevel on go, as in the control block
+  int32_t *dist_base, *lv_block;
+  unsigned long long* cc_sum;
+  const float* sel_w;
 };
 
 constexpr int kSlicesCleared = 4;  // slices zeroed per batch; higher ones on first use
@@ -141,20 +188,17 @@ struct Bits {
   // (a gather then asks L1/TEX for its sector once, not twice).  The
   // vertex's words start on a 32-byte boundary: slots are n x 32 bytes
   // apart from an aligned base.
-  __device__ __forceinline__ static Bits ldg(const u64* p) {
+  // Not through the read-only path: in the persistent launch the words of a
+  // level were written earlier in the same launch.
+  __device__ __forceinline__ static Bits gather(const u64* p) {
     Bits b;
     if constexpr (W == 4) {
-      asm("ld.global.nc.v4.u64 {%0,%1,%2,%3}, [%4];" : "=l"(b.w[0]), "=l"(b.w[1]), "=l"(b.w[2]), "=l"(b.w[3])
-          : "l"(p));
-    } else if (W == 1) {
-      b.w[0] = __ldg(p);
+      asm volatile("ld.global.v4.u64 {%0,%1,%2,%3}, [%4];" : "=l"(b.w[0]), "=l"(b.w[1]), "=l"(b.w[2]), "=l"(b.w[3])
+                   : "l"(p));
+    } else if constexpr (W == 1) {
+      asm volatile("ld.global.u64 %0, [%1];" : "=l"(b.w[0]) : "l"(p));
     } else {
-#pragma unroll
-      for (int i = 0; i < W; i += 2) {
-        const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(p + i));
-        b.w[i] = v.x;
-        b.w[i + 1] = v.y;
-      }
+      asm volatile("ld.global.v2.u64 {%0,%1}, [%2];" : "=l"(b.w[0]), "=l"(b.w[1]) : "l"(p));
     }
     return b;
   }
@@ -243,62 +287,71 @@ struct Bits {
 // From kDeepLevel on the level is stored at once: in the batch's distance
 // rows, or in u's level row (level mode); closeness mode sums it per source
 // instead (add_deep_sums).  The caller owns u.
+__device__ __forceinline__ int batch_of(const BsArgs& a) { return a.batch >= 0 ? a.batch : a.ctl->batch; }
+
 template <int W>
-__device__ __forceinline__ void record_level(const BsCtl* __restrict__ ctl, u64* __restrict__ slices, int32_t n,
-                                             int32_t u, const Bits<W>& nw, int32_t level) {
+__device__ __forceinline__ void record_level(const BsArgs& a, int32_t u, const Bits<W>& nw, int32_t level) {
+  const int32_t n = a.n;
   if (level < kDeepLevel) {
+    u64* const slices = a.slices;
     for (unsigned L = (unsigned)level; L; L &= L - 1) {
       u64* p = slices + ((size_t)(__ffs(L) - 1) * n + u) * W;
       (Bits<W>::ld(p) | nw).st(p);
     }
     return;
   }
-  if (ctl->cc_sum) return;
-  if (ctl->lv_block) {
-    int32_t* row = ctl->lv_block + (size_t)u * 64;
+  if (a.cc_sum) return;
+  if (a.lv_block) {
+    int32_t* row = a.lv_block + (size_t)u * 64;
     for (u64 b = nw.w[0]; b; b &= b - 1) row[__ffsll((long long)b) - 1] = level;
     return;
   }
-  int32_t* dist = ctl->dist_base + (size_t)ctl->batch * 64 * W * n;
+  int32_t* dist = a.dist_base + (size_t)batch_of(a) * 64 * W * n;
 #pragma unroll
   for (int i = 0; i < W; i++)
     for (u64 b = nw.w[i]; b; b &= b - 1) dist[(size_t)(64 * i + __ffsll((long long)b) - 1) * n + u] = level;
 }
 
 // Closeness mode from kDeepLevel on: adds the levels of the warp's new bits
-// to the batch's per-source sums.  The warp's 32 new-bit words are
-// transposed so lane j counts the bits of sources 64i + j and 64i + 32 + j
-// with popc; one atomic per lane and nonzero sum.  All 32 lanes call it (nw
-// zero where a lane has no vertex).
+// to the CTA's per-source sums.  The warp's 32 new-bit words are transposed
+// so lane j counts the bits of sources 64i + j and 64i + 32 + j with popc.
+// All 32 lanes call it (nw zero where a lane has no vertex).
 template <int W>
-__device__ __forceinline__ void add_deep_sums(const BsCtl* __restrict__ ctl, const Bits<W>& nw, int32_t level) {
-  const size_t row0 = (size_t)ctl->batch * 64 * W;
+__device__ __forceinline__ void add_deep_sums(u64* sums, const Bits<W>& nw, int32_t level) {
   const int lane = lane_id();
 #pragma unroll
   for (int i = 0; i < W; i++) {
     if (!__any_sync(kFull, nw.w[i] != 0ull)) continue;
     const unsigned lo = __popc(warp_transpose32((uint32_t)nw.w[i]));
     const unsigned hi = __popc(warp_transpose32((uint32_t)(nw.w[i] >> 32)));
-    if (lo) atomicAdd(ctl->cc_sum + row0 + 64 * i + lane, (unsigned long long)lo * (unsigned)level);
-    if (hi) atomicAdd(ctl->cc_sum + row0 + 64 * i + 32 + lane, (unsigned long long)hi * (unsigned)level);
+    if (lo) atomicAdd(sums + 64 * i + lane, (unsigned long long)lo * (unsigned)level);
+    if (hi) atomicAdd(sums + 64 * i + 32 + lane, (unsigned long long)hi * (unsigned)level);
   }
+}
+// The CTA's sums: cleared before a level, then added to the batch's rows.
+template <int W>
+__device__ __forceinline__ void clear_deep_sums(u64* sums) {
+  for (int t = threadIdx.x; t < 64 * W; t += blockDim.x) sums[t] = 0;
+  __syncthreads();
+}
+template <int W>
+__device__ __forceinline__ void flush_deep_sums(const BsArgs& a, const u64* sums) {
+  __syncthreads();
+  u64* const rows = a.cc_sum + (size_t)batch_of(a) * 64 * W;
+  for (int t = threadIdx.x; t < 64 * W; t += blockDim.x)
+    if (sums[t]) atomicAdd(rows + t, sums[t]);
 }
 
 // Level L is the last one before slice log2(L + 1) is first used: clear it.
 template <int W>
-__device__ __forceinline__ void clear_next_slice(u64* __restrict__ slices, int32_t n, int32_t level, int nbits) {
+__device__ __forceinline__ void clear_next_slice(const Team& tm, u64* slices, int32_t n, int32_t level, int nbits) {
   const unsigned next = (unsigned)level + 1;
   if (next & (next - 1)) return;
   const int b = __ffs(next) - 1;
   if (b < kSlicesCleared || b >= nbits) return;
   u64* p = slices + (size_t)b * n * W;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)n * W; i += stride) p[i] = 0ull;
+  for (size_t i = tm.thread(); i < (size_t)n * W; i += tm.threads()) p[i] = 0ull;
 }
-
-template <int W>
-__device__ __forceinline__ void clear_listed(u64* __restrict__ fr, const int32_t* __restrict__ list, int cnt,
-                                             const Seg* __restrict__ segs, int nsegs);
 
 // Column loads of the pull.  The in-edge columns stream through once per
 // level, so they bypass L1 and are marked first to leave L2 (the frontier
@@ -324,51 +377,45 @@ __device__ __forceinline__ void ld_col8(const int32_t* p, uint64_t pol, int32_t 
       : "l"(p), "l"(pol));
 }
 
-// Zero the frontier words of a stale active list and its segment list
-// (grid-stride).  A list that covers more than a quarter of the vertices is
-// cleared as the whole slot instead: n coalesced word stores cost less than
-// that many scattered partial-sector writes.
+// Zero the frontier words of a stale active list and its segment list.  A
+// list that covers more than a quarter of the vertices is cleared as the
+// whole slot instead: n coalesced word stores cost less than that many
+// scattered partial-sector writes.
+__device__ __forceinline__ bool clears_slot(int cnt, bool unlisted, int32_t n) {
+  return unlisted || (long long)cnt * 4 > n;
+}
 template <int W>
-__device__ __forceinline__ void clear_stale(u64* __restrict__ fr, int32_t n, const int32_t* __restrict__ list,
-                                            int cnt, const Seg* __restrict__ segs, int nsegs, bool unlisted) {
-  if (!unlisted && (long long)cnt * 4 <= n) {
-    clear_listed<W>(fr, list, cnt, segs, nsegs);
+__device__ __forceinline__ void clear_stale(const Team& tm, u64* fr, int32_t n, const int32_t* list, int cnt,
+                                            const Seg* segs, int nsegs, bool unlisted) {
+  const size_t t0 = tm.thread(), stride = tm.threads();
+  if (!clears_slot(cnt, unlisted, n)) {
+    for (size_t i = t0; i < (size_t)cnt; i += stride) Bits<W>::zero().st(fr + (size_t)list[i] * W);
+    for (size_t i = t0; i < (size_t)nsegs; i += stride) Bits<W>::zero().st(fr + (size_t)segs[i].v * W);
     return;
   }
   // 8-byte stores: a slot starts on an 8-byte boundary only (n * W words
   // per slot, n odd possible), and a warp's 32 of them still fill two lines.
-  const size_t words = (size_t)n * W, stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < words; i += stride) fr[i] = 0ull;
+  for (size_t i = t0; i < (size_t)n * W; i += stride) fr[i] = 0ull;
 }
 
-// Zero the frontier words listed in a stale active list and its segment
-// list (grid-stride).
-template <int W>
-__device__ __forceinline__ void clear_listed(u64* __restrict__ fr, const int32_t* __restrict__ list, int cnt,
-                                             const Seg* __restrict__ segs, int nsegs) {
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)cnt; i += stride)
-    Bits<W>::zero().st(fr + (size_t)list[i] * W);
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)nsegs; i += stride)
-    Bits<W>::zero().st(fr + (size_t)segs[i].v * W);
-}
-
-__global__ void __launch_bounds__(kBlock) bs_clear(u64* __restrict__ words, size_t count) {
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
+__device__ __forceinline__ void clear_words(const Team& tm, u64* words, size_t count) {
   ulonglong2* w2 = reinterpret_cast<ulonglong2*>(words);
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count / 2; i += stride)
-    w2[i] = make_ulonglong2(0ull, 0ull);
-  if (blockIdx.x == 0 && threadIdx.x == 0 && (count & 1)) words[count - 1] = 0;
+  for (size_t i = tm.thread(); i < count / 2; i += tm.threads()) w2[i] = make_ulonglong2(0ull, 0ull);
+  if (tm.thread() == 0 && (count & 1)) words[count - 1] = 0;
 }
 
-// One CTA of 64 W threads: thread b seeds source b of the batch.
+// One CTA of at least 64 W threads: thread b seeds source b of the batch.
 template <int W>
-__global__ void bs_init(BsCtl* __restrict__ ctl, const int32_t* __restrict__ row_ptr,
-                        const int32_t* __restrict__ t_row_ptr, u64* __restrict__ visit, u64* __restrict__ fr0,
-                        int32_t* __restrict__ aq0, Seg* __restrict__ segs0, int32_t n, long long m) {
+__device__ __forceinline__ void init_batch(const BsArgs& a) {
   __shared__ u64 s_mf, s_reached, s_dec;
+  BsCtl* const ctl = a.ctl;
+  const int32_t *row_ptr = a.row_ptr, *t_row_ptr = a.t_row_ptr;
+  u64 *visit = a.visit, *fr0 = a.fr;
+  int32_t* aq0 = a.aq;
+  Seg* segs0 = a.segs;
+  const long long m = a.m;
   const int b = threadIdx.x;
-  const int batch = ctl->batch;
+  const int batch = batch_of(a);
   const int per = 64 * W;
   const int nb = min(per, ctl->nsrc - batch * per);
   if (b == 0) {
@@ -397,12 +444,14 @@ __global__ void bs_init(BsCtl* __restrict__ ctl, const int32_t* __restrict__ row
   }
   __syncthreads();
   int32_t s = -1;
+  int rs = 0, deg = 0;
   if (b < nb) {
     s = ctl->sources[batch * per + b];
     const u64 bit = 1ull << (b & 63);
     atomicOr(visit + (size_t)s * W + (b >> 6), bit);
     atomicOr(fr0 + (size_t)s * W + (b >> 6), bit);
-    const int deg = row_ptr[s + 1] - row_ptr[s];
+    rs = row_ptr[s];
+    deg = row_ptr[s + 1] - rs;
     atomicAdd(&s_reached, (u64)deg);
     // A source without out-edges reaches no vertex but itself.  Its bit is
     // left out of `full`, so the other vertices still finish (and leave
@@ -415,23 +464,19 @@ __global__ void bs_init(BsCtl* __restrict__ ctl, const int32_t* __restrict__ row
   // thread of its lowest bit.
   bool lowest = b < nb;
   if (lowest) {
-    for (int i = 0; i < (b >> 6); i++) lowest &= fr0[(size_t)s * W + i] == 0ull;
-    const u64 below = fr0[(size_t)s * W + (b >> 6)] & ((1ull << (b & 63)) - 1ull);
-    lowest &= below == 0ull;
+    const Bits<W> f = Bits<W>::ldcg(fr0 + (size_t)s * W);
+#pragma unroll
+    for (int i = 0; i < W; i++) {
+      const u64 below = i < (b >> 6) ? ~0ull : (i == (b >> 6) ? (1ull << (b & 63)) - 1ull : 0ull);
+      lowest &= (f.w[i] & below) == 0ull;
+    }
   }
   if (lowest) {
-    const int rs = row_ptr[s], deg = row_ptr[s + 1] - rs;
-    if (deg >= kLongRow) {
-      const int nseg = (deg + kSeg - 1) / kSeg;
-      const u64 old = atomicAdd(&ctl->alpack[0], (1ull << 32) | (unsigned)nseg);
-      for (int j = 0; j < nseg; j++) segs0[(uint32_t)old + j] = Seg{s, rs + j * kSeg};
-    } else {
-      aq0[atomicAdd(&ctl->aq_size[0], 1)] = s;
-    }
     atomicAdd(&s_mf, (u64)deg);
-    if (Bits<W>::ld(visit + (size_t)s * W) == Bits<W>::full_of(ctl))
+    if (Bits<W>::ldcg(visit + (size_t)s * W) == Bits<W>::full_of(ctl))
       atomicAdd(&s_dec, (u64)(t_row_ptr[s + 1] - t_row_ptr[s]));
   }
+  if (b < per) emit_routed(lowest, s, deg, rs, aq0, &ctl->aq_size[0], segs0, &ctl->alpack[0]);  // whole warps
   __syncthreads();
   if (b == 0) {
     for (int i = 0; i < 3; i++) ctl->mf[i] = 0;
@@ -449,7 +494,21 @@ __global__ void bs_init(BsCtl* __restrict__ ctl, const int32_t* __restrict__ row
   }
 }
 
-// Per-thread accumulators of a level, flushed once per warp.
+// Shared memory of a level's work: per warp two staging queues (the push
+// keeps its row dealing in the second one's place).
+template <int kWarps>
+struct BsSmem {
+  int32_t q[kWarps][2 * kWarpQueueBig];
+  u64 acc[3];
+  u64 deep[64 * kMaxW];  // closeness: per-source sums of deep levels
+  uint32_t n[2][kWarps];
+  int32_t nf;
+  u64 word[16];
+  BsStep st, next;  // the running phase, and in its last CTA the one it opens
+};
+static_assert(3 * 32 <= kWarpQueueBig, "row dealing fits the second queue");
+
+// Per-thread accumulators of a level.
 struct LevelAcc {
   u64 mf = 0, reached = 0, dec = 0;
   __device__ __forceinline__ void add(u64 out_deg, u64 in_deg, int new_pairs, bool finished) {
@@ -457,17 +516,54 @@ struct LevelAcc {
     reached += out_deg * (u64)new_pairs;
     if (finished) dec += in_deg;
   }
-  __device__ __forceinline__ void flush(BsCtl* ctl, int slot) {
-    mf = warp_sum(mf);
-    reached = warp_sum(reached);
-    dec = warp_sum(dec);
-    if (lane_id() == 0) {
-      if (mf) atomicAdd(&ctl->mf[slot], mf);
-      if (reached) atomicAdd(&ctl->reached, reached);
-      if (dec) atomicAdd(reinterpret_cast<u64*>(&ctl->mu_dec), dec);
+};
+
+// The end of a CTA's share of a level: what its warps still stage goes out
+// with one reservation per queue, and its sums and counts with one atomic
+// each.  A reservation and three sums per warp were 5,000 to 6,000 atomics on
+// each of five words at every level: 10 us even where no vertex was left to
+// visit.  b may be NULL; nf is added to *nf_count when given.
+template <int kWarps>
+__device__ __forceinline__ void end_level(BsSmem<kWarps>& sm, BsCtl* ctl, int slot, LevelAcc& acc, WarpQueueBig& a,
+                                          WarpQueueBig* b, int nf, int32_t* nf_count) {
+  const int lane = lane_id(), wib = threadIdx.x >> 5;
+  if (threadIdx.x < 3) sm.acc[threadIdx.x] = 0;
+  if (threadIdx.x == 3) sm.nf = 0;
+  if (lane == 0) {
+    sm.n[0][wib] = (uint32_t)a.n;
+    sm.n[1][wib] = b ? (uint32_t)b->n : 0u;
+  }
+  __syncthreads();
+  const u64 mf = warp_sum(acc.mf), reached = warp_sum(acc.reached), dec = warp_sum(acc.dec);
+  if (lane == 0) {
+    if (mf) atomicAdd(&sm.acc[0], mf);
+    if (reached) atomicAdd(&sm.acc[1], reached);
+    if (dec) atomicAdd(&sm.acc[2], dec);
+    if (nf) atomicAdd(&sm.nf, nf);
+  }
+  if (wib == 0) {
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const int x = lane < kWarps ? (int)sm.n[q][lane] : 0;
+      const int incl = warp_incl_scan(x);
+      const int tot = __shfl_sync(kFull, incl, 31);
+      int base = 0;
+      if (tot && lane == 0) base = atomicAdd(q ? b->count : a.count, tot);
+      base = __shfl_sync(kFull, base, 0);
+      if (lane < kWarps) sm.n[q][lane] = (uint32_t)(base + incl - x);
     }
   }
-};
+  __syncthreads();
+  for (int i = lane; i < a.n; i += 32) a.out[sm.n[0][wib] + i] = a.buf[i];
+  if (b)
+    for (int i = lane; i < b->n; i += 32) b->out[sm.n[1][wib] + i] = b->buf[i];
+  if (threadIdx.x == 0) {
+    if (sm.acc[0]) atomicAdd(&ctl->mf[slot], sm.acc[0]);
+    if (sm.acc[1]) atomicAdd(&ctl->reached, sm.acc[1]);
+    if (sm.acc[2]) atomicAdd(reinterpret_cast<u64*>(&ctl->mu_dec), sm.acc[2]);
+    if (nf_count && sm.nf) atomicAdd(nf_count, sm.nf);
+  }
+}
 
 // Pull: every vertex of the unfinished list ORs the frontier words of its
 // in-neighbours.  Heavy rows (>= 2 x pull_seg in-edges) come first, one
@@ -479,71 +575,62 @@ struct LevelAcc {
 // entries are swept by the whole warp (4 gathers in flight per lane, early
 // exit once no missing bit is left), shorter ones are walked by one lane
 // each.  The list is filtered into the next unfinished list as it goes.
-template <int W>
-__global__ void __launch_bounds__(kBlock, W == 1 ? 5 : 4) bs_pull(const int32_t* __restrict__ row_ptr,
-                                                     const int32_t* __restrict__ t_row_ptr,
-                                                     const int32_t* __restrict__ t_col, BsCtl* __restrict__ ctl,
-                                                     u64* __restrict__ visit, u64* __restrict__ fr,
-                                                     u64* __restrict__ slices, int32_t* __restrict__ aq,
-                                                     Seg* __restrict__ segs, size_t segcap,
-                                                     const int32_t* __restrict__ ul_static, int32_t ul_static_size,
-                                                     int32_t* __restrict__ ul, const int32_t* __restrict__ hv_static,
-                                                     const int32_t* __restrict__ hv_segoff, u64* __restrict__ hv_acc,
-                                                     int2* __restrict__ hv_tasks, int32_t hv_count, int32_t hv_segs,
-                                                     int32_t pull_seg, int32_t n) {
+template <int W, int kWarps>
+__device__ __forceinline__ void pull_level(const BsArgs& a, const Team& tm, const BsStep& st, BsSmem<kWarps>& sm) {
   using B = Bits<W>;
-  __shared__ int32_t s_qa[kBlock / 32][kWarpQueueBig];
-  __shared__ int32_t s_qu[kBlock / 32][kWarpQueueBig];
-  if (ctl->done || ctl->mode != kModePull) return;
-  const int L = ctl->level;
-  const u64* __restrict__ fin = fr + (size_t)((L - 1) % 3) * n * W;
-  u64* __restrict__ fout = fr + (size_t)(L % 3) * n * W;
-  int32_t* aq_out = aq + (size_t)(L % 3) * n;
-  Seg* seg_out = segs + (size_t)(L % 3) * segcap;
+  BsCtl* const ctl = a.ctl;
+  const int32_t* __restrict__ row_ptr = a.row_ptr;
+  const int32_t* __restrict__ t_row_ptr = a.t_row_ptr;
+  const int32_t* __restrict__ t_col = a.t_col;
+  const int32_t* __restrict__ hv_static = a.hv_static;
+  const int32_t* __restrict__ hv_segoff = a.hv_segoff;
+  u64 *const visit = a.visit, *const hv_acc = a.hv_acc;
+  const int32_t n = a.n, pull_seg = a.pull_seg, hv_segs = a.hv_segs;
+  const int L = st.L;
+  const u64* fin = a.fr + (size_t)((L - 1) % 3) * n * W;
+  u64* fout = a.fr + (size_t)(L % 3) * n * W;
+  int32_t* aq_out = a.aq + (size_t)(L % 3) * n;
+  Seg* seg_out = a.segs + (size_t)(L % 3) * a.segcap;
   int32_t* aq_count = &ctl->aq_size[L % 3];
   u64* al_pack = &ctl->alpack[L % 3];
-  clear_stale<W>(fr + (size_t)((L + 1) % 3) * n * W, n, aq + (size_t)((L + 1) % 3) * n, ctl->aq_size[(L + 1) % 3],
-                 segs + (size_t)((L + 1) % 3) * segcap, seg_count(ctl->alpack[(L + 1) % 3]),
-                 ctl->unlisted[(L + 1) % 3] != 0);
+  clear_stale<W>(tm, a.fr + (size_t)((L + 1) % 3) * n * W, n, a.aq + (size_t)((L + 1) % 3) * n,
+                 st.stale, a.segs + (size_t)((L + 1) % 3) * a.segcap, st.stale_segs, st.stale_unlisted != 0);
   const uint64_t pol = evict_first_policy();
-  clear_next_slice<W>(slices, n, L, ctl->nbits);
-  const int cur = ctl->ul_cur;
-  const int32_t* ul_in = cur < 0 ? ul_static : ul + (size_t)cur * n;
-  const int un = cur < 0 ? ul_static_size : ctl->ul_size[cur];
+  clear_next_slice<W>(tm, a.slices, n, L, a.nbits);
+  const int cur = st.ul_cur;
+  const int32_t* ul_in = cur < 0 ? a.ul_static : a.ul + (size_t)cur * n;
+  const int un = st.un;
   const int nxt = cur < 0 ? 0 : cur ^ 1;
-  int32_t* ul_out = ul + (size_t)nxt * n;
+  int32_t* ul_out = a.ul + (size_t)nxt * n;
   int32_t* ul_count = &ctl->ul_size[nxt];
   const B full = B::full_of(ctl);
   const int lane = lane_id(), wib = threadIdx.x >> 5;
   LevelAcc acc;
-  WarpQueueBig qa(s_qa[wib], aq_out, aq_count);
-  WarpQueueBig qu(s_qu[wib], ul_out, ul_count);
-  const bool deep_cc = ctl->cc_sum && L >= kDeepLevel;
+  WarpQueueBig qa(sm.q[wib], aq_out, aq_count);
+  WarpQueueBig qu(sm.q[wib] + kWarpQueueBig, ul_out, ul_count);
+  const bool deep_cc = a.cc_sum && L >= kDeepLevel;
+  if (deep_cc) clear_deep_sums<W>(sm.deep);
   // A pull level entered with a frontier of at least n / 16 vertices keeps
   // no active list: its output frontier is counted, the next level is made
   // a pull (which reads frontier words), and the slot is cleared densely
   // when it goes stale.  Smaller levels queue their output for a push.
-  const long long nf_in = (long long)ctl->aq_size[(L - 1) % 3] + long_vertices(ctl->alpack[(L - 1) % 3]);
-  const bool lazy = !ctl->force && nf_in * 16 >= n;
+  const bool lazy = !a.force && (long long)st.nf * 16 >= n;
   int my_nf = 0;
   // Heavy-row segments: the first pull level deals every segment of the
   // graph (finding its row by binary search); the finisher of a row that
   // stays unfinished re-lists the row's segments as (row, segment) tasks,
   // and later pull levels deal only those.
-  const int hcur = ctl->hs_cur;
-  const int hn = hcur < 0 ? hv_segs : ctl->hs_size[hcur];
-  const int2* __restrict__ hs_in = hv_tasks + (size_t)(hcur < 0 ? 0 : hcur) * hv_segs;
-  int2* hs_out = hv_tasks + (size_t)(hcur < 0 ? 0 : hcur ^ 1) * hv_segs;
+  const int hcur = st.hs_cur, hn = st.hn;
+  const int2* hs_in = a.hv_tasks + (size_t)(hcur < 0 ? 0 : hcur) * hv_segs;
+  int2* hs_out = a.hv_tasks + (size_t)(hcur < 0 ? 0 : hcur ^ 1) * hv_segs;
   int32_t* hs_count = &ctl->hs_size[hcur < 0 ? 0 : hcur ^ 1];
 
-  for (;;) {
-    int t = 0;
-    if (lane == 0) t = atomicAdd(&ctl->hwork, 1);
-    t = __shfl_sync(kFull, t, 0);
-    if (t >= hn) break;
+  // A warp's first task is its own; the shared counters deal the rest.
+  const int gw = tm.warp(), nw = tm.warps();
+  for (int t = gw; t < hn; t = nw + __shfl_sync(kFull, lane == 0 ? atomicAdd(&ctl->hwork, 1) : 0, 0)) {
     int lo = 0, sidx = t;
     if (hcur < 0) {
-      int hi = hv_count - 1;
+      int hi = a.hv_count - 1;
       while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (__ldg(hv_segoff + mid) <= sidx) lo = mid; else hi = mid - 1;
@@ -568,10 +655,10 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 5 : 4) bs_pull(const int32_t*
       const int32_t v1 = k + 32 < ke ? ld_col(t_col + k + 32, pol) : -1;
       const int32_t v2 = k + 64 < ke ? ld_col(t_col + k + 64, pol) : -1;
       const int32_t v3 = k + 96 < ke ? ld_col(t_col + k + 96, pol) : -1;
-      if (v0 >= 0) w = w | B::ldg(fin + (size_t)v0 * W);
-      if (v1 >= 0) w = w | B::ldg(fin + (size_t)v1 * W);
-      if (v2 >= 0) w = w | B::ldg(fin + (size_t)v2 * W);
-      if (v3 >= 0) w = w | B::ldg(fin + (size_t)v3 * W);
+      if (v0 >= 0) w = w | B::gather(fin + (size_t)v0 * W);
+      if (v1 >= 0) w = w | B::gather(fin + (size_t)v1 * W);
+      if (v2 >= 0) w = w | B::gather(fin + (size_t)v2 * W);
+      if (v3 >= 0) w = w | B::gather(fin + (size_t)v3 * W);
       if ((w.warp_or() | vis | B::ldcg(hacc)) == full) break;
     }
     w = w.warp_or();
@@ -600,7 +687,7 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 5 : 4) bs_pull(const int32_t*
       if (nw.any()) {
         (vis | nw).st(visit + (size_t)u * W);
         nw.st(fout + (size_t)u * W);
-        record_level<W>(ctl, slices, n, u, nw, L);
+        record_level<W>(a, u, nw, L);
         ors = row_ptr[u];
         odeg = row_ptr[u + 1] - ors;
         acc.add((u64)odeg, (u64)(rend - rbeg), nw.popc(), (vis | nw) == full);
@@ -614,22 +701,27 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 5 : 4) bs_pull(const int32_t*
       base = __shfl_sync(kFull, base, 0);
       for (int j = lane; j < nseg; j += 32) hs_out[base + j] = make_int2(lo, s0 + j);
     }
-    if (deep_cc) add_deep_sums<W>(ctl, nw, L);
+    if (deep_cc) add_deep_sums<W>(sm.deep, nw, L);
     if (lazy)
       my_nf += __popc(__ballot_sync(kFull, nw.any()));
     else
       emit_routed(nw.any(), u, odeg, ors, qa, seg_out, al_pack);
   }
 
-  for (;;) {
-    int base = 0;
-    if (lane == 0) base = atomicAdd(&ctl->work, 32);
-    base = __shfl_sync(kFull, base, 0);
-    if (base >= un) break;
+  // Rows per warp task: 32, or fewer where the list is short.  Rows of 64 and
+  // more in-edges go one after another in their task, so graphs that have them
+  // (a mean in-degree of 24 and more) want several tasks per warp; elsewhere
+  // fewer than 32 rows only where half the warps would stay idle (a 29 us pull
+  // of 200,003 mesh vertices took 8 rows a task in four rounds).
+  int rows = 32;
+  const long long spread = a.m >= 24ll * n ? 8ll * nw : (long long)nw;
+  while (rows > 8 && 2ll * un < spread * rows) rows >>= 1;
+  for (int base = gw * rows; base < un;
+       base = nw * rows + __shfl_sync(kFull, lane == 0 ? atomicAdd(&ctl->work, rows) : 0, 0)) {
     const int idx = base + lane;
     int32_t u = -1;
     B vis = full;
-    if (idx < un) {
+    if (lane < rows && idx < un) {
       u = ul_in[idx];
       vis = B::ld(visit + (size_t)u * W);
     }
@@ -654,10 +746,10 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 5 : 4) bs_pull(const int32_t*
         const int32_t v1 = k + 32 < e ? ld_col(t_col + k + 32, pol) : -1;
         const int32_t v2 = k + 64 < e ? ld_col(t_col + k + 64, pol) : -1;
         const int32_t v3 = k + 96 < e ? ld_col(t_col + k + 96, pol) : -1;
-        if (v0 >= 0) w = w | B::ldg(fin + (size_t)v0 * W);
-        if (v1 >= 0) w = w | B::ldg(fin + (size_t)v1 * W);
-        if (v2 >= 0) w = w | B::ldg(fin + (size_t)v2 * W);
-        if (v3 >= 0) w = w | B::ldg(fin + (size_t)v3 * W);
+        if (v0 >= 0) w = w | B::gather(fin + (size_t)v0 * W);
+        if (v1 >= 0) w = w | B::gather(fin + (size_t)v1 * W);
+        if (v2 >= 0) w = w | B::gather(fin + (size_t)v2 * W);
+        if (v3 >= 0) w = w | B::gather(fin + (size_t)v3 * W);
         if ((w.warp_or() | lvis) == full) break;
       }
       w = w.warp_or();
@@ -678,7 +770,7 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 5 : 4) bs_pull(const int32_t*
         ld_col8(t_col + a, pol, c);
 #pragma unroll
         for (int j = 0; j < 8; j++)
-          if (a + j >= rs && a + j < re) w = w | B::ldg(fin + (size_t)c[j] * W);
+          if (a + j >= rs && a + j < re) w = w | B::gather(fin + (size_t)c[j] * W);
         if ((w | vis) == full) break;
       }
       got = w;
@@ -690,25 +782,21 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 5 : 4) bs_pull(const int32_t*
     if (has) {
       (vis | nw).st(visit + (size_t)u * W);
       nw.st(fout + (size_t)u * W);
-      record_level<W>(ctl, slices, n, u, nw, L);
+      record_level<W>(a, u, nw, L);
       ors = row_ptr[u];
       odeg = row_ptr[u + 1] - ors;
       acc.add((u64)odeg, (u64)deg, nw.popc(), !still);
     }
-    if (deep_cc) add_deep_sums<W>(ctl, nw, L);
+    if (deep_cc) add_deep_sums<W>(sm.deep, nw, L);
     qu.push(still, u);
     if (lazy)
       my_nf += __popc(__ballot_sync(kFull, has));
     else
       emit_routed(has, u, odeg, ors, qa, seg_out, al_pack);
   }
-  qa.flush();
-  qu.flush();
-  acc.flush(ctl, L % 3);
-  if (lazy) {
-    if (lane == 0 && my_nf) atomicAdd(aq_count, my_nf);
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->unlisted[L % 3] = 1;
-  }
+  end_level(sm, ctl, L % 3, acc, qa, &qu, my_nf, aq_count);
+  if (deep_cc) flush_deep_sums<W>(a, sm.deep);
+  if (lazy && tm.thread() == 0) ctl->unlisted[L % 3] = 1;
 }
 
 // Push, phase 1: the active vertices' rows (short rows warp-cooperatively,
@@ -717,32 +805,28 @@ __global__ void __launch_bounds__(kBlock, W == 1 ? 5 : 4) bs_pull(const int32_t*
 // the first toucher (claiming the target in a touched bitmap) queues it for
 // phase 2; in dense mode (large frontiers) no queue is kept and phase 2
 // sweeps all vertices instead.
-template <int W>
-__global__ void __launch_bounds__(kBlock) bs_push_scatter(const int32_t* __restrict__ row_ptr,
-                                                          const int32_t* __restrict__ col, BsCtl* __restrict__ ctl,
-                                                          const u64* __restrict__ visit, u64* __restrict__ fr,
-                                                          u64* __restrict__ nxt, u64* __restrict__ slices,
-                                                          int32_t* __restrict__ aq, const Seg* __restrict__ segs,
-                                                          size_t segcap, int32_t* __restrict__ tq,
-                                                          uint32_t* __restrict__ tbm, int32_t n) {
+template <int W, int kWarps>
+__device__ __forceinline__ void scatter_level(const BsArgs& a, const Team& tm, const BsStep& st,
+                                              BsSmem<kWarps>& sm) {
   using B = Bits<W>;
-  __shared__ int s_excl[kBlock / 32][32];
-  __shared__ int s_rs[kBlock / 32][32];
-  __shared__ int s_v[kBlock / 32][32];
-  __shared__ int32_t s_q[kBlock / 32][kWarpQueueBig];
-  if (ctl->done || ctl->mode != kModePush) return;
-  const int L = ctl->level;
-  const u64* __restrict__ fin = fr + (size_t)((L - 1) % 3) * n * W;
-  const int32_t* aq_in = aq + (size_t)((L - 1) % 3) * n;
-  const Seg* seg_in = segs + (size_t)((L - 1) % 3) * segcap;
-  const int qn = ctl->aq_size[(L - 1) % 3];
-  const int ln = seg_count(ctl->alpack[(L - 1) % 3]);
-  const bool dense = ctl->dense != 0;
-  clear_stale<W>(fr + (size_t)((L + 1) % 3) * n * W, n, aq + (size_t)((L + 1) % 3) * n, ctl->aq_size[(L + 1) % 3],
-                 segs + (size_t)((L + 1) % 3) * segcap, seg_count(ctl->alpack[(L + 1) % 3]),
-                 ctl->unlisted[(L + 1) % 3] != 0);
-  clear_next_slice<W>(slices, n, L, ctl->nbits);
+  BsCtl* const ctl = a.ctl;
+  const int32_t* __restrict__ row_ptr = a.row_ptr;
+  const int32_t* __restrict__ col = a.col;
+  const u64* const visit = a.visit;
+  u64* const nxt = a.nxt;
+  uint32_t* const tbm = a.tbm;
+  const int32_t n = a.n;
+  const int L = st.L;
+  const u64* fin = a.fr + (size_t)((L - 1) % 3) * n * W;
+  const int32_t* aq_in = a.aq + (size_t)((L - 1) % 3) * n;
+  const Seg* seg_in = a.segs + (size_t)((L - 1) % 3) * a.segcap;
+  const int qn = st.qn, ln = st.ln;
+  const bool dense = st.dense != 0;
+  clear_stale<W>(tm, a.fr + (size_t)((L + 1) % 3) * n * W, n, a.aq + (size_t)((L + 1) % 3) * n,
+                 st.stale, a.segs + (size_t)((L + 1) % 3) * a.segcap, st.stale_segs, st.stale_unlisted != 0);
+  clear_next_slice<W>(tm, a.slices, n, L, a.nbits);
   const int wib = threadIdx.x >> 5;
+  int32_t* const deal = sm.q[wib] + kWarpQueueBig;
   // The first two levels expand the sources and their neighbours, whose
   // targets are almost never visited yet: there the visited words are not
   // read (one random load per edge fewer), and the update drops the few
@@ -750,7 +834,7 @@ __global__ void __launch_bounds__(kBlock) bs_push_scatter(const int32_t* __restr
   // edges back into the visited region (half of a wavefront's edges on a
   // mesh).
   const bool filter = L > 2;
-  WarpQueueBig wq(s_q[wib], tq, &ctl->tq_size);
+  WarpQueueBig wq(sm.q[wib], a.tq, &ctl->tq_size);
   auto op = [&](int32_t v, int k, bool valid) {
     bool first = false;
     int32_t u = -1;
@@ -759,7 +843,7 @@ __global__ void __launch_bounds__(kBlock) bs_push_scatter(const int32_t* __restr
       // No look at `next` first: its bits are OR-ed in whether or not they
       // are there, which saves a random load per edge (the scatter is bound
       // by the L1/TEX traffic of its random accesses).
-      B bits = B::ldg(fin + (size_t)v * W);
+      B bits = B::gather(fin + (size_t)v * W);
       if (filter) bits = bits.andnot(B::ldcg(visit + (size_t)u * W));
       if (bits.any()) {
         if (W == 1 && !dense) {
@@ -776,46 +860,51 @@ __global__ void __launch_bounds__(kBlock) bs_push_scatter(const int32_t* __restr
     }
     if (!dense) wq.push(first, u);
   };
-  seg_expand(row_ptr, seg_in, ln, op);
-  warp_expand(row_ptr, aq_in, qn, s_excl[wib], s_rs[wib], s_v[wib], op);
-  wq.flush();
+  seg_expand(tm.warp(), tm.warps(), row_ptr, seg_in, ln, op);
+  warp_expand(tm.warp(), tm.warps(), row_ptr, aq_in, qn, deal, deal + 32, deal + 64, op);
+  LevelAcc none;
+  if (!dense) end_level(sm, ctl, L % 3, none, wq, nullptr, 0, nullptr);
 }
 
 // Push, phase 2: fold `next` into visited / frontier / level slices, over
 // the touched list (list mode, clearing the touched bitmap) or over every
 // vertex (dense mode).
-template <int W>
-__global__ void __launch_bounds__(kBlock) bs_push_update(const int32_t* __restrict__ row_ptr,
-                                                         const int32_t* __restrict__ t_row_ptr,
-                                                         BsCtl* __restrict__ ctl, u64* __restrict__ visit,
-                                                         u64* __restrict__ fr, u64* __restrict__ nxt,
-                                                         u64* __restrict__ slices, int32_t* __restrict__ aq,
-                                                         Seg* __restrict__ segs, size_t segcap,
-                                                         const int32_t* __restrict__ tq, uint32_t* __restrict__ tbm,
-                                                         int32_t n) {
+template <int W, int kWarps>
+__device__ __forceinline__ void update_level(const BsArgs& a, const Team& tm, const BsStep& st,
+                                             BsSmem<kWarps>& sm) {
   using B = Bits<W>;
-  __shared__ int32_t s_q[kBlock / 32][kWarpQueueBig];
-  if (ctl->done || ctl->mode != kModePush) return;
-  const int L = ctl->level;
-  u64* __restrict__ fout = fr + (size_t)(L % 3) * n * W;
-  int32_t* aq_out = aq + (size_t)(L % 3) * n;
-  Seg* seg_out = segs + (size_t)(L % 3) * segcap;
+  BsCtl* const ctl = a.ctl;
+  const int32_t* __restrict__ row_ptr = a.row_ptr;
+  const int32_t* __restrict__ t_row_ptr = a.t_row_ptr;
+  u64 *const visit = a.visit, *const nxt = a.nxt;
+  const int32_t* const tq = a.tq;
+  uint32_t* const tbm = a.tbm;
+  const int32_t n = a.n;
+  const int L = st.L;
+  u64* fout = a.fr + (size_t)(L % 3) * n * W;
+  int32_t* aq_out = a.aq + (size_t)(L % 3) * n;
+  Seg* seg_out = a.segs + (size_t)(L % 3) * a.segcap;
   const B full = B::full_of(ctl);
-  const bool dense = ctl->dense != 0;
-  const int tn = dense ? n : ctl->tq_size;
+  const bool dense = st.dense != 0;
+  const int tn = dense ? n : st.tn;
   // A dense level's output frontier is large enough that the next level is
   // a pull (the decide kernel makes it one), which reads frontier words,
   // not an active list: the sweep then only counts the frontier instead of
   // queueing it and cutting its long rows into segments.  Forced-variant
   // runs keep the list (a forced push reads it).
-  const bool lazy = dense && !ctl->force;
+  const bool lazy = dense && !a.force;
   int my_nf = 0;
-  WarpQueueBig wq(s_q[threadIdx.x >> 5], aq_out, &ctl->aq_size[L % 3]);
+  WarpQueueBig wq(sm.q[threadIdx.x >> 5], aq_out, &ctl->aq_size[L % 3]);
   LevelAcc acc;
-  const bool deep_cc = ctl->cc_sum && L >= kDeepLevel;
-  const int total = gridDim.x * blockDim.x;
-  for (int base = blockIdx.x * blockDim.x; base < tn; base += total) {
-    const int i = base + threadIdx.x;
+  const bool deep_cc = a.cc_sum && L >= kDeepLevel;
+  if (deep_cc) clear_deep_sums<W>(sm.deep);
+  // Vertices per warp: fewer than 32 for a short list, so that its scattered
+  // words (some ten sectors a vertex) are spread over all SMs: a level of 45,000
+  // vertices on 70 CTAs took 11 us.
+  int per = 32;
+  while (per > 4 && (long long)(per >> 1) * tm.warps() >= tn) per >>= 1;
+  for (int base = tm.warp() * per; base < tn; base += tm.warps() * per) {
+    const int i = lane_id() < per ? base + lane_id() : tn;
     B nw = B::zero();
     int32_t u = -1;
     int odeg = 0, ors = 0;
@@ -823,32 +912,33 @@ __global__ void __launch_bounds__(kBlock) bs_push_update(const int32_t* __restri
       u = dense ? i : tq[i];
       if (!dense && W > 1) atomicAnd(tbm + (u >> 5), ~(1u << (u & 31)));
       const B x = B::ld(nxt + (size_t)u * W);
-      if (x.any()) {
-        B::zero().st(nxt + (size_t)u * W);
+      // A listed vertex was touched, so all of its words and row bounds are
+      // fetched in one round trip (three of them took a level of a 700 x 700
+      // grid 10 us); a sweep first looks whether it was.
+      if (!dense || x.any()) {
         const B vis = B::ld(visit + (size_t)u * W);
+        ors = row_ptr[u];
+        odeg = row_ptr[u + 1] - ors;
+        const int ideg = t_row_ptr[u + 1] - t_row_ptr[u];
+        B::zero().st(nxt + (size_t)u * W);
         nw = x.andnot(vis);
         if (nw.any()) {
           (vis | nw).st(visit + (size_t)u * W);
           nw.st(fout + (size_t)u * W);
-          record_level<W>(ctl, slices, n, u, nw, L);
-          ors = row_ptr[u];
-          odeg = row_ptr[u + 1] - ors;
-          acc.add((u64)odeg, (u64)(t_row_ptr[u + 1] - t_row_ptr[u]), nw.popc(), (vis | nw) == full);
+          record_level<W>(a, u, nw, L);
+          acc.add((u64)odeg, (u64)ideg, nw.popc(), (vis | nw) == full);
         }
       }
     }
-    if (deep_cc) add_deep_sums<W>(ctl, nw, L);
+    if (deep_cc) add_deep_sums<W>(sm.deep, nw, L);
     if (lazy)
       my_nf += __popc(__ballot_sync(kFull, nw.any()));
     else
       emit_routed(nw.any(), u, odeg, ors, wq, seg_out, &ctl->alpack[L % 3]);
   }
-  wq.flush();
-  acc.flush(ctl, L % 3);
-  if (lazy) {
-    if (lane_id() == 0 && my_nf) atomicAdd(&ctl->aq_size[L % 3], my_nf);
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->unlisted[L % 3] = 1;
-  }
+  end_level(sm, ctl, L % 3, acc, wq, nullptr, my_nf, &ctl->aq_size[L % 3]);
+  if (deep_cc) flush_deep_sums<W>(a, sm.deep);
+  if (lazy && tm.thread() == 0) ctl->unlisted[L % 3] = 1;
 }
 
 // Expands the level slices of one batch into its distance rows: thread per
@@ -859,7 +949,7 @@ __global__ void __launch_bounds__(kBlock) bs_push_update(const int32_t* __restri
 // itself (level 0) or was written out during the traversal, and is kept.
 template <int W, int NB>
 __device__ __forceinline__ void emit_vertex(int32_t* __restrict__ dist, int32_t n, int nb_src, size_t u,
-                                            const u64* __restrict__ visit, const u64* __restrict__ slices,
+                                            const u64* visit, const u64* slices,
                                             const int32_t* __restrict__ src) {
 #pragma unroll
   for (int i = 0; i < W; i++) {
@@ -898,8 +988,7 @@ __device__ __forceinline__ void emit_vertex(int32_t* __restrict__ dist, int32_t 
 // 19 with a shift and mask per slice.
 template <int W, int NB>
 __device__ __forceinline__ void emit_vertex4_packed(int32_t* __restrict__ dist, int32_t n, int nb_src, size_t u0,
-                                                    const u64* __restrict__ visit,
-                                                    const u64* __restrict__ slices) {
+                                                    const u64* visit, const u64* slices) {
 #pragma unroll
   for (int i = 0; i < W; i++) {
     if (64 * i >= nb_src) break;
@@ -945,7 +1034,7 @@ __device__ __forceinline__ void emit_vertex4_packed(int32_t* __restrict__ dist, 
 // the other three.
 template <int W, int NB>
 __device__ __forceinline__ void emit_vertex4(int32_t* __restrict__ dist, int32_t n, int nb_src, size_t u0,
-                                             const u64* __restrict__ visit, const u64* __restrict__ slices,
+                                             const u64* visit, const u64* slices,
                                              const int32_t* __restrict__ src) {
 #pragma unroll
   for (int i = 0; i < W; i++) {
@@ -998,8 +1087,8 @@ __device__ __forceinline__ void emit_vertex4(int32_t* __restrict__ dist, int32_t
 // counts them with popc; CTA totals go to the batch's rows with one atomic
 // per source.
 template <int W>
-__device__ __forceinline__ void emit_closeness(const BsCtl* __restrict__ ctl, const u64* __restrict__ visit,
-                                               const u64* __restrict__ slices, int32_t n, int nb, int nbits) {
+__device__ __forceinline__ void emit_closeness(const Team& tm, const BsCtl* ctl, int batch, const u64* visit,
+                                               const u64* slices, int32_t n, int nb, int nbits) {
   __shared__ unsigned long long s_sum[64 * W], s_cnt[64 * W];
   for (int t = threadIdx.x; t < 64 * W; t += blockDim.x) {
     s_sum[t] = 0;
@@ -1010,30 +1099,36 @@ __device__ __forceinline__ void emit_closeness(const BsCtl* __restrict__ ctl, co
 #pragma unroll
   for (int i = 0; i < W; i++) {
     if (64 * i >= nb) break;
-    unsigned long long sum_lo = 0, sum_hi = 0, cnt_lo = 0, cnt_hi = 0;
-    for (int base = global_warp() * 32; base < n; base += num_warps() * 32) {
+    unsigned long long sum_lo = 0, sum_hi = 0;
+    unsigned cnt_lo = 0, cnt_hi = 0;
+    for (int base = tm.warp() * 32; base < n; base += tm.warps() * 32) {
       const int u = base + lane;
       const bool in = u < n;
+      // the words of every slice are loaded before the first is transposed
+      u64 x[kShallowBits];
+#pragma unroll
+      for (int k = 0; k < kShallowBits; k++) x[k] = in && k < nbits ? slices[((size_t)k * n + u) * W + i] : 0ull;
       const u64 vis = in ? visit[(size_t)u * W + i] : 0ull;
       cnt_lo += __popc(warp_transpose32((uint32_t)vis));
       cnt_hi += __popc(warp_transpose32((uint32_t)(vis >> 32)));
-      for (int k = 0; k < nbits; k++) {
-        const u64 x = in ? slices[((size_t)k * n + u) * W + i] : 0ull;
-        sum_lo += (unsigned long long)__popc(warp_transpose32((uint32_t)x)) << k;
-        sum_hi += (unsigned long long)__popc(warp_transpose32((uint32_t)(x >> 32))) << k;
+#pragma unroll
+      for (int k = 0; k < kShallowBits; k++) {
+        if (k >= nbits) break;
+        sum_lo += (unsigned long long)__popc(warp_transpose32((uint32_t)x[k])) << k;
+        sum_hi += (unsigned long long)__popc(warp_transpose32((uint32_t)(x[k] >> 32))) << k;
       }
     }
     if (cnt_lo | sum_lo) {
-      atomicAdd(&s_cnt[64 * i + lane], cnt_lo);
+      atomicAdd(&s_cnt[64 * i + lane], (unsigned long long)cnt_lo);
       atomicAdd(&s_sum[64 * i + lane], sum_lo);
     }
     if (cnt_hi | sum_hi) {
-      atomicAdd(&s_cnt[64 * i + 32 + lane], cnt_hi);
+      atomicAdd(&s_cnt[64 * i + 32 + lane], (unsigned long long)cnt_hi);
       atomicAdd(&s_sum[64 * i + 32 + lane], sum_hi);
     }
   }
   __syncthreads();
-  const size_t row0 = (size_t)ctl->batch * 64 * W;
+  const size_t row0 = (size_t)batch * 64 * W;
   for (int t = threadIdx.x; t < nb; t += blockDim.x) {
     if (s_sum[t]) atomicAdd(ctl->cc_sum + row0 + t, s_sum[t]);
     if (s_cnt[t]) atomicAdd(ctl->cc_cnt + row0 + t, s_cnt[t]);
@@ -1045,11 +1140,10 @@ __device__ __forceinline__ void emit_closeness(const BsCtl* __restrict__ ctl, co
 // lowest and highest level among them (INT_MAX / -1 when none).  Entries
 // written during the traversal (src set, as in emit_vertex) are kept.
 template <int W>
-__device__ __forceinline__ void emit_levels(const BsCtl* __restrict__ ctl, const u64* __restrict__ visit,
-                                            const u64* __restrict__ slices, int32_t n, int nb, int nbits,
-                                            const int32_t* __restrict__ src) {
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t u = blockIdx.x * (size_t)blockDim.x + threadIdx.x; u < (size_t)n; u += stride) {
+__device__ __forceinline__ void emit_levels(const Team& tm, const BsCtl* ctl, const u64* visit, const u64* slices,
+                                            int32_t n, int nb, int nbits, const int32_t* __restrict__ src) {
+  const size_t stride = tm.threads();
+  for (size_t u = tm.thread(); u < (size_t)n; u += stride) {
     const u64 vis = visit[u * W];
     u64 any = 0ull;
     for (int k = 0; k < nbits; k++) any |= slices[((size_t)k * n + u) * W];
@@ -1084,26 +1178,28 @@ __device__ __forceinline__ void emit_levels(const BsCtl* __restrict__ ctl, const
 }
 
 template <int W>
-__global__ void __launch_bounds__(kBlock) bs_emit_dist(const BsCtl* __restrict__ ctl, const u64* __restrict__ visit,
-                                                       const u64* __restrict__ slices, int32_t n) {
-  const int batch = ctl->batch;
+__device__ __forceinline__ void emit_batch(const BsArgs& a, const Team& tm) {
+  const BsCtl* const ctl = a.ctl;
+  const u64 *const visit = a.visit, *const slices = a.slices;
+  const int32_t n = a.n;
+  const int batch = batch_of(a);
   const int per = 64 * W;
   const int nb = min(per, ctl->nsrc - batch * per);
   // levels below kDeepLevel are in the slices; deeper ones were written out
   const int nbits = min(32 - __clz(max(ctl->level, 1)), kShallowBits);
   const int32_t* src = ctl->level >= kDeepLevel ? ctl->sources + (size_t)batch * per : nullptr;
   if (ctl->lv_block) {
-    if (W == 1) emit_levels<W>(ctl, visit, slices, n, min(64, ctl->nsrc - batch * 64), nbits, src);
+    if (W == 1) emit_levels<W>(tm, ctl, visit, slices, n, min(64, ctl->nsrc - batch * 64), nbits, src);
     return;
   }
   if (ctl->cc_sum) {
-    emit_closeness<W>(ctl, visit, slices, n, nb, nbits);
+    emit_closeness<W>(tm, ctl, batch, visit, slices, n, nb, nbits);
     return;
   }
   int32_t* dist = ctl->dist_base + (size_t)batch * per * n;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  const size_t t0 = tm.thread(), stride = tm.threads();
   if ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(dist) & 15) == 0 && !src) {
-    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < (size_t)n / 4; q += stride) {
+    for (size_t q = t0; q < (size_t)n / 4; q += stride) {
       switch (nbits) {
         case 1: emit_vertex4_packed<W, 1>(dist, n, nb, 4 * q, visit, slices); break;
         case 2: emit_vertex4_packed<W, 2>(dist, n, nb, 4 * q, visit, slices); break;
@@ -1115,7 +1211,7 @@ __global__ void __launch_bounds__(kBlock) bs_emit_dist(const BsCtl* __restrict__
     return;
   }
   if ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(dist) & 15) == 0) {
-    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < (size_t)n / 4; q += stride) {
+    for (size_t q = t0; q < (size_t)n / 4; q += stride) {
       switch (nbits) {
         case 1: emit_vertex4<W, 1>(dist, n, nb, 4 * q, visit, slices, src); break;
         case 2: emit_vertex4<W, 2>(dist, n, nb, 4 * q, visit, slices, src); break;
@@ -1126,7 +1222,7 @@ __global__ void __launch_bounds__(kBlock) bs_emit_dist(const BsCtl* __restrict__
     }
     return;
   }
-  for (size_t u = blockIdx.x * (size_t)blockDim.x + threadIdx.x; u < (size_t)n; u += stride) {
+  for (size_t u = t0; u < (size_t)n; u += stride) {
     switch (nbits) {
       case 1: emit_vertex<W, 1>(dist, n, nb, u, visit, slices, src); break;
       case 2: emit_vertex<W, 2>(dist, n, nb, u, visit, slices, src); break;
@@ -1137,43 +1233,55 @@ __global__ void __launch_bounds__(kBlock) bs_emit_dist(const BsCtl* __restrict__
   }
 }
 
+enum : int32_t { kBsClear = 0, kBsInit, kBsScatter, kBsUpdate, kBsPull };
+
 // One warp.  Ends the batch when the frontier is empty, otherwise picks
 // the next level's variant: the forced one if set, else the learned
 // selector if weights are loaded, else push while
 // push_ratio x frontier edges < unfinished in-edges, dense once the
 // frontier's edges reach n.
-__global__ void bs_decide(BsCtl* __restrict__ ctl, int32_t n, const float* __restrict__ sel_w,
-                          cudaGraphConditionalHandle loop, int in_graph) {
-  const int lane = threadIdx.x;
-  if (sel_w) sel_prefetch(sel_w);
-  // every lane reads the control block before lane 0 changes it
-  const int done = ctl->done;
-  const int L = ctl->level;
-  const int cur_mode = ctl->mode, ul_cur = ctl->ul_cur, hs_cur = ctl->hs_cur;
-  const long long mu = ctl->mu - ctl->mu_dec;
-  const int nf = ctl->aq_size[L % 3] + long_vertices(ctl->alpack[L % 3]);
-  const bool unlisted = ctl->unlisted[L % 3] != 0;
-  const long long mf = (long long)ctl->mf[L % 3];
-  const int policy = ctl->policy, ratio = ctl->push_ratio, force = ctl->force, prev_nf = ctl->prev_nf;
-  const bool sel = ctl->use_sel && sel_w;
-  const float sel_margin = ctl->sel_margin;
-  const long long m = ctl->m;
-  const int per = 64 * ctl->width;
-  const int nb = min(per, ctl->nsrc - ctl->batch * per);
+// Read through volatile loads: inside the persistent launch the counters
+// that other CTAs raised may sit stale in this SM's L1.  All of them are read
+// before lane 0 writes any (one round trip).  Returns whether the batch is
+// done, else what the next level needs in `st`.
+__device__ __forceinline__ bool decide_level(const BsArgs& a, BsStep& st) {
+  BsCtl* const ctl = a.ctl;
+  const float* sel_w = a.sel_w;
+  const int32_t n = a.n;
+  const int lane = lane_id();
+  const volatile BsCtl* vc = ctl;
+  const bool sel = vc->use_sel && sel_w;
+  const int done = vc->done;
+  const int L = vc->level;
+  const int cur_mode = vc->mode, ul_cur = vc->ul_cur, hs_cur = vc->hs_cur;
+  const int ul0 = vc->ul_size[0], ul1 = vc->ul_size[1], hs0 = vc->hs_size[0], hs1 = vc->hs_size[1];
+  const long long mu = vc->mu - vc->mu_dec;
+  const int policy = vc->policy, ratio = vc->push_ratio, force = vc->force, prev_nf = vc->prev_nf;
+  const float sel_margin = vc->sel_margin;
+  const long long m = vc->m;
+  const int per = 64 * vc->width;
+  const int nb = min(per, vc->nsrc - vc->batch * per);
+  const int n_push = vc->n_push, n_pull = vc->n_pull;
+  const int out = L % 3, old = (L + 2) % 3;  // the frontier this level wrote; the slot the next one clears
+  const int qn = vc->aq_size[out], stale = vc->aq_size[old];
+  const unsigned long long al = vc->alpack[out], al_old = vc->alpack[old];
+  const bool unlisted = vc->unlisted[out] != 0, stale_unlisted = vc->unlisted[old] != 0;
+  const long long mf = (long long)vc->mf[out];
+  const int nf = qn + long_vertices(al);
   __syncwarp();
-  if (done) {
-    if (lane == 0 && in_graph) cudaGraphSetConditional(loop, 0);
-    return;
-  }
+  if (done) return true;
+  const bool pulled = cur_mode != kModePush;
+  const int ul_next = pulled ? (ul_cur < 0 ? 0 : ul_cur ^ 1) : ul_cur;
+  const int hs_next = pulled ? (hs_cur < 0 ? 0 : hs_cur ^ 1) : hs_cur;
   if (lane == 0) {
-    if (cur_mode == kModePush) {
-      ctl->n_push++;
+    if (!pulled) {
+      ctl->n_push = n_push + 1;
     } else {
-      ctl->n_pull++;
-      ctl->ul_cur = ul_cur < 0 ? 0 : ul_cur ^ 1;
-      ctl->ul_size[(ul_cur < 0 ? 0 : ul_cur ^ 1) ^ 1] = 0;
-      ctl->hs_cur = hs_cur < 0 ? 0 : hs_cur ^ 1;
-      ctl->hs_size[(hs_cur < 0 ? 0 : hs_cur ^ 1) ^ 1] = 0;
+      ctl->n_pull = n_pull + 1;
+      ctl->ul_cur = ul_next;
+      ctl->ul_size[ul_next ^ 1] = 0;
+      ctl->hs_cur = hs_next;
+      ctl->hs_size[hs_next ^ 1] = 0;
     }
     ctl->mu = mu;
     ctl->mu_dec = 0;
@@ -1182,11 +1290,8 @@ __global__ void bs_decide(BsCtl* __restrict__ ctl, int32_t n, const float* __res
     ctl->hwork = 0;
   }
   if (nf == 0 || L >= n) {
-    if (lane == 0) {
-      ctl->done = 1;
-      if (in_graph) cudaGraphSetConditional(loop, 0);
-    }
-    return;
+    if (lane == 0) ctl->done = 1;
+    return true;
   }
   int variant;
   if (policy == DAWN_VARIANT_PUSH || mf * ratio < mu) {
@@ -1219,15 +1324,283 @@ __global__ void bs_decide(BsCtl* __restrict__ ctl, int32_t n, const float* __res
     ctl->prev_nf = nf;
     ctl->level = L + 1;
   }
+  st.phase = variant == kVarPull ? kBsPull : kBsScatter;
+  st.L = L + 1;
+  st.dense = variant == kVarDense;
+  st.qn = qn;
+  st.ln = seg_count(al);
+  st.stale = stale;
+  st.stale_segs = seg_count(al_old);
+  st.stale_unlisted = stale_unlisted;
+  st.tn = 0;
+  st.ul_cur = ul_next;
+  st.un = ul_next < 0 ? a.ul_static_size : (ul_next ? ul1 : ul0);
+  st.hs_cur = hs_next;
+  st.hn = hs_next < 0 ? a.hv_segs : (hs_next ? hs1 : hs0);
+  st.nf = nf;
+  // Warp tasks of the level, for its CTAs: a vertex or 32 edges of a push,
+  // eight rows or a segment of a pull, 128 words to clear (0: all CTAs).
+  st.ctas = 0;
+  long long work = max((long long)qn + seg_count(al), mf / 32);
+  if (variant == kVarPull) work = (long long)st.un / 8 + st.hn;
+  work = max(work, (long long)(clears_slot(stale, stale_unlisted, n) ? n : stale) / 128);
+  if ((((unsigned)L + 2) & ((unsigned)L + 1)) == 0) work = max(work, (long long)n / 128);  // level L + 2 opens a slice
+  if (variant != kVarDense) st.ctas = (int)min((long long)n, work + 1);
+  return false;
 }
 
-__global__ void bs_next(BsCtl* __restrict__ ctl) {
+// The running level's BsStep from the control block.
+__device__ __forceinline__ BsStep read_step(const BsArgs& a) {
+  const BsCtl* c = a.ctl;
+  BsStep st = {};
+  const int L = c->level, in = (L - 1) % 3, old = (L + 1) % 3;
+  st.L = L;
+  st.dense = c->dense;
+  st.qn = c->aq_size[in];
+  st.ln = seg_count(c->alpack[in]);
+  st.stale = c->aq_size[old];
+  st.stale_segs = seg_count(c->alpack[old]);
+  st.stale_unlisted = c->unlisted[old];
+  st.tn = c->tq_size;
+  st.ul_cur = c->ul_cur;
+  st.un = st.ul_cur < 0 ? a.ul_static_size : c->ul_size[st.ul_cur];
+  st.hs_cur = c->hs_cur;
+  st.hn = st.hs_cur < 0 ? a.hv_segs : c->hs_size[st.hs_cur];
+  st.nf = st.qn + long_vertices(c->alpack[in]);
+  return st;
+}
+
+// One thread: the batch's counters into the call's.
+__device__ __forceinline__ void count_batch(BsCtl* ctl) {
+  const volatile BsCtl* vc = ctl;
+  ctl->total_reached = vc->total_reached + vc->reached;
+  ctl->total_levels = vc->total_levels + vc->level;
+  ctl->total_push = vc->total_push + vc->n_push;
+  ctl->total_pull = vc->total_pull + vc->n_pull;
+}
+
+// --- one launch per step of a level (traced calls) ------------------------------
+
+constexpr int kStepWarps = kBlock / 32;
+
+__global__ void __launch_bounds__(kBlock) bs_clear(const __grid_constant__ BsArgs a) {
+  clear_words(Team{(int)blockIdx.x, (int)gridDim.x}, a.words, a.nwords);
+}
+template <int W>
+__global__ void bs_init(const __grid_constant__ BsArgs a) {
+  init_batch<W>(a);
+}
+template <int W>
+__global__ void __launch_bounds__(kBlock, W == 1 ? 5 : 4) bs_pull(const __grid_constant__ BsArgs a) {
+  __shared__ BsSmem<kStepWarps> sm;
+  if (a.ctl->done || a.ctl->mode != kModePull) return;
+  pull_level<W>(a, Team{(int)blockIdx.x, (int)gridDim.x}, read_step(a), sm);
+}
+template <int W>
+__global__ void __launch_bounds__(kBlock) bs_push_scatter(const __grid_constant__ BsArgs a) {
+  __shared__ BsSmem<kStepWarps> sm;
+  if (a.ctl->done || a.ctl->mode != kModePush) return;
+  scatter_level<W>(a, Team{(int)blockIdx.x, (int)gridDim.x}, read_step(a), sm);
+}
+template <int W>
+__global__ void __launch_bounds__(kBlock) bs_push_update(const __grid_constant__ BsArgs a) {
+  __shared__ BsSmem<kStepWarps> sm;
+  if (a.ctl->done || a.ctl->mode != kModePush) return;
+  update_level<W>(a, Team{(int)blockIdx.x, (int)gridDim.x}, read_step(a), sm);
+}
+template <int W>
+__global__ void __launch_bounds__(kBlock) bs_emit_dist(const __grid_constant__ BsArgs a) {
+  emit_batch<W>(a, Team{(int)blockIdx.x, (int)gridDim.x});
+}
+__global__ void bs_decide(const __grid_constant__ BsArgs a) {
+  BsStep st;
+  decide_level(a, st);
+}
+__global__ void bs_next(const __grid_constant__ BsArgs a) {
   if (threadIdx.x != 0) return;
-  ctl->total_reached += ctl->reached;
-  ctl->total_levels += ctl->level;
-  ctl->total_push += ctl->n_push;
-  ctl->total_pull += ctl->n_pull;
-  ctl->batch += 1;
+  count_batch(a.ctl);
+  a.ctl->batch += 1;
+}
+
+// --- the persistent launch ----------------------------------------------------------
+
+constexpr uint32_t kBsPollLimit = 1u << 27;  // polls of one wait (over 30 s) before the launch gives up
+
+// CTAs for `work` warp tasks.
+__device__ __forceinline__ int bs_ctas(int work, int warps) {
+  const int c = (work + warps - 1) / warps;
+  return c < 1 ? 1 : min(c, (int)gridDim.x);
+}
+
+// One warp of the last CTA to finish phase st; every other participant has
+// arrived and the rest only poll.  Turns st into the next phase; returns false
+// when the batch is done.
+// Not inlined: its registers would be the levels' spills.
+template <int kWarps>
+__device__ __noinline__ bool next_phase(const BsArgs& a, BsStep& step) {
+  BsStep st = step;
+  BsCtl* const ctl = a.ctl;
+  const volatile BsCtl* vc = ctl;
+  if (st.phase == kBsClear) {
+    if (lane_id() == 0) ctl->batch = a.batch;
+    st.phase = kBsInit;
+    st.ctas = 1;
+    step = st;
+    return true;
+  }
+  if (st.phase == kBsScatter) {
+    st.tn = vc->tq_size;
+    st.phase = kBsUpdate;
+    st.ctas = st.dense ? (int)gridDim.x : bs_ctas((st.tn + 3) / 4, kWarps);
+    step = st;
+    return true;
+  }
+  if (st.phase == kBsInit) {
+    const uint32_t arrived = st.arrived;
+    __threadfence();
+    st = read_step(a);
+    st.arrived = arrived;
+    st.phase = vc->mode == kModePush ? kBsScatter : kBsPull;
+    st.ctas = (int)gridDim.x;
+    step = st;
+    return true;
+  }
+  if (decide_level(a, st)) {
+    if (lane_id() == 0) count_batch(ctl);
+    return false;
+  }
+  st.ctas = st.ctas ? bs_ctas(st.ctas, kWarps) : (int)gridDim.x;
+  step = st;
+  return true;
+}
+
+constexpr int kStepWords = 9;
+__device__ __forceinline__ u64 pack_step(const BsStep& st, int i) {
+  const uint32_t lo[kStepWords] = {(uint32_t)st.L, (uint32_t)st.qn, (uint32_t)st.ln, (uint32_t)st.stale,
+                                   (uint32_t)st.stale_segs, (uint32_t)(st.phase == kBsPull ? st.un : st.tn),
+                                   (uint32_t)st.hn, (uint32_t)st.nf, st.arrived};
+  const uint32_t hi = i == 0 ? (uint32_t)st.ctas
+                             : (uint32_t)(st.phase | st.dense << 3 | st.stale_unlisted << 4 | (st.ul_cur + 1) << 5 |
+                                          (st.hs_cur + 1) << 7);
+  uint32_t x = lo[0];
+#pragma unroll
+  for (int k = 1; k < kStepWords; k++) x = i == k ? lo[k] : x;
+  return (u64)(hi & 0xffffu) << 32 | x;
+}
+__device__ __forceinline__ BsStep unpack_step(const u64* w) {
+  BsStep st;
+  const uint32_t f = (uint32_t)(w[1] >> 32) & 0xffffu;
+  st.ctas = (int)((w[0] >> 32) & 0xffffu);
+  st.phase = f & 7;
+  st.dense = (f >> 3) & 1;
+  st.stale_unlisted = (f >> 4) & 1;
+  st.ul_cur = (int)((f >> 5) & 3) - 1;
+  st.hs_cur = (int)((f >> 7) & 3) - 1;
+  st.L = (int)(uint32_t)w[0];
+  st.qn = (int)(uint32_t)w[1];
+  st.ln = (int)(uint32_t)w[2];
+  st.stale = (int)(uint32_t)w[3];
+  st.stale_segs = (int)(uint32_t)w[4];
+  st.tn = st.un = (int)(uint32_t)w[5];
+  st.hn = (int)(uint32_t)w[6];
+  st.nf = (int)(uint32_t)w[7];
+  st.arrived = (uint32_t)w[8];
+  return st;
+}
+
+// One batch in one cooperative launch: clear, seed, levels (the distances
+// follow in a launch of their own, whose 89 registers would cost this one its
+// occupancy).  As launches in a conditional graph a level was four kernels, of
+// which one or two returned at once: 12 to 20 us before any work, the bound of
+// every batch with small or many levels.  Here a step of a level ends with one
+// block barrier and one arrival per CTA, and about 2 us in the last CTA for the
+// decision; steps with little work name fewer CTAs, the others poll.  The CTAs
+// keep the occupancy of the per-level pull: 1,280 threads per SM at 48
+// registers (W = 1), 1,024 at 64.  Per call, graph form -> this:
+//   Erdos-Renyi, 65,536 vertices, 64 sources   201 -> 132 us
+//   RMAT-16, 64 sources                         254 -> 164
+//   RMAT-18, 500 sources                       1068 -> 860
+//   RMAT-22, 64 sources                        1176 -> 1128
+//   grid 700 x 700, 64 sources                26060 -> 22050
+//   kNN, 200,000 vertices, 64 sources         16050 -> 7450
+template <int W>
+__global__ void __launch_bounds__(W == 1 ? 640 : 512, 2) bs_traverse(const __grid_constant__ BsArgs a) {
+  constexpr int kWarps = (W == 1 ? 640 : 512) / 32;
+  __shared__ BsSmem<kWarps> sm;
+  BsCtl* const ctl = a.ctl;
+  const int lane = lane_id(), wib = threadIdx.x >> 5;
+  // no phase can open before every CTA has arrived, so all read the same
+  uint32_t gen = (uint32_t)(*static_cast<const volatile unsigned long long*>(&ctl->sync.word[0]) >> 48);
+  const BsStep& st = sm.st;  // in shared memory: its fields would cost the levels their registers
+  if (threadIdx.x == 0) {
+    sm.st = BsStep{};
+    sm.st.phase = kBsClear;
+    sm.st.ctas = (int)gridDim.x;
+    sm.st.arrived = (uint32_t)(uint32_t)*static_cast<const volatile unsigned long long*>(&ctl->sync.word[8]);
+  }
+  __syncthreads();
+  for (;;) {
+    const Team tm{(int)blockIdx.x, st.ctas};
+    switch (st.phase) {
+      case kBsClear: clear_words(tm, a.words, a.nwords); break;
+      case kBsInit: init_batch<W>(a); break;
+      case kBsScatter: scatter_level<W>(a, tm, st, sm); break;
+      case kBsUpdate: update_level<W>(a, tm, st, sm); break;
+      default: pull_level<W>(a, tm, st, sm);
+    }
+    __syncthreads();
+    if (wib == 0) {
+      int last = 0;
+      if (lane == 0) {
+        __threadfence();
+        last = atomicAdd(&ctl->arrive.n, 1u) + 1 == st.arrived + (uint32_t)st.ctas;
+      }
+      if (__shfl_sync(kFull, last, 0)) {
+        __threadfence();
+        if (lane == 0) {
+          sm.next = st;
+          sm.next.arrived = st.arrived + (uint32_t)st.ctas;
+        }
+        __syncwarp();
+        const bool more = next_phase<kWarps>(a, sm.next);
+        __syncwarp();
+        if (!more && lane == 0) sm.next.ctas = 0;
+        const u64 tag = (u64)((gen + 1) & 0xffffu) << 48;
+        __syncwarp();
+        __threadfence();
+        if (lane < kStepWords) *static_cast<volatile unsigned long long*>(&ctl->sync.word[lane]) = tag | pack_step(sm.next, lane);
+      }
+      __syncwarp();
+      bool idle = false;
+      for (uint32_t polls = 0;; polls++) {
+        u64 w;
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(&ctl->sync.word[lane < kStepWords ? lane : 0]) : "memory");
+        const uint32_t tag = (uint32_t)(w >> 48), tag0 = __shfl_sync(kFull, tag, 0);
+        if (__all_sync(kFull, tag == tag0) && tag != gen) {
+          gen = tag;
+          polls = 0;
+          const uint32_t ctas = (uint32_t)(__shfl_sync(kFull, w, 0) >> 32) & 0xffffu;
+          if (ctas == 0 || blockIdx.x < ctas) {
+            if (lane < kStepWords) sm.word[lane] = w;
+            __syncwarp();
+            if (lane == 0) sm.st = unpack_step(sm.word);
+            break;
+          }
+          idle = true;
+        }
+        if (polls == kBsPollLimit) {
+          if (lane == 0) {
+            ctl->err = DAWN_ERR_TIMEOUT;
+            sm.st.ctas = 0;
+          }
+          break;
+        }
+        if (idle) __nanosleep(64);
+      }
+    }
+    __syncthreads();
+    if (st.ctas == 0) return;
+  }
 }
 
 void probe_bs(const void* p, LevelProbe* out) {
@@ -1272,7 +1645,7 @@ __global__ void scatter_flagged(const int64_t* __restrict__ flags, const int64_t
 // Static pull lists of the in-edge CSR (shared with the weighted pull).
 dawn_status build_static_list(dawn_graph* g) {
   if (g->ul_static.p && g->static_seg == g->pull_seg) return DAWN_OK;
-  // Captured traversal graphs (bitset and weighted single-source) hold these
+  // Captured traversal graphs (weighted, level by level) hold these
   // lists' addresses and sizes; a rebuild for a new segment size may move
   // or resize them.
   if (g->ul_static.p) drop_graphs(g);
@@ -1328,16 +1701,6 @@ dawn_status run_width(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32
                       int32_t* lv_range = nullptr) {
   const int32_t n = g->n;
   const size_t nn = (size_t)n;
-  const int wi = W == 1 ? 0 : (W == 2 ? 1 : 2);
-  if (g->static_seg != g->pull_seg) {
-    // the pull lists are rebuilt for a new segment size; the captured
-    // graphs hold the old list sizes
-    for (cudaGraphExec_t& e : g->bs_exec)
-      if (e) {
-        cudaGraphExecDestroy(e);
-        e = nullptr;
-      }
-  }
   DAWN_CHECK(build_static_list(g));
   if (reinterpret_cast<uintptr_t>(g->t_col) % 32 != 0) {  // the pull's 256-bit column loads
     set_error("in-edge column array is not 32-byte aligned");
@@ -1347,25 +1710,17 @@ dawn_status run_width(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32
   // lists: aq[3] | tq | ul[2] | touched bitmap ; segments[3]
   // Levels never exceed n, and levels from kDeepLevel on bypass the slices.
   const int nbits = std::min(32 - __builtin_clz((unsigned)n), kShallowBits);
-  // The cached graphs hold the word buffer's address: a wider batch that
-  // grows the buffer makes the narrower widths' graphs stale.
-  const void* words_before = g->bs_words.p;
   DAWN_CHECK(ensure(g->bs_words, sizeof(u64) * W * (5 + (size_t)nbits) * nn, g->stream));
-  if (g->bs_words.p != words_before)
-    for (cudaGraphExec_t& e : g->bs_exec)
-      if (e) {
-        cudaGraphExecDestroy(e);
-        e = nullptr;
-      }
+  const bool fresh = g->bs_queues.p == nullptr;
   DAWN_CHECK(ensure(g->bs_queues, sizeof(int32_t) * 6 * nn + sizeof(uint32_t) * (nn / 32 + 1), g->stream));
+  // The touched bitmap starts clear; list-mode updates clear what they set.
+  if (fresh)
+    DAWN_CUDA(cudaMemsetAsync(g->bs_queues.as<int32_t>() + 6 * nn, 0, sizeof(uint32_t) * (nn / 32 + 1), g->stream));
   const size_t segcap = seg_capacity(n, g->m);
   DAWN_CHECK(ensure(g->bs_segs, sizeof(Seg) * 3 * segcap, g->stream));
-  DAWN_CHECK(ensure(g->bs_ctl, sizeof(BsCtl), g->stream));
-  DAWN_CHECK(ensure(g->bs_sources, sizeof(int32_t) * (size_t)nsrc, g->stream));
-  DAWN_CUDA(cudaMemcpyAsync(g->bs_sources.p, sources, sizeof(int32_t) * nsrc, cudaMemcpyHostToDevice,
-                            g->stream));
-  // The touched bitmap must start clear; list-mode updates clear what they set.
-  DAWN_CUDA(cudaMemsetAsync(g->bs_queues.as<int32_t>() + 6 * nn, 0, sizeof(uint32_t) * (nn / 32 + 1), g->stream));
+  // one upload: the control block, then the sources
+  const size_t up_bytes = sizeof(BsCtl) + sizeof(int32_t) * (size_t)nsrc;
+  DAWN_CHECK(ensure(g->bs_ctl, up_bytes, g->stream));
   BsCtl c = {};
   c.nsrc = nsrc;
   c.policy = DAWN_VARIANT_BITSET;
@@ -1373,7 +1728,7 @@ dawn_status run_width(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32
   c.nbits = nbits;
   c.width = W;
   c.dist_base = d_dist;
-  c.sources = g->bs_sources.as<int32_t>();
+  c.sources = reinterpret_cast<const int32_t*>(g->bs_ctl.as<BsCtl>() + 1);
   c.cc_sum = cc_sum;
   c.cc_cnt = cc_cnt;
   c.lv_block = lv_block;
@@ -1382,27 +1737,13 @@ dawn_status run_width(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32
   c.sel_margin = g->sel_margin;
   c.force = g->force_variant;
   c.m = g->m;
-  DAWN_CUDA(cudaMemcpyAsync(g->bs_ctl.p, &c, sizeof(BsCtl), cudaMemcpyHostToDevice, g->stream));
+  std::vector<unsigned char> up(up_bytes);
+  std::memcpy(up.data(), &c, sizeof(c));
+  std::memcpy(up.data() + sizeof(c), sources, sizeof(int32_t) * (size_t)nsrc);
+  // pageable: staged before the call returns
+  DAWN_CUDA(cudaMemcpyAsync(g->bs_ctl.p, up.data(), up_bytes, cudaMemcpyHostToDevice, g->stream));
 
-  struct {
-    BsCtl* ctl;
-    const int32_t *row_ptr, *col, *t_row_ptr, *t_col, *ul_static;
-    u64 *words, *visit, *fr, *fr0, *nxt, *slices;
-    int32_t *aq, *aq0, *tq, *ul;
-    uint32_t* tbm;
-    Seg* segs;
-    size_t segcap;
-    int32_t ul_static_size, hv_count, hv_segs, pull_seg;
-    const int32_t *hv_static, *hv_segoff;
-    u64* hv_acc;
-    int2* hv_tasks;
-    size_t nwords;
-    int32_t n;
-    long long m;
-    cudaGraphConditionalHandle handle;
-    int in_graph;
-    const float* sel_w;
-  } a;
+  BsArgs a = {};
   a.sel_w = g->sel_slot.as<float>();
   a.ctl = g->bs_ctl.as<BsCtl>();
   a.row_ptr = g->row_ptr;
@@ -1421,11 +1762,9 @@ dawn_status run_width(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32
   a.words = g->bs_words.as<u64>();
   a.visit = a.words;
   a.fr = a.words + W * nn;
-  a.fr0 = a.fr;
   a.nxt = a.words + 4 * W * nn;
   a.slices = a.words + 5 * W * nn;
   a.aq = g->bs_queues.as<int32_t>();
-  a.aq0 = a.aq;
   a.tq = a.aq + 3 * nn;
   a.ul = a.aq + 4 * nn;
   a.tbm = reinterpret_cast<uint32_t*>(a.aq + 6 * nn);
@@ -1434,51 +1773,55 @@ dawn_status run_width(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32
   a.nwords = W * (5 + (size_t)(nbits < kSlicesCleared ? nbits : kSlicesCleared)) * nn;
   a.n = n;
   a.m = g->m;
-  a.handle = 0;
-  a.in_graph = 0;
-  void* clear_args[] = {&a.words, &a.nwords};
-  void* init_args[] = {&a.ctl, &a.row_ptr, &a.t_row_ptr, &a.visit, &a.fr0, &a.aq0, &a.segs, &a.n, &a.m};
-  void* pull_args[] = {&a.row_ptr, &a.t_row_ptr, &a.t_col, &a.ctl, &a.visit, &a.fr, &a.slices, &a.aq, &a.segs,
-                       &a.segcap, &a.ul_static, &a.ul_static_size, &a.ul, &a.hv_static, &a.hv_segoff,
-                       &a.hv_acc, &a.hv_tasks, &a.hv_count, &a.hv_segs, &a.pull_seg, &a.n};
-  void* scatter_args[] = {&a.row_ptr, &a.col, &a.ctl, &a.visit, &a.fr, &a.nxt, &a.slices, &a.aq, &a.segs,
-                          &a.segcap, &a.tq, &a.tbm, &a.n};
-  void* update_args[] = {&a.row_ptr, &a.t_row_ptr, &a.ctl, &a.visit, &a.fr, &a.nxt, &a.slices, &a.aq, &a.segs,
-                         &a.segcap, &a.tq, &a.tbm, &a.n};
-  void* emit_args[] = {&a.ctl, &a.visit, &a.slices, &a.n};
-  void* decide_args[] = {&a.ctl, &a.n, &a.sel_w, &a.handle, &a.in_graph};
-  void* next_args[] = {&a.ctl};
+  a.nbits = nbits;
+  a.force = g->force_variant;
+  a.batch = -1;
+  a.dist_base = d_dist;
+  a.lv_block = lv_block;
+  a.cc_sum = cc_sum;
+  const int nbatches = (nsrc + 64 * W - 1) / (64 * W);
+  void* args[] = {&a};
   const int sms = g->geo.sms;
   SsFamily fam;
-  fam.npre = 2;
-  fam.pre[0] = {(const void*)bs_clear, clear_args, dim3(sms * 8), dim3(kBlock), "bs_clear"};
-  fam.pre[1] = {(const void*)bs_init<W>, init_args, dim3(1), dim3(64 * W), "bs_init"};
-  fam.nbody = 4;
-  fam.body[0] = {(const void*)bs_pull<W>, pull_args, dim3(persistent_blocks((const void*)bs_pull<W>, kBlock, 0, g->blocks_per_sm)),
-                 dim3(kBlock), "bs_pull", kModePull};
-  fam.body[1] = {(const void*)bs_push_scatter<W>, scatter_args,
-                 dim3(persistent_blocks((const void*)bs_push_scatter<W>, kBlock, 0, g->blocks_per_sm)), dim3(kBlock),
-                 "bs_push_scatter", kModePush};
-  fam.body[2] = {(const void*)bs_push_update<W>, update_args,
-                 dim3(persistent_blocks((const void*)bs_push_update<W>, kBlock, 0, g->blocks_per_sm)), dim3(kBlock),
-                 "bs_push_update", kModePush};
-  fam.body[3] = {(const void*)bs_decide, decide_args, dim3(1), dim3(32), "bs_decide"};
-  fam.npost = 2;
-  fam.post[0] = {(const void*)bs_emit_dist<W>, emit_args, dim3(sms * 8), dim3(kBlock), "bs_emit_dist"};
-  fam.post[1] = {(const void*)bs_next, next_args, dim3(1), dim3(32), "bs_next"};
-  fam.ctl = a.ctl;
-  fam.ctl_bytes = sizeof(BsCtl);
-  fam.probe = probe_bs;
   if (g->l2_persist) {
     // the three rotating frontier slots: every pull level gathers from one
     fam.l2_base = a.fr;
     fam.l2_bytes = sizeof(u64) * 3 * W * nn;
   }
-  fam.handle = &a.handle;
-  fam.in_graph = &a.in_graph;
-  fam.done_flag = &a.ctl->done;
-  const int nbatches = (nsrc + 64 * W - 1) / (64 * W);
-  return ss_run(g, fam, nbatches, &g->bs_exec[wi]);
+  if (!g->trace) {
+    const void* fn = (const void*)bs_traverse<W>;
+    const int threads = W == 1 ? 640 : 512;
+    const int ctas = persistent_blocks(fn, threads, 0, g->blocks_per_sm);
+    for (a.batch = 0; a.batch < nbatches; a.batch++) {
+      DAWN_CHECK(launch_cooperative(fam, fn, ctas, threads, args, g->stream));
+      DAWN_CUDA(cudaLaunchKernel((const void*)bs_emit_dist<W>, dim3(sms * 8), dim3(kBlock), args, 0, g->stream));
+    }
+    return DAWN_OK;
+  }
+  const Launch step[] = {
+      {(const void*)bs_clear, args, dim3(sms * 8), dim3(kBlock), "bs_clear"},
+      {(const void*)bs_init<W>, args, dim3(1), dim3(64 * W), "bs_init"},
+      {(const void*)bs_pull<W>, args, dim3(persistent_blocks((const void*)bs_pull<W>, kBlock, 0, g->blocks_per_sm)),
+       dim3(kBlock), "bs_pull", kModePull},
+      {(const void*)bs_push_scatter<W>, args,
+       dim3(persistent_blocks((const void*)bs_push_scatter<W>, kBlock, 0, g->blocks_per_sm)), dim3(kBlock),
+       "bs_push_scatter", kModePush},
+      {(const void*)bs_push_update<W>, args,
+       dim3(persistent_blocks((const void*)bs_push_update<W>, kBlock, 0, g->blocks_per_sm)), dim3(kBlock),
+       "bs_push_update", kModePush},
+      {(const void*)bs_decide, args, dim3(1), dim3(32), "bs_decide"},
+      {(const void*)bs_emit_dist<W>, args, dim3(sms * 8), dim3(kBlock), "bs_emit_dist"},
+      {(const void*)bs_next, args, dim3(1), dim3(32), "bs_next"}};
+  fam.npre = 2;
+  fam.nbody = 4;
+  fam.npost = 2;
+  for (int i = 0; i < 2; i++) fam.pre[i] = step[i];
+  for (int i = 0; i < 4; i++) fam.body[i] = step[2 + i];
+  for (int i = 0; i < 2; i++) fam.post[i] = step[6 + i];
+  fam.ctl = a.ctl;
+  fam.ctl_bytes = sizeof(BsCtl);
+  fam.probe = probe_bs;
+  return ss_run_traced(g, fam, nbatches);
 }
 
 }  // namespace
@@ -1515,6 +1858,10 @@ dawn_status bfs_bitset_stats(dawn_graph* g, dawn_stats* st, int32_t nsrc) {
   BsCtl h;
   DAWN_CUDA(cudaMemcpyAsync(&h, g->bs_ctl.p, sizeof(BsCtl), cudaMemcpyDeviceToHost, g->stream));
   DAWN_CUDA(cudaStreamSynchronize(g->stream));
+  if (h.err) {
+    set_error("batched traversal: a device wait ran out");
+    return h.err;
+  }
   st->edges_traversed = (int64_t)h.total_reached;
   st->levels = h.total_levels;
   st->push_levels = h.total_push;

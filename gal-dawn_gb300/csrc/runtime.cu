@@ -271,7 +271,7 @@ constexpr int kPollLevels = 4;  // host-loop form: levels launched between polls
 // Traced form: level by level from the host, CUDA events around each kernel
 // that does work at that level, one trace record per kernel.
 dawn_status ss_run_traced(dawn_graph* g, SsFamily& fam, int32_t nruns) {
-  *fam.in_graph = 0;
+  if (fam.in_graph) *fam.in_graph = 0;
   cudaAccessPolicyWindow win;
   const bool has_win = family_window(fam, &win);
   for (int i = 0; i < 10; i++)
@@ -336,6 +336,27 @@ dawn_status ss_run_traced(dawn_graph* g, SsFamily& fam, int32_t nruns) {
     }
     DAWN_CHECK(timed_stage(fam.post, fam.npost, run, -1));
   }
+  return DAWN_OK;
+}
+
+dawn_status launch_cooperative(const SsFamily& fam, const void* fn, int ctas, int threads, void** args,
+                               cudaStream_t s) {
+  cudaAccessPolicyWindow win;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (family_window(fam, &win)) {
+    attr[1].id = cudaLaunchAttributeAccessPolicyWindow;
+    attr[1].val.accessPolicyWindow = win;
+    cfg.numAttrs = 2;
+  }
+  DAWN_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
   return DAWN_OK;
 }
 

@@ -326,7 +326,7 @@ dawn_status dawn_graph_set_selector(dawn_graph* g, const float* weights,
 /* Per-level trace.  No counterpart in the reference, which only times whole
  * runs with host std::chrono (src/algorithm/gpu/bfs.cu:70,93-95).  While
  * tracing is enabled on a handle, traversals run level by level from the
- * host instead of as one CUDA graph per source batch: before each level the
+ * host instead of as one launch or graph per source batch: before each level the
  * host reads the frontier statistics, launches only the kernels that level
  * uses, brackets each with CUDA events on the handle's stream, and appends
  * one record per kernel.  Results are identical; only speed differs.  The
