@@ -198,14 +198,17 @@ struct dawn_graph {
   dawn::DevBuf ss_ctl;      // SsCtl
   dawn::DevBuf ss_sources;  // int32 source list of the current call
   dawn::DevBuf ss_scratch;  // n x u64 (GOVM source-row resolution)
-  dawn::DevBuf bc_levels;   // betweenness: n x 64 int32 levels of a batch
-  dawn::DevBuf bc_terms;    // n x 64 float (1 / amount + dependency)
-  dawn::DevBuf bc_range;    // 2 x n int32 lowest / highest level per vertex
+  dawn::DevBuf bc_levels;   // betweenness: level blocks of two batches (bfs_bitset_levels)
+  dawn::DevBuf bc_terms;    // per 64 sources of a batch, n x 64 float (1 / amount + dependency)
+  dawn::DevBuf bc_range;    // likewise, 2 x n int32 lowest / highest level per vertex
+  dawn::DevBuf bc_acc;      // likewise, n double: the betweenness from these sources
   dawn::DevBuf bc_out;      // n double (host-pointer calls)
   dawn::DevBuf bc_heavy;    // rows cut into segments: out-rows (ids, segment prefix), in-rows (same)
-  dawn::DevBuf bc_part;     // per-segment partial sums (float) / per-heavy-row counts (int32), 64 each
+  dawn::DevBuf bc_part;     // per 64 sources of a batch: per-segment partial sums (float), per-heavy-row
+                            // counts (int32), 64 each, and segments finished per heavy row
   int32_t bc_hout = -1, bc_segs_out = 0, bc_hin = 0, bc_segs_in = 0;  // -1: lists not built
-  int32_t* bc_h_level = nullptr;  // pinned: the end level of the two batches in flight
+  int32_t bc_blocks = 0;    // 64-source blocks that bc_part is laid out for
+  int32_t* bc_h_level = nullptr;  // pinned: the ends (kLevelsEnd words) of the two batches in flight
   dawn::DevBuf mw_block;    // batched weighted traversal: n x 64 int32 distances
   dawn::DevBuf mw_masks;    // 3 x n uint64 improved-source masks
   dawn::DevBuf mw_ctl;
@@ -338,12 +341,21 @@ dawn_status bfs_bitset(dawn_graph* g, const int32_t* sources, int32_t nsrc,
                        int32_t* d_dist, unsigned long long* cc_sum = nullptr,
                        unsigned long long* cc_cnt = nullptr);
 dawn_status bfs_bitset_stats(dawn_graph* g, dawn_stats* st, int32_t nsrc);
-// One batch of at most 64 sources: levels as n x 64 int32 rows (vertex-major,
-// -1 unreached), per vertex the lowest and highest level (2 x n int32).
-// Enqueued only: the level the batch ended on (the deepest level + 1) is
-// copied to *h_level (pinned host memory) behind the traversal.
-dawn_status bfs_bitset_levels(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32_t* d_levels,
-                              int32_t* d_range, int32_t* h_level);
+// The words of a traversal of 64 w sources.
+dawn_status bitset_reserve(dawn_graph* g, int w);
+// One batch of at most 64 w sources (w = 1, 2 or 4).  d_levels holds a block of
+// n x 64 int32 per 64 sources.  A batch that ends on a level below kDeepLevel
+// leaves, for every level before that, n 64-bit words in each (the sources that
+// reach the vertex at that level), level after level; a deeper one n x 64 level
+// rows (vertex-major, -1 unreached), and in d_range (2 n int32 per 64 sources)
+// the lowest and highest level of each vertex.
+// Enqueued only: the level the batch ended on (the deepest level + 1), its error
+// status and the deepest level of each 64 sources are copied to h_end (pinned
+// host memory) behind the traversal.
+constexpr int kDeepLevel = 32;  // batched traversal: levels from here on are written out directly
+constexpr int kLevelsEnd = 6;
+dawn_status bfs_bitset_levels(dawn_graph* g, int w, const int32_t* sources, int32_t nsrc, int32_t* d_levels,
+                              int32_t* d_range, int32_t* h_end);
 int bitset_width(const dawn_graph* g, int32_t nsrc);
 // govm.cu
 dawn_status sssp_single(dawn_graph* g, const int32_t* sources, int32_t nsrc,

@@ -50,7 +50,10 @@ struct BsCtl {
   int32_t tq_size;              // push: vertices touched this level
   int32_t ul_size[2];           // unfinished-vertex lists (pull work lists)
   int32_t ul_cur;               // list the next pull reads: -1 = the graph's static list
-  int32_t level, mode, done, policy, batch, nsrc, n_push, n_pull;
+  int32_t level;                // with err and depth: read together by level-mode callers
+  int32_t err;                  // persistent launch: a wait ran out
+  int32_t depth[kMaxW];         // level mode: the deepest level of each 64 sources
+  int32_t mode, done, policy, batch, nsrc, n_push, n_pull;
   int32_t push_ratio;           // push while push_ratio * frontier edges < unfinished edges
   int32_t work;                 // dynamic work counter of the current level (light rows)
   int32_t hwork;                // dynamic work counter of the heavy-row segments
@@ -66,19 +69,17 @@ struct BsCtl {
   unsigned long long full[kMaxW];  // this batch's source bits, less those of sources without out-edges
   int32_t* dist_base;
   const int32_t* sources;
-  int32_t* lv_block;            // level mode: n x 64 levels, vertex-major (else NULL)
-  int32_t* lv_range;            // level mode: per vertex, lowest and highest level reached
+  int32_t* lv_block;            // level mode: per 64 sources, their level block (else NULL)
+  int32_t* lv_range;            // level mode: per 64 sources, lowest and highest level of every vertex
   unsigned long long* cc_sum;   // closeness mode: per source, sum of hop distances (else NULL)
   unsigned long long* cc_cnt;   // closeness mode: per source, vertices reached besides itself
   int32_t use_sel;              // decide with the handle's selector weights
   float sel_margin;             // log2 margin by which the selector must beat the heuristic
   int32_t force;                // 0 = decide per level; 1 + variant = always that variant
   int32_t prev_nf;              // frontier size entering the current level
-  int32_t pad3;
   long long m;                  // CSR entries (selector input)
   unsigned long long total_reached;
   int32_t total_levels, total_push, total_pull;
-  int32_t err;                  // persistent launch: a wait ran out
   // 1 = the level that wrote this slot's frontier words kept no active list
   // (a dense push update: the next level is then a pull, which needs none,
   // and the slot is cleared densely when it goes stale); aq_size holds the
@@ -137,7 +138,6 @@ constexpr int kSlicesCleared = 4;  // slices zeroed per batch; higher ones on fi
 // measured 4-10% slower: the pull is bound by its L1/TEX traffic, and the
 // lane walk adds none beyond the column loads and the gathers.
 constexpr int kPullLaneMax = 64;
-constexpr int kDeepLevel = 32;     // levels from here on are written out directly
 constexpr int kShallowBits = 5;    // level slices kept: the bits of levels below kDeepLevel
 static_assert(kDeepLevel == 1 << kShallowBits, "slices hold exactly the levels below kDeepLevel");
 // Heavy pull rows: a row of at least 2 x seg in-edges (seg = the handle's
@@ -302,8 +302,11 @@ __device__ __forceinline__ void record_level(const BsArgs& a, int32_t u, const B
   }
   if (a.cc_sum) return;
   if (a.lv_block) {
-    int32_t* row = a.lv_block + (size_t)u * 64;
-    for (u64 b = nw.w[0]; b; b &= b - 1) row[__ffsll((long long)b) - 1] = level;
+#pragma unroll
+    for (int i = 0; i < W; i++) {
+      int32_t* row = a.lv_block + ((size_t)i * n + u) * 64;
+      for (u64 b = nw.w[i]; b; b &= b - 1) row[__ffsll((long long)b) - 1] = level;
+    }
     return;
   }
   int32_t* dist = a.dist_base + (size_t)batch_of(a) * 64 * W * n;
@@ -1135,46 +1138,95 @@ __device__ __forceinline__ void emit_closeness(const Team& tm, const BsCtl* ctl,
   }
 }
 
-// Level mode of the final pass (one-word batches): each vertex's levels for
-// the batch's sources as one 64-word row (-1 where unreached), and the
-// lowest and highest level among them (INT_MAX / -1 when none).  Entries
-// written during the traversal (src set, as in emit_vertex) are kept.
+// Level mode of the final pass, shallow form (the batch ended below
+// kDeepLevel): per 64 sources, for every level one word per vertex, the sources
+// that reach it there, level after level (n words each) in their level block.
+// top receives the deepest level of each 64.
 template <int W>
-__device__ __forceinline__ void emit_levels(const Team& tm, const BsCtl* ctl, const u64* visit, const u64* slices,
-                                            int32_t n, int nb, int nbits, const int32_t* __restrict__ src) {
+__device__ __forceinline__ void emit_masks(const Team& tm, u64* out, const u64* visit, const u64* slices, int32_t n,
+                                           int nbits, int levels, int (&top)[W]) {
   const size_t stride = tm.threads();
   for (size_t u = tm.thread(); u < (size_t)n; u += stride) {
-    const u64 vis = visit[u * W];
-    u64 any = 0ull;
-    for (int k = 0; k < nbits; k++) any |= slices[((size_t)k * n + u) * W];
-    int lo = 0x7fffffff, hi = -1;
-    int4* row = reinterpret_cast<int4*>(ctl->lv_block + u * 64);
-    for (int s0 = 0; s0 < 64; s0 += 4) {
-      int32_t v[4];
-      int4 old = make_int4(0, 0, 0, 0);
-      if (src && (vis & ~any & (0xfull << s0))) old = row[s0 / 4];
-      const int32_t kept[4] = {old.x, old.y, old.z, old.w};
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int s = s0 + j;
-        v[j] = -1;
-        if (s < nb && ((vis >> s) & 1ull)) {
-          int32_t x = 0;
-          if (src && !((any >> s) & 1ull) && src[s] != (int32_t)u) {
-            x = kept[j];
-          } else {
-            for (int k = 0; k < nbits; k++) x |= (int32_t)((slices[((size_t)k * n + u) * W] >> s) & 1ull) << k;
-          }
-          v[j] = x;
-          lo = min(lo, x);
-          hi = max(hi, x);
-        }
+    for (int i = 0; i < W; i++) {
+      const u64 vis = visit[u * W + i];
+      u64 s[kShallowBits];
+#pragma unroll
+      for (int k = 0; k < kShallowBits; k++) s[k] = k < nbits ? slices[((size_t)k * n + u) * W + i] : 0ull;
+      for (int l = 0; l < levels; l++) {
+        u64 x = vis;
+#pragma unroll
+        for (int k = 0; k < kShallowBits; k++) x &= (l >> k) & 1 ? s[k] : ~s[k];
+        out[((size_t)i * 32 + l) * n + u] = x;
+        if (x) top[i] = max(top[i], l);
       }
-      row[s0 / 4] = make_int4(v[0], v[1], v[2], v[3]);
     }
-    ctl->lv_range[2 * u] = lo;
-    ctl->lv_range[2 * u + 1] = hi;
   }
+}
+static_assert(kDeepLevel * sizeof(u64) <= 64 * sizeof(int32_t), "a level block holds every shallow level's words");
+
+// Deep form: each vertex's levels for 64 sources as one 64-word row (-1 where
+// unreached), and the lowest and highest level among them (INT_MAX / -1 when
+// none).  Entries written during the traversal (src set, as in emit_vertex) are
+// kept.
+template <int W>
+__device__ __forceinline__ void emit_levels(const Team& tm, const BsCtl* ctl, const u64* visit, const u64* slices,
+                                            int32_t n, int nsrc, int nbits, const int32_t* __restrict__ src,
+                                            int (&top)[W]) {
+  const size_t stride = tm.threads();
+#pragma unroll
+  for (int i = 0; i < W; i++) {
+    const int nb = min(64, nsrc - 64 * i);
+    for (size_t u = tm.thread(); nb > 0 && u < (size_t)n; u += stride) {
+      const u64 vis = visit[u * W + i];
+      u64 any = 0ull;
+      for (int k = 0; k < nbits; k++) any |= slices[((size_t)k * n + u) * W + i];
+      int lo = 0x7fffffff, hi = -1;
+      int4* row = reinterpret_cast<int4*>(ctl->lv_block + ((size_t)i * n + u) * 64);
+      for (int s0 = 0; s0 < 64; s0 += 4) {
+        int32_t v[4];
+        int4 old = make_int4(0, 0, 0, 0);
+        if (vis & ~any & (0xfull << s0)) old = row[s0 / 4];
+        const int32_t kept[4] = {old.x, old.y, old.z, old.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const int s = s0 + j;
+          v[j] = -1;
+          if (s < nb && ((vis >> s) & 1ull)) {
+            int32_t x = 0;
+            if (!((any >> s) & 1ull) && src[64 * i + s] != (int32_t)u) {
+              x = kept[j];
+            } else {
+              for (int k = 0; k < nbits; k++) x |= (int32_t)((slices[((size_t)k * n + u) * W + i] >> s) & 1ull) << k;
+            }
+            v[j] = x;
+            lo = min(lo, x);
+            hi = max(hi, x);
+          }
+        }
+        row[s0 / 4] = make_int4(v[0], v[1], v[2], v[3]);
+      }
+      int32_t* const range = ctl->lv_range + 2 * ((size_t)i * n + u);
+      range[0] = lo;
+      range[1] = hi;
+      top[i] = max(top[i], hi);
+    }
+  }
+}
+
+// The deepest level of each 64 sources, one atomic per CTA.
+template <int W>
+__device__ __forceinline__ void record_depth(BsCtl* ctl, const int (&top)[W]) {
+  __shared__ int deepest[W];
+  if (threadIdx.x < W) deepest[threadIdx.x] = 0;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < W; i++) {
+    const int t = __reduce_max_sync(kFull, top[i]);
+    if (lane_id() == 0 && t > 0) atomicMax(&deepest[i], t);
+  }
+  __syncthreads();
+  if (threadIdx.x < W && deepest[threadIdx.x] > 0) atomicMax(&ctl->depth[threadIdx.x], deepest[threadIdx.x]);
 }
 
 template <int W>
@@ -1189,7 +1241,12 @@ __device__ __forceinline__ void emit_batch(const BsArgs& a, const Team& tm) {
   const int nbits = min(32 - __clz(max(ctl->level, 1)), kShallowBits);
   const int32_t* src = ctl->level >= kDeepLevel ? ctl->sources + (size_t)batch * per : nullptr;
   if (ctl->lv_block) {
-    if (W == 1) emit_levels<W>(tm, ctl, visit, slices, n, min(64, ctl->nsrc - batch * 64), nbits, src);
+    int top[W] = {};
+    if (!src)
+      emit_masks<W>(tm, reinterpret_cast<u64*>(ctl->lv_block), visit, slices, n, nbits, ctl->level, top);
+    else
+      emit_levels<W>(tm, ctl, visit, slices, n, nb, nbits, src, top);
+    record_depth<W>(a.ctl, top);
     return;
   }
   if (ctl->cc_sum) {
@@ -1694,6 +1751,15 @@ dawn_status build_static_list(dawn_graph* g) {
 }
 
 namespace {
+int slice_count(int32_t n) { return std::min(32 - __builtin_clz((unsigned)n), kShallowBits); }
+}  // namespace
+
+// words (per vertex w each): visit | fr[3] | nxt | level slices
+dawn_status bitset_reserve(dawn_graph* g, int w) {
+  return ensure(g->bs_words, sizeof(u64) * w * (5 + (size_t)slice_count(g->n)) * (size_t)g->n, g->stream);
+}
+
+namespace {
 
 template <int W>
 dawn_status run_width(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32_t* d_dist,
@@ -1709,8 +1775,8 @@ dawn_status run_width(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32
   // words (per vertex W each): visit | fr[3] | nxt | level slices[nbits]
   // lists: aq[3] | tq | ul[2] | touched bitmap ; segments[3]
   // Levels never exceed n, and levels from kDeepLevel on bypass the slices.
-  const int nbits = std::min(32 - __builtin_clz((unsigned)n), kShallowBits);
-  DAWN_CHECK(ensure(g->bs_words, sizeof(u64) * W * (5 + (size_t)nbits) * nn, g->stream));
+  const int nbits = slice_count(n);
+  DAWN_CHECK(bitset_reserve(g, W));
   const bool fresh = g->bs_queues.p == nullptr;
   DAWN_CHECK(ensure(g->bs_queues, sizeof(int32_t) * 6 * nn + sizeof(uint32_t) * (nn / 32 + 1), g->stream));
   // The touched bitmap starts clear; list-mode updates clear what they set.
@@ -1841,16 +1907,21 @@ dawn_status bfs_bitset(dawn_graph* g, const int32_t* sources, int32_t nsrc, int3
   return run_width<1>(g, sources, nsrc, d_dist, cc_sum, cc_cnt);
 }
 
-dawn_status bfs_bitset_levels(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32_t* d_levels,
-                              int32_t* d_range, int32_t* h_level) {
-  if (nsrc < 1 || nsrc > 64) {
-    set_error("level mode takes 1 to 64 sources per call");
+dawn_status bfs_bitset_levels(dawn_graph* g, int w, const int32_t* sources, int32_t nsrc, int32_t* d_levels,
+                              int32_t* d_range, int32_t* h_end) {
+  if (nsrc < 1 || nsrc > 64 * w) {
+    set_error("level mode takes one batch of sources per call");
     return DAWN_ERR_INVALID_ARG;
   }
-  DAWN_CHECK(run_width<1>(g, sources, nsrc, nullptr, nullptr, nullptr, d_levels, d_range));
-  // the level the batch ended on (an empty one), once the traversal is done
-  DAWN_CUDA(cudaMemcpyAsync(h_level, &g->bs_ctl.as<BsCtl>()->level, sizeof(int32_t), cudaMemcpyDeviceToHost,
-                            g->stream));
+  if (w == 4)
+    DAWN_CHECK(run_width<4>(g, sources, nsrc, nullptr, nullptr, nullptr, d_levels, d_range));
+  else if (w == 2)
+    DAWN_CHECK(run_width<2>(g, sources, nsrc, nullptr, nullptr, nullptr, d_levels, d_range));
+  else
+    DAWN_CHECK(run_width<1>(g, sources, nsrc, nullptr, nullptr, nullptr, d_levels, d_range));
+  static_assert(offsetof(BsCtl, depth) == offsetof(BsCtl, level) + 2 * sizeof(int32_t) && kMaxW == 4, "six words");
+  DAWN_CUDA(cudaMemcpyAsync(h_end, &g->bs_ctl.as<BsCtl>()->level, kLevelsEnd * sizeof(int32_t),
+                            cudaMemcpyDeviceToHost, g->stream));
   return DAWN_OK;
 }
 
