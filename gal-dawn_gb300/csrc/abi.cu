@@ -133,7 +133,8 @@ void destroy(dawn_graph* g) {
   dawn::pool_free(g->row_ptr, g->stream);
   dawn::pool_free(g->col, g->stream);
   if (g->val) dawn::pool_free(g->val, g->stream);
-  DevBuf* bufs[] = {&g->ss_queues, &g->ss_segs, &g->bs_segs, &g->ss_bitmaps, &g->ss_ctl, &g->ss_sources, &g->ss_scratch,
+  DevBuf* bufs[] = {&g->ss_queues, &g->ss_segs, &g->bs_segs, &g->ss_bitmaps, &g->ss_ctl, &g->bfs_sync, &g->bfs_rec,
+                    &g->bfs_long, &g->ss_sources, &g->ss_scratch,
                     &g->bs_words, &g->bs_queues, &g->bs_ctl, &g->ul_static, &g->hv_static, &g->hv_segoff, &g->hv_acc, &g->hv_tasks, &g->cc_out,
                     &g->dist_stage, &g->pt_voff, &g->pt_ctl, &g->pt_scratch, &g->pt_small, &g->pt_tcol, &g->pt_toff, &g->pt_rows,
                     &g->sel_slot, &g->nf_ctl, &g->nf_queue, &g->nf_segbuf, &g->nf_masks, &g->wt_col, &g->wt_val, &g->mw_block, &g->mw_masks,
@@ -175,6 +176,11 @@ dawn_status bfs_device_impl(dawn_graph* g, const int32_t* sources, int32_t nsrc,
       DAWN_CUDA(cudaEventRecord(g->ev1, g->stream));
       dawn::SsCtl c;
       DAWN_CHECK(dawn::download_ctl(g, &c));
+      if (c.err) {
+        dawn::set_error("single-source traversal: a device wait ran out");
+        dawn::release(g->bfs_sync);  // its counts are off: the next call starts a new one
+        return c.err;
+      }
       st->edges_traversed = (int64_t)c.total_reached;
       st->levels = c.total_levels;
       st->push_levels = c.total_push;

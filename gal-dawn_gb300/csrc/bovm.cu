@@ -11,11 +11,12 @@
 //   pull: every still-unvisited vertex scans its in-edges and stops at the
 //         first neighbour in the frontier bitmap (one warp owns 32 vertices,
 //         so bitmap words are written without atomics);
-// and a one-thread decide kernel picks the next level's direction (Beamer's
-// alpha/beta rule) on the device.  Both kernels emit the next frontier as a
-// queue and as a bitmap, so either direction can follow.  Distances are
+// and the device picks the next level's direction (Beamer's alpha/beta rule).
+// Either direction can follow the other: both emit the next frontier as a queue,
+// and its bitmap is written by a level or set from the queue.  Distances are
 // written once, when a vertex is claimed.
 #include <cooperative_groups.h>
+#include <algorithm>
 #include <climits>
 #include <mutex>
 
@@ -46,11 +47,9 @@ __global__ void __launch_bounds__(kBlock) bfs_clear(SsCtl* __restrict__ ctl, uin
 // The first level of the current source (one thread): distance 0, the
 // source in the visited bitmap and the level-0 frontier, its row as the
 // level-1 work, the level counters.
-__device__ __forceinline__ void init_source(SsCtl* __restrict__ ctl, const int32_t* __restrict__ row_ptr,
-                                            int32_t* __restrict__ q, Seg* __restrict__ segs,
-                                            uint32_t* __restrict__ vbm, int32_t n, long long m) {
-  const int32_t s = ctl->sources[ctl->src_idx];
-  int32_t* dist = ctl->dist_base + (size_t)ctl->src_idx * n;
+// lq: the list of long rows in place of the segments (the persistent launch).
+__device__ __forceinline__ void seed(SsCtl* ctl, int32_t s, int32_t* dist, const int32_t* __restrict__ row_ptr,
+                                     int32_t* q, Seg* segs, int32_t* lq, uint32_t* vbm, int32_t n, long long m) {
   const int32_t deg = row_ptr[s + 1] - row_ptr[s];
   ctl->source = s;
   dist[s] = 0;
@@ -58,7 +57,11 @@ __device__ __forceinline__ void init_source(SsCtl* __restrict__ ctl, const int32
   // level-0 frontier bitmap (the first of the three rotating ones, right
   // after the visited words): read when the first level is a pull
   vbm[(n + 31) / 32 + (s >> 5)] |= 1u << (s & 31);
-  if (deg >= kLongRow) {
+  if (deg >= kLongRow && lq) {
+    lq[0] = s;
+    ctl->qsize[0] = 0;
+    ctl->lpack[0] = 1ull << 32;
+  } else if (deg >= kLongRow) {
     const int nseg = (deg + kSeg - 1) / kSeg;
     for (int j = 0; j < nseg; j++) segs[j] = Seg{s, row_ptr[s] + j * kSeg};
     ctl->qsize[0] = 0;
@@ -81,6 +84,25 @@ __device__ __forceinline__ void init_source(SsCtl* __restrict__ ctl, const int32
   ctl->n_push = 0;
   ctl->n_pull = 0;
 }
+__device__ __forceinline__ void init_source(SsCtl* __restrict__ ctl, const int32_t* __restrict__ row_ptr,
+                                            int32_t* __restrict__ q, Seg* __restrict__ segs,
+                                            uint32_t* __restrict__ vbm, int32_t n, long long m) {
+  seed(ctl, ctl->sources[ctl->src_idx], ctl->dist_base + (size_t)ctl->src_idx * n, row_ptr, q, segs, nullptr, vbm, n, m);
+}
+
+// A distance row filled with -1 (16-byte stores over its aligned middle) and
+// the bitmaps cleared.
+__device__ __forceinline__ void fill_row(const Team& tm, int32_t* dist, uint32_t* bitmaps, int32_t n, size_t words) {
+  const size_t tid = tm.thread(), stride = tm.threads();
+  const size_t head = ((16 - (reinterpret_cast<uintptr_t>(dist) & 15)) & 15) / 4;
+  const size_t h = head < (size_t)n ? head : (size_t)n;
+  const size_t nvec = ((size_t)n - h) / 4;
+  if (tid < h) dist[tid] = -1;
+  int4* d4 = reinterpret_cast<int4*>(dist + h);
+  for (size_t i = tid; i < nvec; i += stride) d4[i] = make_int4(-1, -1, -1, -1);
+  for (size_t i = h + 4 * nvec + tid; i < (size_t)n; i += stride) dist[i] = -1;
+  for (size_t i = tid; i < words; i += stride) bitmaps[i] = 0;
+}
 
 __global__ void bfs_init(SsCtl* __restrict__ ctl, const int32_t* __restrict__ row_ptr,
                          int32_t* __restrict__ q, Seg* __restrict__ segs, uint32_t* __restrict__ vbm, int32_t n,
@@ -89,25 +111,15 @@ __global__ void bfs_init(SsCtl* __restrict__ ctl, const int32_t* __restrict__ ro
   init_source(ctl, row_ptr, q, segs, vbm, n, m);
 }
 
-// bfs_clear and bfs_init in one launch: the distance row filled with -1
-// (16-byte stores over its aligned middle) and the bitmaps cleared, then
-// the last CTA to finish (arrival count in the control block, which it
+// bfs_clear and bfs_init in one launch: fill_row, then the last CTA to finish (arrival count in the control block, which it
 // resets) seeds the source.
 __global__ void __launch_bounds__(kBlock) bfs_start(SsCtl* __restrict__ ctl, const int32_t* __restrict__ row_ptr,
                                                     int32_t* __restrict__ q, Seg* __restrict__ segs,
                                                     uint32_t* __restrict__ bitmaps, int32_t n, int32_t nwords,
                                                     long long m) {
   __shared__ int s_last;
-  int32_t* dist = ctl->dist_base + (size_t)ctl->src_idx * n;
-  const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
-  const size_t head = ((16 - (reinterpret_cast<uintptr_t>(dist) & 15)) & 15) / 4;
-  const size_t h = head < (size_t)n ? head : (size_t)n;
-  const size_t nvec = ((size_t)n - h) / 4;
-  if (tid < h) dist[tid] = -1;
-  int4* d4 = reinterpret_cast<int4*>(dist + h);
-  for (size_t i = tid; i < nvec; i += stride) d4[i] = make_int4(-1, -1, -1, -1);
-  for (size_t i = h + 4 * nvec + tid; i < (size_t)n; i += stride) dist[i] = -1;
-  for (size_t i = tid; i < (size_t)4 * nwords; i += stride) bitmaps[i] = 0;
+  fill_row(Team{(int)blockIdx.x, (int)gridDim.x}, ctl->dist_base + (size_t)ctl->src_idx * n, bitmaps, n,
+           4 * (size_t)nwords);
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
@@ -121,58 +133,136 @@ __global__ void __launch_bounds__(kBlock) bfs_start(SsCtl* __restrict__ ctl, con
   }
 }
 
-// Shared memory of one level kernel: the push's row dealing and the
-// queue staging both directions use.
+// Shared memory of one level kernel: the push's row dealing, the queue
+// staging both directions use, and the sums of the level's end.
+template <int kWarps>
 struct LevelSmem {
-  int excl[kBlock / 32][32];
-  int rs[kBlock / 32][32];
-  int v[kBlock / 32][32];
-  int32_t q[kBlock / 32][kWarpQueueBig];
+  int excl[kWarps][32];
+  int rs[kWarps][32];
+  int v[kWarps][32];
+  int32_t q[kWarps][kWarpQueueBig];
+  int32_t lq[kWarps][kWarpQueue];
+  uint32_t n[2][kWarps];
+  unsigned long long mf;
 };
+
+// Where a level's vertices go: short rows to the queue; long rows as segments,
+// reserved per warp step (segs), or by their ids to a list of their own, staged
+// like the queue, for the launch that cuts them only if a push follows (a pull
+// of RMAT-22 finds long rows in most warp steps: 100,000 atomics on one word).
+struct LongQueue {
+  int32_t *buf, *out;
+  unsigned long long* lpack;  // vertices << 32
+  int n = 0;
+  __device__ __forceinline__ void push(bool pred, int32_t v) {
+    const uint32_t m = __ballot_sync(kFull, pred);
+    if (m == 0) return;
+    const int c = __popc(m);
+    if (n + c > kWarpQueue) {
+      uint32_t base = 0;
+      if (lane_id() == 0) base = (uint32_t)(atomicAdd(lpack, (unsigned long long)n << 32) >> 32);
+      base = __shfl_sync(kFull, base, 0);
+      __syncwarp();
+      for (int i = lane_id(); i < n; i += 32) out[base + i] = buf[i];
+      __syncwarp();
+      n = 0;
+    }
+    if (pred) buf[n + __popc(m & lanemask_lt())] = v;
+    n += c;
+  }
+};
+constexpr int kStepWarps = kBlock / 32;
+
+// The end of a CTA's share of a level: what its warps still stage goes out
+// with one reservation per list, and the out-edges with one atomic.
+template <int kWarps>
+__device__ __forceinline__ void end_level(LevelSmem<kWarps>& sm, WarpQueueBig& wq, LongQueue* lq,
+                                          unsigned long long my_mf, unsigned long long* mf) {
+  const int lane = lane_id(), wib = threadIdx.x >> 5;
+  if (threadIdx.x == 0) sm.mf = 0;
+  if (lane == 0) {
+    sm.n[0][wib] = (uint32_t)wq.n;
+    sm.n[1][wib] = lq ? (uint32_t)lq->n : 0u;
+  }
+  __syncthreads();
+  my_mf = warp_sum(my_mf);
+  if (lane == 0 && my_mf) atomicAdd(&sm.mf, my_mf);
+  if (wib == 0) {
+#pragma unroll
+    for (int l = 0; l < 2; l++) {
+      const int x = lane < kWarps ? (int)sm.n[l][lane] : 0;
+      const int incl = warp_incl_scan(x);
+      const int tot = __shfl_sync(kFull, incl, 31);
+      int base = 0;
+      if (tot && lane == 0)
+        base = l ? (int)(atomicAdd(lq->lpack, (unsigned long long)tot << 32) >> 32) : atomicAdd(wq.count, tot);
+      base = __shfl_sync(kFull, base, 0);
+      if (lane < kWarps) sm.n[l][lane] = (uint32_t)(base + incl - x);
+    }
+  }
+  __syncthreads();
+  for (int i = lane; i < wq.n; i += 32) wq.out[sm.n[0][wib] + i] = wq.buf[i];
+  if (lq)
+    for (int i = lane; i < lq->n; i += 32) lq->out[sm.n[1][wib] + i] = lq->buf[i];
+  if (threadIdx.x == 0 && sm.mf) atomicAdd(mf, sm.mf);
+}
 
 // Top-down level: the frontier's rows are dealt to warps; unvisited
 // targets are claimed in the visited bitmap and queued for the next level.
-__device__ __forceinline__ void push_level(const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ col,
-                                           SsCtl* __restrict__ ctl, int32_t* __restrict__ q,
-                                           Seg* __restrict__ segs, size_t segcap, uint32_t* __restrict__ vbm,
-                                           uint32_t* __restrict__ fbm, int32_t n, int32_t nwords, LevelSmem& sm) {
-  const int L = ctl->level;
+// kBits: the next level's frontier goes into its bitmap too (a pull may
+// follow), the bitmap after that is cleared, and long rows go out as segments,
+// not to lq.
+template <bool kBits, int kWarps>
+__device__ __forceinline__ void push_level(const Team& tm, const int32_t* __restrict__ row_ptr,
+                                           const int32_t* __restrict__ col, SsCtl* ctl, int32_t* dist, int L, int qn,
+                                           int ln, int32_t* q, Seg* segs, size_t segcap, int32_t* lq, size_t lcap,
+                                           uint32_t* vbm, uint32_t* fbm, int32_t n, int32_t nwords,
+                                           LevelSmem<kWarps>& sm) {
   const int pin = (L - 1) & 1, pout = L & 1;
   const int32_t* qin = q + (size_t)pin * n;
   const Seg* sin = segs + (size_t)pin * segcap;
-  int32_t* qout = q + (size_t)pout * n;
   Seg* sout = segs + (size_t)pout * segcap;
   uint32_t* fout = rot(fbm, L, nwords);
-  uint32_t* fclr = rot(fbm, L + 1, nwords);
-  int32_t* dist = ctl->dist_base + (size_t)ctl->src_idx * n;
-  int32_t* qcount = &ctl->qsize[pout];
   unsigned long long* lpack = &ctl->lpack[pout];
-  const int qn = ctl->qsize[pin], ln = seg_count(ctl->lpack[pin]);
-  const int lane = lane_id(), wib = threadIdx.x >> 5;
-
-  const size_t gstride = (size_t)gridDim.x * blockDim.x;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)nwords; i += gstride) fclr[i] = 0;
-
+  const int wib = threadIdx.x >> 5;
+  if (kBits) {
+    uint32_t* fclr = rot(fbm, L + 1, nwords);
+    for (size_t i = tm.thread(); i < (size_t)nwords; i += tm.threads()) fclr[i] = 0;
+  }
   unsigned long long my_mf = 0;
-  WarpQueueBig wq(sm.q[wib], qout, qcount);
+  WarpQueueBig wq(sm.q[wib], q + (size_t)pout * n, &ctl->qsize[pout]);
+  LongQueue wl{sm.lq[wib], kBits ? nullptr : lq + (size_t)pout * lcap, lpack};
   auto op = [&](int32_t, int k, bool valid) {
     const int32_t u = valid ? __ldg(col + k) : -1;
     const bool found = valid && claim_bit(vbm, u);
     int deg = 0, rs = 0;
     if (found) {
-      rs = row_ptr[u];
-      deg = row_ptr[u + 1] - rs;
+      rs = __ldg(row_ptr + u);
+      deg = __ldg(row_ptr + u + 1) - rs;
       dist[u] = L;
-      atomicOr(fout + (u >> 5), 1u << (u & 31));
+      if (kBits) atomicOr(fout + (u >> 5), 1u << (u & 31));
       my_mf += (unsigned long long)deg;
     }
-    emit_routed(found, u, deg, rs, wq, sout, lpack);
+    if (kBits) {
+      emit_routed(found, u, deg, rs, wq, sout, lpack);
+    } else {
+      wq.push(found && deg < kLongRow, u);
+      wl.push(found && deg >= kLongRow, u);
+    }
   };
-  seg_expand(row_ptr, sin, ln, op);
-  warp_expand(row_ptr, qin, qn, sm.excl[wib], sm.rs[wib], sm.v[wib], op);
-  wq.flush();
-  my_mf = warp_sum(my_mf);
-  if (lane == 0 && my_mf) atomicAdd(&ctl->mf[pout], my_mf);
+  if (ln * (kSeg / 32) <= tm.warps()) {
+    // few segments: 32 entries a warp, one chain of claims each instead of four
+    for (int i = tm.warp(); i < ln * (kSeg / 32); i += tm.warps()) {
+      const int32_t v = __ldcg(&sin[i / (kSeg / 32)].v);
+      const int k0 = __ldcg(&sin[i / (kSeg / 32)].k0);
+      const int k = k0 + (i % (kSeg / 32)) * 32 + lane_id();
+      op(v, k, k < min(k0 + kSeg, __ldg(row_ptr + v + 1)));
+    }
+  } else {
+    seg_expand<true>(tm.warp(), tm.warps(), row_ptr, sin, ln, op);
+  }
+  warp_expand<true>(tm.warp(), tm.warps(), row_ptr, qin, qn, sm.excl[wib], sm.rs[wib], sm.v[wib], op);
+  end_level(sm, wq, kBits ? nullptr : &wl, my_mf, &ctl->mf[pout]);
 }
 
 __global__ void __launch_bounds__(kBlock) bfs_push(const int32_t* __restrict__ row_ptr,
@@ -180,9 +270,11 @@ __global__ void __launch_bounds__(kBlock) bfs_push(const int32_t* __restrict__ r
                                                    int32_t* __restrict__ q, Seg* __restrict__ segs, size_t segcap,
                                                    uint32_t* __restrict__ vbm, uint32_t* __restrict__ fbm,
                                                    int32_t n, int32_t nwords) {
-  __shared__ LevelSmem sm;
+  __shared__ LevelSmem<kStepWarps> sm;
   if (ctl->done || ctl->mode != kModePush) return;
-  push_level(row_ptr, col, ctl, q, segs, segcap, vbm, fbm, n, nwords, sm);
+  const int L = ctl->level, pin = (L - 1) & 1;
+  push_level<true>(Team{(int)blockIdx.x, (int)gridDim.x}, row_ptr, col, ctl, ctl->dist_base + (size_t)ctl->src_idx * n,
+                   L, ctl->qsize[pin], seg_count(ctl->lpack[pin]), q, segs, segcap, nullptr, 0, vbm, fbm, n, nwords, sm);
 }
 
 // Small frontiers: a single cluster of kSmallCtas CTAs runs push levels one
@@ -210,8 +302,13 @@ __global__ void __launch_bounds__(kBlock) bfs_push(const int32_t* __restrict__ r
 // The first level reads the global queue and segments the kernels before
 // wrote; its input counters are zeroed (behind one extra barrier) before a
 // later level of that parity can spill into them.
-__device__ __forceinline__ void decide_level(SsCtl* __restrict__ ctl, int32_t n, const float* __restrict__ sel_w,
-                                             cudaGraphConditionalHandle loop, int in_graph);
+struct Decision {
+  int done, mode, level;  // of the next level
+  int nf, qn;             // its frontier: vertices, of them with short rows
+};
+template <bool kStaySmall = false>
+__device__ __forceinline__ Decision decide_level(SsCtl* __restrict__ ctl, int32_t n, const float* __restrict__ sel_w,
+                                                 cudaGraphConditionalHandle loop, int in_graph);
 
 __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallBlock)
     bfs_small(const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ col, SsCtl* ctl, int32_t* q,
@@ -413,46 +510,108 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallBlock
   }
 }
 
+// A frontier word written earlier in the same launch: not through the
+// read-only path.
+__device__ __forceinline__ bool frontier_bit(const uint32_t* bm, int32_t u) {
+  uint32_t w;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(w) : "l"(bm + (u >> 5)));
+  return (w >> (u & 31)) & 1u;
+}
+
 // Bottom-up level: a warp owns 32 vertices (one bitmap word); each
 // unvisited one scans its in-edges until a frontier bit.
-__device__ __forceinline__ void pull_level(const int32_t* __restrict__ row_ptr,
-                                           const int32_t* __restrict__ t_row_ptr,
-                                           const int32_t* __restrict__ t_col, SsCtl* __restrict__ ctl,
-                                           int32_t* __restrict__ q, Seg* __restrict__ segs, size_t segcap,
-                                           uint32_t* __restrict__ vbm, uint32_t* __restrict__ fbm, int32_t n,
-                                           int32_t nwords, LevelSmem& sm) {
-  const int L = ctl->level;
+// The bounds of the next 32 rows load while these are scanned.  A lane tests
+// its row's first two columns, where most rows end once the frontier is large,
+// then reads eight (one sector) at a time.  The last few lanes' rows are swept
+// by the whole warp, so that one long row without a hit does not hold it.
+constexpr int kSweepLanes = 4;
+template <bool kSegs, int kWarps>
+__device__ __forceinline__ void pull_level(const Team& tm, const int32_t* __restrict__ row_ptr,
+                                           const int32_t* __restrict__ t_row_ptr, const int32_t* __restrict__ t_col,
+                                           SsCtl* ctl, int32_t* dist, int L, int32_t* q, Seg* segs, size_t segcap,
+                                           int32_t* lq, size_t lcap, uint32_t* vbm, uint32_t* fbm, int32_t n, int32_t nwords,
+                                           LevelSmem<kWarps>& sm) {
   const int pout = L & 1;
-  int32_t* qout = q + (size_t)pout * n;
   Seg* sout = segs + (size_t)pout * segcap;
   unsigned long long* lpack = &ctl->lpack[pout];
   const uint32_t* fin = rot(fbm, L - 1, nwords);
   uint32_t* fout = rot(fbm, L, nwords);
   uint32_t* fclr = rot(fbm, L + 1, nwords);
-  int32_t* dist = ctl->dist_base + (size_t)ctl->src_idx * n;
-  int32_t* qcount = &ctl->qsize[pout];
   const int lane = lane_id();
+  const bool wide = (reinterpret_cast<uintptr_t>(t_col) & 31) == 0;
 
-  const size_t gstride = (size_t)gridDim.x * blockDim.x;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)nwords; i += gstride) fclr[i] = 0;
+  for (size_t i = tm.thread(); i < (size_t)nwords; i += tm.threads()) fclr[i] = 0;
 
   unsigned long long my_mf = 0;
-  WarpQueueBig wq(sm.q[threadIdx.x >> 5], qout, qcount);
-  for (int w = global_warp(); w < nwords; w += num_warps()) {
-    const uint32_t vis = vbm[w];
-    uint32_t unv = ~vis;
-    if (w == nwords - 1 && (n & 31)) unv &= (1u << (n & 31)) - 1u;
-    if (unv == 0) continue;
-    const int32_t u = w * 32 + lane;
-    bool found = false;
-    if ((unv >> lane) & 1u) {
-      const int e = t_row_ptr[u + 1];
-      for (int k = t_row_ptr[u]; k < e; k++) {
-        if (test_bit(fin, __ldg(t_col + k))) {
-          found = true;
-          break;
-        }
+  WarpQueueBig wq(sm.q[threadIdx.x >> 5], q + (size_t)pout * n, &ctl->qsize[pout]);
+  LongQueue wl{sm.lq[threadIdx.x >> 5], kSegs ? nullptr : lq + (size_t)pout * lcap, lpack};
+  const int stride = tm.warps();
+  uint32_t vis_n = ~0u;
+  int k_n = 0, e_n = 0;
+  auto prefetch = [&](int w) {
+    vis_n = ~0u;
+    k_n = e_n = 0;
+    if (w < nwords) {
+      vis_n = __ldcg(vbm + w);
+      const int32_t u = w * 32 + lane;
+      if (u < n) {
+        k_n = __ldg(t_row_ptr + u);
+        e_n = __ldg(t_row_ptr + u + 1);
       }
+    }
+  };
+  prefetch(tm.warp());
+  for (int w = tm.warp(); w < nwords; w += stride) {
+    const uint32_t vis = vis_n;
+    const int k0 = k_n, e = (vis >> lane) & 1u ? k_n : e_n;  // an empty row: nothing to do
+    prefetch(w + stride);
+    if (__all_sync(kFull, k0 == e)) continue;
+    const int32_t u = w * 32 + lane;
+    int k = k0;
+    bool found = false;
+    {
+      const int32_t c0 = k < e ? __ldg(t_col + k) : -1, c1 = k + 1 < e ? __ldg(t_col + k + 1) : -1;
+      const bool h0 = c0 >= 0 && frontier_bit(fin, c0), h1 = c1 >= 0 && frontier_bit(fin, c1);
+      found = h0 || h1;
+      k = found ? e : k + 2;
+    }
+    uint32_t left = __ballot_sync(kFull, k < e);
+    while (__popc(left) > kSweepLanes) {
+      if (k < e) {
+        const int b = k & ~7;
+        int32_t c[8];
+        if (wide) {
+          asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+              : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]), "=r"(c[4]), "=r"(c[5]), "=r"(c[6]), "=r"(c[7])
+              : "l"(t_col + b));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; i++) c[i] = b + i >= k && b + i < e ? __ldg(t_col + b + i) : 0;
+        }
+        bool hit[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) hit[i] = b + i >= k && b + i < e && frontier_bit(fin, c[i]);
+#pragma unroll
+        for (int i = 0; i < 8; i++) found |= hit[i];
+        k = found ? e : b + 8;
+      }
+      left = __ballot_sync(kFull, k < e);
+    }
+    while (left) {
+      const int l = __ffs(left) - 1;
+      left &= left - 1;
+      const int e1 = __shfl_sync(kFull, e, l);
+      bool any = false;
+      for (int k0 = __shfl_sync(kFull, k, l); k0 < e1 && !any; k0 += 128) {
+        int32_t c[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) c[i] = k0 + 32 * i + lane < e1 ? __ldg(t_col + k0 + 32 * i + lane) : -1;
+        bool hit[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) hit[i] = c[i] >= 0 && frontier_bit(fin, c[i]);
+        any = __any_sync(kFull, hit[0] || hit[1] || hit[2] || hit[3]);
+      }
+      if (lane == l) found = any;
     }
     const uint32_t fm = __ballot_sync(kFull, found);
     if (fm) {
@@ -462,28 +621,20 @@ __device__ __forceinline__ void pull_level(const int32_t* __restrict__ row_ptr,
       }
       int deg = 0, rs = 0;
       if (found) {
-        rs = row_ptr[u];
-        deg = row_ptr[u + 1] - rs;
+        rs = row_ptr == t_row_ptr ? k0 : __ldg(row_ptr + u);
+        deg = (row_ptr == t_row_ptr ? e : __ldg(row_ptr + u + 1)) - rs;
         dist[u] = L;
         my_mf += (unsigned long long)deg;
       }
-      emit_routed(found, u, deg, rs, wq, sout, lpack);
+      if (kSegs) {
+        emit_routed(found, u, deg, rs, wq, sout, lpack);
+      } else {
+        wq.push(found && deg < kLongRow, u);
+        wl.push(found && deg >= kLongRow, u);
+      }
     }
   }
-  wq.flush();
-  my_mf = warp_sum(my_mf);
-  if (lane == 0 && my_mf) atomicAdd(&ctl->mf[pout], my_mf);
-}
-
-__global__ void __launch_bounds__(kBlock) bfs_pull(const int32_t* __restrict__ row_ptr,
-                                                   const int32_t* __restrict__ t_row_ptr,
-                                                   const int32_t* __restrict__ t_col, SsCtl* __restrict__ ctl,
-                                                   int32_t* __restrict__ q, Seg* __restrict__ segs, size_t segcap,
-                                                   uint32_t* __restrict__ vbm, uint32_t* __restrict__ fbm,
-                                                   int32_t n, int32_t nwords) {
-  __shared__ LevelSmem sm;
-  if (ctl->done || ctl->mode != kModePull) return;
-  pull_level(row_ptr, t_row_ptr, t_col, ctl, q, segs, segcap, vbm, fbm, n, nwords, sm);
+  end_level(sm, wq, kSegs ? nullptr : &wl, my_mf, &ctl->mf[pout]);
 }
 
 // One warp (all 32 lanes).  Ends the loop when the frontier is empty,
@@ -493,27 +644,32 @@ __global__ void __launch_bounds__(kBlock) bfs_pull(const int32_t* __restrict__ r
 // is read through volatile loads: when this runs at the end of the level
 // kernel itself, counters other CTAs just raised may sit stale in this
 // SM's L1.
-__device__ __forceinline__ void decide_level(SsCtl* __restrict__ ctl, int32_t n, const float* __restrict__ sel_w,
-                                             cudaGraphConditionalHandle loop, int in_graph) {
+// kStaySmall: small levels follow one another without a new decision while
+// the frontier stays small, as inside bfs_small.
+template <bool kStaySmall>
+__device__ __forceinline__ Decision decide_level(SsCtl* __restrict__ ctl, int32_t n, const float* __restrict__ sel_w,
+                                                 cudaGraphConditionalHandle loop, int in_graph) {
   const int lane = lane_id();
   if (sel_w) sel_prefetch(sel_w);
   const volatile SsCtl* vc = ctl;
   // every lane reads the control block before lane 0 changes it
   const int done = vc->done;
   const int L = vc->level, pout = L & 1;
-  const int nf = vc->qsize[pout] + long_vertices(vc->lpack[pout]);
+  const int qn = vc->qsize[pout];
+  const unsigned long long lp = vc->lpack[pout];
+  const int nf = qn + long_vertices(lp);
   const unsigned long long mf = vc->mf[pout];
   const long long mu = vc->mu - (long long)mf;
   const int cur_mode = vc->mode, prev_nf = vc->prev_nf, policy = vc->policy, force = vc->force;
   const bool sel = vc->use_sel && sel_w;
   const long long m = vc->m;
   const int small = vc->small;
-  const unsigned long long nlong = long_vertices(vc->lpack[pout]);
+  const int nlong = long_vertices(lp);
   const float margin = vc->sel_margin;
   __syncwarp();
   if (done) {
     if (lane == 0 && in_graph) cudaGraphSetConditional(loop, 0);
-    return;
+    return {1, 0, L, 0, 0};
   }
   if (lane == 0) {
     ctl->reached += mf;
@@ -525,7 +681,7 @@ __device__ __forceinline__ void decide_level(SsCtl* __restrict__ ctl, int32_t n,
       ctl->done = 1;
       if (in_graph) cudaGraphSetConditional(loop, 0);
     }
-    return;
+    return {1, 0, L, 0, 0};
   }
   int mode = cur_mode == kModePull ? kModePull : kModePush;  // cluster levels are push levels
   if (policy == DAWN_VARIANT_DO) {
@@ -546,9 +702,9 @@ __device__ __forceinline__ void decide_level(SsCtl* __restrict__ ctl, int32_t n,
   }
   // small levels start from frontiers without long rows: a long row's
   // neighbourhood tends to hold more, which end the cluster levels at once
-  if (mode == kModePush && small && !force && policy == DAWN_VARIANT_DO && nf <= kSmallFrontier &&
-      (long long)mf <= kSmallEdges && nlong == 0)
-    mode = kModeSmall;
+  const bool fits = small && !force && policy == DAWN_VARIANT_DO && nf <= kSmallFrontier &&
+                    (long long)mf <= kSmallEdges && nlong == 0;
+  if (fits && (mode == kModePush || (kStaySmall && cur_mode == kModeSmall))) mode = kModeSmall;
   if (lane == 0) {
     ctl->qsize[pout ^ 1] = 0;
     ctl->lpack[pout ^ 1] = 0;
@@ -557,6 +713,7 @@ __device__ __forceinline__ void decide_level(SsCtl* __restrict__ ctl, int32_t n,
     ctl->mode = mode;
     ctl->level = L + 1;
   }
+  return {0, mode, L + 1, nf, qn};
 }
 
 __global__ void bfs_decide(SsCtl* __restrict__ ctl, int32_t n, const float* __restrict__ sel_w,
@@ -576,7 +733,7 @@ __global__ void __launch_bounds__(kBlock, 5) bfs_step(const int32_t* __restrict_
                                                    uint32_t* __restrict__ vbm, uint32_t* __restrict__ fbm,
                                                    int32_t n, int32_t nwords, const float* __restrict__ sel_w,
                                                    cudaGraphConditionalHandle loop, int in_graph) {
-  __shared__ LevelSmem sm;
+  __shared__ LevelSmem<kStepWarps> sm;
   __shared__ int s_last;
   if (ctl->done) {
     // a traversal that ended before its first level (an isolated source)
@@ -585,10 +742,14 @@ __global__ void __launch_bounds__(kBlock, 5) bfs_step(const int32_t* __restrict_
     return;
   }
   const int mode = ctl->mode;
+  const Team tm{(int)blockIdx.x, (int)gridDim.x};
+  int32_t* const dist = ctl->dist_base + (size_t)ctl->src_idx * n;
+  const int L = ctl->level, pin = (L - 1) & 1;
   if (mode == kModePush)
-    push_level(row_ptr, col, ctl, q, segs, segcap, vbm, fbm, n, nwords, sm);
+    push_level<true>(tm, row_ptr, col, ctl, dist, L, ctl->qsize[pin], seg_count(ctl->lpack[pin]), q, segs, segcap,
+                     nullptr, 0, vbm, fbm, n, nwords, sm);
   else if (mode == kModePull)
-    pull_level(row_ptr, t_row_ptr, t_col, ctl, q, segs, segcap, vbm, fbm, n, nwords, sm);
+    pull_level<true>(tm, row_ptr, t_row_ptr, t_col, ctl, dist, L, q, segs, segcap, nullptr, 0, vbm, fbm, n, nwords, sm);
   else
     return;
   __syncthreads();
@@ -602,6 +763,622 @@ __global__ void __launch_bounds__(kBlock, 5) bfs_step(const int32_t* __restrict_
     if (threadIdx.x == 0) ctl->arrive = 0;
     decide_level(ctl, n, sel_w, loop, in_graph);
   }
+}
+
+// --- the persistent launch ----------------------------------------------------------
+
+// One source in one cooperative launch: fill, levels, counters.  In a
+// conditional graph a level is two kernels of which one returns at once, about
+// 10 us before any work; here it ends with one arrival per CTA and a decision
+// in the last one, which names as many CTAs for the next step as it has work
+// for (about 5 us a step, 1.1 us a level in CTA 0).  A small frontier without long rows is CTA 0's, level after level, with
+// the lists in shared memory: a chain of two round trips to L2 (targets; their
+// claims together with their row bounds) and a barrier, against cluster
+// barriers and remote shared memory in bfs_small.  Push levels leave the
+// frontier bitmaps alone: a pull that follows one sets them from the queue.
+// Per call, level kernels -> this:
+//   RMAT-12 (edge factor 8), distances to the host   134 ->   91 us
+//   RMAT-20                                          141 ->   86
+//   RMAT-22                                          261 ->  200
+//   grid 300 x 300                                  1580 ->  818
+//   grid 1000 x 1049                                6511 -> 4297
+constexpr uint32_t kBfPollLimit = 1u << 27;  // polls of one wait (over 30 s)
+constexpr int kBfEntries = 4096;             // vertices and entries per CTA of a small graph
+// Frontiers that go to CTA 0 and that stay there.  One SM makes about one access
+// to L1 or L2 a clock: a row of four entries costs it a dozen (8 us for 1,000
+// rows), with a record and the bitmap in shared memory two.
+constexpr int kSoloStart = 192, kSoloKeep = 256, kSoloCap = 1024;  // the last: vertices that its lists hold
+constexpr uint32_t kSoloEdges = 2048;
+constexpr int kSoloRow = 8;                  // longest row that one lane walks there
+constexpr int kMeshStart = 2048, kMeshKeep = 2560, kMeshCap = 3072;
+constexpr int kRecMax = 32;                  // longest row with a record
+constexpr int32_t kMeshMax = 1600000;        // vertices whose bitmap fits beside the lists
+constexpr int32_t kMeshWide = 32768;
+
+enum : int32_t { kBfStart = 0, kBfWipe, kBfBits, kBfCut, kBfPush, kBfPull, kBfSolo };
+
+struct BfsSync {
+  struct __align__(128) {
+    unsigned long long word[4];
+  } step;  // BfsStep, tagged with the generation in the top 16 bits of each word
+  struct __align__(128) {
+    uint32_t n;
+  } arrive;
+};
+struct BfsStep {
+  int32_t ctas, phase, dirty;  // dirty: a pull has written frontier bitmaps
+  int32_t L, qn, ln;           // the level, its queued vertices and long rows (push: their segments)
+  uint32_t arrived;            // arrivals before the phase
+};
+
+struct BfsArgs {
+  const int32_t *row_ptr, *col, *t_row_ptr, *t_col;
+  SsCtl* ctl;
+  BfsSync* sync;
+  int32_t* dist;
+  int32_t* q;
+  Seg* segs;
+  int32_t* lq;             // long rows, by level parity
+  size_t segcap, lcap;
+  uint32_t *vbm, *fbm;
+  long long m;
+  const float* sel_w;
+  const int32_t* rec;  // n rows of rec_len neighbours, -1 behind the last (NULL: none)
+  int32_t rec_len;
+  int32_t n, nwords, source, first;  // first: of the call's sources
+  int32_t policy, use_sel, force, small;
+  float sel_margin;
+};
+
+struct SoloList {
+  int32_t u[kSoloCap], rs[kSoloCap], deg[kSoloCap];
+};
+struct MeshLists {
+  int32_t u[2][kMeshCap];
+  uint32_t visited[4];  // and the rest of the n bits
+};
+template <int kWarps>
+struct BfsSmem {
+  BfsStep st;
+  int32_t cnt[3];
+  uint32_t mf[3], deg[3];  // solo: out-edges and longest row of the list
+  union {
+    LevelSmem<kWarps> lv;
+    SoloList solo[2];
+    MeshLists mesh;
+  };
+};
+
+// The frontier's bits, from its lists.
+__device__ __forceinline__ void set_bits(const Team& tm, const BfsArgs& a, const BfsStep& st) {
+  const int pin = (st.L - 1) & 1;
+  uint32_t* const f = rot(a.fbm, st.L - 1, a.nwords);
+  const int32_t *const qin = a.q + (size_t)pin * a.n, *const lin = a.lq + (size_t)pin * a.lcap;
+  for (size_t i = tm.thread(); i < (size_t)st.qn + st.ln; i += tm.threads()) {
+    const int32_t v = __ldcg(i < (size_t)st.qn ? qin + i : lin + (i - st.qn));
+    atomicOr(f + (v >> 5), 1u << (v & 31));
+  }
+}
+
+// The segments of the frontier's long rows.
+__device__ __forceinline__ void cut_rows(const Team& tm, const BfsArgs& a, const BfsStep& st) {
+  const int pin = (st.L - 1) & 1, lane = lane_id();
+  const int32_t* const lin = a.lq + (size_t)pin * a.lcap;
+  for (int b = tm.warp() * 32; b < st.ln; b += tm.warps() * 32) {
+    const bool ok = b + lane < st.ln;
+    const int32_t v = ok ? __ldcg(lin + b + lane) : 0;
+    const int rs = ok ? __ldg(a.row_ptr + v) : 0;
+    const int nseg = ok ? (__ldg(a.row_ptr + v + 1) - rs + kSeg - 1) / kSeg : 0;
+    const int incl = warp_incl_scan(nseg);
+    unsigned long long base = 0;
+    if (lane == 31) base = atomicAdd(&a.ctl->lpack[pin], (unsigned long long)incl);
+    const uint32_t first = (uint32_t)__shfl_sync(kFull, base, 31) + incl - nseg;
+    write_segments(__ballot_sync(kFull, ok), v, rs, nseg, first, a.segs + (size_t)pin * a.segcap);
+  }
+}
+
+// A vertex of level L from CTA 0 into its list.
+__device__ __forceinline__ void queue_vertex(const BfsArgs& a, int L, bool is, int32_t v, int deg) {
+  SsCtl* const ctl = a.ctl;
+  const int p = L & 1;
+  const int at = warp_append(is && deg < kLongRow, &ctl->qsize[p]);
+  if (is && deg < kLongRow) a.q[(size_t)p * a.n + at] = v;
+  if (is && deg >= kLongRow)
+    a.lq[(size_t)p * a.lcap + (uint32_t)(atomicAdd(&ctl->lpack[p], 1ull << 32) >> 32)] = v;
+}
+
+// Small levels, by CTA 0 alone.  The last one is left in the queue, with its
+// counters, for the decision at the end of the phase.
+template <int kWarps>
+__device__ __forceinline__ void solo_levels(const BfsArgs& a, const BfsStep& st, BfsSmem<kWarps>& sm) {
+  constexpr int kThreads = 32 * kWarps;
+  SsCtl* const ctl = a.ctl;
+  const int lane = lane_id(), wib = threadIdx.x >> 5;
+  int L = st.L;
+  {
+    const int32_t* qin = a.q + (size_t)((L - 1) & 1) * a.n;
+    if (threadIdx.x < 3) sm.cnt[threadIdx.x] = sm.mf[threadIdx.x] = sm.deg[threadIdx.x] = 0;
+    __syncthreads();
+    uint32_t longest = 0;
+    for (int i = threadIdx.x; i < st.qn; i += kThreads) {
+      const int32_t u = __ldcg(qin + i);
+      const int rs = __ldg(a.row_ptr + u), deg = __ldg(a.row_ptr + u + 1) - rs;
+      sm.solo[0].rs[i] = rs;
+      sm.solo[0].deg[i] = deg;
+      longest = max(longest, (uint32_t)deg);
+    }
+    longest = __reduce_max_sync(kFull, longest);
+    if (lane == 0) atomicMax(&sm.deg[0], longest);
+    if (threadIdx.x == 0) {
+      sm.cnt[0] = st.qn;
+      for (int p = 0; p < 2; p++) {
+        ctl->qsize[p] = 0;
+        ctl->lpack[p] = 0;
+        ctl->mf[p] = 0;
+      }
+    }
+    __syncthreads();
+  }
+  unsigned long long sum_mf = 0;
+  int it = 0, last_nf = 0;
+  for (;; it++, L++) {
+    const int cnt = sm.cnt[it % 3], o = (it + 1) % 3;
+    const SoloList& in = sm.solo[it & 1];
+    SoloList& nx = sm.solo[(it & 1) ^ 1];
+    if (threadIdx.x < 1) sm.cnt[(it + 2) % 3] = sm.mf[(it + 2) % 3] = sm.deg[(it + 2) % 3] = 0;
+    uint32_t my_mf = 0, longest = 0;
+    // claims the targets of up to four entries per lane
+    auto claim = [&](const int (&k)[4], const bool (&ok)[4]) {
+      int32_t u[4];
+      int rs[4], re[4];
+      uint32_t old[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) u[i] = ok[i] ? __ldg(a.col + k[i]) : 0;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        rs[i] = re[i] = 0;
+        old[i] = ~0u;
+        if (ok[i]) {
+          old[i] = atomicOr(a.vbm + (u[i] >> 5), 1u << (u[i] & 31));
+          rs[i] = __ldg(a.row_ptr + u[i]);
+          re[i] = __ldg(a.row_ptr + u[i] + 1);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const bool found = !((old[i] >> (u[i] & 31)) & 1u);
+        const uint32_t m = __ballot_sync(kFull, found);
+        if (m == 0) continue;
+        int base = 0;
+        if (lane == 0) base = atomicAdd(&sm.cnt[o], __popc(m));
+        const int slot = __shfl_sync(kFull, base, 0) + __popc(m & lanemask_lt());
+        const int deg = re[i] - rs[i];
+        if (found) {
+          a.dist[u[i]] = L;
+          my_mf += (uint32_t)deg;
+          longest = max(longest, (uint32_t)deg);
+          if (slot < kSoloCap) {
+            nx.u[slot] = u[i];
+            nx.rs[slot] = rs[i];
+            nx.deg[slot] = deg;
+          }
+        }
+        const bool spill = found && slot >= kSoloCap;
+        if (__any_sync(kFull, spill))
+          queue_vertex(a, L, spill, u[i], deg);
+      }
+    };
+    if (sm.deg[it % 3] <= (uint32_t)kSoloRow) {  // a row per lane
+      int per = 32;
+      while (per > 1 && (per >> 1) * kWarps >= cnt) per >>= 1;
+      for (int b = wib * per; b < cnt; b += kWarps * per) {
+        const bool in_row = lane < per && b + lane < cnt;
+        const int rs = in_row ? in.rs[b + lane] : 0, deg = in_row ? in.deg[b + lane] : 0;
+#pragma unroll
+        for (int j = 0; j < kSoloRow; j += 4) {
+          if (!__any_sync(kFull, deg > j)) break;
+          const int k[4] = {rs + j, rs + j + 1, rs + j + 2, rs + j + 3};
+          const bool ok[4] = {deg > j, deg > j + 1, deg > j + 2, deg > j + 3};
+          claim(k, ok);
+        }
+      }
+    } else {
+      int per = 32;
+      while (per > 1 && (per >> 1) * kWarps >= cnt) per >>= 1;
+      for (int b = wib * per; b < cnt; b += kWarps * per) {
+        const bool in_row = lane < per && b + lane < cnt;
+        const int rs = in_row ? in.rs[b + lane] : 0, deg = in_row ? in.deg[b + lane] : 0;
+        const int incl = warp_incl_scan(deg), excl = incl - deg;
+        const int total = __shfl_sync(kFull, incl, 31);
+        for (int e0 = 0; e0 < total; e0 += 128) {
+          int k[4];
+          bool ok[4];
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const int e = e0 + 32 * j + lane;
+            int lo = 0;  // last lane whose offset is <= e
+#pragma unroll
+            for (int step = 16; step; step >>= 1)
+              if (__shfl_sync(kFull, excl, lo + step) <= e) lo += step;
+            k[j] = __shfl_sync(kFull, rs, lo) + (e - __shfl_sync(kFull, excl, lo));
+            ok[j] = e < total;
+          }
+          claim(k, ok);
+        }
+      }
+    }
+    my_mf = __reduce_add_sync(kFull, my_mf);
+    longest = __reduce_max_sync(kFull, longest);
+    if (lane == 0) {
+      if (my_mf) atomicAdd(&sm.mf[o], my_mf);
+      if (longest) atomicMax(&sm.deg[o], longest);
+    }
+    __syncthreads();
+    const int nf = sm.cnt[o];
+    if (nf == 0 || nf > kSoloKeep || sm.mf[o] > kSoloEdges || sm.deg[o] >= (uint32_t)kLongRow || L + 1 >= a.n) break;
+    sum_mf += sm.mf[o];
+    last_nf = nf;
+  }
+  const SoloList& out = sm.solo[(it & 1) ^ 1];
+  const int o = (it + 1) % 3, p = L & 1, kept = min(sm.cnt[o], kSoloCap);
+  for (int b = wib * 32; b < kept; b += kThreads) {
+    const int i = b + lane;
+    const bool ok = i < kept;
+    queue_vertex(a, L, ok, ok ? out.u[i] : 0, ok ? out.deg[i] : 0);
+  }
+  if (threadIdx.x == 0) {
+    ctl->mf[p] = sm.mf[o];
+    ctl->reached += sum_mf;
+    ctl->mu -= (long long)sum_mf;
+    ctl->n_push += it;
+    if (it) ctl->prev_nf = last_nf;
+    ctl->level = L;
+  }
+}
+
+// Likewise, its out-edges read and counted.
+__device__ __forceinline__ void mesh_queue(const BfsArgs& a, int L, bool is, int32_t v) {
+  uint32_t deg = is ? (uint32_t)(__ldg(a.row_ptr + v + 1) - __ldg(a.row_ptr + v)) : 0u;
+  queue_vertex(a, L, is, v, (int)deg);
+  deg = __reduce_add_sync(kFull, deg);
+  if (lane_id() == 0 && deg) atomicAdd(&a.ctl->mf[L & 1], (unsigned long long)deg);
+}
+
+// Small levels of a graph with records (rows of at most kRecMax entries), by CTA
+// 0 alone, with the visited bitmap in its shared memory: a level is one round
+// trip, for the rows' records, and a store per vertex that no one waits for.
+template <int kWarps>
+__device__ __forceinline__ void mesh_levels(const BfsArgs& a, const BfsStep& st, BfsSmem<kWarps>& sm) {
+  constexpr int kThreads = 32 * kWarps;
+  SsCtl* const ctl = a.ctl;
+  uint32_t* const vis = sm.mesh.visited;
+  const int lane = lane_id(), wib = threadIdx.x >> 5;
+  int L = st.L;
+  const int32_t* qin = a.q + (size_t)((L - 1) & 1) * a.n;
+  for (int i = threadIdx.x; i < a.nwords; i += kThreads) vis[i] = __ldcg(a.vbm + i);
+  for (int i = threadIdx.x; i < st.qn; i += kThreads) sm.mesh.u[0][i] = __ldcg(qin + i);
+  if (threadIdx.x == 0) {
+    sm.cnt[0] = st.qn;
+    sm.cnt[1] = sm.cnt[2] = 0;
+    for (int p = 0; p < 2; p++) {
+      ctl->qsize[p] = 0;
+      ctl->lpack[p] = 0;
+      ctl->mf[p] = 0;
+    }
+  }
+  __syncthreads();
+  uint32_t my_deg = 0;  // entries of the rows walked, but for the first level's
+  int it = 0, last_nf = 0;
+  for (;; it++, L++) {
+    const int cnt = sm.cnt[it % 3], o = (it + 1) % 3;
+    const int32_t* const in = sm.mesh.u[it & 1];
+    int32_t* const out = sm.mesh.u[(it & 1) ^ 1];
+    if (threadIdx.x == 0) sm.cnt[(it + 2) % 3] = 0;
+    int per = 32;
+    while (per > 1 && (per >> 1) * kWarps >= cnt) per >>= 1;
+    for (int b = wib * per; b < cnt; b += kWarps * per) {
+      const bool in_row = lane < per && b + lane < cnt;
+      const int32_t* rec = a.rec + (size_t)(in_row ? in[b + lane] : 0) * a.rec_len;
+      bool go = in_row;
+      for (int j = 0; __any_sync(kFull, go); j += 8) {
+        int32_t c[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) c[i] = -1;
+        if (go)
+          asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+              : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]), "=r"(c[4]), "=r"(c[5]), "=r"(c[6]), "=r"(c[7])
+              : "l"(rec + j));
+        go = c[7] >= 0 && j + 8 < a.rec_len;
+        unsigned is_new = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+          if (c[i] >= 0) {
+            my_deg += it > 0;
+            is_new |= (~vis[c[i] >> 5] >> (c[i] & 31) & 1u) << i;
+          }
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+          if ((is_new >> i) & 1u) {
+            const uint32_t bit = 1u << (c[i] & 31);
+            if (atomicOr(vis + (c[i] >> 5), bit) & bit) is_new &= ~(1u << i);
+          }
+        const int mine = __popc(is_new), incl = warp_incl_scan(mine);
+        const int tot = __shfl_sync(kFull, incl, 31);
+        if (tot == 0) continue;
+        int base = 0;
+        if (lane == 0) base = atomicAdd(&sm.cnt[o], tot);
+        base = __shfl_sync(kFull, base, 0);
+        int slot = base + incl - mine;
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+          if ((is_new >> i) & 1u) {
+            a.dist[c[i]] = L;
+            if (slot < kMeshCap) {
+              out[slot] = c[i];
+              is_new &= ~(1u << i);
+            }
+            slot++;
+          }
+        if (base + tot > kMeshCap) {
+#pragma unroll
+          for (int i = 0; i < 8; i++) mesh_queue(a, L, (is_new >> i) & 1u, c[i]);
+        }
+      }
+    }
+    __syncthreads();
+    const int nf = sm.cnt[o];
+    if (nf == 0 || nf > kMeshKeep || L + 1 >= a.n) break;
+    last_nf = nf;
+  }
+  for (int i = threadIdx.x; i < a.nwords; i += kThreads) a.vbm[i] = vis[i];
+  const int32_t* const out = sm.mesh.u[(it & 1) ^ 1];
+  const int kept = min(sm.cnt[(it + 1) % 3], kMeshCap);
+  for (int b = wib * 32; b < kept; b += kThreads) mesh_queue(a, L, b + lane < kept, b + lane < kept ? out[b + lane] : 0);
+  my_deg = __reduce_add_sync(kFull, my_deg);
+  if (lane == 0 && my_deg) {
+    atomicAdd(&ctl->reached, (unsigned long long)my_deg);
+    atomicAdd(reinterpret_cast<unsigned long long*>(&ctl->mu), -(unsigned long long)my_deg);
+  }
+  if (threadIdx.x == 0) {
+    ctl->n_push += it;
+    if (it) ctl->prev_nf = last_nf;
+    ctl->level = L;
+  }
+}
+
+// CTAs for `work` warp tasks.
+template <int kWarps>
+__device__ __forceinline__ int bf_ctas(int work) {
+  const int c = (work + kWarps - 1) / kWarps;
+  return c < 1 ? 1 : min(c, (int)gridDim.x);
+}
+
+// One warp of the last CTA to finish phase st: the next one.  Returns false
+// when the traversal is done.  Not inlined: its registers would be the
+// levels' spills.
+template <int kWarps>
+__device__ __noinline__ bool next_phase(const BfsArgs& a, BfsStep& step) {
+  BfsStep st = step;
+  SsCtl* const ctl = a.ctl;
+  int phase = kBfPush;
+  if (st.phase == kBfWipe) {
+    phase = kBfBits;
+  } else if (st.phase == kBfBits) {
+    phase = kBfPull;
+  } else if (st.phase == kBfCut) {
+    st.ln = seg_count(static_cast<const volatile SsCtl*>(ctl)->lpack[(st.L - 1) & 1]);
+  } else if (st.phase == kBfStart) {
+    int done = 0, mode = 0, qn = 0, ln = 0;
+    if (lane_id() == 0) {
+      SsCtl c = {};
+      c.policy = a.policy;
+      c.use_sel = a.use_sel;
+      c.sel_margin = a.sel_margin;
+      c.force = a.force;
+      c.small = a.small;
+      c.m = a.m;
+      c.source = a.source;
+      if (!a.first) {
+        const volatile SsCtl* vc = ctl;
+        c.total_reached = vc->total_reached;
+        c.total_levels = vc->total_levels;
+        c.total_push = vc->total_push;
+        c.total_pull = vc->total_pull;
+        c.err = vc->err;
+      }
+      *ctl = c;
+      seed(ctl, a.source, a.dist, a.row_ptr, a.q, a.segs, a.lq, a.vbm, a.n, a.m);
+      done = ctl->done;
+      mode = ctl->mode;
+      qn = ctl->qsize[0];
+      ln = long_vertices(ctl->lpack[0]);
+    }
+    st.L = 1;
+    st.qn = __shfl_sync(kFull, qn, 0);
+    st.ln = __shfl_sync(kFull, ln, 0);
+    mode = __shfl_sync(kFull, mode, 0);
+    if (__shfl_sync(kFull, done, 0)) return false;
+    phase = mode == kModePull ? kBfPull : st.ln ? kBfCut : kBfPush;
+  } else {
+    const Decision d = decide_level<true>(ctl, a.n, a.sel_w, 0, 0);
+    if (d.done) return false;
+    st.L = d.level;
+    st.qn = d.qn;
+    st.ln = d.nf - d.qn;
+    if (st.ln) phase = kBfCut;
+    if (d.mode == kModePull)
+      phase = st.phase == kBfPull ? kBfPull : (st.dirty ? kBfWipe : kBfBits);
+    else if (d.mode == kModeSmall && d.nf <= (a.rec ? kMeshStart : kSoloStart))
+      phase = kBfSolo;
+  }
+  if (phase == kBfPull) st.dirty = 1;
+  if (phase == kBfWipe) st.dirty = 0;
+  st.ctas = phase == kBfSolo ? 1
+            : phase == kBfPush ? bf_ctas<kWarps>(st.qn / 4 + st.ln * (kSeg / 32) + 1)
+            : phase == kBfBits ? bf_ctas<kWarps>((st.qn + st.ln) / 32 + 1)
+            : phase == kBfCut  ? bf_ctas<kWarps>(st.ln / 32 + 1)
+                               : (int)gridDim.x;
+  st.phase = phase;
+  step = st;
+  return true;
+}
+
+// kMesh: with records, 1,024 threads and one CTA per SM (the bitmap takes its
+// shared memory); else two CTAs of 640 threads at 48 registers.
+template <bool kMesh>
+__global__ void __launch_bounds__(kMesh ? 1024 : 640, kMesh ? 1 : 2) bfs_traverse(const __grid_constant__ BfsArgs a) {
+  constexpr int kWarps = kMesh ? 32 : 20;
+  extern __shared__ __align__(16) unsigned char smem[];
+  auto& sm = *reinterpret_cast<BfsSmem<kWarps>*>(smem);
+  const int lane = lane_id(), wib = threadIdx.x >> 5;
+  // no phase can open before every CTA has arrived, so all read the same
+  uint32_t gen = (uint32_t)(*static_cast<const volatile unsigned long long*>(&a.sync->step.word[0]) >> 48);
+  const BfsStep& st = sm.st;
+  if (threadIdx.x == 0) {
+    sm.st = BfsStep{};
+    sm.st.phase = kBfStart;
+    sm.st.ctas = (int)gridDim.x;
+    sm.st.arrived = (uint32_t)*static_cast<const volatile unsigned long long*>(&a.sync->step.word[3]);
+  }
+  __syncthreads();
+  for (;;) {
+    const Team tm{(int)blockIdx.x, st.ctas};
+    switch (st.phase) {
+      case kBfStart: fill_row(tm, a.dist, a.vbm, a.n, 4 * (size_t)a.nwords); break;
+      case kBfWipe:
+        for (size_t i = tm.thread(); i < (size_t)3 * a.nwords; i += tm.threads()) a.fbm[i] = 0;
+        break;
+      case kBfBits: set_bits(tm, a, st); break;
+      case kBfCut: cut_rows(tm, a, st); break;
+      case kBfPush:
+        push_level<false>(tm, a.row_ptr, a.col, a.ctl, a.dist, st.L, st.qn, st.ln, a.q, a.segs, a.segcap, a.lq, a.lcap,
+                          a.vbm, a.fbm, a.n, a.nwords, sm.lv);
+        break;
+      case kBfPull:
+        pull_level<false>(tm, a.row_ptr, a.t_row_ptr, a.t_col, a.ctl, a.dist, st.L, a.q, a.segs, a.segcap, a.lq, a.lcap,
+                          a.vbm, a.fbm, a.n, a.nwords, sm.lv);
+        break;
+      default:
+        if (kMesh)
+          mesh_levels(a, st, sm);
+        else
+          solo_levels(a, st, sm);
+    }
+    __syncthreads();
+    if (wib == 0) {
+      int last = 0;
+      if (lane == 0) {
+        __threadfence();
+        last = atomicAdd(&a.sync->arrive.n, 1u) + 1 == st.arrived + (uint32_t)st.ctas;
+      }
+      if (__shfl_sync(kFull, last, 0)) {
+        __threadfence();
+        BfsStep nx = st;
+        nx.arrived = st.arrived + (uint32_t)st.ctas;
+        const bool more = next_phase<kWarps>(a, nx);
+        if (!more && lane == 0) {
+          SsCtl* const c = a.ctl;
+          c->total_reached += c->reached;
+          c->total_levels += c->level;
+          c->total_push += c->n_push;
+          c->total_pull += c->n_pull;
+        }
+        __syncwarp();
+        __threadfence();
+        if (lane < 4) {
+          const uint32_t lo = lane == 0 ? (uint32_t)nx.qn : lane == 1 ? (uint32_t)nx.ln : lane == 2 ? (uint32_t)nx.L : nx.arrived;
+          const uint32_t hi = lane == 0 ? (more ? (uint32_t)nx.ctas : 0u) : lane == 1 ? (uint32_t)(nx.phase | nx.dirty << 8) : 0u;
+          *static_cast<volatile unsigned long long*>(&a.sync->step.word[lane]) =
+              (unsigned long long)((gen + 1) & 0xffffu) << 48 | (unsigned long long)hi << 32 | lo;
+        }
+      }
+      __syncwarp();
+      bool idle = false;
+      for (uint32_t polls = 0;; polls++) {
+        unsigned long long w;
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(&a.sync->step.word[lane & 3]) : "memory");
+        const uint32_t tag = (uint32_t)(w >> 48), tag0 = __shfl_sync(kFull, tag, 0);
+        if (__all_sync(kFull, tag == tag0) && tag != gen) {
+          gen = tag;
+          polls = 0;
+          const uint32_t hi = (uint32_t)(w >> 32) & 0xffffu, lo = (uint32_t)w;
+          const uint32_t ctas = __shfl_sync(kFull, hi, 0), ph = __shfl_sync(kFull, hi, 1);
+          const uint32_t qn = __shfl_sync(kFull, lo, 0), ln = __shfl_sync(kFull, lo, 1);
+          const uint32_t L = __shfl_sync(kFull, lo, 2), arrived = __shfl_sync(kFull, lo, 3);
+          if (ctas == 0 || blockIdx.x < ctas) {
+            if (lane == 0) sm.st = BfsStep{(int)ctas, (int)(ph & 0xff), (int)(ph >> 8), (int)L, (int)qn, (int)ln, arrived};
+            break;
+          }
+          idle = true;
+        }
+        if (polls == kBfPollLimit) {
+          if (lane == 0) {
+            a.ctl->err = DAWN_ERR_TIMEOUT;
+            sm.st.ctas = 0;
+          }
+          break;
+        }
+        if (idle) __nanosleep(64);
+      }
+    }
+    __syncthreads();
+    if (st.ctas == 0) return;
+  }
+}
+
+__global__ void __launch_bounds__(kBlock) max_degree(const int32_t* __restrict__ row_ptr, int32_t n,
+                                                     int32_t* __restrict__ out) {
+  int deg = 0;
+  for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+    deg = max(deg, row_ptr[v + 1] - row_ptr[v]);
+  deg = __reduce_max_sync(kFull, deg);
+  if (lane_id() == 0 && deg) atomicMax(out, deg);
+}
+
+__global__ void __launch_bounds__(kBlock) fill_records(const int32_t* __restrict__ row_ptr,
+                                                       const int32_t* __restrict__ col, int32_t n, int32_t len,
+                                                       int32_t* __restrict__ rec) {
+  const size_t words = (size_t)n * len, stride = (size_t)gridDim.x * blockDim.x;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < words; i += stride) {
+    const int32_t v = (int32_t)(i / len), k = row_ptr[v] + (int32_t)(i % len);
+    rec[i] = k < row_ptr[v + 1] ? col[k] : -1;
+  }
+}
+
+// The records of a graph of low degree, once per handle: a row in whole sectors,
+// so that a level's rows are one load away from its vertices.  Graphs of up to 12
+// entries a row, none above kRecMax: meshes, street networks, kNN graphs, whose
+// traversals take hundreds of small levels.  Beyond kMeshMax vertices, and with
+// rows of more than eight entries beyond kMeshWide, these keep the level kernels
+// and the cluster levels (kLevelKernels): kNN of 200,000 points takes 1.23 ms that
+// way and 1.54 on one SM, of 2,000 points 161 and 143 us.
+constexpr int32_t kLevelKernels = -2;
+dawn_status records(dawn_graph* g) {
+  if (g->rec_len != -1) return DAWN_OK;
+  int32_t len = 0;
+  if (g->m <= 12 * (int64_t)g->n && g->n > kSoloKeep) {
+    int32_t* d = nullptr;
+    DAWN_CHECK(pool_alloc((void**)&d, sizeof(int32_t), g->stream));
+    DAWN_CUDA(cudaMemsetAsync(d, 0, sizeof(int32_t), g->stream));
+    max_degree<<<g->geo.sms * 4, kBlock, 0, g->stream>>>(g->row_ptr, g->n, d);
+    DAWN_CUDA(cudaGetLastError());
+    int32_t deg = 0;
+    DAWN_CUDA(cudaMemcpyAsync(&deg, d, sizeof(int32_t), cudaMemcpyDeviceToHost, g->stream));
+    pool_free(d, g->stream);
+    DAWN_CUDA(cudaStreamSynchronize(g->stream));
+    len = std::max(8, (deg + 7) / 8 * 8);
+    if (deg > kRecMax) {
+      len = 0;
+    } else if (g->n > kMeshMax || (len > 8 && g->n > kMeshWide)) {
+      len = kLevelKernels;
+    } else {
+      DAWN_CHECK(ensure(g->bfs_rec, sizeof(int32_t) * (size_t)g->n * len, g->stream));
+      fill_records<<<g->geo.sms * 8, kBlock, 0, g->stream>>>(g->row_ptr, g->col, g->n, len, g->bfs_rec.as<int32_t>());
+      DAWN_CUDA(cudaGetLastError());
+    }
+  }
+  g->rec_len = len;
+  return DAWN_OK;
 }
 
 __global__ void ss_next(SsCtl* __restrict__ ctl) {
@@ -636,6 +1413,66 @@ dawn_status bfs_single(dawn_graph* g, const int32_t* sources, int32_t nsrc, int3
   DAWN_CHECK(ensure(g->ss_segs, sizeof(Seg) * 2 * segcap, g->stream));
   DAWN_CHECK(ensure(g->ss_bitmaps, sizeof(uint32_t) * 4 * (size_t)nwords, g->stream));
   DAWN_CHECK(ensure(g->ss_ctl, sizeof(SsCtl), g->stream));
+  const int32_t force = g->force_variant == 3 ? 1 + kVarPush : g->force_variant;
+  if (g->small_levels) DAWN_CHECK(records(g));
+  if (!g->trace && !(g->small_levels && g->rec_len == kLevelKernels)) {
+    if (!g->bfs_sync.p) {
+      DAWN_CHECK(ensure(g->bfs_sync, sizeof(BfsSync), g->stream));
+      DAWN_CUDA(cudaMemsetAsync(g->bfs_sync.p, 0, sizeof(BfsSync), g->stream));
+    }
+    BfsArgs a = {};
+    a.row_ptr = g->row_ptr;
+    a.col = g->col;
+    a.t_row_ptr = g->t_row_ptr;
+    a.t_col = g->t_col;
+    a.ctl = g->ss_ctl.as<SsCtl>();
+    a.sync = g->bfs_sync.as<BfsSync>();
+    a.q = g->ss_queues.as<int32_t>();
+    a.segs = g->ss_segs.as<Seg>();
+    a.segcap = segcap;
+    a.lcap = (size_t)(m / kLongRow) + 1;
+    DAWN_CHECK(ensure(g->bfs_long, sizeof(int32_t) * 2 * a.lcap, g->stream));
+    a.lq = g->bfs_long.as<int32_t>();
+    a.vbm = g->ss_bitmaps.as<uint32_t>();
+    a.fbm = a.vbm + nwords;
+    a.m = m;
+    a.sel_w = g->sel_slot.as<float>();
+    a.n = n;
+    a.nwords = nwords;
+    a.policy = policy;
+    a.use_sel = g->sel_call;
+    a.sel_margin = g->sel_margin;
+    a.force = force;
+    a.small = g->small_levels;
+    const bool mesh = g->small_levels && g->rec_len > 0;
+    a.rec_len = mesh ? g->rec_len : 0;
+    a.rec = mesh ? g->bfs_rec.as<int32_t>() : nullptr;
+    const void* const fn = mesh ? (const void*)bfs_traverse<true> : (const void*)bfs_traverse<false>;
+    const int threads = mesh ? 1024 : 640;
+    constexpr size_t kMeshBytes = offsetof(BfsSmem<32>, mesh) + sizeof(MeshLists);
+    static_assert(kMeshBytes + kMeshMax / 8 >= sizeof(BfsSmem<32>), "the largest size is the bitmap's");
+    const size_t smem = mesh ? std::max(sizeof(BfsSmem<32>), kMeshBytes + sizeof(uint32_t) * (size_t)nwords)
+                             : sizeof(BfsSmem<20>);
+    if (g->bfs_fn != fn || g->bfs_cap != g->blocks_per_sm) {  // 8 us of every call otherwise
+      DAWN_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     mesh ? (int)(kMeshBytes + kMeshMax / 8) : (int)smem));
+      g->bfs_ctas = persistent_blocks(fn, threads, smem, g->blocks_per_sm);
+      g->bfs_fn = fn;
+      g->bfs_cap = g->blocks_per_sm;
+    }
+    // a small graph takes few CTAs: each adds to the arrivals of its phases
+    const int64_t want = (n + m) / kBfEntries + 1;
+    const int ctas = want < g->bfs_ctas ? (int)want : g->bfs_ctas;
+    void* args[] = {&a};
+    for (int32_t i = 0; i < nsrc; i++) {
+      a.source = sources[i];
+      a.first = i == 0;
+      a.dist = d_dist + (size_t)i * n;
+      DAWN_CUDA(cudaLaunchCooperativeKernel(fn, dim3(ctas), dim3(threads), args, smem, g->stream));
+    }
+    return DAWN_OK;
+  }
+  // level kernels: traced calls, and large graphs of low degree
   DAWN_CHECK(ensure(g->ss_sources, sizeof(int32_t) * (size_t)nsrc, g->stream));
   DAWN_CUDA(cudaMemcpyAsync(g->ss_sources.p, sources, sizeof(int32_t) * nsrc, cudaMemcpyHostToDevice,
                             g->stream));
@@ -646,7 +1483,7 @@ dawn_status bfs_single(dawn_graph* g, const int32_t* sources, int32_t nsrc, int3
   c.sources = g->ss_sources.as<int32_t>();
   c.use_sel = g->sel_call;
   c.sel_margin = g->sel_margin;
-  c.force = g->force_variant == 3 ? 1 + kVarPush : g->force_variant;
+  c.force = force;
   c.small = g->small_levels && cluster_fits((const void*)bfs_small, kSmallCtas, kSmallBlock) ? 1 : 0;
   c.m = m;
   DAWN_CHECK(upload_ctl(g, c));

@@ -196,6 +196,12 @@ struct dawn_graph {
   dawn::DevBuf ss_segs;     // 2 x seg_capacity long-row segments
   dawn::DevBuf ss_bitmaps;  // visited + 3 frontier bitmaps (words)
   dawn::DevBuf ss_ctl;      // SsCtl
+  dawn::DevBuf bfs_long;    // 2 x the long rows of a level (single-source BFS)
+  const void* bfs_fn = nullptr;    // the persistent kernel that bfs_ctas and the kernel's limits were set for
+  int32_t bfs_ctas = 0, bfs_cap = 0;
+  dawn::DevBuf bfs_rec;     // rows of low degree as records (single-source BFS)
+  int32_t rec_len = -1;     // words of a record; 0: none, -1: not decided, -2: level kernels instead
+  dawn::DevBuf bfs_sync;    // BfsSync: what the CTAs of the persistent BFS wait on
   dawn::DevBuf ss_sources;  // int32 source list of the current call
   dawn::DevBuf ss_scratch;  // n x u64 (GOVM source-row resolution)
   dawn::DevBuf bc_levels;   // betweenness: level blocks of two batches (bfs_bitset_levels)

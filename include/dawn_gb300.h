@@ -271,10 +271,12 @@ dawn_status dawn_closeness(dawn_graph* g, const int32_t* sources,
  *                          (DAWN_VARIANT_DO) run stretches of levels whose
  *                          frontier holds at most 8192 vertices and 32768
  *                          out-edges, and no row of 128 entries or more,
- *                          inside one launch of a thread-block cluster
- *                          (8 CTAs, one cluster barrier per level), instead
- *                          of a launch per level.  0: every level is its
- *                          own launch.  Distances are the same. */
+ *                          on a single CTA with the lists in shared memory
+ *                          (the smallest of them; on graphs of low degree
+ *                          up to 2048 vertices), or, on large graphs of low
+ *                          degree, in a thread-block cluster (8 CTAs, one
+ *                          cluster barrier per level).  0: every level runs
+ *                          on the whole grid.  Distances are the same. */
 #define DAWN_OPT_SMALL_LEVELS 9
 
 /* Autotuner (no counterpart in the reference, whose launch shapes are fixed
