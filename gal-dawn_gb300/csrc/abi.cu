@@ -243,7 +243,7 @@ dawn_status sssp_device_impl(dawn_graph* g, const int32_t* sources, int32_t nsrc
     DAWN_CHECK(dawn::ensure(g->cc_out, 16 * (size_t)nsrc, g->stream));
     double* sum = g->cc_out.as<double>();
     long long* cnt = reinterpret_cast<long long*>(sum + nsrc);
-    DAWN_CHECK(dawn::row_reduce(g, d_dist, nsrc, g->ss_sources.as<int32_t>(), g->wtype == DAWN_W_F32 ? 2 : 1,
+    DAWN_CHECK(dawn::row_reduce(g, d_dist, nsrc, g->ss_src, g->wtype == DAWN_W_F32 ? 2 : 1,
                                 1, sum, cnt));
     std::vector<long long> h(nsrc);
     DAWN_CUDA(cudaMemcpyAsync(h.data(), sum, sizeof(long long) * nsrc, cudaMemcpyDeviceToHost, g->stream));

@@ -203,6 +203,7 @@ struct dawn_graph {
   int32_t rec_len = -1;     // words of a record; 0: none, -1: not decided, -2: level kernels instead
   dawn::DevBuf bfs_sync;    // BfsSync: what the CTAs of the persistent BFS wait on
   dawn::DevBuf ss_sources;  // int32 source list of the current call
+  const int32_t* ss_src = nullptr;  // weighted: where the current call's list is
   dawn::DevBuf ss_scratch;  // n x u64 (GOVM source-row resolution)
   dawn::DevBuf bc_levels;   // betweenness: level blocks of two batches (bfs_bitset_levels)
   dawn::DevBuf bc_terms;    // per 64 sources of a batch, n x 64 float (1 / amount + dependency)

@@ -25,6 +25,9 @@
 // Any relaxation order reaches the same fixed point (the minimum over paths
 // of the path sums, which rounding leaves monotone), so push, pull and
 // their mix give the distances of the reference CPU path.
+#include <algorithm>
+#include <vector>
+
 #include "dawn_device.cuh"
 #include "selector.cuh"
 
@@ -388,13 +391,15 @@ void probe_sssp(const void* p, LevelProbe* out) {
 
 // One ordered traversal (nearfar.cu) per source.
 dawn_status sssp_ordered(dawn_graph* g, const int32_t* sources, int32_t nsrc, void* d_dist) {
-  DAWN_CHECK(ensure(g->ss_ctl, sizeof(SsCtl), g->stream));
-  DAWN_CHECK(ensure(g->ss_sources, sizeof(int32_t) * (size_t)nsrc, g->stream));
-  DAWN_CUDA(cudaMemcpyAsync(g->ss_sources.p, sources, sizeof(int32_t) * nsrc, cudaMemcpyHostToDevice, g->stream));
-  DAWN_CUDA(cudaMemsetAsync(g->ss_ctl.p, 0, sizeof(SsCtl), g->stream));
+  // one upload: the control block, cleared, and the sources
+  std::vector<int32_t> up(sizeof(SsCtl) / sizeof(int32_t) + (size_t)nsrc, 0);
+  std::copy(sources, sources + nsrc, up.end() - nsrc);
+  DAWN_CHECK(ensure(g->ss_ctl, sizeof(int32_t) * up.size(), g->stream));
+  DAWN_CUDA(cudaMemcpyAsync(g->ss_ctl.p, up.data(), sizeof(int32_t) * up.size(), cudaMemcpyHostToDevice, g->stream));
   SsCtl* ctl = g->ss_ctl.as<SsCtl>();
+  g->ss_src = reinterpret_cast<const int32_t*>(ctl + 1);
   for (int32_t i = 0; i < nsrc; i++)
-    DAWN_CHECK(nearfar_run(g, g->ss_sources.as<int32_t>() + i, 1, 0,
+    DAWN_CHECK(nearfar_run(g, g->ss_src + i, 1, 0,
                            static_cast<int32_t*>(d_dist) + (size_t)i * g->n, &ctl->total_levels, &ctl->total_push, &ctl->err));
   return DAWN_OK;
 }
@@ -421,6 +426,7 @@ dawn_status sssp_single(dawn_graph* g, const int32_t* sources, int32_t nsrc, voi
   DAWN_CHECK(build_static_list(g));
   DAWN_CUDA(cudaMemcpyAsync(g->ss_sources.p, sources, sizeof(int32_t) * nsrc, cudaMemcpyHostToDevice,
                             g->stream));
+  g->ss_src = g->ss_sources.as<int32_t>();
   const int is_float = g->wtype == DAWN_W_F32;
   SsCtl c = {};
   c.policy = DAWN_VARIANT_PUSH;

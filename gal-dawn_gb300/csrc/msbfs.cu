@@ -1481,6 +1481,9 @@ __global__ void bs_next(const __grid_constant__ BsArgs a) {
 
 // --- the persistent launch ----------------------------------------------------------
 
+// Vertices and entries per CTA of a small graph: 1024 / 4096, 64 sources: grid 40 x
+// 60 880 / 1006 us, kNN of 2,127 points 545 / 593, RMAT-12 107 / 114.
+constexpr int kBsEntries = 1024;
 constexpr uint32_t kBsPollLimit = 1u << 27;  // polls of one wait (over 30 s) before the launch gives up
 
 // CTAs for `work` warp tasks.
@@ -1857,7 +1860,10 @@ dawn_status run_width(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32
   if (!g->trace) {
     const void* fn = (const void*)bs_traverse<W>;
     const int threads = W == 1 ? 640 : 512;
-    const int ctas = persistent_blocks(fn, threads, 0, g->blocks_per_sm);
+    // a small graph takes few CTAs: each adds to the arrivals of its phases
+    const int64_t want = ((int64_t)n + g->m) / kBsEntries + 1;
+    const int full = persistent_blocks(fn, threads, 0, g->blocks_per_sm);
+    const int ctas = want < full ? (int)want : full;
     for (a.batch = 0; a.batch < nbatches; a.batch++) {
       DAWN_CHECK(launch_cooperative(fam, fn, ctas, threads, args, g->stream));
       DAWN_CUDA(cudaLaunchKernel((const void*)bs_emit_dist<W>, dim3(sms * 8), dim3(kBlock), args, 0, g->stream));

@@ -48,6 +48,7 @@ namespace {
 constexpr int kNfBlock = 512;
 constexpr int kShortUnroll = 3;  // groups of 32 entries of short rows in flight per warp
 constexpr int kNfWarps = kNfBlock / 32;
+constexpr int kNfEntries = 256;  // vertices and entries per CTA of a small graph (512 the same, 1024: kNN of 2,127 8% slower)
 constexpr uint32_t kPollLimit = 1u << 27;  // polls of one wait (over 30 s) before the launch gives up
 
 enum : int32_t { kPhFill = 0, kPhMark, kPhSeed, kPhNear, kPhFar };
@@ -82,7 +83,11 @@ struct __align__(128) NfCtl {
 };
 
 // Near list of a single-CTA phase.
-constexpr int kSoloMax = 256, kSoloCap = 1024;
+constexpr int kSoloMax = 640, kSoloCap = 1024;
+// At the graph's mean degree: one SM relaxes about 1,900 entries in the time of a
+// phase on the grid (grid 120 x 150: 640 pairs 1005 us, 480 899, 160 1044; kNN of
+// 2,127 points: 310 pairs 451 us, 190 405, 60 416).
+constexpr double kSoloEntries = 1920.0;
 struct Solo {
   uint32_t p[kSoloCap];
   int32_t rs[kSoloCap], deg[kSoloCap];
@@ -101,6 +106,7 @@ struct NfArgs {
   int32_t n, shift;
   uint32_t inf, delta, delta_min, delta_max;
   int32_t has_long;        // some row has at least kLongRow entries
+  uint32_t solo_max;       // pairs of a single-CTA phase
   int32_t* levels_out;     // of the call's control block: levels, push levels, error code
   int32_t* push_out;
   int32_t* err_out;
@@ -189,7 +195,7 @@ __device__ __forceinline__ bool nf_control(const NfArgs& a, uint32_t g, uint32_t
     p.kind = kPhNear;
     p.n = nn;
     p.segs = ns;
-    p.ctas = ns == 0 && nn <= kSoloMax ? 1 : nf_ctas(nn + 2 * ns, kNfWarps * 2);
+    p.ctas = ns == 0 && nn <= a.solo_max ? 1 : nf_ctas(nn + 2 * ns, kNfWarps * 2);
     atomicAdd(&c->far.iters, 1u);
     atomicAdd(&c->far.bucket_iters, 1u);
     atomicAdd(&c->far.bucket_pairs, (unsigned long long)nn + 4ull * ns);
@@ -476,7 +482,7 @@ __global__ void __launch_bounds__(kNfBlock, 2) nf_traverse(const __grid_constant
       }
     };
 
-    if (phase == kPhNear && ph.ctas == 1 && ph.segs == 0 && ph.n <= kSoloMax) {
+    if (phase == kPhNear && ph.ctas == 1 && ph.segs == 0 && ph.n <= a.solo_max) {
       // A few pairs: this CTA alone runs near phases one after another with
       // the lists in shared memory, one barrier per phase, until a list is
       // empty, too long, or holds a long row.  A pair pushed twice in a phase
@@ -555,7 +561,7 @@ __global__ void __launch_bounds__(kNfBlock, 2) nf_traverse(const __grid_constant
         }
         __syncthreads();
         left = *nx_cnt;
-        if (left == 0 || left > kSoloMax || s_long) break;
+        if (left == 0 || left > (int)a.solo_max || s_long) break;
       }
       if (threadIdx.x == 0 && it > 0) {
         atomicAdd(&ctl->far.iters, (uint32_t)it);
@@ -821,10 +827,14 @@ dawn_status nearfar_run(dawn_graph* g, const int32_t* d_sources, int32_t nb, int
   // depends on the work there is.  4 / 8 / 32 / 128: RMAT scale 22 2.14 /
   // 1.83 / 2.75 / 2.85 ms, kNN x 50 sources 10.1 / 10.0 / 10.5 / 13.4 ms; ER
   // (16M entries) 614 / 637 / 529 / 913 us; RMAT scale 12 190 / 160 / 146 /
-  // 130 us, ER (160K entries) 194 / 184 / 151 / 135 us.
+  // 130 us, ER (160K entries) 194 / 184 / 151 / 135 us.  128 / 512: kNN of 2,127
+  // points 406 / 363 us, grid 120 x 150 913 / 945, 10 sources there 1531 / 1387.
   const double work = (double)g->m * nb;
-  const double kStep = work < 1 << 20 ? 128.0 : (work < 1 << 24 ? 32.0 : 8.0);
+  const double kStep = work < 1 << 16 || (nb > 1 && work < 1 << 20) ? 512.0
+                       : work < 1 << 20                               ? 128.0
+                                                                      : (work < 1 << 24 ? 32.0 : 8.0);
   const double deg = g->m > 0 ? (double)g->m / (double)g->n : 1.0;
+  a.solo_max = (uint32_t)std::min((double)kSoloMax, kSoloEntries / std::max(1.0, deg));
   const double step = kStep * g->nf_mean_weight / std::max(1.0, deg);
   const double lo = step / 2, hi = step * 16;
   auto bits = [&](double x) -> uint32_t {
@@ -841,8 +851,11 @@ dawn_status nearfar_run(dawn_graph* g, const int32_t* d_sources, int32_t nb, int
   a.delta_max = bits(hi);
   const void* fn = fl ? (const void*)nf_traverse<true> : (const void*)nf_traverse<false>;
   void* args[] = {&a};
-  DAWN_CUDA(cudaLaunchCooperativeKernel(fn, dim3(persistent_blocks(fn, kNfBlock, 0, g->blocks_per_sm)),
-                                        dim3(kNfBlock), args, 0, g->stream));
+  // a small graph takes few CTAs: each adds to the arrivals of its phases
+  const int64_t want = (int64_t)((double)(g->n + g->m) * nb / kNfEntries) + 1;
+  const int full = persistent_blocks(fn, kNfBlock, 0, g->blocks_per_sm);
+  const int ctas = want < full ? (int)want : full;
+  DAWN_CUDA(cudaLaunchCooperativeKernel(fn, dim3(ctas), dim3(kNfBlock), args, 0, g->stream));
   return DAWN_OK;
 }
 
