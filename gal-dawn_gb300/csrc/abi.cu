@@ -761,6 +761,7 @@ dawn_status dawn_graph_set_option(dawn_graph* g, int32_t option, int64_t value) 
         return DAWN_ERR_INVALID_ARG;
       }
       g->bs_push_ratio = (int32_t)value;
+      g->bs_ratio_set = true;
       return DAWN_OK;
     case DAWN_OPT_FORCE_VARIANT:
       if (value < 0 || value > 3) {

@@ -242,6 +242,7 @@ struct dawn_graph {
   dawn::DevBuf hv_tasks;        // 2 x hv_segs (row, segment): segments of heavy rows still unfinished
   int32_t hv_count = 0, hv_segs = 0;
   int32_t bs_push_ratio = 4;    // push while ratio * frontier edges < unfinished edges
+  bool bs_ratio_set = false;    // by the caller or the autotuner
   int32_t bs_width = 0;         // words per vertex of the bitset traversal (0 = by source count)
   int32_t force_variant = 0;    // 0 = decide per level, else 1 + variant for every level
   int32_t blocks_per_sm = 0;    // CTAs per SM of the persistent traversal grids (0 = occupancy limit)

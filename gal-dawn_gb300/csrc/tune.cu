@@ -59,6 +59,7 @@ std::string class_key(const dawn_graph* g, int32_t nsrc) {
 void apply(dawn_graph* g, const Settings& s) {
   g->bs_width = s.width;
   g->bs_push_ratio = s.ratio;
+  g->bs_ratio_set = true;
   g->pull_seg = s.seg;
   if (g->blocks_per_sm != s.bps) {
     g->blocks_per_sm = s.bps;

@@ -227,7 +227,9 @@ dawn_status dawn_closeness(dawn_graph* g, const int32_t* sources,
  *                          0 = chosen from the source count, or 1, 2, 4
  *                          (64, 128, 256 sources per batch)
  *   DAWN_OPT_PUSH_RATIO    a level pushes while ratio x frontier edges <
- *                          edges of unfinished vertices (default 4) */
+ *                          edges of unfinished vertices (default 4; until it is
+ *                          set, batched traversals of graphs with 16
+ *                          entries a vertex or more use 2) */
 #define DAWN_OPT_BITSET_WIDTH 1
 #define DAWN_OPT_PUSH_RATIO 2
 /*   DAWN_OPT_FORCE_VARIANT every level of BFS and SSSP traversals runs one
