@@ -110,32 +110,7 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x) {
 
 // Light rows go to warps in chunks of `per` vertices whose entries are laid
 // end to end, one entry per lane: a row of three entries then costs three
-// lanes, not a warp's round trips.  Lane i holds row i of the chunk: its first
-// entry, and where its entries start in the chunk.
-struct Chunk {
-  int32_t ks, off, total;
-  __device__ __forceinline__ Chunk(int32_t first, int32_t deg) : ks(first) {
-    int32_t x = deg;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const int32_t y = __shfl_up_sync(kFull, x, d);
-      if (lane_id() >= d) x += y;
-    }
-    off = x - deg;
-    total = __shfl_sync(kFull, x, 31);
-  }
-  // The row of entry f: the last one that starts at or before it.
-  __device__ __forceinline__ int row(int f) const {
-    int lo = 0;
-#pragma unroll
-    for (int step = 16; step; step >>= 1) {
-      const int at = __shfl_sync(kFull, off, (lo + step) & 31);
-      if (lo + step < 32 && at <= f) lo += step;
-    }
-    return lo;
-  }
-};
-
+// lanes, not a warp's round trips.
 // Vertices per chunk: enough chunks for every warp of the grid.
 __host__ __device__ inline int chunk_rows(int32_t n, int warps) {
   int per = 32;
@@ -221,7 +196,7 @@ __global__ void __launch_bounds__(kBlock) bc_amount(const int32_t* __restrict__ 
     }
     if (!set) continue;
     if (!reach) deg = 0;
-    const Chunk ch(ks, deg);
+    const RowChunk ch(ks, deg);
     int ca = 0, cb = 0;
     for (int f0 = 0; f0 < ch.total; f0 += 32) {
       const int f = f0 + lane;
@@ -324,7 +299,7 @@ __global__ void __launch_bounds__(kBlock, 5) bc_sweep(const int32_t* __restrict_
         if (deg >= kHeavy || !w) deg = 0;
       }
     }
-    const Chunk ch(ks, deg);
+    const RowChunk ch(ks, deg);
     int32_t cur = -1;  // the row being summed
     float2 s = make_float2(0.0f, 0.0f), own = s;
     for (int f0 = 0; f0 < ch.total; f0 += 32) {

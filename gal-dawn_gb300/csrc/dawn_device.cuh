@@ -85,6 +85,32 @@ namespace dawn {
 
 constexpr int kWarpRow = 32;  // rows with at least this many entries use the whole warp
 
+// Up to 32 rows of a warp whose entries are laid end to end, one per lane.  Lane
+// i holds row i: its first entry, and where its entries start.
+struct RowChunk {
+  int32_t ks, off, total;
+  __device__ __forceinline__ RowChunk(int32_t first, int32_t deg) : ks(first) {
+    int32_t x = deg;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int32_t y = __shfl_up_sync(kFull, x, d);
+      if (lane_id() >= d) x += y;
+    }
+    off = x - deg;
+    total = __shfl_sync(kFull, x, 31);
+  }
+  // The row of entry f: the last one that starts at or before it.
+  __device__ __forceinline__ int row(int f) const {
+    int lo = 0;
+#pragma unroll
+    for (int step = 16; step; step >>= 1) {
+      const int at = __shfl_sync(kFull, off, (lo + step) & 31);
+      if (lo + step < 32 && at <= f) lo += step;
+    }
+    return lo;
+  }
+};
+
 // Deals the out-edges of a vertex queue to the lanes of every warp of the
 // grid.  Rows of >= kWarpRow entries are swept by the whole warp with
 // coalesced col loads; shorter rows are concatenated through a warp scan and

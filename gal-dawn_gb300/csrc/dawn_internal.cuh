@@ -225,7 +225,12 @@ struct dawn_graph {
   int64_t nf_segs = 0;      // segments of the long out-rows
   double nf_mean_weight = 0.0;
   dawn::DevBuf wt_col;      // weighted in-edge CSR (rows of t_row_ptr): tail vertex
-  dawn::DevBuf wt_val;      // and weight of each in-edge, built on the first weighted pull
+  dawn::DevBuf wt_val;      // and weight of each in-edge, built on the first weighted pull, light entries first
+  dawn::DevBuf wt_light;    // end of the light entries of each row
+  int32_t wt_hub = 0;       // vertex of most in-edges
+  bool wt_has_hub = false;  // it has many times the mean
+  bool wt_has_light = false;  // the light entries are a part of the rows worth a stage of their own
+  dawn::DevBuf mw_bounds;   // batched: per vertex, lowest and highest distance over the sources (mw_bounds)
   dawn::SsCtl* h_ctl = nullptr;  // pinned: [0] upload staging, [1] download
   bool graphs_ok = true;         // conditional CUDA graphs usable
 

@@ -23,6 +23,18 @@
 //     return-free atomicMin where it improves on the fetched value;
 //     the improved sources are OR-ed into the target's next mask, and the
 //     first setter queues the target;
+//   * frontiers whose out-edges reach half the graph are pulled: a vertex reads
+//     its in-edges' tail rows.  What bounds a batch is those 256-byte rows (the
+//     block does not fit L2), so most are left out by bounds (mw_bounds): per
+//     vertex the lowest improved and the highest distance over the sources, both
+//     relative to a hub's distances, which the sources' distances follow
+//     closely.  An edge whose tail's lowest plus its weight is no less than its
+//     head's highest cannot improve any of the 64;
+//   * and the batch starts with pulls along the light in-edges alone (an eighth
+//     of them on RMAT-22): shortest paths run along these, and once the light
+//     edges have settled, one pull over all edges, with every reached pair
+//     taken as improved, leaves out nine tenths of them by the bounds.  RMAT-22
+//     x 64 reads 0.9 m rows so, against 4 m in four whole pulls;
 //   * a final pass transposes the block into the caller's source-major rows
 //     and counts the reached edges.
 // Each source's first frontier is resolved as the single-source path does
@@ -32,6 +44,7 @@
 // reaches the same fixed point, so the distances equal the single-source
 // traversal's.
 #include <algorithm>
+#include <climits>
 
 #include "dawn_device.cuh"
 
@@ -52,12 +65,23 @@ struct MwCtl {
   int32_t work, hwork;          // pull: dynamic work counters (light rows, heavy-row segments)
   int32_t n_pull;
   int32_t n_push, inits;       // inits: mw_init CTAs finished
+  int32_t has_light;           // the batch starts with pulls along light edges
+  int32_t stage;               // of a pull: kLight, kAll or kRest
+  int32_t bounded;             // the pull goes by mw_bounds
+  int32_t has_hub;
+  unsigned long long pairs, prev_pairs;  // (vertex, source) pairs improved by this light pull, by the one before
   unsigned long long reached;   // TEPS numerator of all batches so far
   int32_t* dist_base;           // nsrc x n output (source-major)
   const int32_t* sources;
   int32_t total_levels, total_push, total_pull;
   int32_t err;                  // status of an ordered batch (0 = none)
 };
+
+// Stages of a batch: pulls along light edges; one pull along all edges from every
+// reached pair; whatever is left, from the pairs improved at the last level.
+enum : int32_t { kRest = 0, kLight = 1, kAll = 2 };
+constexpr int kBoundedFrom = 4;   // level from which pulls go by bounds: before it most of a row is unreached
+constexpr int kLightLevels = 24;  // light pulls at most
 
 __device__ __forceinline__ int32_t relax(int32_t d, int32_t w, bool is_float) {
   if (is_float) return __float_as_int(__fadd_rn(__int_as_float(d), __int_as_float(w)));
@@ -78,7 +102,10 @@ __global__ void __launch_bounds__(kBlock) mw_clear(MwCtl* __restrict__ ctl, int3
     ctl->n_push = 0;
     ctl->n_pull = 0;
     ctl->inits = 0;
-    ctl->mode = ctl->force == 2 ? kModePull : kModePush;
+    ctl->stage = ctl->has_light ? kLight : kRest;
+    ctl->mode = ctl->force == 2 || ctl->has_light ? kModePull : kModePush;
+    ctl->bounded = 0;
+    ctl->pairs = ctl->prev_pairs = 0;
     ctl->work = 0;
     ctl->hwork = 0;
   }
@@ -409,37 +436,104 @@ __global__ void __launch_bounds__(kBlock, 4) mw_push(const int32_t* __restrict__
   if (lane == 0 && my_mf) atomicAdd(&ctl->mf[pout], my_mf);
 }
 
-// Pull level (frontiers whose out-edges reach half the graph): every vertex
-// v takes, per source, the minimum of D[u][s] + w over its in-edges (u, w)
-// from tails whose source s improved at the last level, and keeps it where
-// it beats D[v][s].  A warp owns a light row (in-degree below 2 x pull_seg)
-// and writes its row of D and its next mask with plain stores: no atomics
-// per edge, and one improved-source mask per vertex instead of per edge.
-// Heavy rows are cut into pull_seg-entry segment tasks, each a warp, which
-// lower the row with return-free atomicMin where they improve on it and
-// OR their improved sources into the next mask (the first setter queues
-// the vertex).  A tail row (256 bytes) is read by a group of kRowLanes
-// lanes, kPullSrc sources (16 or 32 bytes) per lane, so one warp-wide load
-// brings kRowGroups rows.  Tails are read 32 at a time (vertex coalesced,
-// mask gathered once per lane); the live ones (mask not empty) are packed
-// with their weights into a per-warp shared-memory stage, and the groups
-// walk the stage kPullUnroll rows each, fetching those rows before any is
-// used.  Per-source minima stay in registers; the groups' minima are folded
-// at the end of the vertex and group 0 holds the result.
+// The bounds of a pull: per vertex v, with off[s] the distance of the hub from
+// source s,
+//   x = min D[v][s] - off[s] over the sources improved at v (all reached ones in
+//       the stage kAll), or the type's largest value if there are none;
+//   y = max D[v][s] - off[s] over all sources.
+// An edge (u, v, w) with x[u] + w >= y[v] improves no source: D[u][s] + w is at
+// least D[v][s] for each.  Sources that have not reached the hub have no off: a
+// vertex improved for one of these has the lowest x there is, and y leaves them
+// out.  Float differences are rounded down for x and up for y, and x + w down, so
+// that the comparison holds for the exact values (and then for the rounded sum
+// of the relaxation, which is monotone).  Half a warp per vertex, one pass over
+// the block: 0.17 ms on RMAT-22, where it saves milliseconds.
+template <bool kFloat>
+struct Bound {  // int32 differences, or float ones as their bits
+  __device__ __forceinline__ static int32_t lowest() { return kFloat ? (int32_t)0xff800000u : INT_MIN; }
+  __device__ __forceinline__ static int32_t highest() { return kFloat ? 0x7f800000 : INT_MAX; }
+  __device__ __forceinline__ static int32_t sub_down(int32_t a, int32_t b) {
+    return kFloat ? __float_as_int(__fsub_rd(__int_as_float(a), __int_as_float(b))) : a - b;
+  }
+  __device__ __forceinline__ static int32_t sub_up(int32_t a, int32_t b) {
+    return kFloat ? __float_as_int(__fsub_ru(__int_as_float(a), __int_as_float(b))) : a - b;
+  }
+  __device__ __forceinline__ static int32_t lower(int32_t a, int32_t b) {
+    return kFloat ? __float_as_int(fminf(__int_as_float(a), __int_as_float(b))) : min(a, b);
+  }
+  __device__ __forceinline__ static int32_t higher(int32_t a, int32_t b) {
+    return kFloat ? __float_as_int(fmaxf(__int_as_float(a), __int_as_float(b))) : max(a, b);
+  }
+  // whether an edge of weight w from a tail with lowest x can improve a head with highest y
+  __device__ __forceinline__ static bool may_improve(int32_t x, int32_t w, int32_t y) {
+    if (x == lowest()) return true;
+    if (x == highest()) return false;
+    if (kFloat) return __fadd_rd(__int_as_float(x), __int_as_float(w)) < __int_as_float(y);
+    return (long long)x + w < (long long)y;
+  }
+};
+
+template <bool kFloat>
+__global__ void __launch_bounds__(kBlock) mw_bounds(const MwCtl* __restrict__ ctl, const int32_t* __restrict__ D,
+                                                    const unsigned long long* __restrict__ masks, int32_t inf,
+                                                    int32_t hub, int32_t n, int2* __restrict__ bounds) {
+  using B = Bound<kFloat>;
+  if (ctl->done || ctl->mode != kModePull || !ctl->bounded) return;
+  const unsigned long long* m_in = masks + (size_t)((ctl->level - 1) % 3) * n;
+  const bool all = ctl->stage == kAll;
+  const int lane = lane_id(), sub = lane & 15;
+  const int4 off = __ldcg(reinterpret_cast<const int4*>(D + (size_t)hub * kBatch) + sub);
+  const int warps = num_warps();
+  for (int v0 = global_warp() * 2; v0 < n; v0 += warps * 2) {
+    const int v = v0 + (lane >> 4);
+    int32_t lo = B::highest(), hi = B::lowest();
+    if (v < n) {
+      const int4 d = __ldcs(reinterpret_cast<const int4*>(D + (size_t)v * kBatch) + sub);
+      const unsigned bits = all ? 15u : (unsigned)(__ldcg(m_in + v) >> (4 * sub)) & 15u;
+      const int32_t dd[4] = {d.x, d.y, d.z, d.w}, oo[4] = {off.x, off.y, off.z, off.w};
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const bool reached = dd[i] != inf, has = oo[i] != inf;
+        if (reached && ((bits >> i) & 1u)) lo = has ? B::lower(lo, B::sub_down(dd[i], oo[i])) : B::lowest();
+        if (has) hi = reached ? B::higher(hi, B::sub_up(dd[i], oo[i])) : B::highest();
+      }
+    }
+#pragma unroll
+    for (int k = 8; k; k >>= 1) {
+      lo = B::lower(lo, __shfl_xor_sync(kFull, lo, k));
+      hi = B::higher(hi, __shfl_xor_sync(kFull, hi, k));
+    }
+    if (sub == 0 && v < n) bounds[v] = make_int2(lo, hi);
+  }
+}
+
+// Pull level: every vertex v takes, per source, the minimum of D[u][s] + w over
+// its in-edges (u, w) from tails whose source s improved at the last level (the
+// light ones of them in the stage kLight, from every reached source in the stage
+// kAll), and keeps it where it beats D[v][s].  Edges are tested one per lane,
+// over 32 rows laid end to end; the live ones are packed with their weights and
+// sources into a per-warp shared-memory stage.  A full stage is walked by groups
+// of kRowLanes lanes, a head vertex per group: a tail row (256 bytes) is read by
+// a group, kPullSrc sources (two 16-byte pieces) per lane, kPullUnroll rows in
+// flight.  A warp owns its rows and writes them with plain stores.  Heavy rows
+// (in-degree of 2 x pull_seg and more) are cut into pull_seg-entry segment tasks,
+// each a warp, whose groups walk the stage together and lower the row with
+// return-free atomicMin where they improve on it.
 // Reading a row that another warp lowers in the same level is harmless:
 // every value a row holds is the length of some path, and a value lowered
 // now is relaxed again at the next level through the mask it sets.
-// Eight sources per lane (four rows per warp-wide load) and three rows per
-// group in flight: 64 registers, four CTAs per SM.  RMAT scale 22 x 64
-// sources, int32: 29.3 ms with two sources per lane (one row per load,
-// tails passed by shuffles), 29.7 ms with four (two rows per load), 22.6
-// with eight and two rows per group, 22.3 with three; four rows per group
-// at three CTAs per SM 24.4 ms.
+// Without a hub the bounds leave most of a row until late: there a warp takes one
+// row after another (whole_rows), its groups' minima folded at the end.  That is
+// the better form for whole rows (Erdos-Renyi, 1 M vertices, mean degree 16:
+// 1.0 ms a pull against 1.6) and the worse for the handful that bounds and the
+// light stage leave (RMAT-20 x 64: 2.94 ms a batch, 6.39 with whole rows, by the
+// masks alone and without a light stage).
 constexpr int kPullSrc = 8;                 // sources per lane (4 or 8)
 constexpr int kPullUnroll = 3;              // rows per lane group fetched together
 constexpr int kRowLanes = kBatch / kPullSrc;  // lanes reading one tail row
 constexpr int kRowGroups = 32 / kRowLanes;    // tail rows per warp-wide load
 constexpr int kQuads = kPullSrc / 4;          // 16-byte pieces per lane and row
+static_assert(kRowGroups == 4, "mw_pull splits a warp's groups by two or four");
 static_assert(kPullSrc == 4 || kPullSrc == 8, "a lane reads whole 16-byte pieces of a row");
 
 // Quad q of lane `sub` of a group: sources quad_base(sub, q) .. + 3 (with
@@ -447,130 +541,177 @@ static_assert(kPullSrc == 4 || kPullSrc == 8, "a lane reads whole 16-byte pieces
 // each load instruction of a group covers 128 contiguous bytes).
 __device__ __forceinline__ int quad_base(int sub, int q) { return 4 * sub + q * (kBatch / kQuads); }
 
-__device__ __forceinline__ void pull_min(const int32_t* __restrict__ t_col, const int32_t* __restrict__ t_w,
-                                         const unsigned long long* __restrict__ m_in,
-                                         const int32_t* __restrict__ D, bool fl, int k0, int k1,
-                                         int4* __restrict__ stage, int32_t (&mn)[kPullSrc]) {
-  const int lane = lane_id(), grp = lane / kRowLanes, sub = lane % kRowLanes;
-  for (int kb = k0; kb < k1; kb += 32) {
-    const int k = kb + lane;
-    const int32_t cu = k < k1 ? __ldg(t_col + k) : -1;
-    const unsigned long long cm = cu >= 0 ? __ldcg(m_in + cu) : 0ull;
-    const unsigned live = __ballot_sync(kFull, cm != 0ull);
-    if (cm)
-      stage[__popc(live & lanemask_lt())] =
-          make_int4(cu, __ldg(t_w + k), (int)(unsigned)cm, (int)(unsigned)(cm >> 32));
-    __syncwarp();
-    const int cnt = __popc(live);
-    for (int r0 = 0; r0 < cnt; r0 += kRowGroups * kPullUnroll) {
-      int4 e[kPullUnroll];
-      unsigned bits[kPullUnroll];
-      int4 d[kPullUnroll][kQuads];
-#pragma unroll
-      for (int i = 0; i < kPullUnroll; i++) {
-        const int r = r0 + i * kRowGroups + grp;
-        e[i] = r < cnt ? stage[r] : make_int4(0, 0, 0, 0);
-        bits[i] = 0u;
-#pragma unroll
-        for (int q = 0; q < kQuads; q++) {
-          const int base = quad_base(sub, q);
-          const unsigned word = base >= 32 ? (unsigned)e[i].w : (unsigned)e[i].z;
-          bits[i] |= ((word >> (base & 31)) & 15u) << (4 * q);
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < kPullUnroll; i++) {
-        const int4* du = reinterpret_cast<const int4*>(D + (size_t)e[i].x * kBatch);
-#pragma unroll
-        for (int q = 0; q < kQuads; q++)
-          d[i][q] = ((bits[i] >> (4 * q)) & 15u) ? __ldcg(du + quad_base(sub, q) / 4) : make_int4(0, 0, 0, 0);
-      }
-#pragma unroll
-      for (int i = 0; i < kPullUnroll; i++) {
-#pragma unroll
-        for (int q = 0; q < kQuads; q++) {
-          const unsigned b = bits[i] >> (4 * q);
-          if (b & 1u) mn[4 * q + 0] = min(mn[4 * q + 0], relax(d[i][q].x, e[i].y, fl));
-          if (b & 2u) mn[4 * q + 1] = min(mn[4 * q + 1], relax(d[i][q].y, e[i].y, fl));
-          if (b & 4u) mn[4 * q + 2] = min(mn[4 * q + 2], relax(d[i][q].z, e[i].y, fl));
-          if (b & 8u) mn[4 * q + 3] = min(mn[4 * q + 3], relax(d[i][q].w, e[i].y, fl));
-        }
-      }
-    }
-    __syncwarp();
-  }
-#pragma unroll
-  for (int off = kRowLanes; off < 32; off <<= 1)
-#pragma unroll
-    for (int t = 0; t < kPullSrc; t++) mn[t] = min(mn[t], __shfl_xor_sync(kFull, mn[t], off));
+// What a pull goes by.
+struct PullArgs {
+  const int32_t *t_col, *t_w;
+  const unsigned long long* m_in;
+  const int2* bounds;  // NULL: by the masks alone
+  bool all;            // every reached source counts as improved
+};
+
+// The sources of in-edge k of a head whose highest bound is y, and its tail and
+// weight; 0: leave it out.
+template <bool kFloat>
+__device__ __forceinline__ unsigned long long edge_sources(const PullArgs& a, int k, int32_t y, int32_t& u,
+                                                           int32_t& w) {
+  u = __ldg(a.t_col + k);
+  w = __ldg(a.t_w + k);
+  if (a.bounds && !Bound<kFloat>::may_improve(__ldg(&a.bounds[u].x), w, y)) return 0ull;
+  return a.all ? ~0ull : __ldcg(a.m_in + u);
 }
 
-// The pulled minima of vertex v against its row: group 0 lowers the row
-// (plain stores where the warp owns the row, atomicMin on heavy-row
-// segments) and the warp returns the 64-bit mask of improved sources.
-template <bool kAtomic>
-__device__ __forceinline__ unsigned long long pull_store(int32_t* __restrict__ D, int32_t v,
-                                                         const int32_t (&mn)[kPullSrc]) {
-  const int lane = lane_id(), sub = lane % kRowLanes;
-  unsigned lo = 0u, hi = 0u;
-  if (lane < kRowLanes) {
-    int4* dv = reinterpret_cast<int4*>(D + (size_t)v * kBatch);
+// A relaxation in a pull: unreached tails (kAll) end above every distance.
+template <bool kFloat>
+__device__ __forceinline__ uint32_t pull_relax(int32_t d, int32_t w) {
+  if (kFloat) return __float_as_uint(__fadd_rn(__int_as_float(d), __int_as_float(w)));
+  return (uint32_t)d + (uint32_t)w;
+}
+
+// Entries first, first + step, ... below end of the stage, by a group of lanes:
+// their rows' minima with mn.
+template <bool kFloat>
+__device__ __forceinline__ void pull_rows(const int4* stage, int first, int step, int end,
+                                          const int32_t* __restrict__ D, uint32_t (&mn)[kPullSrc]) {
+  const int sub = lane_id() % kRowLanes;
+  for (int r0 = first; r0 < end; r0 += step * kPullUnroll) {
+    int32_t w[kPullUnroll];
+    unsigned bits[kPullUnroll];
+    int4 d[kPullUnroll][kQuads];
 #pragma unroll
-    for (int q = 0; q < kQuads; q++) {
-      const int base = quad_base(sub, q);
-      const int4 cur = __ldcg(dv + base / 4);
-      const int32_t* m = mn + 4 * q;
-      const unsigned imp = (unsigned)(m[0] < cur.x) | (unsigned)(m[1] < cur.y) << 1 |
-                           (unsigned)(m[2] < cur.z) << 2 | (unsigned)(m[3] < cur.w) << 3;
-      if (imp) {
-        if (kAtomic) {
-          int32_t* p = D + (size_t)v * kBatch + base;
-          if (imp & 1u) atomicMin(p + 0, m[0]);
-          if (imp & 2u) atomicMin(p + 1, m[1]);
-          if (imp & 4u) atomicMin(p + 2, m[2]);
-          if (imp & 8u) atomicMin(p + 3, m[3]);
-        } else {
-          dv[base / 4] = make_int4(imp & 1u ? m[0] : cur.x, imp & 2u ? m[1] : cur.y, imp & 4u ? m[2] : cur.z,
-                                   imp & 8u ? m[3] : cur.w);
-        }
+    for (int i = 0; i < kPullUnroll; i++) {
+      const int r = r0 + i * step;
+      const int4 e = r < end ? stage[r] : make_int4(0, 0, 0, 0);
+      w[i] = e.y;
+      bits[i] = 0u;
+      const int4* du = reinterpret_cast<const int4*>(D + (size_t)e.x * kBatch);
+#pragma unroll
+      for (int q = 0; q < kQuads; q++) {
+        const int base = quad_base(sub, q);
+        const unsigned b = ((base >= 32 ? (unsigned)e.w : (unsigned)e.z) >> (base & 31)) & 15u;
+        bits[i] |= b << (4 * q);
+        d[i][q] = b ? __ldcg(du + base / 4) : make_int4(0, 0, 0, 0);
       }
-      if (base >= 32) hi |= imp << (base & 31);
-      else lo |= imp << base;
+    }
+#pragma unroll
+    for (int i = 0; i < kPullUnroll; i++) {
+#pragma unroll
+      for (int q = 0; q < kQuads; q++) {
+        const unsigned b = bits[i] >> (4 * q);
+        if (b & 1u) mn[4 * q + 0] = min(mn[4 * q + 0], pull_relax<kFloat>(d[i][q].x, w[i]));
+        if (b & 2u) mn[4 * q + 1] = min(mn[4 * q + 1], pull_relax<kFloat>(d[i][q].y, w[i]));
+        if (b & 4u) mn[4 * q + 2] = min(mn[4 * q + 2], pull_relax<kFloat>(d[i][q].z, w[i]));
+        if (b & 8u) mn[4 * q + 3] = min(mn[4 * q + 3], pull_relax<kFloat>(d[i][q].w, w[i]));
+      }
     }
   }
-  lo = __reduce_or_sync(kFull, lo);
-  hi = __reduce_or_sync(kFull, hi);
+}
+
+// A lane's minima against its pieces of v's row, lowered where they improve
+// (kAtomic: other warps lower it too).  Returns the lane's improved sources, four
+// bits per piece.
+template <bool kAtomic>
+__device__ __forceinline__ unsigned pull_lower(int32_t* __restrict__ D, int32_t v, const uint32_t (&mn)[kPullSrc]) {
+  const int sub = lane_id() % kRowLanes;
+  unsigned all = 0u;
+  int4* dv = reinterpret_cast<int4*>(D + (size_t)v * kBatch);
+#pragma unroll
+  for (int q = 0; q < kQuads; q++) {
+    const int base = quad_base(sub, q);
+    const int4 cur = __ldcg(dv + base / 4);
+    const uint32_t* m = mn + 4 * q;
+    const unsigned imp = (unsigned)(m[0] < (uint32_t)cur.x) | (unsigned)(m[1] < (uint32_t)cur.y) << 1 |
+                         (unsigned)(m[2] < (uint32_t)cur.z) << 2 | (unsigned)(m[3] < (uint32_t)cur.w) << 3;
+    if (imp && kAtomic) {
+      int32_t* p = D + (size_t)v * kBatch + base;
+      if (imp & 1u) atomicMin(p + 0, (int32_t)m[0]);
+      if (imp & 2u) atomicMin(p + 1, (int32_t)m[1]);
+      if (imp & 4u) atomicMin(p + 2, (int32_t)m[2]);
+      if (imp & 8u) atomicMin(p + 3, (int32_t)m[3]);
+    } else if (imp) {
+      dv[base / 4] = make_int4(imp & 1u ? (int32_t)m[0] : cur.x, imp & 2u ? (int32_t)m[1] : cur.y,
+                               imp & 4u ? (int32_t)m[2] : cur.z, imp & 8u ? (int32_t)m[3] : cur.w);
+    }
+    all |= imp << (4 * q);
+  }
+  return all;
+}
+
+// The 64-bit mask of a group's improved sources, in its lane 0's eyes (every lane
+// of the warp calls it; the groups' masks apart).
+__device__ __forceinline__ unsigned long long group_mask(unsigned imp) {
+  const int sub = lane_id() % kRowLanes;
+  unsigned lo = 0u, hi = 0u;
+#pragma unroll
+  for (int q = 0; q < kQuads; q++) {
+    const int base = quad_base(sub, q);
+    const unsigned x = ((imp >> (4 * q)) & 15u) << (base & 31);
+    if (base >= 32) hi |= x;
+    else lo |= x;
+  }
+#pragma unroll
+  for (int k = kRowLanes / 2; k; k >>= 1) {
+    lo |= __shfl_xor_sync(kFull, lo, k);
+    hi |= __shfl_xor_sync(kFull, hi, k);
+  }
   return (unsigned long long)hi << 32 | lo;
 }
 
-__global__ void __launch_bounds__(kBlock, 4) mw_pull(const int32_t* __restrict__ row_ptr,
-                                                  const int32_t* __restrict__ t_row_ptr,
-                                                  const int32_t* __restrict__ t_col, const int32_t* __restrict__ t_w,
-                                                  int is_float, MwCtl* __restrict__ ctl, int32_t* __restrict__ D,
-                                                  unsigned long long* __restrict__ masks, int32_t* __restrict__ q,
-                                                  Seg* __restrict__ segs, size_t segcap,
-                                                  const int32_t* __restrict__ ul, int32_t ul_n,
-                                                  const int32_t* __restrict__ hv, const int32_t* __restrict__ hv_segoff,
-                                                  int32_t hv_count, int32_t hv_segs, int32_t pull_seg, int32_t n) {
-  __shared__ int32_t s_q[kBlock / 32][kWarpQueue];
+template <bool kFloat>
+__global__ void __launch_bounds__(kBlock, 4) mw_pull(const int32_t* __restrict__ t_row_ptr,
+                                                     const int32_t* __restrict__ t_light,
+                                                     const int32_t* __restrict__ t_col, const int32_t* __restrict__ t_w,
+                                                     MwCtl* __restrict__ ctl, int32_t* __restrict__ D,
+                                                     unsigned long long* __restrict__ masks,
+                                                     const int2* __restrict__ bounds, const int32_t* __restrict__ ul,
+                                                     int32_t ul_n, const int32_t* __restrict__ hv,
+                                                     const int32_t* __restrict__ hv_segoff, int32_t hv_count,
+                                                     int32_t hv_segs, int32_t pull_seg, int32_t whole_rows, int32_t n) {
   __shared__ int4 s_stage[kBlock / 32][32];
+  __shared__ int32_t s_row[kBlock / 32][32];    // per staged edge, its row in the chunk
+  __shared__ int32_t s_head[kBlock / 32][33];   // where each row's edges start in the stage
+  __shared__ unsigned long long s_pairs;
   if (ctl->done || ctl->mode != kModePull) return;
   const int L = ctl->level;
-  const int pout = L & 1;
-  const unsigned long long* __restrict__ m_in = masks + (size_t)((L - 1) % 3) * n;
   unsigned long long* m_out = masks + (size_t)(L % 3) * n;
   {
     unsigned long long* m_clr = masks + (size_t)((L + 1) % 3) * n;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)n; i += stride) m_clr[i] = 0ull;
   }
-  const int lane = lane_id(), wib = threadIdx.x >> 5;
-  const bool fl = is_float != 0;
-  int4* stage = s_stage[wib];
-  WarpQueue wq(s_q[wib], q + (size_t)pout * n, &ctl->qsize[pout]);
-  Seg* sout = segs + (size_t)pout * segcap;
-  unsigned long long* lpack = &ctl->lpack[pout];
-  unsigned long long my_mf = 0;
+  if (threadIdx.x == 0) s_pairs = 0;
+  __syncthreads();
+  const bool light = ctl->stage == kLight;
+  const PullArgs a{t_col, t_w, masks + (size_t)((L - 1) % 3) * n, ctl->bounded ? bounds : nullptr, ctl->stage == kAll};
+  const int lane = lane_id(), wib = threadIdx.x >> 5, grp = lane / kRowLanes;
+  int4* const stage = s_stage[wib];
+  int32_t *const row = s_row[wib], *const head = s_head[wib];
+  unsigned pairs = 0;
+
+  // The in-edges [ks, ke) of one head by the whole warp: the minima, in every
+  // group.  False if no edge is live.
+  auto row_min = [&](int ks, int ke, int32_t y, uint32_t (&mn)[kPullSrc]) {
+#pragma unroll
+    for (int t = 0; t < kPullSrc; t++) mn[t] = 0xffffffffu;
+    bool any = false;
+    for (int kb = ks; kb < ke; kb += 32) {
+      int32_t u = 0, w = 0;
+      const unsigned long long src = kb + lane < ke ? edge_sources<kFloat>(a, kb + lane, y, u, w) : 0ull;
+      const unsigned live = __ballot_sync(kFull, src != 0ull);
+      if (!live) continue;
+      any = true;
+      if (src) stage[__popc(live & lanemask_lt())] = make_int4(u, w, (int)(unsigned)src, (int)(unsigned)(src >> 32));
+      __syncwarp();
+      pull_rows<kFloat>(stage, grp, kRowGroups, __popc(live), D, mn);
+      __syncwarp();
+    }
+    if (any) {
+#pragma unroll
+      for (int off = kRowLanes; off < 32; off <<= 1)
+#pragma unroll
+        for (int t = 0; t < kPullSrc; t++) mn[t] = min(mn[t], __shfl_xor_sync(kFull, mn[t], off));
+    }
+    return any;
+  };
 
   // heavy rows: segment tasks
   for (;;) {
@@ -584,51 +725,124 @@ __global__ void __launch_bounds__(kBlock, 4) mw_pull(const int32_t* __restrict__
       if (__ldg(hv_segoff + mid) <= sidx) lo = mid; else hi = mid - 1;
     }
     const int32_t v = __ldg(hv + lo);
-    const int rbeg = t_row_ptr[v], rend = t_row_ptr[v + 1];
-    const int ks = rbeg + (sidx - __ldg(hv_segoff + lo)) * pull_seg, ke = min(ks + pull_seg, rend);
-    int32_t mn[kPullSrc];
-#pragma unroll
-    for (int t = 0; t < kPullSrc; t++) mn[t] = 0x7fffffff;
-    pull_min(t_col, t_w, m_in, D, fl, ks, ke, stage, mn);
-    const unsigned long long bits = pull_store<true>(D, v, mn);
-    bool first = false;
-    int deg = 0, rs = 0;
-    if (bits && lane == 0) {
-      first = atomicOr(m_out + v, bits) == 0ull;
-      if (first) {
-        rs = row_ptr[v];
-        deg = row_ptr[v + 1] - rs;
-        my_mf += (unsigned long long)deg;
-      }
+    const int ks = __ldg(t_row_ptr + v) + (sidx - __ldg(hv_segoff + lo)) * pull_seg;
+    const int ke = min(ks + pull_seg, light ? __ldg(t_light + v) : __ldg(t_row_ptr + v + 1));
+    const int32_t y = a.bounds ? __ldg(&a.bounds[v].y) : 0;
+    uint32_t mn[kPullSrc];
+    if (!row_min(ks, ke, y, mn)) continue;
+    const unsigned long long m = group_mask(grp == 0 ? pull_lower<true>(D, v, mn) : 0u);
+    if (lane == 0 && m) {
+      atomicOr(m_out + v, m);
+      pairs += __popcll(m);
     }
-    emit_routed(first, v, deg, rs, wq, sout, lpack);
   }
 
-  // light rows: 32 list entries per warp task, one vertex after another
+  // light rows: 32 list entries per warp task
   for (;;) {
     int base = 0;
     if (lane == 0) base = atomicAdd(&ctl->work, 32);
     base = __shfl_sync(kFull, base, 0);
     if (base >= ul_n) break;
-    const int cnt = min(32, ul_n - base);
-    const int32_t mine = lane < cnt ? __ldg(ul + base + lane) : -1;
-    for (int j = 0; j < cnt; j++) {
-      const int32_t v = __shfl_sync(kFull, mine, j);
-      const int k0 = t_row_ptr[v], k1 = t_row_ptr[v + 1];
-      int32_t mn[kPullSrc];
-#pragma unroll
-      for (int t = 0; t < kPullSrc; t++) mn[t] = 0x7fffffff;
-      pull_min(t_col, t_w, m_in, D, fl, k0, k1, stage, mn);
-      const unsigned long long bits = pull_store<false>(D, v, mn);
-      int deg = 0, rs = 0;
-      if (bits) {
-        if (lane == 0) m_out[v] = bits;
-        rs = row_ptr[v];
-        deg = row_ptr[v + 1] - rs;
-        if (lane == 0) my_mf += (unsigned long long)deg;
-      }
-      emit_routed(bits != 0ull && lane == 0, v, deg, rs, wq, sout, lpack);
+    int32_t v = 0, k0 = 0, k1 = 0, y = 0;
+    if (base + lane < ul_n) {
+      v = __ldg(ul + base + lane);
+      k0 = __ldg(t_row_ptr + v);
+      k1 = light ? __ldg(t_light + v) : __ldg(t_row_ptr + v + 1);
+      if (a.bounds) y = __ldg(&a.bounds[v].y);
     }
+    if (whole_rows) {
+      for (int j = 0; j < min(32, ul_n - base); j++) {
+        const int32_t hvx = __shfl_sync(kFull, v, j);
+        uint32_t mn[kPullSrc];
+        if (!row_min(__shfl_sync(kFull, k0, j), __shfl_sync(kFull, k1, j), __shfl_sync(kFull, y, j), mn)) continue;
+        const unsigned long long m = group_mask(grp == 0 ? pull_lower<false>(D, hvx, mn) : 0u);
+        if (lane == 0 && m) {
+          m_out[hvx] = m;
+          pairs += __popcll(m);
+        }
+      }
+      continue;
+    }
+    const RowChunk ch(k0, k1 - k0);
+    int cnt = 0;  // staged edges
+    // the staged edges, a head vertex per group
+    auto flush = [&]() {
+      __syncwarp();
+      const int r = lane < cnt ? row[lane] : -1;
+      const int before = __shfl_up_sync(kFull, r, 1);
+      const unsigned heads = __ballot_sync(kFull, lane < cnt && (lane == 0 || r != before));
+      const int nh = __popc(heads);
+      if ((heads >> lane) & 1u) head[__popc(heads & lanemask_lt())] = lane;
+      if (lane == 0) head[nh] = cnt;
+      __syncwarp();
+      for (int j0 = 0; j0 < nh;) {
+        // a head per group, or two or four groups per head when few are left
+        const int split = nh - j0 >= 3 ? 1 : nh - j0 == 2 ? kRowGroups / 2 : kRowGroups;
+        const int j = j0 + grp / split, part = grp % split;
+        j0 += kRowGroups / split;
+        const int e0 = j < nh ? head[j] : 0, e1 = j < nh ? head[j + 1] : 0;
+        const int32_t hvx = __shfl_sync(kFull, v, j < nh ? row[e0] : 0);
+        uint32_t mn[kPullSrc];
+#pragma unroll
+        for (int t = 0; t < kPullSrc; t++) mn[t] = 0xffffffffu;
+        pull_rows<kFloat>(stage, e0 + part, split, e1, D, mn);
+        for (int off = kRowLanes; off < kRowLanes * split; off <<= 1)
+#pragma unroll
+          for (int t = 0; t < kPullSrc; t++) mn[t] = min(mn[t], __shfl_xor_sync(kFull, mn[t], off));
+        const unsigned imp = j < nh && part == 0 ? pull_lower<false>(D, hvx, mn) : 0u;
+        const unsigned long long m = group_mask(imp);
+        if (lane % kRowLanes == 0 && m) {
+          atomicOr(m_out + hvx, m);
+          pairs += __popcll(m);
+        }
+      }
+      __syncwarp();
+      cnt = 0;
+    };
+    for (int f0 = 0; f0 < ch.total; f0 += 32) {
+      const int f = f0 + lane;
+      const int q = ch.row(f);
+      const int32_t k = __shfl_sync(kFull, ch.ks, q) + f - __shfl_sync(kFull, ch.off, q);
+      const int32_t yq = __shfl_sync(kFull, y, q);
+      int32_t u = 0, w = 0;
+      const unsigned long long src = f < ch.total ? edge_sources<kFloat>(a, k, yq, u, w) : 0ull;
+      const unsigned live = __ballot_sync(kFull, src != 0ull);
+      if (!live) continue;
+      if (cnt + __popc(live) > 32) flush();
+      if (src) {
+        const int at = cnt + __popc(live & lanemask_lt());
+        stage[at] = make_int4(u, w, (int)(unsigned)src, (int)(unsigned)(src >> 32));
+        row[at] = q;
+      }
+      cnt += __popc(live);
+    }
+    if (cnt) flush();
+  }
+  pairs = __reduce_add_sync(kFull, pairs);
+  if (lane == 0 && pairs) atomicAdd(&s_pairs, (unsigned long long)pairs);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_pairs) atomicAdd(&ctl->pairs, s_pairs);
+}
+
+// The frontier that a pull leaves, from its masks: the queue, the segments and
+// the out-edges.  Light pulls need none.
+__global__ void __launch_bounds__(kBlock) mw_collect(const int32_t* __restrict__ row_ptr, MwCtl* __restrict__ ctl,
+                                                     const unsigned long long* __restrict__ masks,
+                                                     int32_t* __restrict__ q, Seg* __restrict__ segs, size_t segcap,
+                                                     int32_t n) {
+  __shared__ int32_t s_q[kBlock / 32][kWarpQueue];
+  if (ctl->done || ctl->mode != kModePull || ctl->stage == kLight) return;
+  const int pout = ctl->level & 1, lane = lane_id(), wib = threadIdx.x >> 5;
+  const unsigned long long* m_out = masks + (size_t)(ctl->level % 3) * n;
+  WarpQueue wq(s_q[wib], q + (size_t)pout * n, &ctl->qsize[pout]);
+  unsigned long long my_mf = 0;
+  for (int v0 = global_warp() * 32; v0 < n; v0 += num_warps() * 32) {
+    const int v = v0 + lane;
+    const bool in = v < n && __ldcg(m_out + v) != 0ull;
+    if (!__any_sync(kFull, in)) continue;
+    const int rs = in ? __ldg(row_ptr + v) : 0, deg = in ? __ldg(row_ptr + v + 1) - rs : 0;
+    my_mf += (unsigned long long)deg;
+    emit_routed(in, v, deg, rs, wq, segs + (size_t)pout * segcap, &ctl->lpack[pout]);
   }
   wq.flush();
   my_mf = warp_sum(my_mf);
@@ -643,15 +857,33 @@ __global__ void mw_decide(MwCtl* __restrict__ ctl, int32_t n, long long m, int c
     return;
   }
   const int L = ctl->level, pout = L & 1;
-  if (ctl->mode == kModePull) ctl->n_pull++; else ctl->n_push++;
-  if ((ctl->qsize[pout] == 0 && ctl->lpack[pout] == 0) || L >= n) {
+  const bool pulled = ctl->mode == kModePull;
+  if (pulled) ctl->n_pull++; else ctl->n_push++;
+  // (light levels come on top of the n that a shortest path can take)
+  if (ctl->stage != kLight && ((ctl->qsize[pout] == 0 && ctl->lpack[pout] == 0) || L >= n + kLightLevels)) {
     ctl->done = 1;
     if (in_graph) cudaGraphSetConditional(loop, 0);
     return;
   }
-  // a frontier whose out-edges reach half the graph is relaxed by a pull
-  if (ctl->force) ctl->mode = ctl->force == 2 ? kModePull : kModePush;
-  else ctl->mode = can_pull && 2 * (long long)ctl->mf[pout] >= m ? kModePull : kModePush;
+  if (ctl->stage == kLight) {
+    // until few pairs improve, and fewer than before (at first only the
+    // sources' neighbours do)
+    const unsigned long long p = ctl->pairs;
+    const int nb = min(kBatch, ctl->nsrc - ctl->batch * kBatch);
+    if ((p * 50 < (unsigned long long)n * nb && p <= ctl->prev_pairs) || L >= kLightLevels) ctl->stage = kAll;
+    ctl->prev_pairs = p;
+  } else {
+    ctl->stage = kRest;
+    // a frontier whose out-edges reach half the graph is relaxed by a pull
+    if (ctl->force) ctl->mode = ctl->force == 2 ? kModePull : kModePush;
+    else ctl->mode = can_pull && 2 * (long long)ctl->mf[pout] >= m ? kModePull : kModePush;
+  }
+  // without a hub bounds tell nothing while most pairs still improve
+  ctl->bounded = ctl->stage == kAll ||
+                 (L + 1 >= kBoundedFrom &&
+                  (ctl->has_hub ||
+                   (pulled && 2 * ctl->pairs < (unsigned long long)n * min(kBatch, ctl->nsrc - ctl->batch * kBatch))));
+  ctl->pairs = 0;
   ctl->work = 0;
   ctl->hwork = 0;
   ctl->qsize[pout ^ 1] = 0;
@@ -783,10 +1015,13 @@ dawn_status sssp_batched(dawn_graph* g, const int32_t* sources, int32_t nsrc, vo
   // pull levels read in-edges with their weights and the in-degree lists
   DAWN_CHECK(build_weighted_in_edges(g));
   DAWN_CHECK(build_static_list(g));
+  DAWN_CHECK(ensure(g->mw_bounds, sizeof(int2) * nn, g->stream));
   DAWN_CUDA(cudaMemcpyAsync(g->mw_sources.p, sources, sizeof(int32_t) * nsrc, cudaMemcpyHostToDevice,
                             g->stream));
   MwCtl c = {};
   c.force = g->force_variant;
+  c.has_hub = g->wt_has_hub;
+  c.has_light = !g->force_variant && g->wt_has_light;
   c.nsrc = nsrc;
   c.dist_base = static_cast<int32_t*>(d_dist);
   c.sources = g->mw_sources.as<int32_t>();
@@ -805,9 +1040,15 @@ dawn_status sssp_batched(dawn_graph* g, const int32_t* sources, int32_t nsrc, vo
     cudaGraphConditionalHandle handle;
     int in_graph;
     const int32_t *t_row_ptr, *t_col, *t_w, *ul, *hv, *hv_segoff;
-    int32_t ul_n, hv_count, hv_segs, pull_seg, can_pull;
+    int32_t ul_n, hv_count, hv_segs, pull_seg, can_pull, hub, whole_rows;
+    const int32_t* t_light;
+    int2* bounds;
     long long m;
   } a;
+  a.t_light = g->wt_light.as<int32_t>();
+  a.bounds = g->mw_bounds.as<int2>();
+  a.hub = g->wt_hub;
+  a.whole_rows = !g->wt_has_hub;
   a.t_row_ptr = g->t_row_ptr;
   a.t_col = g->wt_col.as<int32_t>();
   a.t_w = g->wt_val.as<int32_t>();  // int32 weights or float32 bit patterns, in in-edge order
@@ -840,9 +1081,10 @@ dawn_status sssp_batched(dawn_graph* g, const int32_t* sources, int32_t nsrc, vo
   void* init_args[] = {&a.ctl, &a.row_ptr, &a.col, &a.w, &a.D, &a.masks, &a.q, &a.segs};
   void* push_args[] = {&a.row_ptr, &a.col, &a.w, &a.is_float, &a.ctl, &a.D, &a.masks, &a.q, &a.segs, &a.segcap,
                        &a.n};
-  void* pull_args[] = {&a.row_ptr, &a.t_row_ptr, &a.t_col, &a.t_w, &a.is_float, &a.ctl, &a.D, &a.masks, &a.q,
-                       &a.segs, &a.segcap, &a.ul, &a.ul_n, &a.hv, &a.hv_segoff, &a.hv_count, &a.hv_segs,
-                       &a.pull_seg, &a.n};
+  void* bounds_args[] = {&a.ctl, &a.D, &a.masks, &a.inf, &a.hub, &a.n, &a.bounds};
+  void* pull_args[] = {&a.t_row_ptr, &a.t_light, &a.t_col, &a.t_w, &a.ctl, &a.D, &a.masks, &a.bounds,
+                       &a.ul, &a.ul_n, &a.hv, &a.hv_segoff, &a.hv_count, &a.hv_segs, &a.pull_seg, &a.whole_rows, &a.n};
+  void* collect_args[] = {&a.row_ptr, &a.ctl, &a.masks, &a.q, &a.segs, &a.segcap, &a.n};
   void* decide_args[] = {&a.ctl, &a.n, &a.m, &a.can_pull, &a.handle, &a.in_graph};
   void* emit_args[] = {&a.ctl, &a.D, &a.row_ptr, &a.inf, &a.n};
   void* next_args[] = {&a.ctl};
@@ -851,14 +1093,17 @@ dawn_status sssp_batched(dawn_graph* g, const int32_t* sources, int32_t nsrc, vo
   fam.npre = 2;
   fam.pre[0] = {(const void*)mw_clear, clear_args, dim3(sms * 8), dim3(kBlock), "mw_clear"};
   fam.pre[1] = {(const void*)mw_init, init_args, dim3(kBatch), dim3(kInitBlock), "mw_init"};
-  fam.nbody = 3;
+  const void* const bounds = is_float ? (const void*)mw_bounds<true> : (const void*)mw_bounds<false>;
+  const void* const pull = is_float ? (const void*)mw_pull<true> : (const void*)mw_pull<false>;
+  fam.nbody = 5;
   fam.body[0] = {(const void*)mw_push, push_args,
                  dim3(persistent_blocks((const void*)mw_push, kBlock, 0, g->blocks_per_sm)), dim3(kBlock),
                  "mw_push", kModePush};
-  fam.body[1] = {(const void*)mw_pull, pull_args,
-                 dim3(persistent_blocks((const void*)mw_pull, kBlock, 0, g->blocks_per_sm)), dim3(kBlock),
+  fam.body[1] = {bounds, bounds_args, dim3(sms * 8), dim3(kBlock), "mw_bounds", kModePull};
+  fam.body[2] = {pull, pull_args, dim3(persistent_blocks(pull, kBlock, 0, g->blocks_per_sm)), dim3(kBlock),
                  "mw_pull", kModePull};
-  fam.body[2] = {(const void*)mw_decide, decide_args, dim3(1), dim3(32), "mw_decide"};
+  fam.body[3] = {(const void*)mw_collect, collect_args, dim3(sms * 4), dim3(kBlock), "mw_collect", kModePull};
+  fam.body[4] = {(const void*)mw_decide, decide_args, dim3(1), dim3(32), "mw_decide"};
   fam.npost = 2;
   fam.post[0] = {(const void*)mw_emit<kBatch>, emit_args, dim3(sms * 8), dim3(kEmitBlock), "mw_emit"};
   fam.post[1] = {(const void*)mw_next, next_args, dim3(1), dim3(32), "mw_next"};

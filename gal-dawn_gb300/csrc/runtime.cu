@@ -2,6 +2,7 @@
 // that runs a single-source traversal as one conditional CUDA graph per
 // source, CSR validation, in-edge (transpose) construction and the exact
 // closeness reductions.
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 #include <utility>
@@ -548,47 +549,108 @@ __global__ void scatter_in_edges(const int32_t* __restrict__ rp, const int32_t* 
   }
 }
 
-__global__ void init_cursor(const int32_t* __restrict__ t_row_ptr, unsigned long long* __restrict__ cursor,
-                            int32_t n) {
+// Where a row's light entries go (from its start up) and its others (from its
+// end down).
+__global__ void init_cursors(const int32_t* __restrict__ t_row_ptr, int2* __restrict__ cursor, int32_t n) {
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)n; i += stride)
-    cursor[i] = (unsigned long long)t_row_ptr[i];
+    cursor[i] = make_int2(t_row_ptr[i], t_row_ptr[i + 1]);
+}
+
+// The light entries' end of every row, and the vertex of most in-edges.
+__global__ void finish_weighted_in_edges(const int32_t* __restrict__ t_row_ptr, const int2* __restrict__ cursor,
+                                         int32_t n, int32_t* __restrict__ light, unsigned long long* __restrict__ hub) {
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  unsigned long long best = 0;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)n; i += stride) {
+    light[i] = cursor[i].x;
+    const unsigned long long x = (unsigned long long)(t_row_ptr[i + 1] - t_row_ptr[i]) << 32 | (unsigned)i;
+    best = x > best ? x : best;
+  }
+#pragma unroll
+  for (int d = 16; d; d >>= 1) {
+    const unsigned long long x = __shfl_xor_sync(kFull, best, d);
+    best = x > best ? x : best;
+  }
+  if ((threadIdx.x & 31) == 0 && best) atomicMax(hub, best);
 }
 
 __global__ void scatter_weighted_in_edges(const int32_t* __restrict__ rp, const int32_t* __restrict__ col,
-                                          const int32_t* __restrict__ val, int32_t n,
-                                          unsigned long long* __restrict__ cursor, int32_t* __restrict__ t_col,
+                                          const int32_t* __restrict__ val, int32_t n, uint32_t most,
+                                          int2* __restrict__ cursor, int32_t* __restrict__ t_col,
                                           int32_t* __restrict__ t_val) {
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
   for (int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n; u += warps) {
     const int e = rp[u + 1];
     for (int k = rp[u] + lane; k < e; k += 32) {
-      const unsigned long long slot = atomicAdd(cursor + col[k], 1ull);
+      const int32_t w = val[k];
+      int2* const c = cursor + col[k];
+      const int slot = (uint32_t)w <= most ? atomicAdd(&c->x, 1) : atomicSub(&c->y, 1) - 1;
       t_col[slot] = u;
-      t_val[slot] = val[k];
+      t_val[slot] = w;
     }
   }
 }
 
+__global__ void sample_weights(const int32_t* __restrict__ val, long long m, int samples, int32_t* __restrict__ out) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < samples; i += gridDim.x * blockDim.x)
+    out[i] = val[(long long)i * m / samples];
+}
+
 }  // namespace
 
+// In-edges with their weights, a row's light entries first: about three a vertex
+// by a sample of the weights (an eighth to a half of them), for the batched
+// traversal, which reaches most of its distances through these alone.  No row
+// has light entries of its own where the weights do not tell them apart.
 dawn_status build_weighted_in_edges(dawn_graph* g) {
   if (g->wt_col.p) return DAWN_OK;
   const int32_t n = g->n;
   const cudaStream_t s = g->stream;
-  unsigned long long* cursor = nullptr;
-  DAWN_CHECK(pool_alloc((void**)&cursor, sizeof(unsigned long long) * ((size_t)n + 1), s));
-  DAWN_CHECK(ensure(g->wt_col, sizeof(int32_t) * (size_t)(g->m > 0 ? g->m : 1) + 16, s));
-  DAWN_CHECK(ensure(g->wt_val, sizeof(int32_t) * (size_t)(g->m > 0 ? g->m : 1) + 16, s));
   const int grid = g->geo.sms * 8;
-  init_cursor<<<grid, kBlock, 0, s>>>(g->t_row_ptr, cursor, n);
+  constexpr int kSamples = 4096;
+  constexpr double kHubDegree = 16.0;  // in mean degrees
+  int2* cursor = nullptr;
+  unsigned long long* hub = nullptr;
+  int32_t* sample = nullptr;
+  DAWN_CHECK(pool_alloc((void**)&cursor, sizeof(int2) * (size_t)n + sizeof(unsigned long long) + 4 * kSamples, s));
+  hub = reinterpret_cast<unsigned long long*>(cursor + n);
+  sample = reinterpret_cast<int32_t*>(hub + 1);
+  DAWN_CUDA(cudaMemsetAsync(hub, 0, sizeof(*hub), s));
+  std::vector<uint32_t> w((size_t)std::min<int64_t>(g->m, kSamples));
+  uint32_t most = 0;
+  g->wt_has_light = false;
+  if (!w.empty()) {
+    sample_weights<<<16, kBlock, 0, s>>>(static_cast<const int32_t*>(g->val), g->m, (int)w.size(), sample);
+    DAWN_CUDA(cudaGetLastError());
+    DAWN_CUDA(cudaMemcpyAsync(w.data(), sample, 4 * w.size(), cudaMemcpyDeviceToHost, s));
+    DAWN_CUDA(cudaStreamSynchronize(s));
+    const double share = std::min(0.5, std::max(0.125, 3.0 * n / (double)g->m));
+    std::sort(w.begin(), w.end());
+    most = w[(size_t)(share * (double)(w.size() - 1))];
+    const size_t cnt = (size_t)(std::upper_bound(w.begin(), w.end(), most) - w.begin());
+    g->wt_has_light = (double)cnt <= 0.6 * (double)w.size();
+  }
+  DAWN_CHECK(ensure(g->wt_light, sizeof(int32_t) * (size_t)n, s));
+  DAWN_CHECK(ensure(g->wt_val, sizeof(int32_t) * (size_t)(g->m > 0 ? g->m : 1) + 16, s));
+  DAWN_CHECK(ensure(g->wt_col, sizeof(int32_t) * (size_t)(g->m > 0 ? g->m : 1) + 16, s));
+  init_cursors<<<grid, kBlock, 0, s>>>(g->t_row_ptr, cursor, n);
   DAWN_CUDA(cudaGetLastError());
-  // 32-bit weights (int32 or float32 bit patterns) move as words
-  scatter_weighted_in_edges<<<grid, kBlock, 0, s>>>(g->row_ptr, g->col, static_cast<const int32_t*>(g->val), n,
+  // 32-bit weights (int32 or float32 bit patterns, not negative) move as words
+  scatter_weighted_in_edges<<<grid, kBlock, 0, s>>>(g->row_ptr, g->col, static_cast<const int32_t*>(g->val), n, most,
                                                     cursor, g->wt_col.as<int32_t>(), g->wt_val.as<int32_t>());
   DAWN_CUDA(cudaGetLastError());
+  finish_weighted_in_edges<<<g->geo.sms * 4, kBlock, 0, s>>>(g->t_row_ptr, cursor, n, g->wt_light.as<int32_t>(), hub);
+  DAWN_CUDA(cudaGetLastError());
+  unsigned long long h = 0;
+  DAWN_CUDA(cudaMemcpyAsync(&h, hub, sizeof(h), cudaMemcpyDeviceToHost, s));
   pool_free(cursor, s);
+  DAWN_CUDA(cudaStreamSynchronize(s));
+  g->wt_hub = (int32_t)(uint32_t)h;
+  // without a hub the bounds leave too much for a light stage to pay
+  g->wt_has_hub = (double)(h >> 32) * n >= kHubDegree * (double)g->m;
+  g->wt_has_light = g->wt_has_light && g->wt_has_hub;
   return DAWN_OK;
 }
 
