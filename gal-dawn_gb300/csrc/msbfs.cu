@@ -455,13 +455,15 @@ __device__ __forceinline__ void init_batch(const BsArgs& a) {
     atomicOr(fr0 + (size_t)s * W + (b >> 6), bit);
     rs = row_ptr[s];
     deg = row_ptr[s + 1] - rs;
-    atomicAdd(&s_reached, (u64)deg);
     // A source without out-edges reaches no vertex but itself.  Its bit is
     // left out of `full`, so the other vertices still finish (and leave
     // the pull lists) once every other source has reached them; a batch
     // of all vertices as sources holds many such sources.
     if (deg == 0) atomicAnd(&ctl->full[b >> 6], ~bit);
   }
+  // (64-bit sums in shared memory are compare-and-swap loops: one per warp)
+  const u64 reached = warp_sum((u64)deg);
+  if (lane_id() == 0 && reached) atomicAdd(&s_reached, reached);
   __syncthreads();
   // A vertex that is the source of several bits is queued once, by the
   // thread of its lowest bit.
@@ -474,10 +476,13 @@ __device__ __forceinline__ void init_batch(const BsArgs& a) {
       lowest &= (f.w[i] & below) == 0ull;
     }
   }
-  if (lowest) {
-    atomicAdd(&s_mf, (u64)deg);
-    if (Bits<W>::ldcg(visit + (size_t)s * W) == Bits<W>::full_of(ctl))
-      atomicAdd(&s_dec, (u64)(t_row_ptr[s + 1] - t_row_ptr[s]));
+  u64 dec = 0;
+  if (lowest && Bits<W>::ldcg(visit + (size_t)s * W) == Bits<W>::full_of(ctl)) dec = (u64)(t_row_ptr[s + 1] - t_row_ptr[s]);
+  const u64 mf = warp_sum(lowest ? (u64)deg : 0ull);
+  dec = warp_sum(dec);
+  if (lane_id() == 0) {
+    if (mf) atomicAdd(&s_mf, mf);
+    if (dec) atomicAdd(&s_dec, dec);
   }
   if (b < per) emit_routed(lowest, s, deg, rs, aq0, &ctl->aq_size[0], segs0, &ctl->alpack[0]);  // whole warps
   __syncthreads();
@@ -989,43 +994,43 @@ __device__ __forceinline__ void emit_vertex(int32_t* __restrict__ dist, int32_t 
 // fifth slice adds its bit separately; an unreached pair becomes -1 by
 // OR-ing (bit - 1).  About 8 instructions per (source, vertex) instead of
 // 19 with a shift and mask per slice.
+// One word i and its bytes c0 .. c1 - 1 per call: the items of a batch of 256
+// sources are then words, not vertices (RMAT-18 has 65,536 groups of four vertices
+// for 311,000 threads: 500 sources 784 -> 757 us a call).
 template <int W, int NB>
 __device__ __forceinline__ void emit_vertex4_packed(int32_t* __restrict__ dist, int32_t n, int nb_src, size_t u0,
-                                                    const u64* visit, const u64* slices) {
+                                                    const u64* visit, const u64* slices, int i, int c0, int c1) {
+  if (64 * i + 8 * c0 >= nb_src) return;
+  u64 vis[4], w[NB][4];
 #pragma unroll
-  for (int i = 0; i < W; i++) {
-    if (64 * i >= nb_src) break;
-    u64 vis[4], w[NB][4];
+  for (int j = 0; j < 4; j++) {
+    vis[j] = visit[(u0 + j) * W + i];
+#pragma unroll
+    for (int k = 0; k < NB; k++) w[k][j] = slices[((size_t)k * n + u0 + j) * W + i];
+  }
+  const int cnt = min(64, nb_src - 64 * i);
+  int32_t* row0 = dist + (size_t)(64 * i) * n + u0;
+  for (int c = c0; c < c1 && 8 * c < cnt; c++) {
+    uint32_t packed[4], five[4], vb[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      vis[j] = visit[(u0 + j) * W + i];
+      uint32_t x = 0;
 #pragma unroll
-      for (int k = 0; k < NB; k++) w[k][j] = slices[((size_t)k * n + u0 + j) * W + i];
+      for (int k = 0; k < (NB < 4 ? NB : 4); k++) x |= (uint32_t)((w[k][j] >> (8 * c)) & 0xffull) << (8 * k);
+      packed[j] = x;
+      five[j] = NB > 4 ? (uint32_t)(w[NB > 4 ? 4 : 0][j] >> (8 * c)) & 0xffu : 0u;
+      vb[j] = (uint32_t)(vis[j] >> (8 * c)) & 0xffu;
     }
-    const int cnt = min(64, nb_src - 64 * i);
-    int32_t* row0 = dist + (size_t)(64 * i) * n + u0;
-    for (int c = 0; c < 8 && 8 * c < cnt; c++) {
-      uint32_t packed[4], five[4], vb[4];
+    const int lim = min(8, cnt - 8 * c);
+    for (int b = 0; b < lim; b++) {
+      int32_t v[4];
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        uint32_t x = 0;
-#pragma unroll
-        for (int k = 0; k < (NB < 4 ? NB : 4); k++) x |= (uint32_t)((w[k][j] >> (8 * c)) & 0xffull) << (8 * k);
-        packed[j] = x;
-        five[j] = NB > 4 ? (uint32_t)(w[NB > 4 ? 4 : 0][j] >> (8 * c)) & 0xffu : 0u;
-        vb[j] = (uint32_t)(vis[j] >> (8 * c)) & 0xffu;
+        uint32_t x = (((packed[j] >> b) & 0x01010101u) * 0x01020408u) >> 24;
+        if (NB > 4) x |= ((five[j] >> b) & 1u) << 4;
+        v[j] = (int32_t)(x | (((vb[j] >> b) & 1u) - 1u));
       }
-      const int lim = min(8, cnt - 8 * c);
-      for (int b = 0; b < lim; b++) {
-        int32_t v[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          uint32_t x = (((packed[j] >> b) & 0x01010101u) * 0x01020408u) >> 24;
-          if (NB > 4) x |= ((five[j] >> b) & 1u) << 4;
-          v[j] = (int32_t)(x | (((vb[j] >> b) & 1u) - 1u));
-        }
-        *reinterpret_cast<int4*>(row0 + (size_t)(8 * c + b) * n) = make_int4(v[0], v[1], v[2], v[3]);
-      }
+      *reinterpret_cast<int4*>(row0 + (size_t)(8 * c + b) * n) = make_int4(v[0], v[1], v[2], v[3]);
     }
   }
 }
@@ -1089,10 +1094,14 @@ __device__ __forceinline__ void emit_vertex4(int32_t* __restrict__ dist, int32_t
 // consecutive vertices so lane j holds bit j (and j + 32) of all of them and
 // counts them with popc; CTA totals go to the batch's rows with one atomic
 // per source.
+// CTAs per SM of the closeness pass: each adds two words per source to the same
+// 512 (closeness of 1,000 sources on RMAT-18, 1 / 2 / 4 / 8: 1603 / 1571 / 1584 /
+// 1610 us, 1717 with eight and 64-bit sums in shared memory).
+constexpr int kClosenessCtas = 2;
 template <int W>
 __device__ __forceinline__ void emit_closeness(const Team& tm, const BsCtl* ctl, int batch, const u64* visit,
                                                const u64* slices, int32_t n, int nb, int nbits) {
-  __shared__ unsigned long long s_sum[64 * W], s_cnt[64 * W];
+  __shared__ uint32_t s_sum[64 * W], s_cnt[64 * W];  // a CTA's vertices x 31 levels fit
   for (int t = threadIdx.x; t < 64 * W; t += blockDim.x) {
     s_sum[t] = 0;
     s_cnt[t] = 0;
@@ -1121,20 +1130,20 @@ __device__ __forceinline__ void emit_closeness(const Team& tm, const BsCtl* ctl,
         sum_hi += (unsigned long long)__popc(warp_transpose32((uint32_t)(x[k] >> 32))) << k;
       }
     }
-    if (cnt_lo | sum_lo) {
-      atomicAdd(&s_cnt[64 * i + lane], (unsigned long long)cnt_lo);
-      atomicAdd(&s_sum[64 * i + lane], sum_lo);
+    if (cnt_lo) {
+      atomicAdd(&s_cnt[64 * i + lane], cnt_lo);
+      atomicAdd(&s_sum[64 * i + lane], (uint32_t)sum_lo);
     }
-    if (cnt_hi | sum_hi) {
-      atomicAdd(&s_cnt[64 * i + 32 + lane], (unsigned long long)cnt_hi);
-      atomicAdd(&s_sum[64 * i + 32 + lane], sum_hi);
+    if (cnt_hi) {
+      atomicAdd(&s_cnt[64 * i + 32 + lane], cnt_hi);
+      atomicAdd(&s_sum[64 * i + 32 + lane], (uint32_t)sum_hi);
     }
   }
   __syncthreads();
   const size_t row0 = (size_t)batch * 64 * W;
   for (int t = threadIdx.x; t < nb; t += blockDim.x) {
-    if (s_sum[t]) atomicAdd(ctl->cc_sum + row0 + t, s_sum[t]);
-    if (s_cnt[t]) atomicAdd(ctl->cc_cnt + row0 + t, s_cnt[t]);
+    if (s_sum[t]) atomicAdd(ctl->cc_sum + row0 + t, (unsigned long long)s_sum[t]);
+    if (s_cnt[t]) atomicAdd(ctl->cc_cnt + row0 + t, (unsigned long long)s_cnt[t]);
   }
 }
 
@@ -1256,13 +1265,19 @@ __device__ __forceinline__ void emit_batch(const BsArgs& a, const Team& tm) {
   int32_t* dist = ctl->dist_base + (size_t)batch * per * n;
   const size_t t0 = tm.thread(), stride = tm.threads();
   if ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(dist) & 15) == 0 && !src) {
-    for (size_t q = t0; q < (size_t)n / 4; q += stride) {
+    const size_t quads = (size_t)n / 4;
+    int split = 1;  // of a word's bytes, while threads are idle
+    while (split < 8 && quads * W * split < stride) split *= 2;
+    const int bytes = 8 / split;
+    for (size_t t = t0; t < quads * W * split; t += stride) {
+      const size_t part = t / quads, u0 = 4 * (t - part * quads);
+      const int i = (int)part / split, c0 = ((int)part % split) * bytes, c1 = c0 + bytes;
       switch (nbits) {
-        case 1: emit_vertex4_packed<W, 1>(dist, n, nb, 4 * q, visit, slices); break;
-        case 2: emit_vertex4_packed<W, 2>(dist, n, nb, 4 * q, visit, slices); break;
-        case 3: emit_vertex4_packed<W, 3>(dist, n, nb, 4 * q, visit, slices); break;
-        case 4: emit_vertex4_packed<W, 4>(dist, n, nb, 4 * q, visit, slices); break;
-        default: emit_vertex4_packed<W, 5>(dist, n, nb, 4 * q, visit, slices); break;
+        case 1: emit_vertex4_packed<W, 1>(dist, n, nb, u0, visit, slices, i, c0, c1); break;
+        case 2: emit_vertex4_packed<W, 2>(dist, n, nb, u0, visit, slices, i, c0, c1); break;
+        case 3: emit_vertex4_packed<W, 3>(dist, n, nb, u0, visit, slices, i, c0, c1); break;
+        case 4: emit_vertex4_packed<W, 4>(dist, n, nb, u0, visit, slices, i, c0, c1); break;
+        default: emit_vertex4_packed<W, 5>(dist, n, nb, u0, visit, slices, i, c0, c1); break;
       }
     }
     return;
@@ -1855,6 +1870,7 @@ dawn_status run_width(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32
   const int nbatches = (nsrc + 64 * W - 1) / (64 * W);
   void* args[] = {&a};
   const int sms = g->geo.sms;
+  const int emit_ctas = cc_sum ? sms * kClosenessCtas : sms * 8;
   SsFamily fam;
   if (g->l2_persist) {
     // the three rotating frontier slots: every pull level gathers from one
@@ -1870,7 +1886,7 @@ dawn_status run_width(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32
     const int ctas = want < full ? (int)want : full;
     for (a.batch = 0; a.batch < nbatches; a.batch++) {
       DAWN_CHECK(launch_cooperative(fam, fn, ctas, threads, args, g->stream));
-      DAWN_CUDA(cudaLaunchKernel((const void*)bs_emit_dist<W>, dim3(sms * 8), dim3(kBlock), args, 0, g->stream));
+      DAWN_CUDA(cudaLaunchKernel((const void*)bs_emit_dist<W>, dim3(emit_ctas), dim3(kBlock), args, 0, g->stream));
     }
     return DAWN_OK;
   }
@@ -1886,7 +1902,7 @@ dawn_status run_width(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32
        dim3(persistent_blocks((const void*)bs_push_update<W>, kBlock, 0, g->blocks_per_sm)), dim3(kBlock),
        "bs_push_update", kModePush},
       {(const void*)bs_decide, args, dim3(1), dim3(32), "bs_decide"},
-      {(const void*)bs_emit_dist<W>, args, dim3(sms * 8), dim3(kBlock), "bs_emit_dist"},
+      {(const void*)bs_emit_dist<W>, args, dim3(emit_ctas), dim3(kBlock), "bs_emit_dist"},
       {(const void*)bs_next, args, dim3(1), dim3(32), "bs_next"}};
   fam.npre = 2;
   fam.nbody = 4;

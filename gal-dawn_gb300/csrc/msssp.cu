@@ -34,7 +34,11 @@
 //     of them on RMAT-22): shortest paths run along these, and once the light
 //     edges have settled, one pull over all edges, with every reached pair
 //     taken as improved, leaves out nine tenths of them by the bounds.  RMAT-22
-//     x 64 reads 0.9 m rows so, against 4 m in four whole pulls;
+//     x 64 reads 0.9 m rows so, against 4 m in four whole pulls.  Per call of 64
+//     sources, whole pulls -> this: RMAT-22 19.9 -> 8.1 ms, RMAT-20 6.4 -> 2.9,
+//     RMAT-20 (edge factor 6) 5.1 -> 2.8, RMAT-17 (32) 2.9 -> 1.3; Erdos-Renyi
+//     (no hub: no light stage, bounds once fewer than half of the pairs still
+//     improve) 300,000 vertices 4.8 -> 4.2, 1 M 12.4 -> 12.5;
 //   * a final pass transposes the block into the caller's source-major rows
 //     and counts the reached edges.
 // Each source's first frontier is resolved as the single-source path does
@@ -528,6 +532,9 @@ __global__ void __launch_bounds__(kBlock) mw_bounds(const MwCtl* __restrict__ ct
 // 1.0 ms a pull against 1.6) and the worse for the handful that bounds and the
 // light stage leave (RMAT-20 x 64: 2.94 ms a batch, 6.39 with whole rows, by the
 // masks alone and without a light stage).
+// Eight sources per lane and three rows per group in flight: 64 registers, four
+// CTAs per SM (two sources per lane, and tails passed by shuffles, took 30% longer
+// in whole pulls, four rows per group at three CTAs 9%).
 constexpr int kPullSrc = 8;                 // sources per lane (4 or 8)
 constexpr int kPullUnroll = 3;              // rows per lane group fetched together
 constexpr int kRowLanes = kBatch / kPullSrc;  // lanes reading one tail row
