@@ -1326,15 +1326,6 @@ __global__ void __launch_bounds__(kMesh ? 1024 : 640, kMesh ? 1 : 2) bfs_travers
   }
 }
 
-__global__ void __launch_bounds__(kBlock) max_degree(const int32_t* __restrict__ row_ptr, int32_t n,
-                                                     int32_t* __restrict__ out) {
-  int deg = 0;
-  for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-    deg = max(deg, row_ptr[v + 1] - row_ptr[v]);
-  deg = __reduce_max_sync(kFull, deg);
-  if (lane_id() == 0 && deg) atomicMax(out, deg);
-}
-
 __global__ void __launch_bounds__(kBlock) fill_records(const int32_t* __restrict__ row_ptr,
                                                        const int32_t* __restrict__ col, int32_t n, int32_t len,
                                                        int32_t* __restrict__ rec) {
@@ -1357,15 +1348,8 @@ dawn_status records(dawn_graph* g) {
   if (g->rec_len != -1) return DAWN_OK;
   int32_t len = 0;
   if (g->m <= 12 * (int64_t)g->n && g->n > kSoloKeep) {
-    int32_t* d = nullptr;
-    DAWN_CHECK(pool_alloc((void**)&d, sizeof(int32_t), g->stream));
-    DAWN_CUDA(cudaMemsetAsync(d, 0, sizeof(int32_t), g->stream));
-    max_degree<<<g->geo.sms * 4, kBlock, 0, g->stream>>>(g->row_ptr, g->n, d);
-    DAWN_CUDA(cudaGetLastError());
-    int32_t deg = 0;
-    DAWN_CUDA(cudaMemcpyAsync(&deg, d, sizeof(int32_t), cudaMemcpyDeviceToHost, g->stream));
-    pool_free(d, g->stream);
-    DAWN_CUDA(cudaStreamSynchronize(g->stream));
+    DAWN_CHECK(longest_row(g));
+    const int32_t deg = g->max_row;
     len = std::max(8, (deg + 7) / 8 * 8);
     if (deg > kRecMax) {
       len = 0;

@@ -200,6 +200,7 @@ struct dawn_graph {
   const void* bfs_fn = nullptr;    // the persistent kernel that bfs_ctas and the kernel's limits were set for
   int32_t bfs_ctas = 0, bfs_cap = 0;
   dawn::DevBuf bfs_rec;     // rows of low degree as records (single-source BFS)
+  int32_t max_row = -1;     // entries of the longest row (-1: not read yet)
   int32_t rec_len = -1;     // words of a record; 0: none, -1: not decided, -2: level kernels instead
   dawn::DevBuf bfs_sync;    // BfsSync: what the CTAs of the persistent BFS wait on
   dawn::DevBuf ss_sources;  // int32 source list of the current call
@@ -378,6 +379,8 @@ dawn_status ss_run(dawn_graph* g, SsFamily& fam, int32_t nsrc,
                    cudaGraphExec_t* exec_cache);
 // Traced form of a family's runs: its kernels one by one, timed.
 dawn_status ss_run_traced(dawn_graph* g, SsFamily& fam, int32_t nruns);
+// Sets max_row, once per handle.
+dawn_status longest_row(dawn_graph* g);
 // A kernel whose CTAs wait for each other, with the family's L2 window if it
 // has one.
 dawn_status launch_cooperative(const SsFamily& fam, const void* fn, int ctas, int threads, void** args,

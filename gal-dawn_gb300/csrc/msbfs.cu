@@ -949,6 +949,71 @@ __device__ __forceinline__ void update_level(const BsArgs& a, const Team& tm, co
   if (lazy && tm.thread() == 0) ctl->unlisted[L % 3] = 1;
 }
 
+// Both phases of a list-mode push at once, for one-word batches in the persistent
+// launch: an edge's bits are claimed in the visited words, and whoever claims a
+// bit records its level and puts it in the frontier (the first one queues the
+// vertex).  Each bit has one claimer, so nothing is written twice.  One step
+// instead of two for the thin levels of meshes and of any graph's first and last
+// levels, which are bound by the chain of round trips of a step, not by the
+// returning atomics that this takes.  Two phases -> this, us a call: grid 700 x 700
+// 23080 -> 15380 (64 sources), 20720 -> 13080 (3); kNN of 75,331 points 3760 ->
+// 3540, 3780 -> 2450; Erdos-Renyi 65,536 x 16 126 -> 118 (64).
+template <int kWarps>
+__device__ __forceinline__ void push_level(const BsArgs& a, const Team& tm, const BsStep& st, BsSmem<kWarps>& sm) {
+  BsCtl* const ctl = a.ctl;
+  const int32_t* __restrict__ row_ptr = a.row_ptr;
+  const int32_t* __restrict__ col = a.col;
+  const int32_t n = a.n;
+  const int L = st.L;
+  const u64* fin = a.fr + (size_t)((L - 1) % 3) * n;
+  u64* fout = a.fr + (size_t)(L % 3) * n;
+  Seg* seg_out = a.segs + (size_t)(L % 3) * a.segcap;
+  clear_stale<1>(tm, a.fr + (size_t)((L + 1) % 3) * n, n, a.aq + (size_t)((L + 1) % 3) * n, st.stale,
+                 a.segs + (size_t)((L + 1) % 3) * a.segcap, st.stale_segs, st.stale_unlisted != 0);
+  clear_next_slice<1>(tm, a.slices, n, L, a.nbits);
+  const int wib = threadIdx.x >> 5;
+  int32_t* const deal = sm.q[wib] + kWarpQueueBig;
+  const u64 full = ctl->full[0];
+  WarpQueueBig wq(sm.q[wib], a.aq + (size_t)(L % 3) * n, &ctl->aq_size[L % 3]);
+  LevelAcc acc;
+  const bool deep_cc = a.cc_sum && L >= kDeepLevel;
+  if (deep_cc) clear_deep_sums<1>(sm.deep);
+  auto op = [&](int32_t v, int k, bool valid) {
+    bool first = false;
+    int32_t u = -1;
+    int ors = 0, odeg = 0;
+    Bits<1> nw = Bits<1>::zero();
+    if (valid) {
+      u = __ldg(col + k);
+      const u64 bits = Bits<1>::gather(fin + v).w[0] & ~__ldcg(a.visit + u);
+      if (bits) {
+        const u64 old = atomicOr(a.visit + u, bits);
+        ors = __ldg(row_ptr + u);
+        odeg = __ldg(row_ptr + u + 1) - ors;
+        nw.w[0] = bits & ~old;
+        if (nw.w[0]) {
+          first = atomicOr(fout + u, nw.w[0]) == 0ull;
+          if (L < kDeepLevel) {
+            for (unsigned l = (unsigned)L; l; l &= l - 1) atomicOr(a.slices + (size_t)(__ffs(l) - 1) * n + u, nw.w[0]);
+          } else {
+            record_level<1>(a, u, nw, L);
+          }
+          acc.reached += (u64)odeg * (u64)nw.popc();
+          if (first) acc.mf += (u64)odeg;
+          if ((old | bits) == full) acc.dec += (u64)(__ldg(a.t_row_ptr + u + 1) - __ldg(a.t_row_ptr + u));
+        }
+      }
+    }
+    if (deep_cc) add_deep_sums<1>(sm.deep, nw, L);
+    emit_routed(first, u, odeg, ors, wq, seg_out, &ctl->alpack[L % 3]);
+  };
+  seg_expand<true>(tm.warp(), tm.warps(), row_ptr, a.segs + (size_t)((L - 1) % 3) * a.segcap, st.ln, op);
+  warp_expand<true>(tm.warp(), tm.warps(), row_ptr, a.aq + (size_t)((L - 1) % 3) * n, st.qn, deal, deal + 32, deal + 64,
+                    op);
+  end_level(sm, ctl, L % 3, acc, wq, nullptr, 0, &ctl->aq_size[L % 3]);
+  if (deep_cc) flush_deep_sums<1>(a, sm.deep);
+}
+
 // Expands the level slices of one batch into its distance rows: thread per
 // vertex, one store per source, consecutive vertices per warp (full lines).
 // NB is the number of level bits in use (<= kShallowBits).  src is the
@@ -1305,7 +1370,8 @@ __device__ __forceinline__ void emit_batch(const BsArgs& a, const Team& tm) {
   }
 }
 
-enum : int32_t { kBsClear = 0, kBsInit, kBsScatter, kBsUpdate, kBsPull };
+// (kBsPush: both phases of a push)
+enum : int32_t { kBsClear = 0, kBsInit, kBsScatter, kBsUpdate, kBsPull, kBsPush };
 
 // One warp.  Ends the batch when the frontier is empty, otherwise picks
 // the next level's variant: the forced one if set, else the learned
@@ -1511,7 +1577,7 @@ __device__ __forceinline__ int bs_ctas(int work, int warps) {
 // arrived and the rest only poll.  Turns st into the next phase; returns false
 // when the batch is done.
 // Not inlined: its registers would be the levels' spills.
-template <int kWarps>
+template <bool kThin, int kWarps>
 __device__ __noinline__ bool next_phase(const BsArgs& a, BsStep& step) {
   BsStep st = step;
   BsCtl* const ctl = a.ctl;
@@ -1535,7 +1601,7 @@ __device__ __noinline__ bool next_phase(const BsArgs& a, BsStep& step) {
     __threadfence();
     st = read_step(a);
     st.arrived = arrived;
-    st.phase = vc->mode == kModePush ? kBsScatter : kBsPull;
+    st.phase = vc->mode != kModePush ? kBsPull : kThin && !st.dense ? kBsPush : kBsScatter;
     st.ctas = (int)gridDim.x;
     step = st;
     return true;
@@ -1544,6 +1610,7 @@ __device__ __noinline__ bool next_phase(const BsArgs& a, BsStep& step) {
     if (lane_id() == 0) count_batch(ctl);
     return false;
   }
+  if (kThin && st.phase == kBsScatter && !st.dense) st.phase = kBsPush;
   st.ctas = st.ctas ? bs_ctas(st.ctas, kWarps) : (int)gridDim.x;
   step = st;
   return true;
@@ -1598,7 +1665,10 @@ __device__ __forceinline__ BsStep unpack_step(const u64* w) {
 //   RMAT-22, 64 sources                        1176 -> 1128
 //   grid 700 x 700, 64 sources                26060 -> 22050
 //   kNN, 200,000 vertices, 64 sources         16050 -> 7450
-template <int W>
+// kThin: list-mode pushes as one phase (push_level), for graphs whose rows are all
+// short.  A kernel of its own: beside it the pull loses registers, and 3 to 7% on
+// RMAT graphs, whose thin levels are few.
+template <int W, bool kThin = false>
 __global__ void __launch_bounds__(W == 1 ? 640 : 512, 2) bs_traverse(const __grid_constant__ BsArgs a) {
   constexpr int kWarps = (W == 1 ? 640 : 512) / 32;
   __shared__ BsSmem<kWarps> sm;
@@ -1621,6 +1691,9 @@ __global__ void __launch_bounds__(W == 1 ? 640 : 512, 2) bs_traverse(const __gri
       case kBsInit: init_batch<W>(a); break;
       case kBsScatter: scatter_level<W>(a, tm, st, sm); break;
       case kBsUpdate: update_level<W>(a, tm, st, sm); break;
+      case kBsPush:
+        if constexpr (kThin) push_level(a, tm, st, sm);
+        break;
       default: pull_level<W>(a, tm, st, sm);
     }
     __syncthreads();
@@ -1637,7 +1710,7 @@ __global__ void __launch_bounds__(W == 1 ? 640 : 512, 2) bs_traverse(const __gri
           sm.next.arrived = st.arrived + (uint32_t)st.ctas;
         }
         __syncwarp();
-        const bool more = next_phase<kWarps>(a, sm.next);
+        const bool more = next_phase<kThin, kWarps>(a, sm.next);
         __syncwarp();
         if (!more && lane == 0) sm.next.ctas = 0;
         const u64 tag = (u64)((gen + 1) & 0xffffu) << 48;
@@ -1879,6 +1952,10 @@ dawn_status run_width(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32
   }
   if (!g->trace) {
     const void* fn = (const void*)bs_traverse<W>;
+    if constexpr (W == 1) {
+      DAWN_CHECK(longest_row(g));
+      if (g->max_row < kLongRow) fn = (const void*)bs_traverse<1, true>;
+    }
     const int threads = W == 1 ? 640 : 512;
     // a small graph takes few CTAs: each adds to the arrivals of its phases
     const int64_t want = ((int64_t)n + g->m) / kBsEntries + 1;

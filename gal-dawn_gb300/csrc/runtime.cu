@@ -458,6 +458,36 @@ dawn_status validate_csr(dawn_graph* g) {
   return DAWN_OK;
 }
 
+// --- longest row --------------------------------------------------------------
+
+namespace {
+
+__global__ void __launch_bounds__(kBlock) max_degree(const int32_t* __restrict__ row_ptr, int32_t n,
+                                                     int32_t* __restrict__ out) {
+  int deg = 0;
+  for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+    deg = max(deg, row_ptr[v + 1] - row_ptr[v]);
+  deg = __reduce_max_sync(kFull, deg);
+  if (lane_id() == 0 && deg) atomicMax(out, deg);
+}
+
+}  // namespace
+
+dawn_status longest_row(dawn_graph* g) {
+  if (g->max_row >= 0) return DAWN_OK;
+  int32_t* d = nullptr;
+  int32_t deg = 0;
+  DAWN_CHECK(pool_alloc((void**)&d, sizeof(int32_t), g->stream));
+  DAWN_CUDA(cudaMemsetAsync(d, 0, sizeof(int32_t), g->stream));
+  max_degree<<<g->geo.sms * 4, kBlock, 0, g->stream>>>(g->row_ptr, g->n, d);
+  DAWN_CUDA(cudaGetLastError());
+  DAWN_CUDA(cudaMemcpyAsync(&deg, d, sizeof(int32_t), cudaMemcpyDeviceToHost, g->stream));
+  pool_free(d, g->stream);
+  DAWN_CUDA(cudaStreamSynchronize(g->stream));
+  g->max_row = deg;
+  return DAWN_OK;
+}
+
 // --- exclusive scan (int64), used for the in-edge CSR ---------------------------
 
 namespace {
