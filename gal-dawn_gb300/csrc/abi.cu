@@ -139,7 +139,7 @@ void destroy(dawn_graph* g) {
                     &g->dist_stage, &g->pt_voff, &g->pt_ctl, &g->pt_scratch, &g->pt_small, &g->pt_tcol, &g->pt_toff, &g->pt_rows,
                     &g->sel_slot, &g->nf_ctl, &g->nf_queue, &g->nf_segbuf, &g->nf_masks, &g->wt_col, &g->wt_val, &g->wt_light, &g->mw_bounds, &g->mw_block, &g->mw_masks,
                     &g->mw_ctl, &g->mw_sources, &g->bc_levels, &g->bc_terms, &g->bc_range, &g->bc_out,
-                    &g->bc_heavy, &g->bc_part, &g->bc_acc};
+                    &g->bc_heavy, &g->bc_part, &g->bc_acc, &g->bc_pairs};
   for (DevBuf* b : bufs) dawn::release(*b);
   if (g->stream) cudaStreamSynchronize(g->stream);
   if (g->bfs_exec) cudaGraphExecDestroy(g->bfs_exec);

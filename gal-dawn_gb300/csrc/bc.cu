@@ -29,7 +29,8 @@
 // level rows (256 bytes an edge too) beside every term row the passes of a
 // block took 580 us, now 200 (of three blocks together); the sweep of the widest
 // level moves 0.7 sectors per SM clock, near what L1/TEX gathers reach.  Batches
-// of kDeepLevel levels and more have no such words: they keep the level rows.
+// of kDeepLevel levels and more have no such words: they have level rows, and on
+// graphs of short rows go by pairs (bc_pairs).
 // Rows of at least kHeavy entries (the hubs of power-law graphs) would keep
 // one warp busy for thousands of dependent row loads while the rest of the
 // grid idles, so they are cut into kBcSeg-entry segments, each a warp task
@@ -386,6 +387,174 @@ __global__ void __launch_bounds__(kBlock) bc_fold(const double* __restrict__ acc
   }
 }
 
+// --- deeper batches on short rows: (vertex, source) pairs by level ------------------
+//
+// On a mesh a vertex is at 40 levels for 64 sources, and a sweep over vertices
+// reads 512 bytes an edge for the one source or two that are at its level: 44 us a
+// level on a kNN graph of 50,000 points.  Here the pairs are sorted by level
+// once, and a lane takes one pair and walks its row, eight bytes an edge.  The
+// additions are those of the level rows: along a row, one after another.  Rows
+// of kHeavy entries and more would hold a lane too long, so graphs with one keep
+// the level rows.  Per call, sweeps over vertices -> pairs: kNN of 50,000 points, 60
+// sources 8.2 -> 4.5 ms, of 3,000 points, 200 sources 4.6 -> 2.2, grid 150 x 150,
+// 60 sources 6.5 -> 4.4.
+
+constexpr int kPairLevels = 4096;  // levels counted in shared memory
+
+// Counts the pairs of every level (kPlace false), or puts pair ids (vertex x 64 +
+// source) in their level's part of the list, where cursor[l] stands (kPlace).
+// Level 0 is left out.
+template <bool kPlace>
+__global__ void __launch_bounds__(kBlock) bc_pairs(const int32_t* __restrict__ L, size_t quads, int levels,
+                                                   uint32_t* __restrict__ cursor, uint32_t* __restrict__ list) {
+  __shared__ uint32_t cnt[kPairLevels];
+  const bool local = levels <= kPairLevels;
+  const size_t per = (quads + gridDim.x - 1) / gridDim.x, q0 = blockIdx.x * per, q1 = min(q0 + per, quads);
+  if (local) {
+    for (int l = threadIdx.x; l < levels; l += kBlock) cnt[l] = 0;
+    __syncthreads();
+    for (size_t q = q0 + threadIdx.x; q < q1; q += kBlock) {
+      const int4 x = __ldg(reinterpret_cast<const int4*>(L) + q);
+      if (x.x > 0) atomicAdd(cnt + x.x, 1u);
+      if (x.y > 0) atomicAdd(cnt + x.y, 1u);
+      if (x.z > 0) atomicAdd(cnt + x.z, 1u);
+      if (x.w > 0) atomicAdd(cnt + x.w, 1u);
+    }
+    __syncthreads();
+    for (int l = threadIdx.x; l < levels; l += kBlock)
+      if (cnt[l]) cnt[l] = atomicAdd(cursor + l, cnt[l]);
+    if (!kPlace) return;
+    __syncthreads();
+  }
+  uint32_t* const at = local ? cnt : cursor;
+  for (size_t q = q0 + threadIdx.x; q < q1; q += kBlock) {
+    const int4 x = __ldg(reinterpret_cast<const int4*>(L) + q);
+    const int32_t l[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      if (l[i] > 0) {
+        const uint32_t pos = atomicAdd(at + l[i], 1u);
+        if (kPlace) list[pos] = (uint32_t)(4 * q + i);
+      }
+  }
+}
+
+// Counts to first positions: off[l], and the same in cursor for the placing.  One
+// CTA.
+__global__ void __launch_bounds__(1024) bc_pair_offsets(uint32_t* __restrict__ cursor, uint32_t* __restrict__ off,
+                                                        int levels) {
+  __shared__ uint32_t warp_tot[32];
+  __shared__ uint32_t base;
+  if (threadIdx.x == 0) base = 0;
+  const int lane = lane_id(), w = threadIdx.x >> 5;
+  for (int l0 = 0; l0 <= levels; l0 += 1024) {
+    const int l = l0 + threadIdx.x;
+    const uint32_t x = l < levels ? cursor[l] : 0u;
+    const uint32_t incl = (uint32_t)warp_incl_scan((int)x);
+    __syncthreads();
+    if (lane == 31) warp_tot[w] = incl;
+    __syncthreads();
+    if (w == 0) warp_tot[lane] = (uint32_t)warp_incl_scan((int)warp_tot[lane]);
+    __syncthreads();
+    const uint32_t first = base + (w ? warp_tot[w - 1] : 0u) + incl - x;
+    if (l <= levels) off[l] = first;
+    if (l < levels) cursor[l] = first;
+    __syncthreads();
+    if (threadIdx.x == 0) base += warp_tot[31];
+  }
+}
+
+// 1 / amount of the pairs at level 2 and deeper.
+__global__ void __launch_bounds__(kBlock) bc_pair_amounts(const int32_t* __restrict__ t_row_ptr,
+                                                          const int32_t* __restrict__ t_col,
+                                                          const int32_t* __restrict__ L, float* __restrict__ T,
+                                                          const uint32_t* __restrict__ list,
+                                                          const uint32_t* __restrict__ off, int levels) {
+  const size_t stride = (size_t)gridDim.x * kBlock;
+  for (size_t i = off[2] + blockIdx.x * (size_t)kBlock + threadIdx.x; i < off[levels]; i += stride) {
+    const uint32_t p = list[i], src = p & 63u;
+    const int l = L[p], ke = __ldg(t_row_ptr + (p >> 6) + 1);
+    int amount = 0;
+    for (int k = __ldg(t_row_ptr + (p >> 6)); k < ke; k += kUnroll) {
+      int32_t x[kUnroll];
+#pragma unroll
+      for (int j = 0; j < kUnroll; j++) x[j] = k + j < ke ? __ldg(L + (size_t)__ldg(t_col + k + j) * kLanes + src) : -2;
+#pragma unroll
+      for (int j = 0; j < kUnroll; j++) amount += x[j] == l - 1;
+    }
+    T[p] = amount ? 1.0f / (float)amount : 0.0f;
+  }
+}
+
+// Level l of the backward sweep.
+__global__ void __launch_bounds__(kBlock) bc_pair_sweep(const int32_t* __restrict__ row_ptr,
+                                                        const int32_t* __restrict__ col,
+                                                        const int32_t* __restrict__ L, float* __restrict__ T,
+                                                        float* __restrict__ delta, const uint32_t* __restrict__ list,
+                                                        const uint32_t* __restrict__ off, int level) {
+  const size_t stride = (size_t)gridDim.x * kBlock, end = off[level + 1];
+  for (size_t i = off[level] + blockIdx.x * (size_t)kBlock + threadIdx.x; i < end; i += stride) {
+    const uint32_t p = list[i], src = p & 63u;
+    const int ke = __ldg(row_ptr + (p >> 6) + 1);
+    const float own = level > 1 ? __ldcg(T + p) : 0.0f;
+    float sum = 0.0f;
+    for (int k = __ldg(row_ptr + (p >> 6)); k < ke; k += kUnroll) {
+      int32_t x[kUnroll];
+      float t[kUnroll];
+#pragma unroll
+      for (int j = 0; j < kUnroll; j++) {
+        const size_t c = k + j < ke ? (size_t)__ldg(col + k + j) * kLanes + src : 0;
+        x[j] = k + j < ke ? __ldg(L + c) : -2;
+        t[j] = k + j < ke ? __ldcg(T + c) : 0.0f;
+      }
+#pragma unroll
+      for (int j = 0; j < kUnroll; j++)
+        if (x[j] == level + 1) sum += t[j];
+    }
+    delta[p] = sum;
+    if (level > 1) T[p] = own + sum;
+  }
+}
+
+// The vertices' betweenness from the block: half a warp per vertex.
+__global__ void __launch_bounds__(kBlock) bc_pair_sums(const int32_t* __restrict__ L, const float* __restrict__ delta,
+                                                       double* __restrict__ bc, int32_t n, int levels) {
+  const int lane = lane_id(), sub = lane & 15;
+  for (int v0 = global_warp() * 2; v0 < n; v0 += num_warps() * 2) {
+    const int v = v0 + (lane >> 4);
+    double sum = 0.0;
+    if (v < n) {
+      const int4 l = __ldg(reinterpret_cast<const int4*>(L + (size_t)v * kLanes) + sub);
+      const float4 d = __ldg(reinterpret_cast<const float4*>(delta + (size_t)v * kLanes) + sub);
+      // pairs at level 1 to the last but one have a delta
+      if (l.x > 0 && l.x < levels - 1) sum += (double)d.x;
+      if (l.y > 0 && l.y < levels - 1) sum += (double)d.y;
+      if (l.z > 0 && l.z < levels - 1) sum += (double)d.z;
+      if (l.w > 0 && l.w < levels - 1) sum += (double)d.w;
+    }
+#pragma unroll
+    for (int k = 8; k; k >>= 1) sum += __shfl_xor_sync(kFull, sum, k);
+    if (sub == 0 && v < n && sum != 0.0) bc[v] += sum;
+  }
+}
+
+// The passes of one deep block of 64 sources whose deepest level is deepest.
+void pair_passes(dawn_graph* g, const int32_t* L, float* T, double* out, int deepest) {
+  const size_t nn = (size_t)g->n;
+  const int levels = deepest + 1, sms = g->geo.sms;
+  uint32_t* const list = g->bc_pairs.as<uint32_t>();
+  float* const delta = reinterpret_cast<float*>(list + kLanes * nn);
+  uint32_t *const off = list + 2 * kLanes * nn, *const cursor = off + nn + 2;
+  cudaMemsetAsync(cursor, 0, sizeof(uint32_t) * (size_t)levels, g->stream);
+  bc_pairs<false><<<sms * 4, kBlock, 0, g->stream>>>(L, 16 * nn, levels, cursor, nullptr);
+  bc_pair_offsets<<<1, 1024, 0, g->stream>>>(cursor, off, levels);
+  bc_pairs<true><<<sms * 4, kBlock, 0, g->stream>>>(L, 16 * nn, levels, cursor, list);
+  if (levels > 2) bc_pair_amounts<<<sms * 8, kBlock, 0, g->stream>>>(g->t_row_ptr, g->t_col, L, T, list, off, levels);
+  for (int l = deepest - 1; l >= 1; l--)
+    bc_pair_sweep<<<sms, kBlock, 0, g->stream>>>(g->row_ptr, g->col, L, T, delta, list, off, l);
+  bc_pair_sums<<<sms * 8, kBlock, 0, g->stream>>>(L, delta, out, g->n, levels);
+}
+
 // --- deeper batches: level rows -----------------------------------------------------
 
 // Per lane, the entries j -> c in [ks, ke) whose level row holds la - 1
@@ -641,6 +810,7 @@ dawn_status reserve(dawn_graph* g, int blocks) {
 dawn_status betweenness(dawn_graph* g, const int32_t* sources, int32_t nsrc, double* d_bc, dawn_stats* st) {
   const size_t nn = (size_t)g->n;
   DAWN_CHECK(prepare_heavy(g));
+  DAWN_CHECK(longest_row(g));
   // Batches of up to 256 sources: RMAT-16, 150 sources, takes 810 us in one and
   // took 1150 in three of 64.  A block of 64 takes about 0.9 KB a vertex and 5 bytes an
   // edge, so large graphs take fewer at a time, and so do devices with little
@@ -728,9 +898,20 @@ dawn_status betweenness(dawn_graph* g, const int32_t* sources, int32_t nsrc, dou
       for (int32_t l = end[0] - 2; l >= 1; l--)
         bc_sweep<<<grid, kBlock, 0, g->stream>>>(g->row_ptr, g->col, M, T, acc, g->n, l, per, hout, part, done_out);
     } else {
+      // pair ids are 32-bit, and the lists are scratch that large graphs may not get
+      bool pairs = g->max_row < kHeavy && nn < (size_t)1 << 25;
+      if (pairs && ensure(g->bc_pairs, sizeof(uint32_t) * (2 * kLanes + 2) * (nn + 2), g->stream) != DAWN_OK) {
+        cudaGetLastError();
+        clear_error();
+        pairs = false;
+      }
       for (int32_t i = 0; i < k; i++) {
         const int32_t *const L = Ls[p] + i * kLanes * nn, *const R = Rs[p] + i * 2 * nn;
         double* const out = acc + i * nn;
+        if (pairs) {
+          pair_passes(g, L, T, out, end[2 + i]);
+          continue;
+        }
         bc_rows_amount<<<ctas, kBlock, 0, g->stream>>>(g->t_row_ptr, g->t_col, L, T, g->n, hin, cnt);
         if (hin.count) bc_rows_amount_heavy<<<ctas, kBlock, 0, g->stream>>>(L, T, hin, cnt);
         for (int32_t l = end[2 + i] - 1; l >= 1; l--) {

@@ -212,6 +212,7 @@ struct dawn_graph {
   dawn::DevBuf bc_acc;      // likewise, n double: the betweenness from these sources
   dawn::DevBuf bc_out;      // n double (host-pointer calls)
   dawn::DevBuf bc_heavy;    // rows cut into segments: out-rows (ids, segment prefix), in-rows (same)
+  dawn::DevBuf bc_pairs;    // deep batches: pairs by level, their deltas, level offsets and cursors
   dawn::DevBuf bc_part;     // per 64 sources of a batch: per-segment partial sums (float), per-heavy-row
                             // counts (int32), 64 each, and segments finished per heavy row
   int32_t bc_hout = -1, bc_segs_out = 0, bc_hin = 0, bc_segs_in = 0;  // -1: lists not built
