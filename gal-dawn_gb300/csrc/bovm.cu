@@ -520,7 +520,9 @@ __device__ __forceinline__ bool frontier_bit(const uint32_t* bm, int32_t u) {
 
 // Bottom-up level: a warp owns 32 vertices (one bitmap word); each
 // unvisited one scans its in-edges until a frontier bit.
-// The bounds of the next 32 rows load while these are scanned.  A lane tests
+// While 32 rows are scanned, the first columns of the next 32 load and the bounds
+// of the 32 after (from DRAM on RMAT-22: the pull is a chain of such loads, 21
+// times per warp at its widest level).  A lane tests
 // its row's first two columns, where most rows end once the frontier is large,
 // then reads eight (one sector) at a time.  The last few lanes' rows are swept
 // by the whole warp, so that one long row without a hit does not hold it.
@@ -546,31 +548,42 @@ __device__ __forceinline__ void pull_level(const Team& tm, const int32_t* __rest
   WarpQueueBig wq(sm.q[threadIdx.x >> 5], q + (size_t)pout * n, &ctl->qsize[pout]);
   LongQueue wl{sm.lq[threadIdx.x >> 5], kSegs ? nullptr : lq + (size_t)pout * lcap, lpack};
   const int stride = tm.warps();
-  uint32_t vis_n = ~0u;
-  int k_n = 0, e_n = 0;
-  auto prefetch = [&](int w) {
-    vis_n = ~0u;
-    k_n = e_n = 0;
+  uint32_t vis_a = ~0u, vis_b = ~0u;
+  int k_a = 0, e_a = 0, k_b = 0, e_b = 0;  // rows to scan: empty where the vertex is visited
+  int32_t c0_b = -1, c1_b = -1;
+  auto load_bounds = [&](int w) {
+    vis_a = ~0u;
+    k_a = e_a = 0;
     if (w < nwords) {
-      vis_n = __ldcg(vbm + w);
+      vis_a = __ldcg(vbm + w);
       const int32_t u = w * 32 + lane;
       if (u < n) {
-        k_n = __ldg(t_row_ptr + u);
-        e_n = __ldg(t_row_ptr + u + 1);
+        k_a = __ldg(t_row_ptr + u);
+        e_a = __ldg(t_row_ptr + u + 1);
       }
     }
   };
-  prefetch(tm.warp());
+  auto load_columns = [&]() {
+    vis_b = vis_a;
+    k_b = k_a;
+    e_b = (vis_a >> lane) & 1u ? k_a : e_a;
+    c0_b = k_b < e_b ? __ldg(t_col + k_b) : -1;
+    c1_b = k_b + 1 < e_b ? __ldg(t_col + k_b + 1) : -1;
+  };
+  load_bounds(tm.warp());
+  load_columns();
+  load_bounds(tm.warp() + stride);
   for (int w = tm.warp(); w < nwords; w += stride) {
-    const uint32_t vis = vis_n;
-    const int k0 = k_n, e = (vis >> lane) & 1u ? k_n : e_n;  // an empty row: nothing to do
-    prefetch(w + stride);
+    const uint32_t vis = vis_b;
+    const int k0 = k_b, e = e_b;
+    const int32_t c0 = c0_b, c1 = c1_b;
+    load_columns();
+    load_bounds(w + 2 * stride);
     if (__all_sync(kFull, k0 == e)) continue;
     const int32_t u = w * 32 + lane;
     int k = k0;
     bool found = false;
     {
-      const int32_t c0 = k < e ? __ldg(t_col + k) : -1, c1 = k + 1 < e ? __ldg(t_col + k + 1) : -1;
       const bool h0 = c0 >= 0 && frontier_bit(fin, c0), h1 = c1 >= 0 && frontier_bit(fin, c1);
       found = h0 || h1;
       k = found ? e : k + 2;
