@@ -168,6 +168,14 @@ __device__ __forceinline__ uint32_t warp_transpose32(uint32_t x) {
   return x;
 }
 
+// *p |= x without waiting for the old value.  As a reduction by name: beside an
+// atomicOr whose result is used, the compiler makes one returning atomic of both
+// (the dense scatter of RMAT-22 then takes 224 us, not 164; a call for 500 sources
+// on RMAT-18 763, not 720).
+__device__ __forceinline__ void or_word(u64* p, u64 x) {
+  asm volatile("red.relaxed.gpu.global.or.b64 [%0], %1;" ::"l"(p), "l"(x) : "memory");
+}
+
 // W words of one vertex.
 template <int W>
 struct Bits {
@@ -861,7 +869,7 @@ __device__ __forceinline__ void scatter_level(const BsArgs& a, const Team& tm, c
         } else {
 #pragma unroll
           for (int i = 0; i < W; i++)
-            if (bits.w[i]) atomicOr(nxt + (size_t)u * W + i, bits.w[i]);
+            if (bits.w[i]) or_word(nxt + (size_t)u * W + i, bits.w[i]);
           if (!dense) first = claim_bit(tbm, u);
         }
       }
