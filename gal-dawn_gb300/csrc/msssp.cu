@@ -30,13 +30,13 @@
 //     relative to a hub's distances, which the sources' distances follow
 //     closely.  An edge whose tail's lowest plus its weight is no less than its
 //     head's highest cannot improve any of the 64;
-//   * and the batch starts with pulls along the light in-edges alone (an eighth
-//     of them on RMAT-22): shortest paths run along these, and once the light
+//   * and a batch's second level on are pulls along the light in-edges alone (an
+//     eighth of them on RMAT-22): shortest paths run along these, and once the light
 //     edges have settled, one pull over all edges, with every reached pair
 //     taken as improved, leaves out nine tenths of them by the bounds.  RMAT-22
 //     x 64 reads 0.9 m rows so, against 4 m in four whole pulls.  Per call of 64
-//     sources, whole pulls -> this: RMAT-22 19.9 -> 8.1 ms, RMAT-20 6.4 -> 2.9,
-//     RMAT-20 (edge factor 6) 5.1 -> 2.8, RMAT-17 (32) 2.9 -> 1.3; Erdos-Renyi
+//     sources, whole pulls -> this: RMAT-22 19.9 -> 8.1 ms, RMAT-20 6.4 -> 2.8,
+//     RMAT-20 (edge factor 6) 5.1 -> 2.7, RMAT-17 (32) 2.9 -> 1.3; Erdos-Renyi
 //     (no hub: no light stage, bounds once fewer than half of the pairs still
 //     improve) 300,000 vertices 4.8 -> 4.2, 1 M 12.4 -> 12.5;
 //   * a final pass transposes the block into the caller's source-major rows
@@ -69,7 +69,7 @@ struct MwCtl {
   int32_t work, hwork;          // pull: dynamic work counters (light rows, heavy-row segments)
   int32_t n_pull;
   int32_t n_push, inits;       // inits: mw_init CTAs finished
-  int32_t has_light;           // the batch starts with pulls along light edges
+  int32_t has_light;           // levels 2 and on begin with pulls along light edges
   int32_t stage;               // of a pull: kLight, kAll or kRest
   int32_t bounded;             // the pull goes by mw_bounds
   int32_t has_hub;
@@ -106,8 +106,8 @@ __global__ void __launch_bounds__(kBlock) mw_clear(MwCtl* __restrict__ ctl, int3
     ctl->n_push = 0;
     ctl->n_pull = 0;
     ctl->inits = 0;
-    ctl->stage = ctl->has_light ? kLight : kRest;
-    ctl->mode = ctl->force == 2 || ctl->has_light ? kModePull : kModePush;
+    ctl->stage = kRest;
+    ctl->mode = ctl->force == 2 ? kModePull : kModePush;
     ctl->bounded = 0;
     ctl->pairs = ctl->prev_pairs = 0;
     ctl->work = 0;
@@ -879,6 +879,15 @@ __global__ void mw_decide(MwCtl* __restrict__ ctl, int32_t n, long long m, int c
     const int nb = min(kBatch, ctl->nsrc - ctl->batch * kBatch);
     if ((p * 50 < (unsigned long long)n * nb && p <= ctl->prev_pairs) || L >= kLightLevels) ctl->stage = kAll;
     ctl->prev_pairs = p;
+  } else if (L == 1 && ctl->has_light) {
+    // The first level pushed every edge: a source whose neighbours have no light
+    // edges would otherwise not start before the pull over all edges, and then
+    // take such pulls of its own.  Light pulls from the first level -> this, by
+    // the sources drawn: with such a source, RMAT-22 16.3 -> 8.7 ms, RMAT-20
+    // (edge factor 6) 4.4 -> 2.7, RMAT-18 2.9 -> 1.45; with none, RMAT-22 8.01 ->
+    // 8.06, RMAT-20 2.89 -> 2.82 (33 sources 2.35 -> 2.42), RMAT-18 1.39 -> 1.42.
+    ctl->stage = kLight;
+    ctl->mode = kModePull;
   } else {
     ctl->stage = kRest;
     // a frontier whose out-edges reach half the graph is relaxed by a pull
