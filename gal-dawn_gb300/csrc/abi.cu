@@ -73,7 +73,10 @@ dawn_status check_sources(const dawn_graph* g, const int32_t* sources, int32_t n
 }
 
 dawn_status finish_graph(dawn_graph* g, uint32_t flags) {
-  if (!(flags & DAWN_GRAPH_NO_VALIDATE)) DAWN_CHECK(dawn::validate_csr(g));
+  if (!(flags & DAWN_GRAPH_NO_VALIDATE))
+    DAWN_CHECK(dawn::validate_csr(g));
+  else
+    DAWN_CHECK(dawn::read_weight_signs(g));
   if (g->symmetric) {
     g->t_row_ptr = g->row_ptr;
     g->t_col = g->col;

@@ -188,6 +188,7 @@ struct dawn_graph {
   int32_t* row_ptr = nullptr;
   int32_t* col = nullptr;
   void* val = nullptr;
+  bool negative_weights = false;  // (unvalidated handles) some: distances may fall below zero, and without end
   int32_t* t_row_ptr = nullptr;
   int32_t* t_col = nullptr;
 
@@ -409,7 +410,10 @@ dawn_status row_reduce(dawn_graph* g, const void* d_dist, int32_t nsrc,
                        const int32_t* d_sources, int kind, int degree,
                        double* d_sum, long long* d_cnt);
 const char* last_error();
+// Both leave 0.0 for -0.0 in the handle's weights; the second, for handles that
+// are not validated, sets negative_weights.
 dawn_status validate_csr(dawn_graph* g);
+dawn_status read_weight_signs(dawn_graph* g);
 dawn_status exclusive_scan_i64(const int64_t* d_in, int64_t* d_out, int64_t n,
                                cudaStream_t s);
 

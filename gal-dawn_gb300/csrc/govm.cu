@@ -409,7 +409,9 @@ dawn_status sssp_ordered(dawn_graph* g, const int32_t* sources, int32_t nsrc, vo
 dawn_status sssp_single(dawn_graph* g, const int32_t* sources, int32_t nsrc, void* d_dist) {
   const int32_t n = g->n;
   const int32_t nwords = (n + 31) / 32;
-  if (!g->force_variant && !g->trace) return sssp_ordered(g, sources, nsrc, d_dist);
+  // (below zero the ordered form's unsigned comparisons are wrong, and a cycle
+  // would keep it going: the levels compare signed and stop after n)
+  if (!g->force_variant && !g->trace && !g->negative_weights) return sssp_ordered(g, sources, nsrc, d_dist);
   DAWN_CHECK(ensure(g->ss_queues, sizeof(int32_t) * 2 * (size_t)n, g->stream));
   size_t segcap = seg_capacity(n, g->m);
   DAWN_CHECK(ensure(g->ss_segs, sizeof(Seg) * 2 * segcap, g->stream));

@@ -867,7 +867,7 @@ __global__ void mw_decide(MwCtl* __restrict__ ctl, int32_t n, long long m, int c
   const bool pulled = ctl->mode == kModePull;
   if (pulled) ctl->n_pull++; else ctl->n_push++;
   // (light levels come on top of the n that a shortest path can take)
-  if (ctl->stage != kLight && ((ctl->qsize[pout] == 0 && ctl->lpack[pout] == 0) || L >= n + kLightLevels)) {
+  if (ctl->stage != kLight && ((ctl->qsize[pout] == 0 && ctl->lpack[pout] == 0) || L >= n + (ctl->has_light ? kLightLevels : 0))) {
     ctl->done = 1;
     if (in_graph) cudaGraphSetConditional(loop, 0);
     return;
@@ -1019,7 +1019,7 @@ dawn_status sssp_batched(dawn_graph* g, const int32_t* sources, int32_t nsrc, vo
   const size_t nn = (size_t)n;
   const int is_float = g->wtype == DAWN_W_F32;
   bool ordered = false;
-  if (!g->force_variant && !g->trace) DAWN_CHECK(nearfar_batch_fits(g, nsrc, &ordered));
+  if (!g->force_variant && !g->trace && !g->negative_weights) DAWN_CHECK(nearfar_batch_fits(g, nsrc, &ordered));
   if (ordered) return run_ordered(g, sources, nsrc, d_dist);
   const size_t segcap = seg_capacity(n, g->m);
   DAWN_CHECK(ensure(g->mw_block, sizeof(int32_t) * kBatch * nn, g->stream));
@@ -1035,9 +1035,10 @@ dawn_status sssp_batched(dawn_graph* g, const int32_t* sources, int32_t nsrc, vo
   DAWN_CUDA(cudaMemcpyAsync(g->mw_sources.p, sources, sizeof(int32_t) * nsrc, cudaMemcpyHostToDevice,
                             g->stream));
   MwCtl c = {};
-  c.force = g->force_variant;
+  // negative weights: pushes alone, which compare distances as signed words
+  c.force = g->negative_weights ? 1 : g->force_variant;
   c.has_hub = g->wt_has_hub;
-  c.has_light = !g->force_variant && g->wt_has_light;
+  c.has_light = !c.force && g->wt_has_light;
   c.nsrc = nsrc;
   c.dist_base = static_cast<int32_t*>(d_dist);
   c.sources = g->mw_sources.as<int32_t>();

@@ -210,8 +210,14 @@ __device__ __forceinline__ bool nf_control(const NfArgs& a, uint32_t g, uint32_t
     uint32_t delta = __ldcg(&c->far.delta);
     p.t_old = p.T;
     if (p.kind == kPhFar) {
-      // the scan moved nothing: step past the gap
+      // The scan moved nothing: step past the gap.  Every pair left lies above T
+      // and below `inf`, so T rises; a launch in which it does not would never
+      // end.
       p.T = nf_threshold<kFloat>(__ldcg(&c->far.min_far), delta, a.inf);
+      if (p.T <= p.t_old) {
+        *a.err_out = DAWN_ERR_TIMEOUT;
+        return false;
+      }
     } else {
       const uint32_t iters = __ldcg(&c->far.bucket_iters);
       const unsigned long long pairs = __ldcg(&c->far.bucket_pairs);

@@ -3,6 +3,7 @@
 // source, CSR validation, in-edge (transpose) construction and the exact
 // closeness reductions.
 #include <algorithm>
+#include <climits>
 #include <cstring>
 #include <mutex>
 #include <utility>
@@ -398,13 +399,22 @@ dawn_status ss_run(dawn_graph* g, SsFamily& fam, int32_t nruns, cudaGraphExec_t*
 
 namespace {
 
-__device__ __forceinline__ int check_entry(int32_t c, int32_t n, const void* val, int wtype, size_t k) {
+// Weight k of the handle's own copy, as a word; a float -0.0 (what -log(1.0f)
+// gives) becomes 0.0 there first.  The traversals compare distances as words, and
+// its word, 0x80000000, sorts above every distance as unsigned and below them as
+// signed.
+__device__ __forceinline__ int32_t weight_word(int32_t* val, int wtype, size_t k) {
+  const int32_t w = val[k];
+  if (wtype != DAWN_W_F32 || w != INT_MIN) return w;
+  val[k] = 0;
+  return 0;
+}
+
+__device__ __forceinline__ int check_entry(int32_t c, int32_t n, int32_t* val, int wtype, size_t k) {
   int f = (c < 0 || c >= n) ? 8 : 0;
-  if (wtype == DAWN_W_I32 && static_cast<const int32_t*>(val)[k] < 0) f |= 16;
-  if (wtype == DAWN_W_F32) {
-    const float w = static_cast<const float*>(val)[k];
-    if (!(w >= 0.0f) || isinf(w)) f |= 16;
-  }
+  if (wtype == DAWN_W_NONE) return f;
+  const int32_t w = weight_word(val, wtype, k);
+  if (w < 0 || (wtype == DAWN_W_F32 && !isfinite(__int_as_float(w)))) f |= 16;
   return f;
 }
 
@@ -412,7 +422,7 @@ __device__ __forceinline__ int check_entry(int32_t c, int32_t n, const void* val
 // the kernels rely on: monotone row_ptr from 0 to m, columns in [0, n),
 // weights finite and non-negative.
 __global__ void validate_csr_kernel(const int32_t* __restrict__ rp, const int32_t* __restrict__ col,
-                                    const void* __restrict__ val, int wtype, int32_t n, long long m,
+                                    int32_t* __restrict__ val, int wtype, int32_t n, long long m,
                                     int* __restrict__ flags) {
   const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -435,14 +445,37 @@ __global__ void validate_csr_kernel(const int32_t* __restrict__ rp, const int32_
   if (f) atomicOr(flags, f);
 }
 
+// Whether any weight has its sign bit set (-0.0 aside).
+__global__ void weight_signs(int32_t* __restrict__ val, int wtype, long long m, int* __restrict__ flag) {
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  bool neg = false;
+  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < (size_t)m; k += stride)
+    neg |= weight_word(val, wtype, k) < 0;
+  if (neg) atomicOr(flag, 1);
+}
+
 }  // namespace
+
+dawn_status read_weight_signs(dawn_graph* g) {
+  if (g->wtype == DAWN_W_NONE) return DAWN_OK;
+  int *d_flag = nullptr, flag = 0;
+  DAWN_CHECK(pool_alloc((void**)&d_flag, sizeof(int), g->stream));
+  DAWN_CUDA(cudaMemsetAsync(d_flag, 0, sizeof(int), g->stream));
+  weight_signs<<<g->geo.sms * 8, kBlock, 0, g->stream>>>(static_cast<int32_t*>(g->val), g->wtype, g->m, d_flag);
+  DAWN_CUDA(cudaGetLastError());
+  DAWN_CUDA(cudaMemcpyAsync(&flag, d_flag, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
+  pool_free(d_flag, g->stream);
+  DAWN_CUDA(cudaStreamSynchronize(g->stream));
+  g->negative_weights = flag != 0;
+  return DAWN_OK;
+}
 
 dawn_status validate_csr(dawn_graph* g) {
   int* d_flags = nullptr;
   DAWN_CUDA(cudaMallocAsync(&d_flags, sizeof(int), g->stream));
   DAWN_CUDA(cudaMemsetAsync(d_flags, 0, sizeof(int), g->stream));
-  validate_csr_kernel<<<g->geo.sms * 8, kBlock, 0, g->stream>>>(g->row_ptr, g->col, g->val, g->wtype, g->n, g->m,
-                                                                 d_flags);
+  validate_csr_kernel<<<g->geo.sms * 8, kBlock, 0, g->stream>>>(g->row_ptr, g->col, static_cast<int32_t*>(g->val),
+                                                                 g->wtype, g->n, g->m, d_flags);
   DAWN_CUDA(cudaGetLastError());
   int flags = 0;
   DAWN_CUDA(cudaMemcpyAsync(&flags, d_flags, sizeof(int), cudaMemcpyDeviceToHost, g->stream));

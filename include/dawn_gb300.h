@@ -12,6 +12,7 @@
  *   int32 weights  int32 distance, INT32_MAX = unreachable.
  *   float weights  float distance, FLT_MAX = unreachable, as the reference
  *                  (src/algorithm/cpu/sssp.cpp:36).
+ *                  A float weight of -0.0 counts as 0.0.
  *   dist arrays    row-major nsrc x n: row i belongs to sources[i].
  *
  * Threading: a graph handle is not thread safe; calls on one handle are
