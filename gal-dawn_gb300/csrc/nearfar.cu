@@ -664,11 +664,11 @@ __global__ void __launch_bounds__(kNfBlock, 2) nf_traverse(const __grid_constant
           const bool win = k < re && __ldcg(a.D + p) == -(k + 1);
           bool near = false, far = false;
           if (win) {
-            const uint32_t d = u == s ? 0u : (uint32_t)__ldg(a.w + k);
+            const uint32_t d = u == s ? 0u : min((uint32_t)__ldg(a.w + k), a.inf);
             a.D[p] = (int32_t)d;
             if (d <= T)
               near = set_pair(near_out, p);
-            else
+            else if (d < a.inf)  // a weight of `inf` reaches nothing, and no T covers it
               far = set_pair(far_mask, p);
           }
           emit_near(near, p);

@@ -1,7 +1,9 @@
-"""Float weights of -0.0 (what -log(1.0f) gives) count as 0.0 in every weighted
+"""Weights whose words need care.  Float weights of -0.0 (what -log(1.0f) gives) count as 0.0 in every weighted
 form: on a bridge, in a cycle, on a leaf, and where a longer path is found
 first.  Compared with the oracle on the same graph with 0.0 in their place;
-distances are sums of whole numbers below 2^24, so the tolerance is zero."""
+distances are sums of whole numbers below 2^24, so the tolerance is zero.  A
+weight in the source's row that equals the encoding of "unreached" reaches
+nothing."""
 
 import numpy as np
 import pytest
@@ -56,3 +58,14 @@ def test_negative_weights_of_an_unvalidated_handle_end():
         for srcs, variant in (([0], abi.VARIANT_DO), ([0, 1], abi.VARIANT_AUTO)):
             d, st = dg.sssp(srcs, variant=variant)
             assert d.shape == (len(srcs), 4) and st.levels <= 2 * g.n
+
+
+@pytest.mark.parametrize("weights", ["i32", "f32"])
+def test_source_row_weight_of_unreached(weights):
+    top = abi.INT32_MAX if weights == "i32" else abi.FLT_MAX
+    g = weighted(5, [0, 1, 0, 3], [1, 2, 3, 4], [1, 1, 5, 2])
+    g.w_i32[0], g.w_f32[0] = abi.INT32_MAX, abi.FLT_MAX
+    with abi.Graph(g, weights=weights) as dg:
+        for srcs, variant in (([0], abi.VARIANT_DO), ([0, 0, 0], abi.VARIANT_AUTO)):
+            d, _ = dg.sssp(srcs, variant=variant)
+            assert (d == np.array([0, top, top, 5, 7], d.dtype)).all(), (variant, d)

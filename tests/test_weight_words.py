@@ -24,8 +24,9 @@ def add(a, b, kind):
         return int((np.uint32(a).view(np.float32) + np.uint32(b).view(np.float32)).view(np.uint32))
 
 
-def distances(n, edges, source, kind, step, raw=False, most=10000):
-    """Words of the distances, None if the rule does not end."""
+def distances(n, edges, source, kind, step, raw=False, queue_all=False, most=10000):
+    """Words of the distances, None if the rule does not end.  queue_all: neighbours
+    of the source are queued whatever their weight."""
     inf, w_of = INF[kind], (lambda x: int(np.float32(x).view(np.uint32))) if raw else (lambda x: word(x, kind))
     rows = [[] for _ in range(n)]
     for u, v, w in edges:
@@ -37,7 +38,8 @@ def distances(n, edges, source, kind, step, raw=False, most=10000):
     for v, w in last.items():
         d = 0 if v == source else w
         D[v] = d
-        (near if d <= T else far).append(v)
+        if d < inf or queue_all:
+            (near if d <= T else far).append(v)
     D[source] = 0
     scanned = False
     for _ in range(most):
@@ -107,3 +109,13 @@ def test_rule_ends(kind):
         got = got.view(np.float32).astype(np.float64) if kind == "f32" else got.astype(np.float64)
         got[got >= (np.float64(np.finfo(np.float32).max) if kind == "f32" else INF["i32"])] = np.inf
         assert np.array_equal(got, want), trial
+
+
+@pytest.mark.parametrize("kind", ["i32", "f32"])
+def test_source_row_weight_of_unreached(kind):
+    # the largest weight there is equals the encoding of "unreached"
+    top = INF[kind] if kind == "i32" else float(np.finfo(np.float32).max)
+    edges = [(0, 1, top), (1, 2, 1.0), (0, 3, 5.0), (3, 4, 2.0)]
+    step = word(3, kind)
+    assert distances(5, edges, 0, kind, step, queue_all=True) is None
+    assert distances(5, edges, 0, kind, step) == [0, INF[kind], INF[kind], word(5, kind), word(7, kind)]
