@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(kNfBlock, 2) nf_traverse(const __grid_constant
   __shared__ uint32_t s_nn[kNfWarps], s_nf[kNfWarps];
   __shared__ unsigned long long s_word[4];
   __shared__ Solo s_solo[2];
-  __shared__ int32_t s_cnt[3], s_long;
+  __shared__ int32_t s_cnt[3], s_long[3];  // of the lists of three phases in a row
   const int shift = a.shift;
   const uint32_t smask = (1u << shift) - 1u;
   NfCtl* const ctl = a.ctl;
@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(kNfBlock, 2) nf_traverse(const __grid_constant
       if (threadIdx.x == 0) {
         s_cnt[0] = (int)ph.n;
         s_cnt[1] = s_cnt[2] = 0;
-        s_long = 0;
+        s_long[0] = s_long[1] = s_long[2] = 0;
       }
       __syncthreads();
       int left = 0, it = 0;
@@ -515,8 +515,9 @@ __global__ void __launch_bounds__(kNfBlock, 2) nf_traverse(const __grid_constant
         const int cnt = s_cnt[it % 3];
         const Solo& in = s_solo[it & 1];
         Solo& nx = s_solo[(it & 1) ^ 1];
-        int32_t* const nx_cnt = &s_cnt[(it + 1) % 3];
-        if (threadIdx.x == 0) s_cnt[(it + 2) % 3] = 0;
+        const int o = (it + 1) % 3;
+        int32_t* const nx_cnt = &s_cnt[o];
+        if (threadIdx.x == 0) s_cnt[(it + 2) % 3] = s_long[(it + 2) % 3] = 0;
         auto push = [&](auto& k, auto& ok, auto& d, auto& src) {
           constexpr int kU = sizeof(k) / sizeof(k[0]);
           uint32_t pu[kU], c[kU];
@@ -547,7 +548,7 @@ __global__ void __launch_bounds__(kNfBlock, 2) nf_traverse(const __grid_constant
               nx.p[base] = pu[i];
               nx.rs[base] = rs[i];
               nx.deg[base] = re[i] - rs[i];
-              if (re[i] - rs[i] >= kLongRow) s_long = 1;
+              if (re[i] - rs[i] >= kLongRow) s_long[o] = 1;
             }
             bool over = near && base >= kSoloCap;
             if (over) over = set_pair(near_out, pu[i]);
@@ -566,8 +567,9 @@ __global__ void __launch_bounds__(kNfBlock, 2) nf_traverse(const __grid_constant
           expand(p, ok ? in.rs[i] : 0, ok ? in.deg[i] : 0, ok ? (uint32_t)__ldcg(a.D + p) : 0u, push);
         }
         __syncthreads();
+        // a warp that goes on writes the next phase's words, not these
         left = *nx_cnt;
-        if (left == 0 || left > (int)a.solo_max || s_long) break;
+        if (left == 0 || left > (int)a.solo_max || s_long[o]) break;
       }
       if (threadIdx.x == 0 && it > 0) {
         atomicAdd(&ctl->far.iters, (uint32_t)it);
