@@ -1422,7 +1422,7 @@ dawn_status bfs_single(dawn_graph* g, const int32_t* sources, int32_t nsrc, int3
     a.col = g->col;
     a.t_row_ptr = g->t_row_ptr;
     a.t_col = g->t_col;
-    a.ctl = g->ss_ctl.as<SsCtl>();
+    a.ctl = g->ss_call = g->ss_ctl.as<SsCtl>();
     a.sync = g->bfs_sync.as<BfsSync>();
     a.q = g->ss_queues.as<int32_t>();
     a.segs = g->ss_segs.as<Seg>();

@@ -196,7 +196,7 @@ struct dawn_graph {
   dawn::DevBuf ss_queues;   // 2 x n int32 short-row queues
   dawn::DevBuf ss_segs;     // 2 x seg_capacity long-row segments
   dawn::DevBuf ss_bitmaps;  // visited + 3 frontier bitmaps (words)
-  dawn::DevBuf ss_ctl;      // SsCtl
+  dawn::DevBuf ss_ctl;      // SsCtl: one size for good, the captured graphs hold its address
   dawn::DevBuf bfs_long;    // 2 x the long rows of a level (single-source BFS)
   const void* bfs_fn = nullptr;    // the persistent kernel that bfs_ctas and the kernel's limits were set for
   int32_t bfs_ctas = 0, bfs_cap = 0;
@@ -204,8 +204,9 @@ struct dawn_graph {
   int32_t max_row = -1;     // entries of the longest row (-1: not read yet)
   int32_t rec_len = -1;     // words of a record; 0: none, -1: not decided, -2: level kernels instead
   dawn::DevBuf bfs_sync;    // BfsSync: what the CTAs of the persistent BFS wait on
-  dawn::DevBuf ss_sources;  // int32 source list of the current call
+  dawn::DevBuf ss_sources;  // int32 source list of the current call (ordered weighted: a control block before it)
   const int32_t* ss_src = nullptr;  // weighted: where the current call's list is
+  dawn::SsCtl* ss_call = nullptr;   // the current call's control block
   dawn::DevBuf ss_scratch;  // n x u64 (GOVM source-row resolution)
   dawn::DevBuf bc_levels;   // betweenness: level blocks of two batches (bfs_bitset_levels)
   dawn::DevBuf bc_terms;    // per 64 sources of a batch, n x 64 float (1 / amount + dependency)

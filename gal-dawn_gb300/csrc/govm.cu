@@ -391,12 +391,14 @@ void probe_sssp(const void* p, LevelProbe* out) {
 
 // One ordered traversal (nearfar.cu) per source.
 dawn_status sssp_ordered(dawn_graph* g, const int32_t* sources, int32_t nsrc, void* d_dist) {
-  // one upload: the control block, cleared, and the sources
+  // One upload: a control block, cleared, and the sources.  In a buffer of their
+  // own: ss_ctl must not move, whatever the number of sources.
   std::vector<int32_t> up(sizeof(SsCtl) / sizeof(int32_t) + (size_t)nsrc, 0);
   std::copy(sources, sources + nsrc, up.end() - nsrc);
-  DAWN_CHECK(ensure(g->ss_ctl, sizeof(int32_t) * up.size(), g->stream));
-  DAWN_CUDA(cudaMemcpyAsync(g->ss_ctl.p, up.data(), sizeof(int32_t) * up.size(), cudaMemcpyHostToDevice, g->stream));
-  SsCtl* ctl = g->ss_ctl.as<SsCtl>();
+  DAWN_CHECK(ensure(g->ss_sources, sizeof(int32_t) * up.size(), g->stream));
+  DAWN_CUDA(cudaMemcpyAsync(g->ss_sources.p, up.data(), sizeof(int32_t) * up.size(), cudaMemcpyHostToDevice,
+                            g->stream));
+  SsCtl* ctl = g->ss_call = g->ss_sources.as<SsCtl>();
   g->ss_src = reinterpret_cast<const int32_t*>(ctl + 1);
   for (int32_t i = 0; i < nsrc; i++)
     DAWN_CHECK(nearfar_run(g, g->ss_src + i, 1, 0,

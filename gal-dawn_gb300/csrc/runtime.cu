@@ -119,12 +119,13 @@ int persistent_blocks(const void* fn, int block, size_t smem, int cap) {
 dawn_status upload_ctl(dawn_graph* g, const SsCtl& c) {
   // Pageable source: the runtime stages it before returning, so the stack
   // copy may go out of scope while the transfer is still queued.
+  g->ss_call = g->ss_ctl.as<SsCtl>();
   DAWN_CUDA(cudaMemcpyAsync(g->ss_ctl.p, &c, sizeof(SsCtl), cudaMemcpyHostToDevice, g->stream));
   return DAWN_OK;
 }
 
 dawn_status download_ctl(dawn_graph* g, SsCtl* out) {
-  DAWN_CUDA(cudaMemcpyAsync(&g->h_ctl[1], g->ss_ctl.p, sizeof(SsCtl), cudaMemcpyDeviceToHost, g->stream));
+  DAWN_CUDA(cudaMemcpyAsync(&g->h_ctl[1], g->ss_call, sizeof(SsCtl), cudaMemcpyDeviceToHost, g->stream));
   DAWN_CUDA(cudaStreamSynchronize(g->stream));
   *out = g->h_ctl[1];
   return DAWN_OK;
