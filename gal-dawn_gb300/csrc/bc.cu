@@ -827,7 +827,7 @@ dawn_status betweenness(dawn_graph* g, const int32_t* sources, int32_t nsrc, dou
   }
   if (!g->bc_h_level) DAWN_CHECK(pinned_slot((void**)&g->bc_h_level));
   const int32_t nb = (nsrc + kLanes - 1) / kLanes, nbatches = (nb + width - 1) / width;
-  const int32_t nacc = std::min<int32_t>(nb, width);
+  const int32_t nacc = std::max(1, std::min<int32_t>(nb, width));  // no sources: zeros all the same
   double* const acc = nacc > 1 ? g->bc_acc.as<double>() : d_bc;
   DAWN_CUDA(cudaMemsetAsync(acc, 0, sizeof(double) * nn * nacc, g->stream));
   // Level blocks and ranges are double-buffered: the traversal of batch b runs
