@@ -85,6 +85,8 @@ dawn_status finish_graph(dawn_graph* g, uint32_t flags) {
   }
   static_assert(2 * sizeof(dawn::SsCtl) <= dawn::kPinnedSlot, "control-block copies exceed a pinned slot");
   DAWN_CHECK(dawn::pinned_slot((void**)&g->h_ctl));
+  DAWN_CHECK(dawn::pinned_slot((void**)&g->h_err));
+  *g->h_err = 0;
   DAWN_CHECK(dawn::ensure(g->sel_slot, sizeof(float) * DAWN_SELECTOR_WEIGHTS, g->stream));
   DAWN_CUDA(cudaEventCreate(&g->ev0));
   DAWN_CUDA(cudaEventCreate(&g->ev1));
@@ -150,6 +152,7 @@ void destroy(dawn_graph* g) {
   if (g->pt_exec) cudaGraphExecDestroy(g->pt_exec);
   if (g->mw_exec) cudaGraphExecDestroy(g->mw_exec);
   dawn::pinned_slot_release(g->h_ctl);
+  dawn::pinned_slot_release(g->h_err);
   dawn::pinned_slot_release(g->bc_h_level);
   for (cudaEvent_t e : g->trace_ev)
     if (e) cudaEventDestroy(e);
@@ -167,6 +170,7 @@ int32_t resolve_variant(const dawn_graph* g, int32_t variant, int32_t nsrc) {
 
 dawn_status bfs_device_impl(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32_t* d_dist,
                             int32_t variant, dawn_stats* st) {
+  DAWN_CHECK(dawn::device_status(g));
   variant = resolve_variant(g, variant, nsrc);
   DAWN_CHECK(dawn::call_selector(g, variant, &g->sel_call));
   if (st) {
@@ -179,11 +183,7 @@ dawn_status bfs_device_impl(dawn_graph* g, const int32_t* sources, int32_t nsrc,
       DAWN_CUDA(cudaEventRecord(g->ev1, g->stream));
       dawn::SsCtl c;
       DAWN_CHECK(dawn::download_ctl(g, &c));
-      if (c.err) {
-        dawn::set_error("single-source traversal: a device wait ran out");
-        dawn::release(g->bfs_sync);  // its counts are off: the next call starts a new one
-        return c.err;
-      }
+      DAWN_CHECK(dawn::device_status(g));
       st->edges_traversed = (int64_t)c.total_reached;
       st->levels = c.total_levels;
       st->push_levels = c.total_push;
@@ -215,6 +215,7 @@ bool sssp_uses_batch(int32_t variant, int32_t nsrc) {
 
 dawn_status sssp_device_impl(dawn_graph* g, const int32_t* sources, int32_t nsrc, void* d_dist,
                              dawn_stats* st, int32_t variant = DAWN_VARIANT_AUTO) {
+  DAWN_CHECK(dawn::device_status(g));
   if (st) {
     std::memset(st, 0, sizeof(*st));
     DAWN_CUDA(cudaEventRecord(g->ev0, g->stream));
@@ -233,10 +234,7 @@ dawn_status sssp_device_impl(dawn_graph* g, const int32_t* sources, int32_t nsrc
     DAWN_CUDA(cudaEventRecord(g->ev1, g->stream));
     dawn::SsCtl c;
     DAWN_CHECK(dawn::download_ctl(g, &c));
-    if (c.err) {
-      dawn::set_error("weighted traversal: a device wait ran out");
-      return c.err;
-    }
+    DAWN_CHECK(dawn::device_status(g));
     st->levels = c.total_levels;
     st->push_levels = c.total_push;
     st->pull_levels = c.total_pull;
@@ -287,7 +285,7 @@ dawn_status staged(dawn_graph* g, const int32_t* sources, int32_t nsrc, void* ho
     // link: no device staging and no separate copy.
     DAWN_CHECK(run(sources, nsrc, host_dist, st));
     DAWN_CUDA(cudaStreamSynchronize(g->stream));
-    return DAWN_OK;
+    return dawn::device_status(g);
   }
   int32_t chunk = (int32_t)(kStageBytes / row_bytes);
   if (chunk >= 64) chunk -= chunk % 64;
@@ -305,7 +303,7 @@ dawn_status staged(dawn_graph* g, const int32_t* sources, int32_t nsrc, void* ho
     if (st) add_stats(st, s);
   }
   DAWN_CUDA(cudaStreamSynchronize(g->stream));
-  return DAWN_OK;
+  return dawn::device_status(g);
 }
 
 long long multi_out_elems(const dawn_graph* g, const int32_t* source_offset) {
@@ -440,7 +438,7 @@ dawn_status dawn_graph_synchronize(dawn_graph* g) {
     return DAWN_ERR_INVALID_ARG;
   }
   DAWN_CUDA(cudaStreamSynchronize(g->stream));
-  return DAWN_OK;
+  return dawn::device_status(g);
 }
 
 dawn_status dawn_bfs_device(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32_t* d_dist,
@@ -534,6 +532,7 @@ dawn_status dawn_closeness(dawn_graph* g, const int32_t* sources, int32_t nsrc, 
   DAWN_CHECK(check_sources(g, sources, nsrc));
   if (stats) std::memset(stats, 0, sizeof(*stats));
   if (nsrc == 0) return DAWN_OK;
+  DAWN_CHECK(dawn::device_status(g));
   const int kind = !weighted ? 0 : (g->wtype == DAWN_W_F32 ? 2 : 1);
   if (kind == 0) {
     // Hop closeness straight from the batched traversal's level words: its
@@ -556,6 +555,7 @@ dawn_status dawn_closeness(dawn_graph* g, const int32_t* sources, int32_t nsrc, 
     DAWN_CUDA(cudaMemcpyAsync(h.data(), d_sum, sizeof(unsigned long long) * h.size(), cudaMemcpyDeviceToHost,
                               g->stream));
     DAWN_CUDA(cudaStreamSynchronize(g->stream));
+    DAWN_CHECK(dawn::device_status(g));
     for (int32_t i = 0; i < nsrc; i++) {
       const double total = (double)h[i];
       cc[i] = total > 0 ? (double)(g->n - 1) / total : 0.0;
@@ -605,6 +605,7 @@ dawn_status dawn_closeness(dawn_graph* g, const int32_t* sources, int32_t nsrc, 
       s = DAWN_ERR_CUDA;
       break;
     }
+    if ((s = dawn::device_status(g)) != DAWN_OK) break;
     for (int32_t i = 0; i < c; i++) {
       double total;
       if (kind == 2) {
@@ -631,6 +632,7 @@ dawn_status dawn_betweenness_device(dawn_graph* g, const int32_t* sources, int32
     return DAWN_ERR_INVALID_ARG;
   }
   DAWN_CHECK(check_sources(g, sources, nsrc));
+  DAWN_CHECK(dawn::device_status(g));
   if (stats) DAWN_CUDA(cudaEventRecord(g->ev0, g->stream));
   DAWN_CHECK(dawn::betweenness(g, sources, nsrc, d_bc, stats));
   if (stats) {
@@ -821,6 +823,13 @@ dawn_status dawn_graph_set_option(dawn_graph* g, int32_t option, int64_t value) 
       }
       g->small_levels = value != 0;  // read from the control block at every call
       return DAWN_OK;
+    case DAWN_OPT_WAIT_POLLS:
+      if (value < 1 || value > INT32_MAX) {
+        dawn::set_error("polls of a wait must lie in [1, 2^31)");
+        return DAWN_ERR_INVALID_ARG;
+      }
+      g->wait_polls = (uint32_t)value;
+      return DAWN_OK;
     default:
       dawn::set_error("unknown option %d", option);
       return DAWN_ERR_INVALID_ARG;
@@ -913,6 +922,9 @@ dawn_status dawn_graph_get_option(const dawn_graph* g, int32_t option, int64_t* 
       return DAWN_OK;
     case DAWN_OPT_SMALL_LEVELS:
       *value = g->small_levels ? 1 : 0;
+      return DAWN_OK;
+    case DAWN_OPT_WAIT_POLLS:
+      *value = g->wait_polls;
       return DAWN_OK;
     default:
       dawn::set_error("unknown option %d", option);

@@ -880,14 +880,10 @@ dawn_status betweenness(dawn_graph* g, const int32_t* sources, int32_t nsrc, dou
       status = DAWN_ERR_CUDA;
       break;
     }
-    const int32_t* const end = g->bc_h_level + kLevelsEnd * p;  // level, status, depth of each 64
-    if (end[1]) {
-      set_error("betweenness: a device wait ran out");
-      status = end[1];
-      break;
-    }
+    if ((status = device_status(g)) != DAWN_OK) break;
+    const int32_t* const end = g->bc_h_level + kLevelsEnd * p;  // level, depth of each 64
     const int32_t k = (in_batch(b - 1) + kLanes - 1) / kLanes;  // blocks
-    for (int32_t i = 0; i < k; i++) levels += end[2 + i];
+    for (int32_t i = 0; i < k; i++) levels += end[1 + i];
     if (end[0] < kDeepLevel) {
       const u64* M = reinterpret_cast<const u64*>(Ls[p]);
       const dim3 grid(std::max(1, ctas / k), k), grid_amount(std::max(1, ctas_amount / k), k);
@@ -909,12 +905,12 @@ dawn_status betweenness(dawn_graph* g, const int32_t* sources, int32_t nsrc, dou
         const int32_t *const L = Ls[p] + i * kLanes * nn, *const R = Rs[p] + i * 2 * nn;
         double* const out = acc + i * nn;
         if (pairs) {
-          pair_passes(g, L, T, out, end[2 + i]);
+          pair_passes(g, L, T, out, end[1 + i]);
           continue;
         }
         bc_rows_amount<<<ctas, kBlock, 0, g->stream>>>(g->t_row_ptr, g->t_col, L, T, g->n, hin, cnt);
         if (hin.count) bc_rows_amount_heavy<<<ctas, kBlock, 0, g->stream>>>(L, T, hin, cnt);
-        for (int32_t l = end[2 + i] - 1; l >= 1; l--) {
+        for (int32_t l = end[1 + i] - 1; l >= 1; l--) {
           bc_rows_sweep<<<ctas, kBlock, 0, g->stream>>>(g->row_ptr, g->col, L, R, T, out, g->n, l, hout, part);
           if (hout.count) bc_rows_sweep_heavy<<<ctas, kBlock, 0, g->stream>>>(L, R, T, out, l, hout, part);
         }

@@ -795,7 +795,6 @@ __global__ void __launch_bounds__(kBlock, 5) bfs_step(const int32_t* __restrict_
 //   RMAT-22                                          261 ->  200
 //   grid 300 x 300                                  1580 ->  818
 //   grid 1000 x 1049                                6511 -> 4297
-constexpr uint32_t kBfPollLimit = 1u << 27;  // polls of one wait (over 30 s)
 constexpr int kBfEntries = 4096;             // vertices and entries per CTA of a small graph
 // Frontiers that go to CTA 0 and that stay there.  One SM makes about one access
 // to L1 or L2 a clock: a row of four entries costs it a dozen (8 us for 1,000
@@ -813,6 +812,7 @@ enum : int32_t { kBfStart = 0, kBfWipe, kBfBits, kBfCut, kBfPush, kBfPull, kBfSo
 struct BfsSync {
   struct __align__(128) {
     unsigned long long word[4];
+    uint32_t broken;  // a wait of an earlier launch gave up: its arrivals are missing
   } step;  // BfsStep, tagged with the generation in the top 16 bits of each word
   struct __align__(128) {
     uint32_t n;
@@ -841,6 +841,8 @@ struct BfsArgs {
   int32_t n, nwords, source, first;  // first: of the call's sources
   int32_t policy, use_sel, force, small;
   float sel_margin;
+  uint32_t polls;      // of one wait
+  int32_t* err;        // pinned host word
 };
 
 struct SoloList {
@@ -1197,7 +1199,6 @@ __device__ __noinline__ bool next_phase(const BfsArgs& a, BfsStep& step) {
         c.total_levels = vc->total_levels;
         c.total_push = vc->total_push;
         c.total_pull = vc->total_pull;
-        c.err = vc->err;
       }
       *ctl = c;
       seed(ctl, a.source, a.dist, a.row_ptr, a.q, a.segs, a.lq, a.vbm, a.n, a.m);
@@ -1250,10 +1251,11 @@ __global__ void __launch_bounds__(kMesh ? 1024 : 640, kMesh ? 1 : 2) bfs_travers
   if (threadIdx.x == 0) {
     sm.st = BfsStep{};
     sm.st.phase = kBfStart;
-    sm.st.ctas = (int)gridDim.x;
+    sm.st.ctas = *static_cast<const volatile uint32_t*>(&a.sync->step.broken) ? 0 : (int)gridDim.x;
     sm.st.arrived = (uint32_t)*static_cast<const volatile unsigned long long*>(&a.sync->step.word[3]);
   }
   __syncthreads();
+  if (st.ctas == 0) return;
   for (;;) {
     const Team tm{(int)blockIdx.x, st.ctas};
     switch (st.phase) {
@@ -1324,9 +1326,10 @@ __global__ void __launch_bounds__(kMesh ? 1024 : 640, kMesh ? 1 : 2) bfs_travers
           }
           idle = true;
         }
-        if (polls == kBfPollLimit) {
+        if (polls == a.polls) {
           if (lane == 0) {
-            a.ctl->err = DAWN_ERR_TIMEOUT;
+            *a.err = DAWN_ERR_TIMEOUT;
+            *static_cast<volatile uint32_t*>(&a.sync->step.broken) = 1;
             sm.st.ctas = 0;
           }
           break;
@@ -1441,6 +1444,8 @@ dawn_status bfs_single(dawn_graph* g, const int32_t* sources, int32_t nsrc, int3
     a.sel_margin = g->sel_margin;
     a.force = force;
     a.small = g->small_levels;
+    a.polls = g->wait_polls;
+    a.err = g->h_err;
     const bool mesh = g->small_levels && g->rec_len > 0;
     a.rec_len = mesh ? g->rec_len : 0;
     a.rec = mesh ? g->bfs_rec.as<int32_t>() : nullptr;

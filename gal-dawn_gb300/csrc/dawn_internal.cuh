@@ -85,7 +85,6 @@ struct SsCtl {
   int32_t source;               // current source vertex
   int32_t policy;               // DAWN_VARIANT_PUSH or DAWN_VARIANT_DO
   int32_t weighted;             // GOVM: 0 int32, 1 float32 distances
-  int32_t err;                  // first device-side error code (0 = none)
   int32_t nsrc;                 // sources of the current call
   // per-call parameters (host-written before the first launch)
   int32_t* dist_base;           // nsrc x n output, row src_idx is current
@@ -236,6 +235,8 @@ struct dawn_graph {
   bool wt_has_light = false;  // the light entries are a part of the rows worth a stage of their own
   dawn::DevBuf mw_bounds;   // batched: per vertex, lowest and highest distance over the sources (mw_bounds)
   dawn::SsCtl* h_ctl = nullptr;  // pinned: [0] upload staging, [1] download
+  int32_t* h_err = nullptr;      // pinned: status that a launch of this handle wrote (device_status), 0 = none
+  uint32_t wait_polls = 1u << 27;  // DAWN_OPT_WAIT_POLLS: polls of a wait between CTAs before it gives up
   bool graphs_ok = true;         // conditional CUDA graphs usable
 
   // batched bitset workspace
@@ -328,9 +329,9 @@ dawn_status sssp_batched_stats(dawn_graph* g, dawn_stats* st, int32_t nsrc);
 // relaxation in one persistent launch.  D[(v << shift) + s] receives the
 // distance of vertex v from source s (shift 0 for one source, else
 // nearfar_shift(nb)).  The steps taken are added to *levels_out and *push_out
-// (device); *err_out (device) receives DAWN_ERR_TIMEOUT when a wait ran out.
+// (device).
 dawn_status nearfar_run(dawn_graph* g, const int32_t* d_sources, int32_t nb, int shift, int32_t* D,
-                        int32_t* levels_out, int32_t* push_out, int32_t* err_out);
+                        int32_t* levels_out, int32_t* push_out);
 int nearfar_shift(int32_t nb);
 // Whether batches of up to 64 of nsrc sources run through nearfar_run.
 dawn_status nearfar_batch_fits(dawn_graph* g, int32_t nsrc, bool* fits);
@@ -366,11 +367,11 @@ dawn_status bitset_reserve(dawn_graph* g, int w);
 // reach the vertex at that level), level after level; a deeper one n x 64 level
 // rows (vertex-major, -1 unreached), and in d_range (2 n int32 per 64 sources)
 // the lowest and highest level of each vertex.
-// Enqueued only: the level the batch ended on (the deepest level + 1), its error
-// status and the deepest level of each 64 sources are copied to h_end (pinned
-// host memory) behind the traversal.
+// Enqueued only: the level the batch ended on (the deepest level + 1) and the
+// deepest level of each 64 sources are copied to h_end (pinned host memory)
+// behind the traversal.
 constexpr int kDeepLevel = 32;  // batched traversal: levels from here on are written out directly
-constexpr int kLevelsEnd = 6;
+constexpr int kLevelsEnd = 5;
 dawn_status bfs_bitset_levels(dawn_graph* g, int w, const int32_t* sources, int32_t nsrc, int32_t* d_levels,
                               int32_t* d_range, int32_t* h_end);
 int bitset_width(const dawn_graph* g, int32_t nsrc);
@@ -384,6 +385,12 @@ dawn_status ss_run(dawn_graph* g, SsFamily& fam, int32_t nsrc,
 dawn_status ss_run_traced(dawn_graph* g, SsFamily& fam, int32_t nruns);
 // Sets max_row, once per handle.
 dawn_status longest_row(dawn_graph* g);
+// The status of the handle's launches that the host has waited for: not DAWN_OK
+// once after a wait between the CTAs of a launch gave up.  Every call on a handle
+// asks at its start (for what earlier calls left enqueued) and after its own last
+// synchronisation; a launch that gave up says so by one store to pinned memory,
+// and the others cost nothing.
+dawn_status device_status(dawn_graph* g);
 // A kernel whose CTAs wait for each other, with the family's L2 window if it
 // has one.
 dawn_status launch_cooperative(const SsFamily& fam, const void* fn, int ctas, int threads, void** args,

@@ -402,7 +402,7 @@ dawn_status sssp_ordered(dawn_graph* g, const int32_t* sources, int32_t nsrc, vo
   g->ss_src = reinterpret_cast<const int32_t*>(ctl + 1);
   for (int32_t i = 0; i < nsrc; i++)
     DAWN_CHECK(nearfar_run(g, g->ss_src + i, 1, 0,
-                           static_cast<int32_t*>(d_dist) + (size_t)i * g->n, &ctl->total_levels, &ctl->total_push, &ctl->err));
+                           static_cast<int32_t*>(d_dist) + (size_t)i * g->n, &ctl->total_levels, &ctl->total_push));
   return DAWN_OK;
 }
 

@@ -50,8 +50,7 @@ struct BsCtl {
   int32_t tq_size;              // push: vertices touched this level
   int32_t ul_size[2];           // unfinished-vertex lists (pull work lists)
   int32_t ul_cur;               // list the next pull reads: -1 = the graph's static list
-  int32_t level;                // with err and depth: read together by level-mode callers
-  int32_t err;                  // persistent launch: a wait ran out
+  int32_t level;                // with depth: read together by level-mode callers
   int32_t depth[kMaxW];         // level mode: the deepest level of each 64 sources
   int32_t mode, done, policy, batch, nsrc, n_push, n_pull;
   int32_t push_ratio;           // push while push_ratio * frontier edges < unfinished edges
@@ -88,7 +87,8 @@ struct BsCtl {
   // persistent launch: the words that all CTAs poll (BsStep), and the
   // arrivals of all phases so far
   struct __align__(128) {
-    unsigned long long word[16];
+    unsigned long long word[15];
+    uint32_t broken;  // a wait of an earlier batch gave up: its arrivals are missing
   } sync;
   struct __align__(128) {
     uint32_t n;
@@ -129,6 +129,8 @@ struct BsArgs {
   int32_t *dist_base, *lv_block;
   unsigned long long* cc_sum;
   const float* sel_w;
+  uint32_t polls;               // persistent launch: of one wait
+  int32_t* err;                 // pinned host word
 };
 
 constexpr int kSlicesCleared = 4;  // slices zeroed per batch; higher ones on first use
@@ -1573,7 +1575,6 @@ __global__ void bs_next(const __grid_constant__ BsArgs a) {
 // Vertices and entries per CTA of a small graph: 1024 / 4096, 64 sources: grid 40 x
 // 60 880 / 1006 us, kNN of 2,127 points 545 / 593, RMAT-12 107 / 114.
 constexpr int kBsEntries = 1024;
-constexpr uint32_t kBsPollLimit = 1u << 27;  // polls of one wait (over 30 s) before the launch gives up
 
 // CTAs for `work` warp tasks.
 __device__ __forceinline__ int bs_ctas(int work, int warps) {
@@ -1688,10 +1689,11 @@ __global__ void __launch_bounds__(W == 1 ? 640 : 512, 2) bs_traverse(const __gri
   if (threadIdx.x == 0) {
     sm.st = BsStep{};
     sm.st.phase = kBsClear;
-    sm.st.ctas = (int)gridDim.x;
-    sm.st.arrived = (uint32_t)(uint32_t)*static_cast<const volatile unsigned long long*>(&ctl->sync.word[8]);
+    sm.st.ctas = *static_cast<const volatile uint32_t*>(&ctl->sync.broken) ? 0 : (int)gridDim.x;
+    sm.st.arrived = (uint32_t)*static_cast<const volatile unsigned long long*>(&ctl->sync.word[8]);
   }
   __syncthreads();
+  if (st.ctas == 0) return;
   for (;;) {
     const Team tm{(int)blockIdx.x, st.ctas};
     switch (st.phase) {
@@ -1744,9 +1746,10 @@ __global__ void __launch_bounds__(W == 1 ? 640 : 512, 2) bs_traverse(const __gri
           }
           idle = true;
         }
-        if (polls == kBsPollLimit) {
+        if (polls == a.polls) {
           if (lane == 0) {
-            ctl->err = DAWN_ERR_TIMEOUT;
+            *a.err = DAWN_ERR_TIMEOUT;
+            *static_cast<volatile uint32_t*>(&ctl->sync.broken) = 1;
             sm.st.ctas = 0;
           }
           break;
@@ -1945,6 +1948,8 @@ dawn_status run_width(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32
   a.nbits = nbits;
   a.force = g->force_variant;
   a.batch = -1;
+  a.polls = g->wait_polls;
+  a.err = g->h_err;
   a.dist_base = d_dist;
   a.lv_block = lv_block;
   a.cc_sum = cc_sum;
@@ -2030,7 +2035,7 @@ dawn_status bfs_bitset_levels(dawn_graph* g, int w, const int32_t* sources, int3
     DAWN_CHECK(run_width<2>(g, sources, nsrc, nullptr, nullptr, nullptr, d_levels, d_range));
   else
     DAWN_CHECK(run_width<1>(g, sources, nsrc, nullptr, nullptr, nullptr, d_levels, d_range));
-  static_assert(offsetof(BsCtl, depth) == offsetof(BsCtl, level) + 2 * sizeof(int32_t) && kMaxW == 4, "six words");
+  static_assert(offsetof(BsCtl, depth) == offsetof(BsCtl, level) + sizeof(int32_t) && kMaxW == 4, "five words");
   DAWN_CUDA(cudaMemcpyAsync(h_end, &g->bs_ctl.as<BsCtl>()->level, kLevelsEnd * sizeof(int32_t),
                             cudaMemcpyDeviceToHost, g->stream));
   return DAWN_OK;
@@ -2040,10 +2045,7 @@ dawn_status bfs_bitset_stats(dawn_graph* g, dawn_stats* st, int32_t nsrc) {
   BsCtl h;
   DAWN_CUDA(cudaMemcpyAsync(&h, g->bs_ctl.p, sizeof(BsCtl), cudaMemcpyDeviceToHost, g->stream));
   DAWN_CUDA(cudaStreamSynchronize(g->stream));
-  if (h.err) {
-    set_error("batched traversal: a device wait ran out");
-    return h.err;
-  }
+  DAWN_CHECK(device_status(g));
   st->edges_traversed = (int64_t)h.total_reached;
   st->levels = h.total_levels;
   st->push_levels = h.total_push;

@@ -78,7 +78,6 @@ struct MwCtl {
   int32_t* dist_base;           // nsrc x n output (source-major)
   const int32_t* sources;
   int32_t total_levels, total_push, total_pull;
-  int32_t err;                  // status of an ordered batch (0 = none)
 };
 
 // Stages of a batch: pulls along light edges; one pull along all edges from every
@@ -1004,7 +1003,7 @@ dawn_status run_ordered(dawn_graph* g, const int32_t* sources, int32_t nsrc, voi
                      : shift == 3 ? mw_emit<8> : mw_emit<4>;
   for (int32_t b0 = 0; b0 < nsrc; b0 += kBatch) {
     DAWN_CHECK(nearfar_run(g, g->mw_sources.as<int32_t>() + b0, std::min(kBatch, nsrc - b0), shift, D,
-                           &ctl->total_levels, &ctl->total_push, &ctl->err));
+                           &ctl->total_levels, &ctl->total_push));
     emit<<<g->geo.sms * 8, kEmitBlock, 0, g->stream>>>(ctl, D, g->row_ptr, inf, g->n);
     mw_next<<<1, 32, 0, g->stream>>>(ctl);
     DAWN_CUDA(cudaGetLastError());
@@ -1142,10 +1141,7 @@ dawn_status sssp_batched_stats(dawn_graph* g, dawn_stats* st, int32_t nsrc) {
   MwCtl h;
   DAWN_CUDA(cudaMemcpyAsync(&h, g->mw_ctl.p, sizeof(MwCtl), cudaMemcpyDeviceToHost, g->stream));
   DAWN_CUDA(cudaStreamSynchronize(g->stream));
-  if (h.err) {
-    set_error("weighted traversal: a device wait ran out");
-    return h.err;
-  }
+  DAWN_CHECK(device_status(g));
   st->edges_traversed = (int64_t)h.reached;
   st->levels = h.total_levels;
   st->push_levels = h.total_push;

@@ -49,7 +49,6 @@ constexpr int kNfBlock = 512;
 constexpr int kShortUnroll = 3;  // groups of 32 entries of short rows in flight per warp
 constexpr int kNfWarps = kNfBlock / 32;
 constexpr int kNfEntries = 256;  // vertices and entries per CTA of a small graph (512 the same, 1024: kNN of 2,127 8% slower)
-constexpr uint32_t kPollLimit = 1u << 27;  // polls of one wait (over 30 s) before the launch gives up
 
 enum : int32_t { kPhFill = 0, kPhMark, kPhSeed, kPhNear, kPhFar };
 
@@ -107,9 +106,10 @@ struct NfArgs {
   uint32_t inf, delta, delta_min, delta_max;
   int32_t has_long;        // some row has at least kLongRow entries
   uint32_t solo_max;       // pairs of a single-CTA phase
-  int32_t* levels_out;     // of the call's control block: levels, push levels, error code
+  int32_t* levels_out;     // of the call's control block: levels, push levels
   int32_t* push_out;
-  int32_t* err_out;
+  uint32_t polls;          // of one wait
+  int32_t* err;            // pinned host word
 };
 
 __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p) {
@@ -215,7 +215,7 @@ __device__ __forceinline__ bool nf_control(const NfArgs& a, uint32_t g, uint32_t
       // end.
       p.T = nf_threshold<kFloat>(__ldcg(&c->far.min_far), delta, a.inf);
       if (p.T <= p.t_old) {
-        *a.err_out = DAWN_ERR_TIMEOUT;
+        *a.err = DAWN_ERR_TIMEOUT;
         return false;
       }
     } else {
@@ -355,9 +355,9 @@ __global__ void __launch_bounds__(kNfBlock, 2) nf_traverse(const __grid_constant
           }
           idle = true;
         }
-        if (polls == kPollLimit) {
+        if (polls == a.polls) {
           if (lane == 0) {
-            *a.err_out = DAWN_ERR_TIMEOUT;
+            *a.err = DAWN_ERR_TIMEOUT;
             s_word[0] = 0;
           }
           break;
@@ -799,7 +799,7 @@ dawn_status nearfar_batch_fits(dawn_graph* g, int32_t nsrc, bool* fits) {
 }
 
 dawn_status nearfar_run(dawn_graph* g, const int32_t* d_sources, int32_t nb, int shift, int32_t* D,
-                        int32_t* levels_out, int32_t* push_out, int32_t* err_out) {
+                        int32_t* levels_out, int32_t* push_out) {
   DAWN_CHECK(shape_of(g));
   const size_t nn = (size_t)g->n;
   const bool fl = g->wtype == DAWN_W_F32;
@@ -829,7 +829,8 @@ dawn_status nearfar_run(dawn_graph* g, const int32_t* d_sources, int32_t nb, int
   a.inf = fl ? 0x7f7fffffu : 0x7fffffffu;
   a.levels_out = levels_out;
   a.push_out = push_out;
-  a.err_out = err_out;
+  a.polls = g->wait_polls;
+  a.err = g->h_err;
   // First step, in mean weights per mean out-degree.  A short step relaxes
   // few entries twice but takes more phases; which of the two costs more
   // depends on the work there is.  4 / 8 / 32 / 128: RMAT scale 22 2.14 /

@@ -363,6 +363,22 @@ dawn_status launch_cooperative(const SsFamily& fam, const void* fn, int ctas, in
   return DAWN_OK;
 }
 
+dawn_status device_status(dawn_graph* g) {
+  const int32_t e = *static_cast<volatile int32_t*>(g->h_err);
+  if (!e) return DAWN_OK;
+  DAWN_CUDA(cudaStreamSynchronize(g->stream));
+  *static_cast<volatile int32_t*>(g->h_err) = 0;
+  // what the launches expect as the last one should have left it: the arrivals of
+  // bfs_traverse, the touched bitmap, the accumulators of heavy rows, the counts
+  // of betweenness
+  release(g->bfs_sync);
+  release(g->bs_queues);
+  if (g->hv_acc.p) DAWN_CUDA(cudaMemsetAsync(g->hv_acc.p, 0, g->hv_acc.bytes, g->stream));
+  g->bc_blocks = 0;
+  set_error("a device wait ran out: the results of this call, or of an earlier one on this handle, are unfinished");
+  return e;
+}
+
 dawn_status ss_run(dawn_graph* g, SsFamily& fam, int32_t nruns, cudaGraphExec_t* exec) {
   if (g->trace && fam.probe) return ss_run_traced(g, fam, nruns);
   if (g->graphs_ok && !*exec) {

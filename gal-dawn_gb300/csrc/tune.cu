@@ -92,6 +92,7 @@ dawn_status time_sample(dawn_graph* g, const int32_t* src, int32_t k, bool batch
     DAWN_CUDA(cudaEventSynchronize(g->ev1));
     float t = 0.0f;
     DAWN_CUDA(cudaEventElapsedTime(&t, g->ev0, g->ev1));
+    DAWN_CHECK(device_status(g));
     if (best < 0.0f || t < best) best = t;
   }
   *ms = best;

@@ -281,6 +281,14 @@ dawn_status dawn_closeness(dawn_graph* g, const int32_t* sources,
  *                          cluster barrier per level).  0: every level runs
  *                          on the whole grid.  Distances are the same. */
 #define DAWN_OPT_SMALL_LEVELS 9
+/*   DAWN_OPT_WAIT_POLLS    polls after which a wait between the CTAs of one
+ *                          launch gives up with DAWN_ERR_TIMEOUT; 1..2^31-1,
+ *                          default 2^27 (over 30 s).  The results of such a
+ *                          call are unfinished.  Calls that synchronise with
+ *                          the host report it themselves, asynchronous ones
+ *                          through the next call on the handle or
+ *                          dawn_graph_synchronize; the handle stays usable. */
+#define DAWN_OPT_WAIT_POLLS 10
 
 /* Autotuner (no counterpart in the reference, whose launch shapes are fixed
  * in its tools, algorithm/gpu/mssp_gpu/mssp_gpu.cu:16-17).  Times the
