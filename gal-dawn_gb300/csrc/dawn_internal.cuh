@@ -163,6 +163,7 @@ struct PartRow {
   int32_t part;
 };
 constexpr int32_t kPartMaxVertices = DAWN_PART_MAX_VERTICES;
+constexpr int32_t kPushRatio = 4;  // what DAWN_OPT_PUSH_RATIO answers until it is set
 
 // Launch geometry for persistent grids on this device.
 struct Geometry {
@@ -251,7 +252,7 @@ struct dawn_graph {
   dawn::DevBuf hv_acc;          // per heavy row: OR accumulator + finished-segment count
   dawn::DevBuf hv_tasks;        // 2 x hv_segs (row, segment): segments of heavy rows still unfinished
   int32_t hv_count = 0, hv_segs = 0;
-  int32_t bs_push_ratio = 4;    // push while ratio * frontier edges < unfinished edges
+  int32_t bs_push_ratio = dawn::kPushRatio;  // push while ratio * frontier edges < unfinished edges
   bool bs_ratio_set = false;    // by the caller or the autotuner
   int32_t bs_width = 0;         // words per vertex of the bitset traversal (0 = by source count)
   int32_t force_variant = 0;    // 0 = decide per level, else 1 + variant for every level
@@ -375,6 +376,8 @@ constexpr int kLevelsEnd = 5;
 dawn_status bfs_bitset_levels(dawn_graph* g, int w, const int32_t* sources, int32_t nsrc, int32_t* d_levels,
                               int32_t* d_range, int32_t* h_end);
 int bitset_width(const dawn_graph* g, int32_t nsrc);
+// The push ratio of batched traversals until one is set.
+int default_push_ratio(const dawn_graph* g);
 // govm.cu
 dawn_status sssp_single(dawn_graph* g, const int32_t* sources, int32_t nsrc,
                         void* d_dist);

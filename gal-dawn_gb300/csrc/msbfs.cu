@@ -1892,11 +1892,7 @@ dawn_status run_width(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32
   BsCtl c = {};
   c.nsrc = nsrc;
   c.policy = DAWN_VARIANT_BITSET;
-  // Unless it was set, 2 from 16 entries a vertex on: there a push, which reads a
-  // frontier's rows once, beats a pull of half as many entries (4 / 2: RMAT-18, 500
-  // sources 859 / 794 us, closeness of 1,000 1798 / 1670, RMAT-16 x 64 168 / 149;
-  // RMAT-22 and Erdos-Renyi the same; grid 60 x 40 x 20 1165 / 1184).
-  c.push_ratio = g->bs_ratio_set || g->m < 16 * (int64_t)n ? g->bs_push_ratio : 2;
+  c.push_ratio = g->bs_ratio_set ? g->bs_push_ratio : default_push_ratio(g);
   c.nbits = nbits;
   c.width = W;
   c.dist_base = d_dist;
@@ -2007,6 +2003,12 @@ dawn_status run_width(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32
 }
 
 }  // namespace
+
+// 2 from 16 entries a vertex on: there a push, which reads a frontier's rows once,
+// beats a pull of half as many entries (4 / 2: RMAT-18, 500 sources 859 / 794 us,
+// closeness of 1,000 1798 / 1670, RMAT-16 x 64 168 / 149; RMAT-22 and Erdos-Renyi
+// the same; grid 60 x 40 x 20 1165 / 1184).
+int default_push_ratio(const dawn_graph* g) { return g->m < 16 * (int64_t)g->n ? kPushRatio : 2; }
 
 int bitset_width(const dawn_graph* g, int32_t nsrc) {
   if (g->bs_width > 0) return g->bs_width;

@@ -25,7 +25,7 @@ namespace dawn {
 namespace {
 
 struct Settings {
-  int32_t width, ratio, seg, bps, learned;
+  int32_t width, ratio, seg, bps, learned;  // ratio 0: none set (no batch was tuned)
 };
 
 std::mutex g_cache_mu;
@@ -58,8 +58,8 @@ std::string class_key(const dawn_graph* g, int32_t nsrc) {
 
 void apply(dawn_graph* g, const Settings& s) {
   g->bs_width = s.width;
-  g->bs_push_ratio = s.ratio;
-  g->bs_ratio_set = true;
+  g->bs_push_ratio = s.ratio ? s.ratio : kPushRatio;
+  g->bs_ratio_set = s.ratio != 0;
   g->pull_seg = s.seg;
   if (g->blocks_per_sm != s.bps) {
     g->blocks_per_sm = s.bps;
@@ -106,20 +106,21 @@ int32_t default_width(int32_t nsrc) { return nsrc > 128 ? 4 : nsrc > 64 ? 2 : 1;
 dawn_status autotune(dawn_graph* g, const int32_t* sources, int32_t nsrc, uint32_t flags, dawn_tuning* out) {
   std::memset(out, 0, sizeof(*out));
   const std::string key = class_key(g, nsrc);
+  const bool batched = nsrc >= 2;
   if (flags & DAWN_TUNE_USE_CACHE) {
     std::lock_guard<std::mutex> lock(g_cache_mu);
     auto it = g_cache.find(key);
     if (it != g_cache.end()) {
       *out = it->second;
       out->from_cache = 1;
-      apply(g, Settings{out->bitset_width, out->push_ratio, out->pull_segment, out->blocks_per_sm, out->learned});
+      apply(g, Settings{out->bitset_width, batched ? out->push_ratio : 0, out->pull_segment, out->blocks_per_sm,
+                        out->learned});
       return DAWN_OK;
     }
   }
-  const bool batched = nsrc >= 2;
   const int32_t k = batched ? (nsrc < 256 ? nsrc : 256) : 1;
   const int32_t ks = batched ? k : (nsrc < 4 ? nsrc : 4);
-  Settings cur{batched && nsrc > 64 ? default_width(nsrc) : 0, 4, 1024, 0, 0};
+  Settings cur{batched && nsrc > 64 ? default_width(nsrc) : 0, batched ? default_push_ratio(g) : 0, 1024, 0, 0};
   apply(g, cur);
   float cur_ms = 0.0f;
   // one untimed run builds the pull lists and the captured graphs
@@ -153,7 +154,7 @@ dawn_status autotune(dawn_graph* g, const int32_t* sources, int32_t nsrc, uint32
   DAWN_CHECK(try_values(&Settings::bps, {0, 1, 2, 4}));
 
   out->bitset_width = cur.width;
-  out->push_ratio = cur.ratio;
+  out->push_ratio = batched ? cur.ratio : kPushRatio;
   out->pull_segment = cur.seg;
   out->blocks_per_sm = cur.bps;
   out->learned = cur.learned;
