@@ -1173,10 +1173,15 @@ __device__ __forceinline__ void emit_vertex4(int32_t* __restrict__ dist, int32_t
 // 512 (closeness of 1,000 sources on RMAT-18, 1 / 2 / 4 / 8: 1603 / 1571 / 1584 /
 // 1610 us, 1717 with eight and 64-bit sums in shared memory).
 constexpr int kClosenessCtas = 2;
+// And in all: a CTA's sums are 32-bit, and exact while its share of the vertices (at
+// most 2^31 in all, dealt 256 at a time) times 31 levels stays below 2^32, on
+// however few SMs.
+constexpr int kClosenessMin = 16;
+static_assert(((1ull << 31) / kClosenessMin + 256) * (kDeepLevel - 1) < 1ull << 32, "a CTA's sums fit 32 bits");
 template <int W>
 __device__ __forceinline__ void emit_closeness(const Team& tm, const BsCtl* ctl, int batch, const u64* visit,
                                                const u64* slices, int32_t n, int nb, int nbits) {
-  __shared__ uint32_t s_sum[64 * W], s_cnt[64 * W];  // a CTA's vertices x 31 levels fit
+  __shared__ uint32_t s_sum[64 * W], s_cnt[64 * W];
   for (int t = threadIdx.x; t < 64 * W; t += blockDim.x) {
     s_sum[t] = 0;
     s_cnt[t] = 0;
@@ -1952,7 +1957,7 @@ dawn_status run_width(dawn_graph* g, const int32_t* sources, int32_t nsrc, int32
   const int nbatches = (nsrc + 64 * W - 1) / (64 * W);
   void* args[] = {&a};
   const int sms = g->geo.sms;
-  const int emit_ctas = cc_sum ? sms * kClosenessCtas : sms * 8;
+  const int emit_ctas = cc_sum ? std::max(sms * kClosenessCtas, kClosenessMin) : sms * 8;
   SsFamily fam;
   if (g->l2_persist) {
     // the three rotating frontier slots: every pull level gathers from one
