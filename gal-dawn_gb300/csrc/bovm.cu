@@ -1030,7 +1030,9 @@ __device__ __forceinline__ void solo_levels(const BfsArgs& a, const BfsStep& st,
     }
     __syncthreads();
     const int nf = sm.cnt[o];
-    if (nf == 0 || nf > kSoloKeep || sm.mf[o] > kSoloEdges || sm.deg[o] >= (uint32_t)kLongRow || L + 1 >= a.n) break;
+    if (nf == 0 || nf > kSoloKeep || sm.mf[o] > kSoloEdges || sm.deg[o] >= (uint32_t)kLongRow || L + 1 >= a.n ||
+        it + 1 == kSoloSteps)
+      break;
     sum_mf += sm.mf[o];
     last_nf = nf;
   }
@@ -1142,7 +1144,7 @@ __device__ __forceinline__ void mesh_levels(const BfsArgs& a, const BfsStep& st,
     }
     __syncthreads();
     const int nf = sm.cnt[o];
-    if (nf == 0 || nf > kMeshKeep || L + 1 >= a.n) break;
+    if (nf == 0 || nf > kMeshKeep || L + 1 >= a.n || it + 1 == kSoloSteps) break;
     last_nf = nf;
   }
   for (int i = threadIdx.x; i < a.nwords; i += kThreads) a.vbm[i] = vis[i];

@@ -79,6 +79,12 @@ struct Team {
   __device__ __forceinline__ size_t threads() const { return ctas * (size_t)blockDim.x; }
 };
 
+// Levels or phases that one CTA of a persistent launch runs alone before it gives
+// the decision back: the others poll meanwhile, for a limited number of times, and
+// a path of a hundred million vertices takes minutes.  32,768 take up to 0.3 s, and
+// the round trip after them 10 us.
+constexpr int kSoloSteps = 1 << 15;
+
 }  // namespace dawn
 
 namespace dawn {

@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(kNfBlock, 2) nf_traverse(const __grid_constant
         __syncthreads();
         // a warp that goes on writes the next phase's words, not these
         left = *nx_cnt;
-        if (left == 0 || left > (int)a.solo_max || s_long[o]) break;
+        if (left == 0 || left > (int)a.solo_max || s_long[o] || it + 1 == kSoloSteps) break;
       }
       if (threadIdx.x == 0 && it > 0) {
         atomicAdd(&ctl->far.iters, (uint32_t)it);
