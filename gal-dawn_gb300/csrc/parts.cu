@@ -849,9 +849,11 @@ int small_bits(int64_t np, size_t bytes) {
   return 0;
 }
 
-// Launch shape and scratch of the single-CTA tasks.  Small parts run as
-// smaller CTAs, more of them per SM, with the SM's memory shared out.
+// Launch shape, columns and scratch of the single-CTA tasks.  Small parts run as
+// smaller CTAs, more of them per SM, with the SM's memory shared out.  Until it
+// has succeeded, no part counts as small (pt_small_smem is 0).
 dawn_status small_slots(dawn_graph* g) {
+  g->pt_small_smem = 0;
   int optin = 0;
   DAWN_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, g->device));
   const size_t all = ((size_t)optin - 1024) & ~(size_t)127;
@@ -874,31 +876,33 @@ dawn_status small_slots(dawn_graph* g) {
     word_bytes = std::max(word_bytes, ((size_t)np * (size_t)(bits / 8) + 15) & ~(size_t)15);
     listed = std::max(listed, np);
   }
-  const int32_t nparts = (int32_t)g->pt_off.size() - 1;
-  const size_t n1 = (size_t)g->n + 1;
-  int64_t* tmp = nullptr;
-  DAWN_CHECK(pool_alloc((void**)&tmp, sizeof(int64_t) * 2 * n1, g->stream));
-  parts_pieces<<<g->geo.sms * 8, kBlock, 0, g->stream>>>(g->t_row_ptr, g->n, tmp);
-  DAWN_CUDA(cudaGetLastError());
-  DAWN_CHECK(exclusive_scan_i64(tmp, tmp + n1, (int64_t)n1, g->stream));
-  // a row of d entries takes at most d / 8 + 1 pieces
-  DAWN_CHECK(ensure(g->pt_tcol, sizeof(uint16_t) * ((size_t)g->m + 8 * n1), g->stream));
-  DAWN_CHECK(ensure(g->pt_toff, sizeof(int32_t) * n1, g->stream));
-  const int gx = std::min(nparts, 65535);
-  parts_local_cols<<<dim3(gx, (nparts + gx - 1) / gx, 8), kBlock, 0, g->stream>>>(
-      g->t_row_ptr, g->t_col, g->pt_voff.as<int32_t>(), nparts, tmp + n1, g->pt_toff.as<int32_t>(),
-      g->pt_tcol.as<uint16_t>());
-  DAWN_CUDA(cudaGetLastError());
-  pool_free(tmp, g->stream);
   const void* fn = small_kernel(threads);
   DAWN_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)all));
   DAWN_CUDA(cudaFuncSetAttribute(small_kernel(1024), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)all));
   g->pt_small_threads = threads;
-  g->pt_small_smem = smem;
   g->pt_small_ctas = persistent_blocks(fn, threads, smem);
   g->pt_small_words = word_bytes;
   g->pt_small_slot = ((1 + kPartDeep) * word_bytes + sizeof(int32_t) * ((size_t)listed / 8 + 64) + 127) & ~(size_t)127;
   DAWN_CHECK(ensure(g->pt_small, g->pt_small_slot * (size_t)g->pt_small_ctas, g->stream));
+  const int32_t nparts = (int32_t)g->pt_off.size() - 1;
+  const size_t n1 = (size_t)g->n + 1;
+  // a row of d entries takes at most d / 8 + 1 pieces
+  DAWN_CHECK(ensure(g->pt_tcol, sizeof(uint16_t) * ((size_t)g->m + 8 * n1), g->stream));
+  DAWN_CHECK(ensure(g->pt_toff, sizeof(int32_t) * n1, g->stream));
+  int64_t* tmp = nullptr;
+  DAWN_CHECK(pool_alloc((void**)&tmp, sizeof(int64_t) * 2 * n1, g->stream));
+  parts_pieces<<<g->geo.sms * 8, kBlock, 0, g->stream>>>(g->t_row_ptr, g->n, tmp);
+  dawn_status s = exclusive_scan_i64(tmp, tmp + n1, (int64_t)n1, g->stream);
+  if (s == DAWN_OK) {
+    const int gx = std::min(nparts, 65535);
+    parts_local_cols<<<dim3(gx, (nparts + gx - 1) / gx, 8), kBlock, 0, g->stream>>>(
+        g->t_row_ptr, g->t_col, g->pt_voff.as<int32_t>(), nparts, tmp + n1, g->pt_toff.as<int32_t>(),
+        g->pt_tcol.as<uint16_t>());
+  }
+  pool_free(tmp, g->stream);
+  DAWN_CHECK(s);
+  DAWN_CUDA(cudaGetLastError());
+  g->pt_small_smem = smem;
   return DAWN_OK;
 }
 
@@ -949,6 +953,40 @@ dawn_status cluster_slots(dawn_graph* g) {
   return DAWN_OK;
 }
 
+// Uploads offsets, reads the edge positions there and checks that no edge leaves
+// its part.  Waits for the stream.
+dawn_status read_parts(dawn_graph* g, int32_t nparts, const int32_t* offsets, DevBuf& voff,
+                       std::vector<long long>& pos) {
+  const size_t count = (size_t)nparts + 1;
+  DAWN_CHECK(ensure(voff, sizeof(int32_t) * count, g->stream));
+  DAWN_CUDA(cudaMemcpyAsync(voff.p, offsets, sizeof(int32_t) * count, cudaMemcpyHostToDevice, g->stream));
+  long long* d_pos = nullptr;  // and the flag behind them
+  DAWN_CHECK(pool_alloc((void**)&d_pos, sizeof(long long) * (count + 1), g->stream));
+  pos.assign(count + 1, 0);
+  int* const d_flag = reinterpret_cast<int*>(d_pos + count);
+  cudaError_t e = cudaMemsetAsync(d_flag, 0, sizeof(long long), g->stream);
+  parts_bounds<<<((int)count + kBlock - 1) / kBlock, kBlock, 0, g->stream>>>(g->row_ptr, voff.as<int32_t>(), (int)count,
+                                                                            d_pos);
+  if (!(g->flags & DAWN_GRAPH_NO_VALIDATE)) {
+    const int gx = std::min(nparts, 65535);
+    const int gy = (nparts + gx - 1) / gx;
+    parts_check<<<dim3(gx, gy), kBlock, 0, g->stream>>>(g->row_ptr, g->col, voff.as<int32_t>(), nparts, d_flag);
+  }
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(pos.data(), d_pos, sizeof(long long) * (count + 1), cudaMemcpyDeviceToHost, g->stream);
+  pool_free(d_pos, g->stream);
+  DAWN_CUDA(e);
+  DAWN_CUDA(cudaStreamSynchronize(g->stream));
+  const bool leaves = pos.back() != 0;
+  pos.pop_back();
+  if (leaves) {
+    set_error("parts: an edge leaves its part (the graph is not the disjoint union the offsets describe)");
+    return DAWN_ERR_INVALID_ARG;
+  }
+  return DAWN_OK;
+}
+
 }  // namespace
 
 dawn_status parts_set(dawn_graph* g, int32_t nparts, const int32_t* offsets) {
@@ -974,49 +1012,33 @@ dawn_status parts_set(dawn_graph* g, int32_t nparts, const int32_t* offsets) {
               maxn, kPartMaxVertices);
     return DAWN_ERR_INVALID_ARG;
   }
-  DAWN_CHECK(ensure(g->pt_voff, sizeof(int32_t) * ((size_t)nparts + 1), g->stream));
-  DAWN_CUDA(cudaMemcpyAsync(g->pt_voff.p, offsets, sizeof(int32_t) * ((size_t)nparts + 1), cudaMemcpyHostToDevice,
-                            g->stream));
-  {
-    long long* d_pos = nullptr;
-    DAWN_CHECK(pool_alloc((void**)&d_pos, sizeof(long long) * ((size_t)nparts + 1), g->stream));
-    parts_bounds<<<(nparts + 1 + kBlock - 1) / kBlock, kBlock, 0, g->stream>>>(g->row_ptr, g->pt_voff.as<int32_t>(),
-                                                                              nparts + 1, d_pos);
-    g->pt_pos.resize((size_t)nparts + 1);
-    const cudaError_t le = cudaGetLastError();
-    const cudaError_t ce = cudaMemcpyAsync(g->pt_pos.data(), d_pos, sizeof(long long) * ((size_t)nparts + 1),
-                                           cudaMemcpyDeviceToHost, g->stream);
-    pool_free(d_pos, g->stream);
-    DAWN_CUDA(le);
-    DAWN_CUDA(ce);
+  // The parts that a handle has stay as they are until the new ones are known to
+  // hold.
+  DevBuf voff;
+  std::vector<long long> pos;
+  const dawn_status read = read_parts(g, nparts, offsets, voff, pos);
+  if (read != DAWN_OK) {
+    release(voff);
+    return read;
   }
-  if (!(g->flags & DAWN_GRAPH_NO_VALIDATE)) {
-    int* d_flag = nullptr;
-    DAWN_CHECK(pool_alloc((void**)&d_flag, sizeof(int), g->stream));
-    DAWN_CUDA(cudaMemsetAsync(d_flag, 0, sizeof(int), g->stream));
-    const int gx = std::min(nparts, 65535);
-    const int gy = (nparts + gx - 1) / gx;
-    parts_check<<<dim3(gx, gy), kBlock, 0, g->stream>>>(g->row_ptr, g->col, g->pt_voff.as<int32_t>(), nparts,
-                                                         d_flag);
-    DAWN_CUDA(cudaGetLastError());
-    int flag = 0;
-    DAWN_CUDA(cudaMemcpyAsync(&flag, d_flag, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
-    pool_free(d_flag, g->stream);
-    DAWN_CUDA(cudaStreamSynchronize(g->stream));
-    if (flag) {
-      set_error("parts: an edge leaves its part (the graph is not the disjoint union the offsets describe)");
-      return DAWN_ERR_INVALID_ARG;
-    }
-  }
+  release(g->pt_voff);
+  g->pt_voff = voff;
+  g->pt_pos.swap(pos);
   g->pt_off.assign(offsets, offsets + nparts + 1);
   g->pt_maxn = maxn;
   g->pt_cluster_ready = false;
   if (g->pt_exec) {  // it holds the earlier parts' addresses and sizes
-    DAWN_CUDA(cudaStreamSynchronize(g->stream));
     cudaGraphExecDestroy(g->pt_exec);
     g->pt_exec = nullptr;
   }
-  DAWN_CHECK(small_slots(g));
+  const dawn_status small = small_slots(g);
+  if (small == DAWN_ERR_OOM) {  // then every part is a cluster's
+    cudaGetLastError();
+    clear_error();
+    for (DevBuf* b : {&g->pt_small, &g->pt_tcol, &g->pt_toff}) release(*b);
+  } else {
+    DAWN_CHECK(small);
+  }
   DAWN_CUDA(cudaStreamSynchronize(g->stream));
   return DAWN_OK;
 }
