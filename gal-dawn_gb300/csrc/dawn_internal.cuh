@@ -334,6 +334,8 @@ dawn_status sssp_batched_stats(dawn_graph* g, dawn_stats* st, int32_t nsrc);
 dawn_status nearfar_run(dawn_graph* g, const int32_t* d_sources, int32_t nb, int shift, int32_t* D,
                         int32_t* levels_out, int32_t* push_out);
 int nearfar_shift(int32_t nb);
+// Its buffers for nb sources (nearfar_run makes them too).
+dawn_status nearfar_reserve(dawn_graph* g, int32_t nb, int shift);
 // Whether batches of up to 64 of nsrc sources run through nearfar_run.
 dawn_status nearfar_batch_fits(dawn_graph* g, int32_t nsrc, bool* fits);
 

@@ -984,13 +984,19 @@ void probe_mw(const void* p, LevelProbe* out) {
   out->unvisited_edges = 0;
 }
 
+dawn_status ordered_buffers(dawn_graph* g, int32_t nsrc) {
+  const int32_t nb = std::min(kBatch, nsrc);
+  const int shift = nearfar_shift(nb);
+  DAWN_CHECK(ensure(g->mw_block, sizeof(int32_t) * ((size_t)g->n << shift), g->stream));
+  DAWN_CHECK(ensure(g->mw_ctl, sizeof(MwCtl), g->stream));
+  DAWN_CHECK(ensure(g->mw_sources, sizeof(int32_t) * (size_t)nsrc, g->stream));
+  return nearfar_reserve(g, nb, shift);
+}
+
 // Batches through the ordered traversal (nearfar.cu), which leaves the
 // distances in the vertex-major block that mw_emit writes out.
 dawn_status run_ordered(dawn_graph* g, const int32_t* sources, int32_t nsrc, void* d_dist) {
   const int shift = nearfar_shift(std::min(kBatch, nsrc));
-  DAWN_CHECK(ensure(g->mw_block, sizeof(int32_t) * ((size_t)g->n << shift), g->stream));
-  DAWN_CHECK(ensure(g->mw_ctl, sizeof(MwCtl), g->stream));
-  DAWN_CHECK(ensure(g->mw_sources, sizeof(int32_t) * (size_t)nsrc, g->stream));
   DAWN_CUDA(cudaMemcpyAsync(g->mw_sources.p, sources, sizeof(int32_t) * nsrc, cudaMemcpyHostToDevice, g->stream));
   MwCtl c = {};
   c.nsrc = nsrc;
@@ -1019,7 +1025,16 @@ dawn_status sssp_batched(dawn_graph* g, const int32_t* sources, int32_t nsrc, vo
   const int is_float = g->wtype == DAWN_W_F32;
   bool ordered = false;
   if (!g->force_variant && !g->trace && !g->negative_weights) DAWN_CHECK(nearfar_batch_fits(g, nsrc, &ordered));
-  if (ordered) return run_ordered(g, sources, nsrc, d_dist);
+  if (ordered) {
+    // The lists take 16 bytes per pair, 1 KB a vertex for 64 sources where the rows
+    // take 0.3: where they cannot be had, rows.
+    const dawn_status s = ordered_buffers(g, nsrc);
+    if (s == DAWN_OK) return run_ordered(g, sources, nsrc, d_dist);
+    if (s != DAWN_ERR_OOM) return s;
+    cudaGetLastError();
+    clear_error();
+    for (DevBuf* b : {&g->nf_queue, &g->nf_segbuf, &g->nf_masks}) release(*b);
+  }
   const size_t segcap = seg_capacity(n, g->m);
   DAWN_CHECK(ensure(g->mw_block, sizeof(int32_t) * kBatch * nn, g->stream));
   DAWN_CHECK(ensure(g->mw_masks, sizeof(unsigned long long) * 3 * nn, g->stream));

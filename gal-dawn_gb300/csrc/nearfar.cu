@@ -798,10 +798,33 @@ dawn_status nearfar_batch_fits(dawn_graph* g, int32_t nsrc, bool* fits) {
   return DAWN_OK;
 }
 
+namespace {
+
+// Lists, segments and masks of a traversal of nb sources.
+struct NfSizes {
+  size_t cap, segcap, nwords;
+  NfSizes(const dawn_graph* g, int32_t nb, int shift)
+      : cap((size_t)g->n * (size_t)nb),
+        segcap(g->nf_max_deg >= kLongRow ? (size_t)g->nf_segs * (size_t)nb + 64 : 64),
+        nwords((((size_t)g->n << shift) + 31) / 32) {}
+};
+
+}  // namespace
+
+dawn_status nearfar_reserve(dawn_graph* g, int32_t nb, int shift) {
+  DAWN_CHECK(shape_of(g));
+  const NfSizes z(g, nb, shift);
+  DAWN_CHECK(ensure(g->nf_ctl, sizeof(NfCtl), g->stream));
+  DAWN_CHECK(ensure(g->nf_queue, sizeof(int32_t) * 4 * z.cap, g->stream));
+  DAWN_CHECK(ensure(g->nf_segbuf, sizeof(Seg) * 2 * z.segcap, g->stream));
+  DAWN_CHECK(ensure(g->nf_masks, sizeof(uint32_t) * 3 * z.nwords, g->stream));
+  return DAWN_OK;
+}
+
 dawn_status nearfar_run(dawn_graph* g, const int32_t* d_sources, int32_t nb, int shift, int32_t* D,
                         int32_t* levels_out, int32_t* push_out) {
-  DAWN_CHECK(shape_of(g));
-  const size_t nn = (size_t)g->n;
+  DAWN_CHECK(nearfar_reserve(g, nb, shift));
+  const NfSizes z(g, nb, shift);
   const bool fl = g->wtype == DAWN_W_F32;
   NfArgs a = {};
   a.row_ptr = g->row_ptr;
@@ -812,16 +835,12 @@ dawn_status nearfar_run(dawn_graph* g, const int32_t* d_sources, int32_t nb, int
   a.shift = shift;
   a.nb = nb;
   a.sources = d_sources;
-  a.cap = nn * (size_t)nb;
-  a.nwords = ((nn << shift) + 31) / 32;
+  a.cap = z.cap;
+  a.nwords = z.nwords;
   a.has_long = g->nf_max_deg >= kLongRow;
-  a.segcap = a.has_long ? (size_t)g->nf_segs * (size_t)nb + 64 : 64;
-  DAWN_CHECK(ensure(g->nf_ctl, sizeof(NfCtl), g->stream));
+  a.segcap = z.segcap;
   // the arrival counts start at zero, also after a launch that gave up
   DAWN_CUDA(cudaMemsetAsync(g->nf_ctl.p, 0, sizeof(NfCtl), g->stream));
-  DAWN_CHECK(ensure(g->nf_queue, sizeof(int32_t) * 4 * a.cap, g->stream));
-  DAWN_CHECK(ensure(g->nf_segbuf, sizeof(Seg) * 2 * a.segcap, g->stream));
-  DAWN_CHECK(ensure(g->nf_masks, sizeof(uint32_t) * 3 * a.nwords, g->stream));
   a.ctl = g->nf_ctl.as<NfCtl>();
   a.queue = g->nf_queue.as<int32_t>();
   a.segs = g->nf_segbuf.as<Seg>();
