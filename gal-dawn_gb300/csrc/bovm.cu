@@ -1374,12 +1374,27 @@ dawn_status records(dawn_graph* g) {
     } else if (g->n > kMeshMax || (len > 8 && g->n > kMeshWide)) {
       len = kLevelKernels;
     } else {
-      DAWN_CHECK(ensure(g->bfs_rec, sizeof(int32_t) * (size_t)g->n * len, g->stream));
+      const dawn_status s = ensure(g->bfs_rec, sizeof(int32_t) * (size_t)g->n * len, g->stream);
+      if (s == DAWN_ERR_OOM) {  // not decided: the next call tries again
+        cudaGetLastError();
+        clear_error();
+        return DAWN_OK;
+      }
+      DAWN_CHECK(s);
       fill_records<<<g->geo.sms * 8, kBlock, 0, g->stream>>>(g->row_ptr, g->col, g->n, len, g->bfs_rec.as<int32_t>());
       DAWN_CUDA(cudaGetLastError());
     }
   }
   g->rec_len = len;
+  return DAWN_OK;
+}
+
+// What the persistent launch needs beside the level kernels' buffers.
+dawn_status persistent_buffers(dawn_graph* g, size_t lcap) {
+  DAWN_CHECK(ensure(g->bfs_long, sizeof(int32_t) * 2 * lcap, g->stream));
+  if (g->bfs_sync.p) return DAWN_OK;
+  DAWN_CHECK(ensure(g->bfs_sync, sizeof(BfsSync), g->stream));
+  DAWN_CUDA(cudaMemsetAsync(g->bfs_sync.p, 0, sizeof(BfsSync), g->stream));
   return DAWN_OK;
 }
 
@@ -1417,11 +1432,19 @@ dawn_status bfs_single(dawn_graph* g, const int32_t* sources, int32_t nsrc, int3
   DAWN_CHECK(ensure(g->ss_ctl, sizeof(SsCtl), g->stream));
   const int32_t force = g->force_variant == 3 ? 1 + kVarPush : g->force_variant;
   if (g->small_levels) DAWN_CHECK(records(g));
-  if (!g->trace && !(g->small_levels && g->rec_len == kLevelKernels)) {
-    if (!g->bfs_sync.p) {
-      DAWN_CHECK(ensure(g->bfs_sync, sizeof(BfsSync), g->stream));
-      DAWN_CUDA(cudaMemsetAsync(g->bfs_sync.p, 0, sizeof(BfsSync), g->stream));
+  const size_t lcap = (size_t)(m / kLongRow) + 1;
+  bool persistent = !g->trace && !(g->small_levels && g->rec_len == kLevelKernels);
+  if (persistent) {
+    const dawn_status s = persistent_buffers(g, lcap);
+    if (s == DAWN_ERR_OOM) {  // the level kernels need neither
+      cudaGetLastError();
+      clear_error();
+      persistent = false;
+    } else {
+      DAWN_CHECK(s);
     }
+  }
+  if (persistent) {
     BfsArgs a = {};
     a.row_ptr = g->row_ptr;
     a.col = g->col;
@@ -1432,8 +1455,7 @@ dawn_status bfs_single(dawn_graph* g, const int32_t* sources, int32_t nsrc, int3
     a.q = g->ss_queues.as<int32_t>();
     a.segs = g->ss_segs.as<Seg>();
     a.segcap = segcap;
-    a.lcap = (size_t)(m / kLongRow) + 1;
-    DAWN_CHECK(ensure(g->bfs_long, sizeof(int32_t) * 2 * a.lcap, g->stream));
+    a.lcap = lcap;
     a.lq = g->bfs_long.as<int32_t>();
     a.vbm = g->ss_bitmaps.as<uint32_t>();
     a.fbm = a.vbm + nwords;

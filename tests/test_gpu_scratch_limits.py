@@ -28,3 +28,22 @@ def test_ordered_batch_without_lists():
                 dg.sssp_device(srcs[:k], out.data_ptr())
                 assert np.array_equal(to_ref(out[:k].cpu().numpy()), want[:k]), k
             dg.close()
+
+
+def test_bfs_without_records():
+    # records of 1.5 M grid vertices 48 MB, the queues and bitmaps 13 and the segments
+    import torch
+    g = gen.grid(1250, 1200, seed=3)
+    srcs = np.array([0, g.n // 2], np.int32)
+    want = O.hops_ref_to_api(O.mssp(g, srcs)[0], srcs)
+    out = torch.empty((2, g.n), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    with abi.Graph(g) as dg:
+        with pool_limit(32 << 20):
+            for _ in range(2):
+                out.fill_(0)
+                torch.cuda.synchronize()
+                dg.bfs_device(srcs, out.data_ptr(), variant=abi.VARIANT_DO)
+                assert np.array_equal(out.cpu().numpy(), want)
+        dg.bfs_device(srcs, out.data_ptr(), variant=abi.VARIANT_DO)  # with them
+        assert np.array_equal(out.cpu().numpy(), want)
