@@ -209,15 +209,10 @@ __device__ __forceinline__ bool nf_control(const NfArgs& a, uint32_t g, uint32_t
     }
     uint32_t delta = __ldcg(&c->far.delta);
     p.t_old = p.T;
-    if (p.kind == kPhFar) {
-      // The scan moved nothing: step past the gap.  Every pair left lies above T
-      // and below `inf`, so T rises; a launch in which it does not would never
-      // end.
+    const bool scanned = p.kind == kPhFar;
+    if (scanned) {
+      // the scan moved nothing: step past the gap
       p.T = nf_threshold<kFloat>(__ldcg(&c->far.min_far), delta, a.inf);
-      if (p.T <= p.t_old) {
-        *a.err = DAWN_ERR_TIMEOUT;
-        return false;
-      }
     } else {
       const uint32_t iters = __ldcg(&c->far.bucket_iters);
       const unsigned long long pairs = __ldcg(&c->far.bucket_pairs);
@@ -237,6 +232,13 @@ __device__ __forceinline__ bool nf_control(const NfArgs& a, uint32_t g, uint32_t
     p.fcur ^= 1;
     p.n = far_n;
     p.ctas = nf_ctas(far_n, kNfBlock);
+    // Every pair that a scan leaves lies above T and below `inf`, so T rises past
+    // it; a launch in which it does not would never end.  (After a near list T may
+    // stay where it is: a step below its rounding.)
+    if (scanned && p.T <= p.t_old) {
+      *a.err = DAWN_ERR_TIMEOUT;
+      p.ctas = 0;
+    }
   }
   c->cnt[(g + 2) & 3].tally = 0;
   c->cnt[(g + 2) & 3].lpack = 0;
@@ -291,7 +293,7 @@ __global__ void __launch_bounds__(kNfBlock, 2) nf_traverse(const __grid_constant
   __shared__ uint32_t s_nn[kNfWarps], s_nf[kNfWarps];
   __shared__ unsigned long long s_word[4];
   __shared__ Solo s_solo[2];
-  __shared__ int32_t s_cnt[3], s_long[3];  // of the lists of three phases in a row
+  __shared__ int2 s_cl[3];  // lists of three phases in a row: entries, and whether a long row is among them
   const int shift = a.shift;
   const uint32_t smask = (1u << shift) - 1u;
   NfCtl* const ctl = a.ctl;
@@ -505,19 +507,17 @@ __global__ void __launch_bounds__(kNfBlock, 2) nf_traverse(const __grid_constant
         clear_pair(near_in, p);
       }
       if (threadIdx.x == 0) {
-        s_cnt[0] = (int)ph.n;
-        s_cnt[1] = s_cnt[2] = 0;
-        s_long[0] = s_long[1] = s_long[2] = 0;
+        s_cl[0] = make_int2((int)ph.n, 0);
+        s_cl[1] = s_cl[2] = make_int2(0, 0);
       }
       __syncthreads();
       int left = 0, it = 0;
       for (;; it++) {
-        const int cnt = s_cnt[it % 3];
+        const int cnt = s_cl[it % 3].x;
         const Solo& in = s_solo[it & 1];
         Solo& nx = s_solo[(it & 1) ^ 1];
-        const int o = (it + 1) % 3;
-        int32_t* const nx_cnt = &s_cnt[o];
-        if (threadIdx.x == 0) s_cnt[(it + 2) % 3] = s_long[(it + 2) % 3] = 0;
+        int32_t* const nx_cnt = &s_cl[(it + 1) % 3].x;
+        if (threadIdx.x == 0) s_cl[(it + 2) % 3] = make_int2(0, 0);
         auto push = [&](auto& k, auto& ok, auto& d, auto& src) {
           constexpr int kU = sizeof(k) / sizeof(k[0]);
           uint32_t pu[kU], c[kU];
@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(kNfBlock, 2) nf_traverse(const __grid_constant
               nx.p[base] = pu[i];
               nx.rs[base] = rs[i];
               nx.deg[base] = re[i] - rs[i];
-              if (re[i] - rs[i] >= kLongRow) s_long[o] = 1;
+              if (re[i] - rs[i] >= kLongRow) nx_cnt[1] = 1;
             }
             bool over = near && base >= kSoloCap;
             if (over) over = set_pair(near_out, pu[i]);
@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(kNfBlock, 2) nf_traverse(const __grid_constant
         __syncthreads();
         // a warp that goes on writes the next phase's words, not these
         left = *nx_cnt;
-        if (left == 0 || left > (int)a.solo_max || s_long[o] || it + 1 == kSoloSteps) break;
+        if (left == 0 || left > (int)a.solo_max || nx_cnt[1] || it + 1 == kSoloSteps) break;
       }
       if (threadIdx.x == 0 && it > 0) {
         atomicAdd(&ctl->far.iters, (uint32_t)it);

@@ -35,3 +35,26 @@ def test_long_rows_come_and_go(leaves, spacing):
                 assert np.array_equal(to_ref(d), want[:1])
                 d, _ = dg.sssp(srcs)
                 assert np.array_equal(to_ref(d), want)
+
+
+def test_threshold_below_its_own_rounding():
+    # a distance of 1e11 behind an edge that the sample of the weights misses: the
+    # threshold's step, some mean weights of 1, does not raise it at all, and pairs
+    # beyond it are reached by the least distance that a scan leaves
+    m = 200000
+    w = np.ones(m, np.float32)
+    free = np.setdiff1d(np.arange(m), np.arange(65536, dtype=np.int64) * m // 65536)
+    w[free[0]] = 1e11
+    w[free[5::700]] = 1e6
+    k = np.arange(m)
+    g = weighted(m + 1, k, k + 1, np.ones(m))
+    g.w_f32 = w
+    want = np.zeros(m + 1, np.float32)
+    for i in range(m):
+        want[i + 1] = want[i] + w[i]
+    assert np.float32(1e11) + np.float32(512 * 16) > np.float32(1e11) == np.float32(1e11) + np.float32(512)
+    with abi.Graph(g, weights="f32") as dg:
+        d, _ = dg.sssp([0], variant=abi.VARIANT_DO)
+        assert np.array_equal(d[0], want)
+        d, _ = dg.sssp([0, 0, 0])
+        assert (d == want).all()
