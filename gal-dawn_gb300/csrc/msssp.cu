@@ -85,6 +85,7 @@ struct MwCtl {
 enum : int32_t { kRest = 0, kLight = 1, kAll = 2 };
 constexpr int kBoundedFrom = 4;   // level from which pulls go by bounds: before it most of a row is unreached
 constexpr int kLightLevels = 24;  // light pulls at most
+constexpr long long kBoundDegree = 14;  // mean degree from which pulls without a hub go by bounds
 
 __device__ __forceinline__ int32_t relax(int32_t d, int32_t w, bool is_float) {
   if (is_float) return __float_as_int(__fadd_rn(__int_as_float(d), __int_as_float(w)));
@@ -836,11 +837,13 @@ __global__ void __launch_bounds__(kBlock) mw_collect(const int32_t* __restrict__
                                                      const unsigned long long* __restrict__ masks,
                                                      int32_t* __restrict__ q, Seg* __restrict__ segs, size_t segcap,
                                                      int32_t n) {
-  __shared__ int32_t s_q[kBlock / 32][kWarpQueue];
+  __shared__ int32_t s_q[kBlock / 32][kWarpQueueBig];
+  __shared__ uint32_t s_n[kBlock / 32];
+  __shared__ unsigned long long s_mf;
   if (ctl->done || ctl->mode != kModePull || ctl->stage == kLight) return;
   const int pout = ctl->level & 1, lane = lane_id(), wib = threadIdx.x >> 5;
   const unsigned long long* m_out = masks + (size_t)(ctl->level % 3) * n;
-  WarpQueue wq(s_q[wib], q + (size_t)pout * n, &ctl->qsize[pout]);
+  WarpQueueBig wq(s_q[wib], q + (size_t)pout * n, &ctl->qsize[pout]);
   unsigned long long my_mf = 0;
   for (int v0 = global_warp() * 32; v0 < n; v0 += num_warps() * 32) {
     const int v = v0 + lane;
@@ -850,9 +853,25 @@ __global__ void __launch_bounds__(kBlock) mw_collect(const int32_t* __restrict__
     my_mf += (unsigned long long)deg;
     emit_routed(in, v, deg, rs, wq, segs + (size_t)pout * segcap, &ctl->lpack[pout]);
   }
-  wq.flush();
+  // One reservation and one sum per CTA: per warp, and with a quarter of the
+  // staging, they were 20,000 atomics on one word where every vertex has improved
+  // (25 us a pass of 1 M vertices, 8 so).
+  if (threadIdx.x == 0) s_mf = 0;
+  if (lane == 0) s_n[wib] = (uint32_t)wq.n;
+  __syncthreads();
   my_mf = warp_sum(my_mf);
-  if (lane == 0 && my_mf) atomicAdd(&ctl->mf[pout], my_mf);
+  if (lane == 0 && my_mf) atomicAdd(&s_mf, my_mf);
+  if (wib == 0) {
+    const int x = lane < kBlock / 32 ? (int)s_n[lane] : 0;
+    const int incl = warp_incl_scan(x), tot = __shfl_sync(kFull, incl, 31);
+    int base = 0;
+    if (tot && lane == 0) base = atomicAdd(wq.count, tot);
+    base = __shfl_sync(kFull, base, 0);
+    if (lane < kBlock / 32) s_n[lane] = (uint32_t)(base + incl - x);
+  }
+  __syncthreads();
+  for (int i = lane; i < wq.n; i += 32) wq.out[s_n[wib] + i] = wq.buf[i];
+  if (threadIdx.x == 0 && s_mf) atomicAdd(&ctl->mf[pout], s_mf);
 }
 
 __global__ void mw_decide(MwCtl* __restrict__ ctl, int32_t n, long long m, int can_pull,
@@ -893,11 +912,15 @@ __global__ void mw_decide(MwCtl* __restrict__ ctl, int32_t n, long long m, int c
     if (ctl->force) ctl->mode = ctl->force == 2 ? kModePull : kModePush;
     else ctl->mode = can_pull && 2 * (long long)ctl->mf[pout] >= m ? kModePull : kModePush;
   }
-  // without a hub bounds tell nothing while most pairs still improve
+  // Without a hub bounds tell nothing while most pairs still improve, and spare too
+  // little of short rows later on: a pass over the block costs 75 us per million
+  // vertices (bounded / not: Erdos-Renyi, 64 sources, mean degree 12 11.6 / 11.2 ms,
+  // 16 11.8 / 12.3, 22 12.9 / 14.0, 30 4.0 / 4.3).
   ctl->bounded = ctl->stage == kAll ||
                  (L + 1 >= kBoundedFrom &&
                   (ctl->has_hub ||
-                   (pulled && 2 * ctl->pairs < (unsigned long long)n * min(kBatch, ctl->nsrc - ctl->batch * kBatch))));
+                   (m >= kBoundDegree * n && pulled &&
+                    2 * ctl->pairs < (unsigned long long)n * min(kBatch, ctl->nsrc - ctl->batch * kBatch))));
   ctl->pairs = 0;
   ctl->work = 0;
   ctl->hwork = 0;
