@@ -232,8 +232,9 @@ struct dawn_graph {
   dawn::DevBuf wt_val;      // and weight of each in-edge, built on the first weighted pull, light entries first
   dawn::DevBuf wt_light;    // end of the light entries of each row
   int32_t wt_hub = 0;       // vertex of most in-edges
-  bool wt_has_hub = false;  // it has many times the mean
-  bool wt_has_light = false;  // the light entries are a part of the rows worth a stage of their own
+  bool wt_has_light = false;  // the light entries are worth a stage of their own, and the hub bounds by it
+  bool light_read = false, light_pays = false;  // light_weights
+  uint32_t light_most = 0;  // word of the largest light weight
   dawn::DevBuf mw_bounds;   // batched: per vertex, lowest and highest distance over the sources (mw_bounds)
   dawn::SsCtl* h_ctl = nullptr;  // pinned: [0] upload staging, [1] download
   int32_t* h_err = nullptr;      // pinned: status that a launch of this handle wrote (device_status), 0 = none
@@ -412,6 +413,8 @@ bool cluster_fits(const void* fn, int ctas, int threads);
 dawn_status build_transpose(dawn_graph* g);
 // In-edge tails and weights in the row layout of t_row_ptr (g->wt_col, g->wt_val).
 dawn_status build_weighted_in_edges(dawn_graph* g);
+// Sets light_most and light_pays, once per handle.
+dawn_status light_weights(dawn_graph* g);
 // msbfs.cu: light/heavy in-degree lists of the pull kernels (g->ul_static, g->hv_*).
 dawn_status build_static_list(dawn_graph* g);
 // Per-row reductions over a distance block (kind 0 hops, 1 int32, 2 float):

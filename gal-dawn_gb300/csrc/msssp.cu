@@ -1074,7 +1074,7 @@ dawn_status sssp_batched(dawn_graph* g, const int32_t* sources, int32_t nsrc, vo
   MwCtl c = {};
   // negative weights: pushes alone, which compare distances as signed words
   c.force = g->negative_weights ? 1 : g->force_variant;
-  c.has_hub = g->wt_has_hub;
+  c.has_hub = g->wt_has_light;
   c.has_light = !c.force && g->wt_has_light;
   c.nsrc = nsrc;
   c.dist_base = static_cast<int32_t*>(d_dist);
@@ -1102,7 +1102,7 @@ dawn_status sssp_batched(dawn_graph* g, const int32_t* sources, int32_t nsrc, vo
   a.t_light = g->wt_light.as<int32_t>();
   a.bounds = g->mw_bounds.as<int2>();
   a.hub = g->wt_hub;
-  a.whole_rows = !g->wt_has_hub;
+  a.whole_rows = !g->wt_has_light;
   a.t_row_ptr = g->t_row_ptr;
   a.t_col = g->wt_col.as<int32_t>();
   a.t_w = g->wt_val.as<int32_t>();  // int32 weights or float32 bit patterns, in in-edge order

@@ -680,46 +680,70 @@ __global__ void sample_weights(const int32_t* __restrict__ val, long long m, int
 
 }  // namespace
 
-// In-edges with their weights, a row's light entries first: about three a vertex
-// by a sample of the weights (an eighth to a half of them), for the batched
-// traversal, which reaches most of its distances through these alone.  No row
-// has light entries of its own where the weights do not tell them apart.
+// The light weights, from a sample of 4,096: about three entries a vertex (an eighth
+// to a half of them).  A stage of their own pays where two of them in a row are
+// shorter than most other edges.  64 sources on RMAT-18, ms with the stage / without
+// / whole pulls alone: lengths 1-63 1.25 / 1.9 / 2.5, 1-4 1.49 / 1.66 / 1.88, 1-3
+// 1.56 / 1.60 / 1.83, 1-2 1.93 / 1.50 / 1.54, 61-123 1.95 / 1.51 / 1.55, equal
+// 2.1 / 1.48 / 1.50; on RMAT-20 with four entries a vertex 1-63 2.4 / 3.5 / 3.4.
+dawn_status light_weights(dawn_graph* g) {
+  if (g->light_read) return DAWN_OK;
+  constexpr int kSamples = 4096;
+  constexpr double kHeavier = 2.6;  // mean of the others, in means of the light ones
+  const int samples = (int)std::min<int64_t>(g->m, kSamples);
+  g->light_most = 0;
+  g->light_pays = false;
+  if (samples > 0) {
+    std::vector<uint32_t> w((size_t)samples);
+    int32_t* d = nullptr;
+    DAWN_CHECK(pool_alloc((void**)&d, sizeof(int32_t) * w.size(), g->stream));
+    sample_weights<<<16, kBlock, 0, g->stream>>>(static_cast<const int32_t*>(g->val), g->m, samples, d);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(w.data(), d, sizeof(uint32_t) * w.size(), cudaMemcpyDeviceToHost, g->stream);
+    pool_free(d, g->stream);
+    DAWN_CUDA(e);
+    DAWN_CUDA(cudaStreamSynchronize(g->stream));
+    const double share = std::min(0.5, std::max(0.125, 3.0 * g->n / (double)g->m));
+    std::sort(w.begin(), w.end());
+    g->light_most = w[(size_t)(share * (double)(w.size() - 1))];
+    double sum[2] = {0.0, 0.0};
+    size_t cnt[2] = {0, 0};
+    for (uint32_t x : w) {
+      float f;
+      std::memcpy(&f, &x, sizeof(f));
+      const int heavy = x > g->light_most;
+      sum[heavy] += g->wtype == DAWN_W_F32 ? (double)f : (double)x;
+      cnt[heavy]++;
+    }
+    g->light_pays = (double)cnt[0] <= 0.6 * samples && kHeavier * sum[0] / cnt[0] < sum[1] / cnt[1];
+  }
+  g->light_read = true;
+  return DAWN_OK;
+}
+
+// In-edges with their weights, a row's light entries first, for the batched
+// traversal, which reaches most of its distances through these alone.
 dawn_status build_weighted_in_edges(dawn_graph* g) {
   if (g->wt_col.p) return DAWN_OK;
   const int32_t n = g->n;
   const cudaStream_t s = g->stream;
   const int grid = g->geo.sms * 8;
-  constexpr int kSamples = 4096;
   constexpr double kHubDegree = 16.0;  // in mean degrees
+  DAWN_CHECK(light_weights(g));
   int2* cursor = nullptr;
-  unsigned long long* hub = nullptr;
-  int32_t* sample = nullptr;
-  DAWN_CHECK(pool_alloc((void**)&cursor, sizeof(int2) * (size_t)n + sizeof(unsigned long long) + 4 * kSamples, s));
-  hub = reinterpret_cast<unsigned long long*>(cursor + n);
-  sample = reinterpret_cast<int32_t*>(hub + 1);
+  DAWN_CHECK(pool_alloc((void**)&cursor, sizeof(int2) * (size_t)n + sizeof(unsigned long long), s));
+  unsigned long long* const hub = reinterpret_cast<unsigned long long*>(cursor + n);
   DAWN_CUDA(cudaMemsetAsync(hub, 0, sizeof(*hub), s));
-  std::vector<uint32_t> w((size_t)std::min<int64_t>(g->m, kSamples));
-  uint32_t most = 0;
-  g->wt_has_light = false;
-  if (!w.empty()) {
-    sample_weights<<<16, kBlock, 0, s>>>(static_cast<const int32_t*>(g->val), g->m, (int)w.size(), sample);
-    DAWN_CUDA(cudaGetLastError());
-    DAWN_CUDA(cudaMemcpyAsync(w.data(), sample, 4 * w.size(), cudaMemcpyDeviceToHost, s));
-    DAWN_CUDA(cudaStreamSynchronize(s));
-    const double share = std::min(0.5, std::max(0.125, 3.0 * n / (double)g->m));
-    std::sort(w.begin(), w.end());
-    most = w[(size_t)(share * (double)(w.size() - 1))];
-    const size_t cnt = (size_t)(std::upper_bound(w.begin(), w.end(), most) - w.begin());
-    g->wt_has_light = (double)cnt <= 0.6 * (double)w.size();
-  }
   DAWN_CHECK(ensure(g->wt_light, sizeof(int32_t) * (size_t)n, s));
   DAWN_CHECK(ensure(g->wt_val, sizeof(int32_t) * (size_t)(g->m > 0 ? g->m : 1) + 16, s));
   DAWN_CHECK(ensure(g->wt_col, sizeof(int32_t) * (size_t)(g->m > 0 ? g->m : 1) + 16, s));
   init_cursors<<<grid, kBlock, 0, s>>>(g->t_row_ptr, cursor, n);
   DAWN_CUDA(cudaGetLastError());
   // 32-bit weights (int32 or float32 bit patterns, not negative) move as words
-  scatter_weighted_in_edges<<<grid, kBlock, 0, s>>>(g->row_ptr, g->col, static_cast<const int32_t*>(g->val), n, most,
-                                                    cursor, g->wt_col.as<int32_t>(), g->wt_val.as<int32_t>());
+  scatter_weighted_in_edges<<<grid, kBlock, 0, s>>>(g->row_ptr, g->col, static_cast<const int32_t*>(g->val), n,
+                                                    g->light_most, cursor, g->wt_col.as<int32_t>(),
+                                                    g->wt_val.as<int32_t>());
   DAWN_CUDA(cudaGetLastError());
   finish_weighted_in_edges<<<g->geo.sms * 4, kBlock, 0, s>>>(g->t_row_ptr, cursor, n, g->wt_light.as<int32_t>(), hub);
   DAWN_CUDA(cudaGetLastError());
@@ -728,9 +752,9 @@ dawn_status build_weighted_in_edges(dawn_graph* g) {
   pool_free(cursor, s);
   DAWN_CUDA(cudaStreamSynchronize(s));
   g->wt_hub = (int32_t)(uint32_t)h;
-  // without a hub the bounds leave too much for a light stage to pay
-  g->wt_has_hub = (double)(h >> 32) * n >= kHubDegree * (double)g->m;
-  g->wt_has_light = g->wt_has_light && g->wt_has_hub;
+  // Without a hub the bounds leave too much for a light stage to pay, and without a
+  // light stage they leave too much of a hub's rows: both or neither.
+  g->wt_has_light = g->light_pays && (double)(h >> 32) * n >= kHubDegree * (double)g->m;
   return DAWN_OK;
 }
 
