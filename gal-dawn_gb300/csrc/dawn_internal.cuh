@@ -163,6 +163,7 @@ struct PartRow {
   int32_t part;
 };
 constexpr int32_t kPartMaxVertices = DAWN_PART_MAX_VERTICES;
+constexpr double kHubDegree = 16.0;  // entries of a hub's row, in mean degrees
 constexpr int32_t kPushRatio = 4;  // what DAWN_OPT_PUSH_RATIO answers until it is set
 
 // Launch geometry for persistent grids on this device.
@@ -202,6 +203,7 @@ struct dawn_graph {
   int32_t bfs_ctas = 0, bfs_cap = 0;
   dawn::DevBuf bfs_rec;     // rows of low degree as records (single-source BFS)
   int32_t max_row = -1;     // entries of the longest row (-1: not read yet)
+  double growth = -1.0;     // per level (read_growth; -1: not read yet)
   int32_t rec_len = -1;     // words of a record; 0: none, -1: not decided, -2: level kernels instead
   dawn::DevBuf bfs_sync;    // BfsSync: what the CTAs of the persistent BFS wait on
   dawn::DevBuf ss_sources;  // int32 source list of the current call (ordered weighted: a control block before it)
@@ -391,6 +393,13 @@ dawn_status ss_run(dawn_graph* g, SsFamily& fam, int32_t nsrc,
 dawn_status ss_run_traced(dawn_graph* g, SsFamily& fam, int32_t nruns);
 // Sets max_row, once per handle.
 dawn_status longest_row(dawn_graph* g);
+// Sets growth, once per handle: by what factor a level widens the neighbourhood of a
+// vertex, on average until it holds 8,192 vertices or half of them.  Random graphs
+// grow by about their mean degree; meshes, road networks and kNN graphs by 1.1 to
+// 1.7, whatever their degree, and take hundreds of levels.  (For graphs of low
+// degree: a row is one warp's.)
+dawn_status read_growth(dawn_graph* g);
+constexpr double kGrows = 2.0;
 // The status of the handle's launches that the host has waited for: not DAWN_OK
 // once after a wait between the CTAs of a launch gave up.  Every call on a handle
 // asks at its start (for what earlier calls left enqueued) and after its own last

@@ -777,24 +777,39 @@ int nearfar_shift(int32_t nb) {
   return shift == 1 ? 2 : shift;  // rows of at least 16 bytes in a batch
 }
 
-// Where the pairs beat the 64-source rows of msssp.cu (measured, float32
-// weights, ms ordered / by rows; ER: 200,000 vertices):
-//   mean degree 12: 5 sources 0.51 / 1.54, 32: 1.67 / 2.16, 50: 2.59 / 2.22
-//   mean degree 20: 16 sources 1.39 / 2.14, 32: 2.18 / 2.41, 50: 3.35 / 2.63
-//   RMAT scale 14: 64 sources 1.14 / 1.57
-//   RMAT scale 18: 4 sources 0.81 / 2.54, 16: 2.43 / 2.69, 32: 4.43 / 3.18
-//   RMAT scale 22: 4 sources 7.7 / 14.2, 12: 30.2 / 17.4
-// The pairs take about 16 ps per entry and source, the rows 1.3 ms of levels
-// and 120 ps per entry whatever the number of sources: the line below.  On
-// graphs of low degree without hubs (meshes, street networks) the rows take
-// hundreds of levels and lose by 5 to 6 times at any number of sources (kNN
-// mesh, 50 sources: 10.0 / 56.9).
+// Where the pairs beat the rows of msssp.cu.  The pairs cost 13 to 60 ps per entry
+// and source, the more the less of the block fits L2; the rows have a price per
+// entry that 64 sources pay as well as two, so the line lies in the sources beyond a
+// few times the entries.  Measured, ms ordered / by rows, int32 lengths 1 to 63 (m:
+// million entries):
+//   hub, light stage:  RMAT-14 (0.4 m) 32 sources 0.67 / 0.77, 48 1.34 / 0.81; RMAT-16 (1.0)
+//     16 0.69 / 0.87, 24 1.26 / 0.89; RMAT-18 (7.6) 4 0.69 / 0.90, 6 1.16 / 0.96;
+//     RMAT-20 (15.7) 2 1.09 / 1.61, 4 1.88 / 1.81; RMAT-22 (128) 2 3.7 / 5.3, 4 6.2 / 5.8
+//   hub, equal lengths: RMAT-18 16 1.00 / 1.32, 24 1.51 / 1.35; RMAT-20 16 2.35 / 2.25
+//   no hub: Erdos-Renyi 300,000 x 8 32 1.96 / 2.68, 48 3.14 / 2.91; 1 M x 4 32 5.7 / 6.9,
+//     48 11.9 / 8.0; 1 M x 12 24 8.7 / 8.7; 1 M x 22 16 6.0 / 9.6, 24 12.1 / 10.3; 2 M x 6 16
+//     8.2 / 13.2, 24 16.2 / 14.4; 4 M x 16 16 37.4 / 37.8
+//   meshes: kNN of 100,000, 64 sources 6.9 / 30.9; grid 300 x 300 5.7 / 34.7: the rows take
+//     hundreds of levels, at any number of sources
+// A graph of low degree without long rows is a mesh if it does not grow like a random
+// one.
+constexpr int64_t kNfLine = 72000000, kNfLightLine = 13000000;
+
 dawn_status nearfar_batch_fits(dawn_graph* g, int32_t nsrc, bool* fits) {
   *fits = false;
   const int32_t nb = nsrc < 64 ? nsrc : 64;
   if ((int64_t)g->n << nearfar_shift(nb) > kNfMaxPairs) return DAWN_OK;
   DAWN_CHECK(shape_of(g));
-  *fits = (g->nf_max_deg < kLongRow && g->m < 10 * (int64_t)g->n) || (int64_t)(nb - 7) * g->m <= 70000000;
+  if ((double)g->nf_max_deg * g->n >= kHubDegree * (double)g->m) {
+    if ((nb - 3) * g->m > kNfLightLine) DAWN_CHECK(light_weights(g));
+    *fits = (nb - 3) * g->m <= kNfLightLine || (!g->light_pays && (nb - 12) * g->m <= kNfLine);
+    return DAWN_OK;
+  }
+  *fits = (nb - 16) * g->m <= kNfLine;
+  if (!*fits && g->nf_max_deg < kLongRow && g->m < 10 * (int64_t)g->n) {
+    DAWN_CHECK(read_growth(g));
+    *fits = g->growth < kGrows;
+  }
   return DAWN_OK;
 }
 

@@ -4,6 +4,7 @@
 // closeness reductions.
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 #include <utility>
@@ -538,6 +539,95 @@ dawn_status longest_row(dawn_graph* g) {
   return DAWN_OK;
 }
 
+// --- growth ---------------------------------------------------------------------
+
+namespace {
+
+constexpr int kGrowthSamples = 4, kGrowthReach = 8192, kGrowthLevels = 16;
+
+// How fast the neighbourhoods of a few vertices grow: one CTA per sample walks
+// levels until it has seen `reach` vertices, for kGrowthLevels at most.
+// out: levels, vertices seen.
+__global__ void __launch_bounds__(1024) grow(const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ col,
+                                             int32_t n, int reach, uint32_t* bitmaps, size_t nwords, int32_t* queues,
+                                             int2* __restrict__ out) {
+  __shared__ int s_count, s_start;
+  uint32_t* const seen = bitmaps + blockIdx.x * nwords;
+  int32_t* const q = queues + (size_t)blockIdx.x * reach;
+  const int lane = lane_id();
+  if (threadIdx.x == 0) s_start = n;
+  __syncthreads();
+  // the first vertex with a row, of 1,024 from the sample's place on
+  const int32_t v0 = (int32_t)((long long)n * (2 * blockIdx.x + 1) / (2 * kGrowthSamples));
+  if (threadIdx.x < n - v0 && row_ptr[v0 + threadIdx.x] < row_ptr[v0 + threadIdx.x + 1])
+    atomicMin(&s_start, v0 + (int)threadIdx.x);
+  __syncthreads();
+  if (s_start == n) {
+    if (threadIdx.x == 0) out[blockIdx.x] = make_int2(0, 0);
+    return;
+  }
+  if (threadIdx.x == 0) {
+    q[0] = s_start;
+    seen[s_start >> 5] |= 1u << (s_start & 31);
+    s_count = 1;
+  }
+  int lo = 0, L = 0;
+  for (;; L++) {
+    __syncthreads();
+    const int hi = s_count;
+    __syncthreads();
+    if (hi >= reach || hi == lo || L == kGrowthLevels) break;
+    for (int i = lo + (int)(threadIdx.x >> 5); i < hi; i += 32) {
+      const int32_t v = q[i];
+      const int e = row_ptr[v + 1];
+      for (int k = row_ptr[v] + lane; k < e; k += 32) {
+        const int32_t u = col[k];
+        const uint32_t bit = 1u << (u & 31);
+        if (atomicOr(seen + (u >> 5), bit) & bit) continue;
+        const int at = atomicAdd(&s_count, 1);
+        if (at < reach) q[at] = u;
+      }
+    }
+    lo = hi;
+  }
+  if (threadIdx.x == 0) out[blockIdx.x] = make_int2(L, s_count);
+}
+
+}  // namespace
+
+dawn_status read_growth(dawn_graph* g) {
+  if (g->growth >= 0.0) return DAWN_OK;
+  const int reach = std::max(64, std::min(kGrowthReach, g->n / 2));
+  const size_t nwords = ((size_t)g->n + 31) / 32;
+  const size_t words = 2 * kGrowthSamples + kGrowthSamples * (nwords + (size_t)reach);
+  int32_t* d = nullptr;
+  int2 h[kGrowthSamples];
+  const dawn_status s = pool_alloc((void**)&d, sizeof(int32_t) * words, g->stream);
+  if (s == DAWN_ERR_OOM) {  // not read: taken as a mesh by this call
+    cudaGetLastError();
+    clear_error();
+    return DAWN_OK;
+  }
+  DAWN_CHECK(s);
+  uint32_t* const bitmaps = reinterpret_cast<uint32_t*>(d + 2 * kGrowthSamples);
+  cudaError_t e = cudaMemsetAsync(bitmaps, 0, sizeof(uint32_t) * kGrowthSamples * nwords, g->stream);
+  grow<<<kGrowthSamples, 1024, 0, g->stream>>>(g->row_ptr, g->col, g->n, reach, bitmaps, nwords,
+                                                d + 2 * kGrowthSamples + kGrowthSamples * nwords,
+                                                reinterpret_cast<int2*>(d));
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, g->stream);
+  pool_free(d, g->stream);
+  DAWN_CUDA(e);
+  DAWN_CUDA(cudaStreamSynchronize(g->stream));
+  // per level, of the samples that reached far enough; 1 for those that did not
+  // within the levels or at all
+  double most = 1.0;
+  for (const int2& x : h)
+    if (x.x > 0 && x.y >= reach) most = std::max(most, std::pow((double)x.y, 1.0 / x.x));
+  g->growth = most;
+  return DAWN_OK;
+}
+
 // --- exclusive scan (int64), used for the in-edge CSR ---------------------------
 
 namespace {
@@ -729,7 +819,6 @@ dawn_status build_weighted_in_edges(dawn_graph* g) {
   const int32_t n = g->n;
   const cudaStream_t s = g->stream;
   const int grid = g->geo.sms * 8;
-  constexpr double kHubDegree = 16.0;  // in mean degrees
   DAWN_CHECK(light_weights(g));
   int2* cursor = nullptr;
   DAWN_CHECK(pool_alloc((void**)&cursor, sizeof(int2) * (size_t)n + sizeof(unsigned long long), s));
