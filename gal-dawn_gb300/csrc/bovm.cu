@@ -1359,29 +1359,44 @@ __global__ void __launch_bounds__(kBlock) fill_records(const int32_t* __restrict
 // entries a row, none above kRecMax: meshes, street networks, kNN graphs, whose
 // traversals take hundreds of small levels.  Beyond kMeshMax vertices, and with
 // rows of more than eight entries beyond kMeshWide, these keep the level kernels
-// and the cluster levels (kLevelKernels): kNN of 200,000 points takes 1.23 ms that
-// way and 1.54 on one SM, of 2,000 points 161 and 143 us.
+// and the cluster levels (kLevelKernels; records / level kernels, us a call: kNN of
+// 9,000 points 280 / 291, 20,000 455 / 471, 32,000 545 / 575, of 200,000 1.54 / 1.23 ms).
+// Random graphs of low degree have a few wide levels instead, which one SM with
+// records is slow at: from kRandomFrom vertices on they go by their growth.  Records /
+// level kernels / neither, us a call on Erdos-Renyi graphs of mean degree 11, 9,000
+// vertices 101 / 89 / 74, 20,000 107 / 90 / 76, 32,000 126 / 97 / 82; of 7, 20,000
+// 102 / 100 / 87; of 4 (growth 4.2 to 4.6) 9,000 88 / 90 / 101, 20,000 109 / 100 / 105,
+// 32,000 113 / 122 / 111, 50,000 - / 131 / 108; of 2.5 20,000 117 / 115 / 136, 32,000 128 / 126 /
+// 141, 50,000 - / 160 / 152; of 5, 3 M - / 365 / 297.
 constexpr int32_t kLevelKernels = -2;
+constexpr int32_t kRandomFrom = 6000, kRandomSlow = 26000, kRandomWide = 45000;
+constexpr double kGrowsFast = 4.8, kGrowsWell = 3.5;
 dawn_status records(dawn_graph* g) {
   if (g->rec_len != -1) return DAWN_OK;
+  const int32_t n = g->n;
   int32_t len = 0;
-  if (g->m <= 12 * (int64_t)g->n && g->n > kSoloKeep) {
+  if (g->m <= 12 * (int64_t)n && n > kSoloKeep) {
     DAWN_CHECK(longest_row(g));
     const int32_t deg = g->max_row;
     len = std::max(8, (deg + 7) / 8 * 8);
-    if (deg > kRecMax) {
+    double growth = 0.0;
+    if (deg <= kRecMax && n >= kRandomFrom) {
+      DAWN_CHECK(read_growth(g));
+      growth = g->growth;
+    }
+    if (deg > kRecMax || growth >= kGrowsFast || (growth >= kGrows && n > kRandomWide)) {
       len = 0;
-    } else if (g->n > kMeshMax || (len > 8 && g->n > kMeshWide)) {
+    } else if (n > kMeshMax || (len > 8 && n > kMeshWide) || (growth >= kGrowsWell && n < kRandomSlow)) {
       len = kLevelKernels;
     } else {
-      const dawn_status s = ensure(g->bfs_rec, sizeof(int32_t) * (size_t)g->n * len, g->stream);
+      const dawn_status s = ensure(g->bfs_rec, sizeof(int32_t) * (size_t)n * len, g->stream);
       if (s == DAWN_ERR_OOM) {  // not decided: the next call tries again
         cudaGetLastError();
         clear_error();
         return DAWN_OK;
       }
       DAWN_CHECK(s);
-      fill_records<<<g->geo.sms * 8, kBlock, 0, g->stream>>>(g->row_ptr, g->col, g->n, len, g->bfs_rec.as<int32_t>());
+      fill_records<<<g->geo.sms * 8, kBlock, 0, g->stream>>>(g->row_ptr, g->col, n, len, g->bfs_rec.as<int32_t>());
       DAWN_CUDA(cudaGetLastError());
     }
   }
