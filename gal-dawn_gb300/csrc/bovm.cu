@@ -809,10 +809,12 @@ constexpr int32_t kMeshWide = 32768;
 
 enum : int32_t { kBfStart = 0, kBfWipe, kBfBits, kBfCut, kBfPush, kBfPull, kBfSolo };
 
+// What a wait that gives up adds to the arrivals: more than a launch's CTAs, so that
+// no later arrival counts as a step's last.
+constexpr uint32_t kBfBroken = 1u << 30;
 struct BfsSync {
   struct __align__(128) {
     unsigned long long word[4];
-    uint32_t broken;  // a wait of an earlier launch gave up: its arrivals are missing
   } step;  // BfsStep, tagged with the generation in the top 16 bits of each word
   struct __align__(128) {
     uint32_t n;
@@ -910,6 +912,7 @@ __device__ __forceinline__ void solo_levels(const BfsArgs& a, const BfsStep& st,
   SsCtl* const ctl = a.ctl;
   const int lane = lane_id(), wib = threadIdx.x >> 5;
   int L = st.L;
+  const int last = min(a.n, L + kSoloSteps);
   {
     const int32_t* qin = a.q + (size_t)((L - 1) & 1) * a.n;
     if (threadIdx.x < 3) sm.cnt[threadIdx.x] = sm.mf[threadIdx.x] = sm.deg[threadIdx.x] = 0;
@@ -1030,9 +1033,7 @@ __device__ __forceinline__ void solo_levels(const BfsArgs& a, const BfsStep& st,
     }
     __syncthreads();
     const int nf = sm.cnt[o];
-    if (nf == 0 || nf > kSoloKeep || sm.mf[o] > kSoloEdges || sm.deg[o] >= (uint32_t)kLongRow || L + 1 >= a.n ||
-        it + 1 == kSoloSteps)
-      break;
+    if (nf == 0 || nf > kSoloKeep || sm.mf[o] > kSoloEdges || sm.deg[o] >= (uint32_t)kLongRow || L + 1 >= last) break;
     sum_mf += sm.mf[o];
     last_nf = nf;
   }
@@ -1144,7 +1145,7 @@ __device__ __forceinline__ void mesh_levels(const BfsArgs& a, const BfsStep& st,
     }
     __syncthreads();
     const int nf = sm.cnt[o];
-    if (nf == 0 || nf > kMeshKeep || L + 1 >= a.n || it + 1 == kSoloSteps) break;
+    if (nf == 0 || nf > kMeshKeep || L + 1 >= a.n) break;  // (kMeshMax levels at most: a few seconds)
     last_nf = nf;
   }
   for (int i = threadIdx.x; i < a.nwords; i += kThreads) a.vbm[i] = vis[i];
@@ -1245,6 +1246,7 @@ template <bool kMesh>
 __global__ void __launch_bounds__(kMesh ? 1024 : 640, kMesh ? 1 : 2) bfs_traverse(const __grid_constant__ BfsArgs a) {
   constexpr int kWarps = kMesh ? 32 : 20;
   extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ uint32_t s_polls;  // of one wait
   auto& sm = *reinterpret_cast<BfsSmem<kWarps>*>(smem);
   const int lane = lane_id(), wib = threadIdx.x >> 5;
   // no phase can open before every CTA has arrived, so all read the same
@@ -1253,11 +1255,14 @@ __global__ void __launch_bounds__(kMesh ? 1024 : 640, kMesh ? 1 : 2) bfs_travers
   if (threadIdx.x == 0) {
     sm.st = BfsStep{};
     sm.st.phase = kBfStart;
-    sm.st.ctas = *static_cast<const volatile uint32_t*>(&a.sync->step.broken) ? 0 : (int)gridDim.x;
+    sm.st.ctas = (int)gridDim.x;
     sm.st.arrived = (uint32_t)*static_cast<const volatile unsigned long long*>(&a.sync->step.word[3]);
+    // after a launch that gave up, none of the next ones' steps completes (its
+    // arrivals are missing): they wait once and end
+    const uint32_t now = *static_cast<const volatile uint32_t*>(&a.sync->arrive.n);
+    s_polls = now - sm.st.arrived >= kBfBroken ? 1 : a.polls;
   }
   __syncthreads();
-  if (st.ctas == 0) return;
   for (;;) {
     const Team tm{(int)blockIdx.x, st.ctas};
     switch (st.phase) {
@@ -1328,10 +1333,11 @@ __global__ void __launch_bounds__(kMesh ? 1024 : 640, kMesh ? 1 : 2) bfs_travers
           }
           idle = true;
         }
-        if (polls == a.polls) {
+        if (polls == s_polls) {
+          const uint32_t base = __shfl_sync(kFull, (uint32_t)w, 3);
           if (lane == 0) {
+            atomicExch(&a.sync->arrive.n, base + kBfBroken);
             *a.err = DAWN_ERR_TIMEOUT;
-            *static_cast<volatile uint32_t*>(&a.sync->step.broken) = 1;
             sm.st.ctas = 0;
           }
           break;

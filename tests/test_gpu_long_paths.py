@@ -52,14 +52,17 @@ def test_weighted(weights, weight):
 @pytest.mark.parametrize("hub", [0, 200])
 def test_others_wait_for_one_step_only(hub):
     # half a million levels by one CTA are a second or two; the other CTAs wait a
-    # third of one at most, which one step's levels do not take
+    # third of one at most, which one step's levels do not take (without a hub the
+    # levels go by records, all in one step, on graphs of 1.6 million vertices at
+    # most: a few seconds)
     n = 500001
     k, leaf = np.arange(n - 1), n + np.arange(hub)
     g = weighted(n + hub, np.concatenate([k, np.full(hub, n - 1)]), np.concatenate([k + 1, leaf]), np.full(n - 1 + hub, 0))
     want = np.concatenate([np.arange(n), np.full(hub, n)])
     with abi.Graph(g, weights="i32") as dg:
-        dg.set_option(abi.OPT_WAIT_POLLS, 1 << 19)
+        dg.set_option(abi.OPT_WAIT_POLLS, 1 << (19 if hub else 23))
         d, _ = dg.bfs([0], variant=abi.VARIANT_DO)
         assert np.array_equal(d[0], want)
+        dg.set_option(abi.OPT_WAIT_POLLS, 1 << 19)
         d, _ = dg.sssp([0], variant=abi.VARIANT_DO)
         assert not d.any()
