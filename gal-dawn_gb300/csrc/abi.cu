@@ -83,9 +83,10 @@ dawn_status finish_graph(dawn_graph* g, uint32_t flags) {
   } else {
     DAWN_CHECK(dawn::build_transpose(g));
   }
-  static_assert(2 * sizeof(dawn::SsCtl) <= dawn::kPinnedSlot, "control-block copies exceed a pinned slot");
+  static_assert(2 * sizeof(dawn::SsCtl) + sizeof(int32_t) <= dawn::kPinnedSlot,
+                "control-block copies and status exceed a pinned slot");
   DAWN_CHECK(dawn::pinned_slot((void**)&g->h_ctl));
-  DAWN_CHECK(dawn::pinned_slot((void**)&g->h_err));
+  g->h_err = reinterpret_cast<int32_t*>(g->h_ctl + 2);
   *g->h_err = 0;
   DAWN_CHECK(dawn::ensure(g->sel_slot, sizeof(float) * DAWN_SELECTOR_WEIGHTS, g->stream));
   DAWN_CUDA(cudaEventCreate(&g->ev0));
@@ -152,7 +153,6 @@ void destroy(dawn_graph* g) {
   if (g->pt_exec) cudaGraphExecDestroy(g->pt_exec);
   if (g->mw_exec) cudaGraphExecDestroy(g->mw_exec);
   dawn::pinned_slot_release(g->h_ctl);
-  dawn::pinned_slot_release(g->h_err);
   dawn::pinned_slot_release(g->bc_h_level);
   for (cudaEvent_t e : g->trace_ev)
     if (e) cudaEventDestroy(e);

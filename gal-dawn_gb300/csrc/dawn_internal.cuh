@@ -239,7 +239,7 @@ struct dawn_graph {
   uint32_t light_most = 0;  // word of the largest light weight
   dawn::DevBuf mw_bounds;   // batched: per vertex, lowest and highest distance over the sources (mw_bounds)
   dawn::SsCtl* h_ctl = nullptr;  // pinned: [0] upload staging, [1] download
-  int32_t* h_err = nullptr;      // pinned: status that a launch of this handle wrote (device_status), 0 = none
+  int32_t* h_err = nullptr;      // behind it: status that a launch of this handle wrote (device_status), 0 = none
   uint32_t wait_polls = 1u << 27;  // DAWN_OPT_WAIT_POLLS: polls of a wait between CTAs before it gives up
   bool graphs_ok = true;         // conditional CUDA graphs usable
 
