@@ -344,7 +344,7 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallBlock
     const int p = L & 1;
     uint32_t my_mf = 0;
     bool my_long = false;
-    auto op = [&](int k, bool valid, int32_t) {
+    auto op = [&](int k, bool valid) {
       const int32_t u = valid ? __ldg(col + k) : -1;
       bool found = false;
       int rs = 0, deg = 0;
@@ -382,7 +382,7 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallBlock
       const int pin = p ^ 1;
       const int32_t* qin = q + (size_t)pin * n;
       const int qn = ctl->qsize[pin], ln = seg_count(ctl->lpack[pin]);
-      seg_expand(row_ptr, segs + (size_t)pin * segcap, ln, [&](int32_t, int k, bool valid) { op(k, valid, 0); });
+      seg_expand(row_ptr, segs + (size_t)pin * segcap, ln, [&](int32_t, int k, bool valid) { op(k, valid); });
       const int bs = batch_rows(qn);
       for (int b = cwarp * bs; b < qn; b += kSmallCtas * kWarps * bs) {
         const int i = b + lane;
@@ -393,7 +393,7 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallBlock
           rs = row_ptr[v];
           deg = row_ptr[v + 1] - rs;
         }
-        expand_rows(ok, rs, deg, 0, op);
+        expand_rows(ok, rs, deg, op);
       }
     } else {
       // the previous level's slices, across the cluster
@@ -414,7 +414,7 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallBlock
           deg = src->deg[off];
           dist[src->u[off]] = L - 1;
         }
-        expand_rows(e < tot, rs, deg, 0, op);
+        expand_rows(e < tot, rs, deg, op);
       }
     }
     my_mf = __reduce_add_sync(kFull, my_mf);

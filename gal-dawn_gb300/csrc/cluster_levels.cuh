@@ -21,13 +21,13 @@ constexpr long long kSmallEdges = 32768;
 constexpr int kSmallMaxLevels = 512;
 
 // Expands one warp batch of frontier rows: lane i holds row (rs, deg) when
-// valid, and a value of its row (the row vertex's distance, for instance).
+// valid.
 // Rows of >= kWarpRow entries are swept by the whole warp, shorter ones are
 // concatenated through a warp scan and dealt 32 edges at a time (the owning
 // lane is found by a binary search over the lanes' exclusive offsets,
-// through shuffles).  op(k, valid, value of k's row) runs on all 32 lanes.
+// through shuffles).  op(k, valid) runs on all 32 lanes.
 template <class Op>
-__device__ __forceinline__ void expand_rows(bool valid, int rs, int deg, int32_t val, Op&& op) {
+__device__ __forceinline__ void expand_rows(bool valid, int rs, int deg, Op&& op) {
   const int lane = lane_id();
   if (!valid) deg = 0;
   uint32_t big = __ballot_sync(kFull, deg >= kWarpRow);
@@ -35,8 +35,7 @@ __device__ __forceinline__ void expand_rows(bool valid, int rs, int deg, int32_t
     const int leader = __ffs(big) - 1;
     big &= big - 1;
     const int s = __shfl_sync(kFull, rs, leader), d = __shfl_sync(kFull, deg, leader);
-    const int32_t lv = __shfl_sync(kFull, val, leader);
-    for (int k0 = 0; k0 < d; k0 += 32) op(s + k0 + lane, k0 + lane < d, lv);
+    for (int k0 = 0; k0 < d; k0 += 32) op(s + k0 + lane, k0 + lane < d);
   }
   const int sdeg = deg < kWarpRow ? deg : 0;
   const int incl = warp_incl_scan(sdeg);
@@ -51,7 +50,7 @@ __device__ __forceinline__ void expand_rows(bool valid, int rs, int deg, int32_t
       if (ex <= e) lo += step;
     }
     const int k = __shfl_sync(kFull, rs, lo) + (e - __shfl_sync(kFull, excl, lo));
-    op(k, e < total, __shfl_sync(kFull, val, lo));
+    op(k, e < total);
   }
 }
 
