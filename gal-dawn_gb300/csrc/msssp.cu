@@ -30,15 +30,17 @@
 //     relative to a hub's distances, which the sources' distances follow
 //     closely.  An edge whose tail's lowest plus its weight is no less than its
 //     head's highest cannot improve any of the 64;
-//   * and a batch's second level on are pulls along the light in-edges alone (an
+//   * and on graphs with a hub whose lengths spread (light_weights), a batch's
+//     second level on are pulls along the light in-edges alone (an
 //     eighth of them on RMAT-22): shortest paths run along these, and once the light
 //     edges have settled, one pull over all edges, with every reached pair
 //     taken as improved, leaves out nine tenths of them by the bounds.  RMAT-22
 //     x 64 reads 0.9 m rows so, against 4 m in four whole pulls.  Per call of 64
 //     sources, whole pulls -> this: RMAT-22 19.9 -> 8.1 ms, RMAT-20 6.4 -> 2.8,
-//     RMAT-20 (edge factor 6) 5.1 -> 2.7, RMAT-17 (32) 2.9 -> 1.3; Erdos-Renyi
-//     (no hub: no light stage, bounds once fewer than half of the pairs still
-//     improve) 300,000 vertices 4.8 -> 4.2, 1 M 12.4 -> 12.5;
+//     RMAT-20 (edge factor 6) 5.1 -> 2.7, RMAT-17 (32) 2.9 -> 1.3.  Other graphs
+//     keep whole pulls, a warp a row, by bounds only from a mean degree of
+//     kBoundDegree and once fewer than half of the pairs still improve
+//     (Erdos-Renyi, 1 M x 22 14.0 -> 12.9 ms, 300,000 x 30 4.3 -> 4.0);
 //   * a final pass transposes the block into the caller's source-major rows
 //     and counts the reached edges.
 // Each source's first frontier is resolved as the single-source path does

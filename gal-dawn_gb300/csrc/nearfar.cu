@@ -27,12 +27,16 @@
 // arrival: 6 to 7 us, 1.6 us within one CTA); on RMAT the gather of a
 // target's distance per entry, 100 to 140 G entries/s in the large phases
 // against the 230 G/s of the L1/TEX sector rate.  Times per call, before
-// (level by level) and now:
-//   kNN mesh, 200,003 points, 50 sources, float32     56.9 -> 10.0 ms
-//   RMAT scale 22, one source, float32                2.97 -> 1.83 ms
-//   grid 1000 x 1049, one source, float32             23.4 -> 9.3 ms
-//   kNN mesh, 20,000 points, one source               1.71 -> 0.97 ms
-//   RMAT scale 12 (edge factor 8), one source         178 -> 133 us
+// (level by level) and now, float32, on one GPU in turn, from the fastest to the
+// slowest of three sources (source lists):
+//   kNN mesh, 200,003 points, 50 sources     55.9-57.2 -> 10.2-10.5 ms
+//   RMAT scale 22, one source                1.90-2.32 -> 1.87-2.00 ms (real-valued lengths 2.55 -> 2.0-2.2)
+//   grid 1000 x 1049, one source             24.0-29.1 -> 9.9-12.4 ms
+//   kNN mesh, 20,000 points, one source      1.41-1.64 -> 0.88-1.04 ms
+//   RMAT scale 12 (edge factor 8), one       143-163 -> 131-141 us
+// Slower than cluster levels were (one launch for many small levels): one source on
+// meshes of 20,000 to 90,000 vertices whose levels hold 500 to 1,500 pairs, a phase of
+// 6.8 us each (grid 200 x 200 by a tenth, a street network of 62,500 by a quarter).
 #include <algorithm>
 #include <cstring>
 

@@ -410,15 +410,16 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kPartBlock, 1)
 //     padded to eight (made when the parts are declared; the padding names a
 //     word that is always 0), so a 16-byte load brings eight of them, a row of
 //     average length comes in one round trip and no entry is checked against
-//     the row's bounds (with 32-bit columns and checks the loop was bound by
-//     instruction issue, 2.6 per clock).
+//     the row's bounds.
 //   * The word arrays of levels 1 .. kPartDeep - 1 are expanded into the
 //     distance rows at the end, in full lines; deeper levels are stored at
 //     once (and share the last array).
 // 300 directed ER graphs (1,024 to 65,536 vertices, degrees 4 to 32, 8 to 64
 // sources): 5.08 ms as cluster tasks, 1.64 ms here (3.44 with global-memory
-// accumulators and 32-bit columns, 2.21 with a word array per level).  It is
-// bound by instruction issue, 2.6 per clock: per vertex and level about 1 ns.
+// accumulators and 32-bit columns, 2.21 with a word array per level).  What bounds
+// it is latency at the 32 warps an SM holds beside a part's words: 512 such graphs
+// issue 1.6 instructions a clock with L1 and shared memory at 44% and HBM at 2.55 TB/s
+// (2.76 ms), about 1 ns per vertex and level.
 constexpr int kPartDeep = 15;
 constexpr int kPartPush = 4;  // times the handle's push ratio
 constexpr int kPartLanePieces = 8;  // in-rows of this many pieces are swept by the warp

@@ -173,7 +173,10 @@ dawn_status dawn_graph_set_parts(dawn_graph* g, int32_t nparts,
  * receives, part after part, a (sources of p) x (vertices of p) int32 block
  * in part-local ids, -1 where unreachable: the values dawn_bfs gives on
  * each part as a graph of its own.  stats->batches counts the
- * (part, 64-source) tasks. */
+ * (part, 64-source) tasks; stats->levels, push_levels and pull_levels are
+ * summed over the tasks as the library cuts them, up to 16 or 32 sources of a
+ * part that fits one SM's shared memory and up to 64 of any other, or of a
+ * traced call. */
 dawn_status dawn_multi_bfs(dawn_graph* g, const int32_t* source_offset,
                            const int32_t* sources, int32_t* dist,
                            dawn_stats* stats);
